@@ -42,7 +42,8 @@ struct KOperator {
   using C = cplx_t<R>;
   int npw = 0, n1 = 0, n2 = 0, n3 = 0, g1min = 0, nplanes = 0, np = 0, max_rows = 0;
   AxisPlan ax, ay, az;
-  DeviceBuffer<int> plane_start, spos, row_start, row_list, plane_xpos;
+  DeviceBuffer<int> plane_start, spos, row_start, row_list, slot_plane;
+  DeviceBuffer<C> tw;        // exp(-2 pi i t / n) of the x, y and z axes, one after another
   DeviceBuffer<R> veff;      // Veff / N_r, C order
   DeviceBuffer<R> kinetic;
   DeviceBuffer<C> work;      // chunk x nplanes x n2 x n3
@@ -70,110 +71,239 @@ KOperatorSet::~KOperatorSet() = default;
 namespace {
 
 constexpr int kXTile = 16;
+constexpr int kPlaneThreads = 512;
 
 template <typename C>
 __device__ __forceinline__ C czero() { C c; c.x = 0; c.y = 0; return c; }
 
+// The local operator's three kernels are bound by instruction issue and
+// shared-memory accesses, not by HBM (a chunk's planes stay in L2), so every
+// pass over a plane or line that can be saved is: the first and last
+// transform passes read and write global memory directly, rows known to be
+// zero are neither cleared nor loaded, and rows nobody reads are not stored.
+// Rows of a plane are padded by one element in shared memory so that the z
+// passes, whose threads run over rows, are free of bank conflicts.  Kernel
+// time of one mixed solve of the 216-atom cell (96^3 box, B200), against
+// four radix <= 5 passes per axis with separate clear, scatter, product and
+// gather passes: K2 FP32 96.5 -> 26.7 ms, K2 FP64 67.0 -> 27.1 ms, K1 + K3
+// FP32 56.8 -> 27.3 ms, FP64 64.4 -> 28.2 ms.
+
+// Shared memory of a plane kernel: twiddles of both axes, the plane with
+// padded rows, the occupied rows and a flag per row.
 template <typename R>
-__global__ void __launch_bounds__(512) k1_sphere_to_planes(const cplx_t<R>* __restrict__ psi, long long ld, int b0,
-                                                           int n2, int n3, int nplanes, const int* __restrict__ plane_start,
-                                                           const int* __restrict__ spos, const int* __restrict__ row_start,
-                                                           const int* __restrict__ row_list, AxisPlan ay, AxisPlan az,
-                                                           cplx_t<R>* __restrict__ work) {
+size_t plane_smem(int n2, int n3) {
+  return (n2 + n3 + size_t(n2) * (n3 + 1)) * sizeof(cplx_t<R>) + size_t(n2) * 2 * sizeof(int);
+}
+
+// Threads of a plane kernel: 512 where shared memory holds one plane (FP64)
+// or two (FP32) per SM, which is also what the registers allow; smaller
+// planes run as more and smaller CTAs of the same total, so that one CTA's
+// barriers and loads overlap another's transforms.
+template <typename R>
+int plane_threads(size_t smem) {
+  const int total = sizeof(R) == 4 ? 1024 : 512;   // resident threads per SM (64 / 128 registers)
+  int th = kPlaneThreads;
+  while (th > 128 && size_t(total / (th / 2)) * (smem + 1024) <= 227 * 1024) th /= 2;
+  return th;
+}
+
+// Threads of an x-line kernel: one per item of the pass with most items.
+inline int xline_threads(const FFTPlan& p) {
+  int items = 0;
+  for (int s = 0; s < p.nstages; ++s) items = std::max(items, p.n / p.radix[s] * kXTile);
+  return std::min(256, (items + 31) / 32 * 32);
+}
+
+template <typename R>
+struct PlaneSmem {
+  using C = cplx_t<R>;
+  C *twy, *twz, *plane;
+  int *rows, *occ;
+  __device__ __forceinline__ PlaneSmem(unsigned char* raw, int n2, int n3) {
+    twy = reinterpret_cast<C*>(raw);
+    twz = twy + n2;
+    plane = twz + n3;
+    rows = reinterpret_cast<int*>(plane + size_t(n2) * (n3 + 1));
+    occ = rows + n2;
+  }
+};
+
+// tw: the twiddles of the x, y and z axes one after another.
+template <typename R>
+__global__ void __launch_bounds__(kPlaneThreads, sizeof(R) == 4 ? 2 : 1)
+    k1_sphere_to_planes(const cplx_t<R>* __restrict__ psi, long long ld, int b0, int n2, int n3, int nplanes,
+                        const int* __restrict__ plane_start, const int* __restrict__ spos,
+                        const int* __restrict__ row_start, const int* __restrict__ row_list, FFTPlan py, FFTPlan pz,
+                        const cplx_t<R>* __restrict__ tw_yz, cplx_t<R>* __restrict__ work) {
   using C = cplx_t<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* twy = reinterpret_cast<C*>(smem_raw);
-  C* twz = twy + kMaxFFT;
-  C* plane = twz + kMaxFFT;
-  int* rows = reinterpret_cast<int*>(plane + n2 * n3);
+  const PlaneSmem<R> sm(smem_raw, n2, n3);
+  C* const plane = sm.plane;
+  const int n3p = n3 + 1;
   const int j = blockIdx.x, b = blockIdx.y;
-  fill_twiddles(twy, n2);
-  fill_twiddles(twz, n3);
-  const int npl = n2 * n3;
-  for (int t = threadIdx.x; t < npl; t += blockDim.x) plane[t] = czero<C>();
+  for (int t = threadIdx.x; t < n2 + n3; t += blockDim.x) sm.twy[t] = tw_yz[t];
   const int r0 = row_start[j], nrows = row_start[j + 1] - r0;
-  for (int t = threadIdx.x; t < nrows; t += blockDim.x) rows[t] = row_list[r0 + t];
+  for (int t = threadIdx.x; t < n2; t += blockDim.x) sm.occ[t] = 0;
+  for (int r = threadIdx.x >> 5; r < nrows; r += blockDim.x >> 5) {   // one warp per occupied row
+    const int row = row_list[r0 + r];
+    if ((threadIdx.x & 31) == 0) sm.rows[r] = row * n3p;
+    for (int t = threadIdx.x & 31; t < n3; t += 32) plane[row * n3p + t] = czero<C>();
+  }
   __syncthreads();
+  for (int t = threadIdx.x; t < nrows; t += blockDim.x) sm.occ[sm.rows[t] / n3p] = 1;
   const C* col = psi + (long long)(b0 + b) * ld;
   const int p0 = plane_start[j], p1 = plane_start[j + 1];
   for (int p = p0 + threadIdx.x; p < p1; p += blockDim.x) plane[spos[p]] = col[p];
   __syncthreads();
-  fft_pencils<true, C, R>(plane, nrows, n3, 1, az.plan, twz, +1, rows);
-  fft_pencils<true, C, R>(plane, n3, 1, n3, ay.plan, twy, +1);
-  C* dst = work + ((long long)b * nplanes + j) * npl;
-  for (int t = threadIdx.x; t < npl; t += blockDim.x) dst[t] = plane[t];
+  const int* const rows = sm.rows;
+  for (int s = pz.nstages - 1; s >= 0; --s) {
+    fft_pass<true, +1, C, R>(
+        pz, s, nrows, sm.twz, [&](int p, int i) { return plane[rows[p] + i]; },
+        [&](int p, int i, C v) { plane[rows[p] + i] = v; });
+    __syncthreads();
+  }
+  C* const dst = work + ((long long)b * nplanes + j) * n2 * n3;
+  const int* const occ = sm.occ;
+  auto ld_occ = [&](int p, int i) { return occ[i] ? plane[i * n3p + p] : czero<C>(); };
+  auto st_plane = [&](int p, int i, C v) { plane[i * n3p + p] = v; };
+  auto st_work = [&](int p, int i, C v) { dst[i * n3 + p] = v; };
+  if (py.nstages == 1) {
+    fft_pass<true, +1, C, R>(py, 0, n3, sm.twy, ld_occ, st_work);
+    return;
+  }
+  fft_pass<true, +1, C, R>(py, py.nstages - 1, n3, sm.twy, ld_occ, st_plane);
+  __syncthreads();
+  auto ld_plane = [&](int p, int i) { return plane[i * n3p + p]; };
+  if (py.nstages == 3) {
+    fft_pass<true, +1, C, R>(py, 1, n3, sm.twy, ld_plane, st_plane);
+    __syncthreads();
+  }
+  fft_pass<true, +1, C, R>(py, 0, n3, sm.twy, ld_plane, st_work);
 }
 
+// Shared memory of an x-line kernel: twiddles, the tile's box points, one
+// real per point (Veff / N_r, or the density) and the plane of each slot.
 template <typename R>
-__global__ void __launch_bounds__(256) k2_xlines(cplx_t<R>* __restrict__ work, int n1, int n2, int n3, int nplanes,
-                                                 const int* __restrict__ plane_xpos, AxisPlan ax,
-                                                 const R* __restrict__ veff, int nb, int bands_per_cta) {
-  // One CTA per (i2, z tile) and group of bands_per_cta of the chunk's nb
-  // bands, looping over its bands: the twiddles, the occupied-slot map and
-  // the tile's Veff are set up once per CTA.
+size_t xline_smem(int n1) {
+  return (n1 + size_t(n1) * kXTile) * sizeof(cplx_t<R>) + size_t(n1) * kXTile * sizeof(R) + size_t(n1) * sizeof(int);
+}
+
+// One CTA per (i2, z tile) and group of bands_per_cta of the chunk's nb
+// bands, looping over its bands: the twiddles, the plane of every slot
+// (slot_plane, -1 where the sphere has none) and the tile's Veff are set up
+// once per CTA.  Per band, three passes for a two-pass axis: the first
+// inverse pass loads the occupied planes from global memory, the last
+// inverse pass, the product with Veff and the first forward pass are one
+// pass in registers, and the last forward pass stores the occupied planes.
+template <typename R>
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k2_xlines(cplx_t<R>* __restrict__ work, int n1, int n2, int n3, int nplanes,
+                                                 const int* __restrict__ slot_plane, FFTPlan px,
+                                                 const cplx_t<R>* __restrict__ tw_x, const R* __restrict__ veff, int nb,
+                                                 int bands_per_cta) {
   using C = cplx_t<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* tw = reinterpret_cast<C*>(smem_raw);
-  C* X = tw + kMaxFFT;                                 // [i1][tz]
-  R* vt = reinterpret_cast<R*>(X + n1 * kXTile);       // [i1][tz] Veff / N_r
-  int* xpos = reinterpret_cast<int*>(vt + n1 * kXTile);
+  C* const tw = reinterpret_cast<C*>(smem_raw);
+  C* const X = tw + n1;                                      // [slot][tz]
+  R* const vt = reinterpret_cast<R*>(X + n1 * kXTile);       // [i1][tz] Veff / N_r
+  int* const slot = reinterpret_cast<int*>(vt + n1 * kXTile);
   const int tiles = (n3 + kXTile - 1) / kXTile;
   const int i2 = blockIdx.x / tiles, z0 = (blockIdx.x - i2 * tiles) * kXTile;
   const int nz = min(kXTile, n3 - z0);
-  fill_twiddles(tw, n1);
-  for (int t = threadIdx.x; t < nplanes; t += blockDim.x) xpos[t] = plane_xpos[t];
+  const int npl = n2 * n3;
+  for (int t = threadIdx.x; t < n1; t += blockDim.x) {
+    tw[t] = tw_x[t];
+    const int jj = slot_plane[t];
+    slot[t] = jj < 0 ? -1 : jj * npl;
+  }
   for (int t = threadIdx.x; t < n1 * kXTile; t += blockDim.x) {
     const int i1 = t / kXTile, c = t - i1 * kXTile;
     vt[t] = c < nz ? veff[((long long)i1 * n2 + i2) * n3 + z0 + c] : R(0);
   }
-  const long long npl = (long long)n2 * n3;
+  __syncthreads();
+  auto ld_x = [&](int p, int i) { return X[i * kXTile + p]; };
+  auto st_x = [&](int p, int i, C v) { X[i * kXTile + p] = v; };
+  auto times_v = [&](int p, int i, C v) { return cscale(v, vt[i * kXTile + p]); };
+  const int last = px.nstages - 1;
   const int bend = min(nb, (blockIdx.y + 1) * bands_per_cta);
   for (int b = blockIdx.y * bands_per_cta; b < bend; ++b) {
-    for (int t = threadIdx.x; t < n1 * kXTile; t += blockDim.x) X[t] = czero<C>();
-    __syncthreads();
-    C* base = work + (long long)b * nplanes * npl + (long long)i2 * n3 + z0;
-    for (int t = threadIdx.x; t < nplanes * kXTile; t += blockDim.x) {
-      int jj = t / kXTile, c = t - jj * kXTile;
-      if (c < nz) X[xpos[jj] * kXTile + c] = base[jj * npl + c];
+    C* const base = work + (long long)b * nplanes * npl + (long long)i2 * n3 + z0;
+    auto ld_work = [&](int p, int i) {
+      const int o = slot[i];
+      return o >= 0 && p < nz ? base[o + p] : czero<C>();
+    };
+    auto st_work = [&](int p, int i, C v) {
+      const int o = slot[i];
+      if (o >= 0 && p < nz) base[o + p] = v;
+    };
+    if (last == 0) {
+      fft_pass_fused<C, R>(px, kXTile, tw, ld_work, times_v, st_work);
+      continue;
     }
+    fft_pass<true, +1, C, R>(px, last, kXTile, tw, ld_work, st_x);
     __syncthreads();
-    fft_pencils<true, C, R>(X, kXTile, 1, kXTile, ax.plan, tw, +1);
-    for (int t = threadIdx.x; t < n1 * kXTile; t += blockDim.x) X[t] = cscale(X[t], vt[t]);
-    __syncthreads();
-    fft_pencils<false, C, R>(X, kXTile, 1, kXTile, ax.plan, tw, -1);
-    for (int t = threadIdx.x; t < nplanes * kXTile; t += blockDim.x) {
-      int jj = t / kXTile, c = t - jj * kXTile;
-      if (c < nz) base[jj * npl + c] = X[xpos[jj] * kXTile + c];
+    if (last == 2) {
+      fft_pass<true, +1, C, R>(px, 1, kXTile, tw, ld_x, st_x);
+      __syncthreads();
     }
+    fft_pass_fused<C, R>(px, kXTile, tw, ld_x, times_v, st_x);
+    __syncthreads();
+    if (last == 2) {
+      fft_pass<false, -1, C, R>(px, 1, kXTile, tw, ld_x, st_x);
+      __syncthreads();
+    }
+    fft_pass<false, -1, C, R>(px, last, kXTile, tw, ld_x, st_work);
     __syncthreads();
   }
 }
 
 template <typename R>
-__global__ void __launch_bounds__(512) k3_planes_to_sphere(const cplx_t<R>* __restrict__ work, int n2, int n3,
-                                                           int nplanes, const int* __restrict__ plane_start,
-                                                           const int* __restrict__ spos, const int* __restrict__ row_start,
-                                                           const int* __restrict__ row_list, AxisPlan ay, AxisPlan az,
-                                                           const cplx_t<R>* __restrict__ psi, long long ld, int b0,
-                                                           const R* __restrict__ kinetic, cplx_t<R>* __restrict__ hpsi,
-                                                           cplx_t<R>* __restrict__ spsi) {
+__global__ void __launch_bounds__(kPlaneThreads, sizeof(R) == 4 ? 2 : 1)
+    k3_planes_to_sphere(const cplx_t<R>* __restrict__ work, int n2, int n3, int nplanes,
+                        const int* __restrict__ plane_start, const int* __restrict__ spos,
+                        const int* __restrict__ row_start, const int* __restrict__ row_list, FFTPlan py, FFTPlan pz,
+                        const cplx_t<R>* __restrict__ tw_yz, const cplx_t<R>* __restrict__ psi, long long ld, int b0,
+                        const R* __restrict__ kinetic, cplx_t<R>* __restrict__ hpsi, cplx_t<R>* __restrict__ spsi) {
   using C = cplx_t<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* twy = reinterpret_cast<C*>(smem_raw);
-  C* twz = twy + kMaxFFT;
-  C* plane = twz + kMaxFFT;
-  int* rows = reinterpret_cast<int*>(plane + n2 * n3);
+  const PlaneSmem<R> sm(smem_raw, n2, n3);
+  C* const plane = sm.plane;
+  const int n3p = n3 + 1;
   const int j = blockIdx.x, b = blockIdx.y;
-  fill_twiddles(twy, n2);
-  fill_twiddles(twz, n3);
-  const int npl = n2 * n3;
-  const C* src = work + ((long long)b * nplanes + j) * npl;
-  for (int t = threadIdx.x; t < npl; t += blockDim.x) plane[t] = src[t];
+  for (int t = threadIdx.x; t < n2 + n3; t += blockDim.x) sm.twy[t] = tw_yz[t];
   const int r0 = row_start[j], nrows = row_start[j + 1] - r0;
-  for (int t = threadIdx.x; t < nrows; t += blockDim.x) rows[t] = row_list[r0 + t];
+  for (int t = threadIdx.x; t < n2; t += blockDim.x) sm.occ[t] = 0;
   __syncthreads();
-  fft_pencils<false, C, R>(plane, n3, 1, n3, ay.plan, twy, -1);
-  fft_pencils<false, C, R>(plane, nrows, n3, 1, az.plan, twz, -1, rows);
+  for (int t = threadIdx.x; t < nrows; t += blockDim.x) {
+    const int row = row_list[r0 + t];
+    sm.rows[t] = row * n3p;
+    sm.occ[row] = 1;
+  }
+  const C* const src = work + ((long long)b * nplanes + j) * n2 * n3;
+  const int* const occ = sm.occ;
+  auto ld_work = [&](int p, int i) { return src[i * n3 + p]; };
+  auto ld_plane = [&](int p, int i) { return plane[i * n3p + p]; };
+  auto st_plane = [&](int p, int i, C v) { plane[i * n3p + p] = v; };
+  auto st_occ = [&](int p, int i, C v) { if (occ[i]) plane[i * n3p + p] = v; };
+  if (py.nstages == 1) {
+    __syncthreads();   // occ
+    fft_pass<false, -1, C, R>(py, 0, n3, sm.twy, ld_work, st_occ);
+  } else {
+    fft_pass<false, -1, C, R>(py, 0, n3, sm.twy, ld_work, st_plane);
+    __syncthreads();
+    if (py.nstages == 3) {
+      fft_pass<false, -1, C, R>(py, 1, n3, sm.twy, ld_plane, st_plane);
+      __syncthreads();
+    }
+    fft_pass<false, -1, C, R>(py, py.nstages - 1, n3, sm.twy, ld_plane, st_occ);
+  }
+  __syncthreads();
+  const int* const rows = sm.rows;
+  for (int s = 0; s < pz.nstages; ++s) {
+    fft_pass<false, -1, C, R>(
+        pz, s, nrows, sm.twz, [&](int p, int i) { return plane[rows[p] + i]; },
+        [&](int p, int i, C v) { plane[rows[p] + i] = v; });
+    __syncthreads();
+  }
   const long long off = (long long)(b0 + b) * ld;
   const int p0 = plane_start[j], p1 = plane_start[j + 1];
   for (int p = p0 + threadIdx.x; p < p1; p += blockDim.x) {
@@ -192,38 +322,52 @@ __global__ void __launch_bounds__(512) k3_planes_to_sphere(const cplx_t<R>* __re
 // transform, accumulating bw[b] |psi_b(r)|^2; the chunk total is added to
 // density (C order) once.  No atomics: each point has one owner.
 __global__ void __launch_bounds__(256) k2_density(const double2* __restrict__ work, int n1, int n2, int n3,
-                                                  int nplanes, const int* __restrict__ plane_xpos, AxisPlan ax,
-                                                  const double* __restrict__ bw, int nb,
-                                                  double* __restrict__ density) {
+                                                  int nplanes, const int* __restrict__ slot_plane, FFTPlan px,
+                                                  const double2* __restrict__ tw_x, const double* __restrict__ bw,
+                                                  int nb, double* __restrict__ density) {
+  using C = double2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double2* tw = reinterpret_cast<double2*>(smem_raw);
-  double2* X = tw + kMaxFFT;                                   // [i1][tz]
-  double* acc = reinterpret_cast<double*>(X + n1 * kXTile);    // [i1][tz]
-  int* xpos = reinterpret_cast<int*>(acc + n1 * kXTile);
+  C* const tw = reinterpret_cast<C*>(smem_raw);
+  C* const X = tw + n1;                                              // [slot][tz]
+  double* const acc = reinterpret_cast<double*>(X + n1 * kXTile);    // [i1][tz]
+  int* const slot = reinterpret_cast<int*>(acc + n1 * kXTile);
   const int tiles = (n3 + kXTile - 1) / kXTile;
   const int i2 = blockIdx.x / tiles, z0 = (blockIdx.x - i2 * tiles) * kXTile;
   const int nz = min(kXTile, n3 - z0);
-  fill_twiddles(tw, n1);
+  const int npl = n2 * n3;
+  for (int t = threadIdx.x; t < n1; t += blockDim.x) {
+    tw[t] = tw_x[t];
+    const int jj = slot_plane[t];
+    slot[t] = jj < 0 ? -1 : jj * npl;
+  }
   for (int t = threadIdx.x; t < n1 * kXTile; t += blockDim.x) acc[t] = 0.0;
-  for (int t = threadIdx.x; t < nplanes; t += blockDim.x) xpos[t] = plane_xpos[t];
-  const long long npl = (long long)n2 * n3;
+  __syncthreads();
+  auto ld_x = [&](int p, int i) { return X[i * kXTile + p]; };
+  auto st_x = [&](int p, int i, C v) { X[i * kXTile + p] = v; };
+  const int last = px.nstages - 1;
   for (int b = 0; b < nb; ++b) {
-    for (int t = threadIdx.x; t < n1 * kXTile; t += blockDim.x) X[t] = czero<double2>();
-    __syncthreads();
-    const double2* base = work + (long long)b * nplanes * npl + (long long)i2 * n3 + z0;
-    for (int t = threadIdx.x; t < nplanes * kXTile; t += blockDim.x) {
-      int jj = t / kXTile, c = t - jj * kXTile;
-      if (c < nz) X[xpos[jj] * kXTile + c] = base[jj * npl + c];
-    }
-    __syncthreads();
-    fft_pencils<true, double2, double>(X, kXTile, 1, kXTile, ax.plan, tw, +1);
+    const C* const base = work + (long long)b * nplanes * npl + (long long)i2 * n3 + z0;
     const double w = bw[b];
-    for (int t = threadIdx.x; t < n1 * kXTile; t += blockDim.x) {
-      const double2 v = X[t];
-      acc[t] += w * (v.x * v.x + v.y * v.y);
+    auto ld_work = [&](int p, int i) {
+      const int o = slot[i];
+      return o >= 0 && p < nz ? base[o + p] : czero<C>();
+    };
+    // every pass maps points to threads alike, so each sum has one writer
+    auto add = [&](int p, int i, C v) { acc[i * kXTile + p] += w * (v.x * v.x + v.y * v.y); };
+    if (last == 0) {
+      fft_pass<true, +1, C, double>(px, 0, kXTile, tw, ld_work, add);
+      continue;
     }
+    fft_pass<true, +1, C, double>(px, last, kXTile, tw, ld_work, st_x);
+    __syncthreads();
+    if (last == 2) {
+      fft_pass<true, +1, C, double>(px, 1, kXTile, tw, ld_x, st_x);
+      __syncthreads();
+    }
+    fft_pass<true, +1, C, double>(px, 0, kXTile, tw, ld_x, add);
     __syncthreads();
   }
+  __syncthreads();
   for (int t = threadIdx.x; t < n1 * kXTile; t += blockDim.x) {
     int i1 = t / kXTile, c = t - i1 * kXTile;
     if (c < nz) density[((long long)i1 * n2 + i2) * n3 + z0 + c] += acc[t];
@@ -320,19 +464,10 @@ __global__ void scale_copy_kernel(const double* __restrict__ in, R* __restrict__
   if (i < n) out[i] = R(in[i] * s);
 }
 
-template <typename R>
-size_t plane_smem(int n2, int n3) {
-  return (2 * kMaxFFT + size_t(n2) * n3) * sizeof(cplx_t<R>) + size_t(n2) * sizeof(int);
-}
-template <typename R>
-size_t xline_smem(int n1, int nplanes) {
-  return (kMaxFFT + size_t(n1) * kXTile) * sizeof(cplx_t<R>) + size_t(n1) * kXTile * sizeof(R) +
-         size_t(nplanes) * sizeof(int);
-}
-
 struct HostGeom {
   int g1min = 0, nplanes = 0, max_rows = 0;
-  std::vector<int> plane_start, spos, row_start, row_list, plane_xpos;
+  std::vector<int> plane_start, spos, row_start, row_list;
+  std::vector<int> slot_plane;   // plane of each x slot, -1 where the sphere has none
 };
 
 HostGeom plane_geometry(const Basis& b, const AxisPlan& ax, const AxisPlan& ay, const AxisPlan& az) {
@@ -344,6 +479,7 @@ HostGeom plane_geometry(const Basis& b, const AxisPlan& ax, const AxisPlan& ay, 
   h.nplanes = g1max - g1min + 1;
   if (h.nplanes > n1) fail(kInternal, "sphere x-extent exceeds the FFT box");
   h.plane_start.assign(h.nplanes + 1, 0);
+  h.slot_plane.assign(n1, -1);
   h.spos.resize(npw);
   long long p = 0;
   for (int j = 0; j < h.nplanes; ++j) {
@@ -354,15 +490,26 @@ HostGeom plane_geometry(const Basis& b, const AxisPlan& ax, const AxisPlan& ay, 
       int i2 = ((b.gvec[3 * p + 1] % n2) + n2) % n2, i3 = ((b.gvec[3 * p + 2] % n3) + n3) % n3;
       int row = ay.pos[i2];
       if (i2 != last_i2) { h.row_list.push_back(row); last_i2 = i2; }
-      h.spos[p] = row * n3 + az.pos[i3];
+      h.spos[p] = row * (n3 + 1) + az.pos[i3];   // rows are padded in shared memory
       ++p;
     }
     int i1 = (((g1min + j) % n1) + n1) % n1;
-    h.plane_xpos.push_back(ax.pos[i1]);
+    h.slot_plane[ax.pos[i1]] = j;
   }
   h.plane_start[h.nplanes] = int(p);
   h.row_start.push_back(int(h.row_list.size()));
-  for (int j = 0; j < h.nplanes; ++j) h.max_rows = std::max(h.max_rows, h.row_start[j + 1] - h.row_start[j]);
+  // z passes: threads run over a plane's rows, so neighbours in the list get
+  // different shared-memory banks where the occupied rows allow it
+  for (int j = 0; j < h.nplanes; ++j) {
+    const int a = h.row_start[j], e = h.row_start[j + 1];
+    std::vector<std::vector<int>> by_bank(16);
+    for (int r = a; r < e; ++r) by_bank[h.row_list[r] % 16].push_back(h.row_list[r]);
+    int o = a;
+    for (size_t i = 0; o < e; ++i)
+      for (auto& v : by_bank)
+        if (i < v.size()) h.row_list[o++] = v[i];
+    h.max_rows = std::max(h.max_rows, e - a);
+  }
   if (p != npw) fail(kInternal, "basis is not ordered by g1");
   return h;
 }
@@ -384,6 +531,7 @@ template <typename R>
 void fill_operator(Context& ctx, Runtime& rt, const Basis& basis, const HostGeom& hg, const DeviceBuffer<double2>& B64, int np,
                    const std::vector<int>& cb, const std::vector<int>& ca, const std::vector<int>& cn,
                    const std::vector<int>& cd, const std::vector<int>& cq, const ProjGen& gen, KOperator<R>& op) {
+  using C = cplx_t<R>;
   cudaStream_t s = rt.stream;
   op.npw = int(basis.npw());
   op.n1 = basis.shape[0]; op.n2 = basis.shape[1]; op.n3 = basis.shape[2];
@@ -396,7 +544,13 @@ void fill_operator(Context& ctx, Runtime& rt, const Basis& basis, const HostGeom
   op.spos.upload(hg.spos, s);
   op.row_start.upload(hg.row_start, s);
   op.row_list.upload(hg.row_list, s);
-  op.plane_xpos.upload(hg.plane_xpos, s);
+  op.slot_plane.upload(hg.slot_plane, s);
+  std::vector<C> tw;
+  const int axes[3] = {op.n1, op.n2, op.n3};
+  for (int a = 0; a < 3; ++a)
+    for (int t = 0; t < axes[a]; ++t)
+      tw.push_back(cmake(R(std::cos(2.0 * kPi * t / axes[a])), R(-std::sin(2.0 * kPi * t / axes[a]))));
+  op.tw.upload(tw, s);
   const long long nr = ctx.nr();
   op.veff.resize(nr);
   scale_copy_kernel<R><<<ceil_div(nr, 256), 256, 0, s>>>(ctx.veff.get(), op.veff.get(), nr, 1.0 / double(nr));
@@ -455,7 +609,7 @@ void fill_operator(Context& ctx, Runtime& rt, const Basis& basis, const HostGeom
   HALF_CUDA(cudaStreamSynchronize(s));
   raise_smem_limit(k1_sphere_to_planes<R>, plane_smem<R>(op.n2, op.n3));
   raise_smem_limit(k3_planes_to_sphere<R>, plane_smem<R>(op.n2, op.n3));
-  raise_smem_limit(k2_xlines<R>, xline_smem<R>(op.n1, op.nplanes));
+  raise_smem_limit(k2_xlines<R>, xline_smem<R>(op.n1));
 }
 
 }  // namespace
@@ -620,7 +774,8 @@ void apply_hs(Context& ctx, KOperatorSet& ks, const cplx_t<R>* x, long long ld, 
     op.work.resize((size_t)chunk * op.nplanes * op.n2 * op.n3);
     op.work_chunk = chunk;
   }
-  const size_t psm = plane_smem<R>(op.n2, op.n3), xsm = xline_smem<R>(op.n1, op.nplanes);
+  const size_t psm = plane_smem<R>(op.n2, op.n3), xsm = xline_smem<R>(op.n1);
+  const int pth = plane_threads<R>(psm);
   const int tiles = (op.n3 + kXTile - 1) / kXTile;
   int sms = 148, dev = 0;
   HALF_CUDA(cudaGetDevice(&dev));
@@ -630,18 +785,19 @@ void apply_hs(Context& ctx, KOperatorSet& ks, const cplx_t<R>* x, long long ld, 
   const int ev_local = ev_sweep;
   for (int b0 = 0; b0 < nb; b0 += chunk) {
     int nbc = std::min(chunk, nb - b0);
-    k1_sphere_to_planes<R><<<dim3(op.nplanes, nbc), 512, psm, s>>>(
+    k1_sphere_to_planes<R><<<dim3(op.nplanes, nbc), pth, psm, s>>>(
         x, ld, b0, op.n2, op.n3, op.nplanes, op.plane_start.get(), op.spos.get(), op.row_start.get(), op.row_list.get(),
-        op.ay, op.az, op.work.get());
+        op.ay.plan, op.az.plan, op.tw.get() + op.n1, op.work.get());
     // bands per K2 CTA: as many as keep about eight CTAs per SM busy
     const int lines = op.n2 * tiles;
     const int groups = std::max(1, std::min(nbc, ceil_div(8 * sms, lines)));
     const int bpc = ceil_div(nbc, groups);
-    k2_xlines<R><<<dim3(lines, ceil_div(nbc, bpc)), 256, xsm, s>>>(op.work.get(), op.n1, op.n2, op.n3, op.nplanes,
-                                                                  op.plane_xpos.get(), op.ax, op.veff.get(), nbc, bpc);
-    k3_planes_to_sphere<R><<<dim3(op.nplanes, nbc), 512, psm, s>>>(
+    k2_xlines<R><<<dim3(lines, ceil_div(nbc, bpc)), xline_threads(op.ax.plan), xsm, s>>>(
+        op.work.get(), op.n1, op.n2, op.n3, op.nplanes, op.slot_plane.get(), op.ax.plan, op.tw.get(), op.veff.get(), nbc,
+        bpc);
+    k3_planes_to_sphere<R><<<dim3(op.nplanes, nbc), pth, psm, s>>>(
         op.work.get(), op.n2, op.n3, op.nplanes, op.plane_start.get(), op.spos.get(), op.row_start.get(),
-        op.row_list.get(), op.ay, op.az, x, ld, b0, op.kinetic.get(), hx, sx);
+        op.row_list.get(), op.ay.plan, op.az.plan, op.tw.get() + op.n1, x, ld, b0, op.kinetic.get(), hx, sx);
     pf.launches += 3;
   }
   HALF_LAUNCH("local operator");
@@ -744,16 +900,18 @@ void accumulate_band_density(KOperatorSet& ks, const double2* x, long long ld, i
     op.work_chunk = chunk;
   }
   const size_t psm = plane_smem<double>(op.n2, op.n3);
-  const size_t dsm = xline_smem<double>(op.n1, op.nplanes);   // its accumulator takes the Veff tile's place
+  const int pth = plane_threads<double>(psm);
+  const size_t dsm = xline_smem<double>(op.n1);   // its accumulator takes the Veff tile's place
   raise_smem_limit(k2_density, dsm);
   const int tiles = (op.n3 + kXTile - 1) / kXTile;
   for (int b0 = 0; b0 < nb; b0 += chunk) {
     const int nbc = std::min(chunk, nb - b0);
-    k1_sphere_to_planes<double><<<dim3(op.nplanes, nbc), 512, psm, s>>>(
+    k1_sphere_to_planes<double><<<dim3(op.nplanes, nbc), pth, psm, s>>>(
         x, ld, b0, op.n2, op.n3, op.nplanes, op.plane_start.get(), op.spos.get(), op.row_start.get(),
-        op.row_list.get(), op.ay, op.az, op.work.get());
-    k2_density<<<op.n2 * tiles, 256, dsm, s>>>(op.work.get(), op.n1, op.n2, op.n3, op.nplanes, op.plane_xpos.get(),
-                                                op.ax, bw + b0, nbc, density_c);
+        op.row_list.get(), op.ay.plan, op.az.plan, op.tw.get() + op.n1, op.work.get());
+    k2_density<<<op.n2 * tiles, xline_threads(op.ax.plan), dsm, s>>>(
+        op.work.get(), op.n1, op.n2, op.n3, op.nplanes, op.slot_plane.get(), op.ax.plan, op.tw.get(), bw + b0, nbc,
+        density_c);
     ks.rt->prof.launches += 2;
   }
   HALF_LAUNCH("band density");

@@ -88,8 +88,8 @@ namespace {
 constexpr int kTile = 16;   // pencils per block for strided axes
 
 // FFT along the contiguous axis (i3): each block transforms `rows` pencils.
-template <typename C, typename R>
-__global__ void fft_rows_kernel(C* data, long long npencils, AxisPlan ap, int sign) {
+template <int SIGN, typename C, typename R>
+__global__ void fft_rows_kernel(C* data, long long npencils, AxisPlan ap) {
   extern __shared__ unsigned char smem_raw[];
   C* tw = reinterpret_cast<C*>(smem_raw);
   const int n = ap.plan.n;
@@ -99,7 +99,7 @@ __global__ void fft_rows_kernel(C* data, long long npencils, AxisPlan ap, int si
   const int np = int(min((long long)kTile, npencils - p0));
   for (int t = threadIdx.x; t < np * n; t += blockDim.x) buf[t] = data[p0 * n + t];
   __syncthreads();
-  fft_pencils<false, C, R>(buf, np, n, 1, ap.plan, tw, sign);
+  fft_pencils<SIGN, C, R>(buf, np, n, 1, ap.plan, tw);
   for (int t = threadIdx.x; t < np * n; t += blockDim.x) {
     int p = t / n, k = t - p * n;
     data[(p0 + p) * n + k] = buf[p * n + ap.pos[k]];
@@ -108,9 +108,8 @@ __global__ void fft_rows_kernel(C* data, long long npencils, AxisPlan ap, int si
 
 // FFT along a strided axis: pencil (o, c) starts at o*outer_stride + c and
 // steps by axis_stride; a block takes kTile consecutive c (coalesced).
-template <typename C, typename R>
-__global__ void fft_strided_kernel(C* data, int ncols, long long axis_stride, long long outer_stride, AxisPlan ap,
-                                   int sign) {
+template <int SIGN, typename C, typename R>
+__global__ void fft_strided_kernel(C* data, int ncols, long long axis_stride, long long outer_stride, AxisPlan ap) {
   extern __shared__ unsigned char smem_raw[];
   C* tw = reinterpret_cast<C*>(smem_raw);
   const int n = ap.plan.n;
@@ -125,7 +124,7 @@ __global__ void fft_strided_kernel(C* data, int ncols, long long axis_stride, lo
     else buf[t] = cmake(R(0), R(0));
   }
   __syncthreads();
-  fft_pencils<false, C, R>(buf, kTile, 1, kTile, ap.plan, tw, sign);
+  fft_pencils<SIGN, C, R>(buf, kTile, 1, kTile, ap.plan, tw);
   for (int t = threadIdx.x; t < n * kTile; t += blockDim.x) {
     int k = t / kTile, c = t - k * kTile;
     if (c < nc) data[base + k * axis_stride + c] = buf[ap.pos[k] * kTile + c];
@@ -134,21 +133,31 @@ __global__ void fft_strided_kernel(C* data, int ncols, long long axis_stride, lo
 
 }  // namespace
 
-void fft3d_inplace(double2* data, const std::array<int, 3>& shape, int sign, cudaStream_t s) {
+namespace {
+
+template <int SIGN>
+void fft3d(double2* data, const std::array<int, 3>& shape, cudaStream_t s) {
   const int n1 = shape[0], n2 = shape[1], n3 = shape[2];
   AxisPlan a1 = make_axis_plan(n1), a2 = make_axis_plan(n2), a3 = make_axis_plan(n3);
   const long long rows = (long long)n1 * n2;
   size_t sm3 = (kMaxFFT + size_t(kTile) * n3) * sizeof(double2);
-  fft_rows_kernel<double2, double><<<ceil_div(rows, kTile), 256, sm3, s>>>(data, rows, a3, sign);
+  fft_rows_kernel<SIGN, double2, double><<<ceil_div(rows, kTile), 256, sm3, s>>>(data, rows, a3);
   HALF_LAUNCH("fft rows");
   size_t sm2 = (kMaxFFT + size_t(kTile) * n2) * sizeof(double2);
-  fft_strided_kernel<double2, double><<<dim3(ceil_div(n3, kTile), n1), 256, sm2, s>>>(data, n3, n3, (long long)n2 * n3,
-                                                                                       a2, sign);
+  fft_strided_kernel<SIGN, double2, double><<<dim3(ceil_div(n3, kTile), n1), 256, sm2, s>>>(
+      data, n3, n3, (long long)n2 * n3, a2);
   HALF_LAUNCH("fft axis 2");
   size_t sm1 = (kMaxFFT + size_t(kTile) * n1) * sizeof(double2);
-  fft_strided_kernel<double2, double><<<dim3(ceil_div((long long)n2 * n3, kTile), 1), 256, sm1, s>>>(
-      data, n2 * n3, (long long)n2 * n3, 0, a1, sign);
+  fft_strided_kernel<SIGN, double2, double><<<dim3(ceil_div((long long)n2 * n3, kTile), 1), 256, sm1, s>>>(
+      data, n2 * n3, (long long)n2 * n3, 0, a1);
   HALF_LAUNCH("fft axis 1");
+}
+
+}  // namespace
+
+void fft3d_inplace(double2* data, const std::array<int, 3>& shape, int sign, cudaStream_t s) {
+  if (sign > 0) fft3d<+1>(data, shape, s);
+  else fft3d<-1>(data, shape, s);
 }
 
 // ------------------------------------------------------------------ Veff
