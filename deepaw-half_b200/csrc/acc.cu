@@ -285,7 +285,7 @@ struct SmallSolver {
     if (const char* po = std::getenv("HALF_PENCIL_OWN")) own_large = own && std::string(po) != "0";
     info.resize(3);
     info.zero(rt.stream);
-    if (own && (2 * m <= SmallEigen::kOwnMaxOrder || own_large)) eig.reserve(rt, 2 * m);
+    if (own) eig.reserve(rt, own_large ? 2 * m : std::min(2 * m, SmallEigen::kOwnMaxOrder));   // locking shrinks pencils below it
     int l1 = 0, l2 = 0, l3 = 0;
     cusolver_check(cusolverDnZheevd_bufferSize(rt.solver, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, m,
                                                reinterpret_cast<cuDoubleComplex*>(a), m, w, &l1),

@@ -25,6 +25,8 @@
 // The eigenvectors are finally Y = U^-1 V (trsm), giving Y^H B Y = I, the
 // same normalisation as zhegvd (itype 1, upper).
 #include <algorithm>
+#include <cooperative_groups.h>
+
 #include <cfloat>
 #include <cmath>
 #include <string>
@@ -35,40 +37,55 @@
 
 namespace hb {
 
+namespace cg = cooperative_groups;
+
 namespace {
 
 constexpr int kExtraEig = 8;   // eigenvalues located beyond the wanted ones (cluster at the cut)
-constexpr int kMetricMax = 164;   // packed triangle + two m-vectors within kSmemMax
 constexpr size_t kSmemMax = 226 * 1024;   // dynamic shared memory per CTA, leaving room for static
 
-// Number of eigenvalues of T below x (Sylvester inertia of T - x I).  The
+// Number of eigenvalues of T below x (Sylvester inertia of T - x I), T scaled
+// to a norm of at most 1 with squared off-diagonals floored at kE2Floor.  The
 // pivots of the LDL^T factorisation are ratios q_i = p_i / p_{i-1} of the
 // continuant p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2}, so the count is the
 // number of sign changes along p_0 = 1, p_1, ..., p_n.  Carrying p instead of
-// q keeps divisions off the dependent chain (one FMA per step).  A pivot of
-// magnitude below kPivFloor is replaced by -kPivFloor (LAPACK dstebz does the
-// same with its pivmin), and the pair (p_{i-1}, p_i) is rescaled by a power
-// of two whenever p_i leaves [2^-300, 2^300], which changes no ratio.
-constexpr double kPivFloor = 0x1p-400;
+// q keeps divisions off the dependent chain, which is one FMA per step: the
+// sign test works on the high words beside it, and the pair (p_{i-1}, p_i) is
+// rescaled by a power of two (which changes no ratio) only every four steps.
+// Per step the larger of the pair grows by at most |d - x| + e^2 <= 3 and
+// shrinks by at most kE2Floor / 4, so four steps from 2^-300 stay above
+// 2^-790.  That also means no pivot needs a floor of its own: a zero p_i is
+// followed by -e^2 p_{i-1}, and either sign given to it counts one change.
+// (One rescaling branch and a pivot test per step made a step about 170
+// cycles; order 144, 80 values: 116 us.)
+constexpr double kE2Floor = 0x1p-120;   // moves e by 2^-60 of the norm at most, below eps / 2 of it
+
+__device__ __forceinline__ void sturm_step(double di, double e2, double x, double& p0, double& p1, int& c) {
+  const double p2 = fma(di - x, p1, -e2 * p0);
+  c += (__double2hiint(p2) ^ __double2hiint(p1)) < 0;
+  p0 = p1;
+  p1 = p2;
+}
+
+__device__ __forceinline__ void sturm_rescale(double& p0, double& p1) {
+  const int ex = (__double2hiint(fabs(p0) > fabs(p1) ? p0 : p1) >> 20) & 0x7ff;   // biased exponent of the larger
+  if (ex > 1023 + 300 || ex < 1023 - 300) {
+    const double sc = __hiloint2double((2046 - max(ex, 1)) << 20, 0);   // 2^-(ex - 1023)
+    p0 *= sc;
+    p1 *= sc;
+  }
+}
 
 __device__ int sturm_count(const double* d, const double* e2, int n, double x) {
   double p0 = 1.0, p1 = d[0] - x;
-  if (fabs(p1) < kPivFloor) p1 = -kPivFloor;
-  int c = p1 < 0.0;
-  for (int i = 1; i < n; ++i) {
-    double p2 = fma(d[i] - x, p1, -e2[i - 1] * p0);
-    const double lim = kPivFloor * fabs(p1);
-    if (fabs(p2) < lim) p2 = p1 < 0.0 ? lim : -lim;
-    c += (p2 < 0.0) != (p1 < 0.0);
-    p0 = p1;
-    p1 = p2;
-    const double a = fabs(p1);
-    if (a > 0x1p300 || a < 0x1p-300) {   // |p_i| in [2^-700, 2^330] here; bring it to [1, 2)
-      const double sc = scalbn(1.0, -ilogb(p1));
-      p0 *= sc;
-      p1 *= sc;
-    }
+  int c = __double2hiint(p1) < 0;
+  int i = 1;
+  for (; i + 3 < n; i += 4) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sturm_step(d[i + q], e2[i + q - 1], x, p0, p1, c);
+    sturm_rescale(p0, p1);
   }
+  for (; i < n; ++i) sturm_step(d[i], e2[i - 1], x, p0, p1, c);
   return c;
 }
 
@@ -135,16 +152,22 @@ __device__ void tri_solve(int n, const double* ai, const double* b1, const doubl
   }
 }
 
-// Padded Gershgorin interval of T and the norm max_i (|d_i| + |e_{i-1}| + |e_i|);
-// both tridiagonal kernels evaluate it with this one routine, so they agree bit for bit.
+// Padded Gershgorin interval of T and the norm max_i (|d_i| + |e_{i-1}| + |e_i|),
+// by one warp; every lane gets the results.  Both tridiagonal kernels evaluate
+// it with this one routine, so they agree bit for bit.
 __device__ void gershgorin(const double* d, const double* e, int n, double& lo, double& hi, double& nrm) {
   double gl = d[0], gu = d[0];
   nrm = 0;
-  for (int i = 0; i < n; ++i) {
+  for (int i = threadIdx.x & 31; i < n; i += 32) {
     const double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i < n - 1 ? fabs(e[i]) : 0.0);
     gl = fmin(gl, d[i] - r);
     gu = fmax(gu, d[i] + r);
     nrm = fmax(nrm, fabs(d[i]) + r);
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    gl = fmin(gl, __shfl_xor_sync(0xffffffffu, gl, off));
+    gu = fmax(gu, __shfl_xor_sync(0xffffffffu, gu, off));
+    nrm = fmax(nrm, __shfl_xor_sync(0xffffffffu, nrm, off));
   }
   const double pad = 2.0 * DBL_EPSILON * fmax(fabs(gl), fabs(gu)) * n + 1e-300;
   lo = gl - pad;
@@ -152,15 +175,39 @@ __device__ void gershgorin(const double* d, const double* e, int n, double& lo, 
   nrm = fmax(nrm, DBL_MIN);
 }
 
+// Power of two that brings a norm below 1.
+__device__ __forceinline__ double norm_scale(double nrm) { return scalbn(1.0, -(ilogb(nrm) + 1)); }
+
+// Squared off-diagonal of the scaled T, floored for sturm_count.
+__device__ __forceinline__ double scaled_e2(double e, double sc) { return fmax((e * sc) * (e * sc), kE2Floor); }
+
 constexpr int kValueWarps = 8;       // eigenvalues per CTA of the value kernel, one warp each
 constexpr int kVectorThreads = 32;   // eigenvectors per CTA of the vector kernel, one thread each
 
-// Eigenvalues 0..ne-1 of T (ascending) by multisection: the 32 lanes of a warp
-// count at 32 interior points of its eigenvalue's bracket per round, which
-// shrinks to the pair of neighbouring points whose counts straddle the index
-// (33-fold per round).  Brackets end at 2 eps |lambda| + eps ||T|| (absolute
-// accuracy eps ||T||, as bisection guarantees).  Also clears *status for the
-// vector kernel that follows on the stream.
+// Eigenvalue k of the scaled T in [lo, hi] by multisection: the 32 lanes of a
+// warp count at 32 interior points of the bracket per round, which shrinks to
+// the pair of neighbouring points whose counts straddle the index (33-fold
+// per round).  Brackets end at 2 eps |lambda| + eps ||T|| (absolute accuracy
+// eps ||T||, as bisection guarantees).
+__device__ double multisect(const double* d, const double* e2, int n, int k, double lo, double hi, double tnorm) {
+  const int lane = threadIdx.x & 31;
+  for (int round = 0; round < 200; ++round) {   // lo and hi are warp-uniform throughout
+    if (hi - lo <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + DBL_EPSILON * tnorm) break;
+    const double x = lo + (hi - lo) * double(lane + 1) / 33.0;
+    const unsigned b = __ballot_sync(0xffffffffu, sturm_count(d, e2, n, x) > k);   // lambda_k < x
+    const int first = b ? __ffs(b) - 1 : 32;                                          // first point above
+    const double xlo = __shfl_sync(0xffffffffu, x, first > 0 ? first - 1 : 0);
+    const double xhi = __shfl_sync(0xffffffffu, x, first < 32 ? first : 31);
+    const double nlo = first > 0 ? xlo : lo, nhi = first < 32 ? xhi : hi;
+    if (!(nlo > lo || nhi < hi)) break;   // no progress left in floating point
+    lo = nlo;
+    hi = nhi;
+  }
+  return 0.5 * (lo + hi);
+}
+
+// Eigenvalues 0..ne-1 of T (ascending), one warp each.  Also clears *status
+// for the vector kernel that follows on the stream.
 __global__ void __launch_bounds__(32 * kValueWarps) tridiag_values_kernel(const double* __restrict__ d_in,
                                                                           const double* __restrict__ e_in, int n,
                                                                           int ne, double* __restrict__ lam,
@@ -173,31 +220,26 @@ __global__ void __launch_bounds__(32 * kValueWarps) tridiag_values_kernel(const 
   if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     d[i] = d_in[i];
-    const double ei = i < n - 1 ? e_in[i] : 0.0;
-    e[i] = ei;
-    e2[i] = ei * ei;
+    e[i] = i < n - 1 ? e_in[i] : 0.0;
   }
   __syncthreads();
-  if (threadIdx.x == 0) gershgorin(d, e, n, s_gl, s_gu, s_norm);
+  if (threadIdx.x < 32) {
+    double gl, gu, nrm;
+    gershgorin(d, e, n, gl, gu, nrm);
+    if (threadIdx.x == 0) { s_gl = gl; s_gu = gu; s_norm = nrm; }
+  }
+  __syncthreads();
+  const double sc = norm_scale(s_norm);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    d[i] *= sc;
+    e2[i] = scaled_e2(e[i], sc);
+  }
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int k = blockIdx.x * kValueWarps + (threadIdx.x >> 5);
   if (k >= ne) return;   // whole warps; no barrier follows
-  const double tnorm = s_norm;
-  double lo = s_gl, hi = s_gu;   // warp-uniform throughout
-  for (int round = 0; round < 200; ++round) {
-    if (hi - lo <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + DBL_EPSILON * tnorm) break;
-    const double x = lo + (hi - lo) * double(lane + 1) / 33.0;
-    const unsigned b = __ballot_sync(0xffffffffu, sturm_count(d, e2, n, x) > k);   // lambda_k < x
-    const int first = b ? __ffs(b) - 1 : 32;                                          // first point above
-    const double xlo = __shfl_sync(0xffffffffu, x, first > 0 ? first - 1 : 0);
-    const double xhi = __shfl_sync(0xffffffffu, x, first < 32 ? first : 31);
-    const double nlo = first > 0 ? xlo : lo, nhi = first < 32 ? xhi : hi;
-    if (!(nlo > lo || nhi < hi)) break;   // no progress left in floating point
-    lo = nlo;
-    hi = nhi;
-  }
-  if (lane == 0) lam[k] = 0.5 * (lo + hi);
+  const double v = multisect(d, e2, n, k, s_gl * sc, s_gu * sc, s_norm * sc);
+  if (lane == 0) lam[k] = v / sc;
 }
 
 // Eigenvectors of lam[0..nev) by inverse iteration on the pivoted LU of
@@ -210,9 +252,12 @@ __global__ void __launch_bounds__(32 * kValueWarps) tridiag_values_kernel(const 
 // |<z_i, z_j>| <= eps ||T|| / gap <~ 1e-9.  Scratch: five n-vectors and the
 // pivot flags per thread, interleaved by thread (a warp touches consecutive
 // words), in shared memory after the tables when gscratch is null, else in
-// global memory with one slot per thread of the grid.
+// global memory with one slot per eigenvector.  A CTA takes `per` eigenvectors,
+// as many as its shared memory holds (32 at order 138, 8 at order 432): the
+// threads run serial chains, so few of them per SM cost nothing, while
+// scratch in global memory puts a cache miss into every link.
 __global__ void __launch_bounds__(kVectorThreads) tridiag_vectors_kernel(
-    const double* __restrict__ d_in, const double* __restrict__ e_in, int n, int nev, int ne,
+    const double* __restrict__ d_in, const double* __restrict__ e_in, int n, int nev, int ne, int per,
     const double* __restrict__ lam_g, double* __restrict__ w, double* __restrict__ Z, double* __restrict__ gscratch,
     int* __restrict__ status) {
   extern __shared__ double sm[];
@@ -220,25 +265,23 @@ __global__ void __launch_bounds__(kVectorThreads) tridiag_vectors_kernel(
   double* e = d + n;
   double* lam = e + n;
   int* cl_first = reinterpret_cast<int*>(lam + ne);
-  __shared__ double s_gl, s_gu, s_norm;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     d[i] = d_in[i];
     e[i] = i < n - 1 ? e_in[i] : 0.0;
   }
   for (int i = threadIdx.x; i < ne; i += blockDim.x) lam[i] = lam_g[i];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    gershgorin(d, e, n, s_gl, s_gu, s_norm);
-    const double ortol = 1.0e-7 * s_norm;
-    int first = 0;
-    for (int k = 0; k < ne; ++k) {
-      if (k > 0 && lam[k] - lam[k - 1] > ortol) first = k;
-      cl_first[k] = first;
-    }
+  double gl, gu, tnorm;   // one warp (kVectorThreads) evaluates, every thread holds the results
+  gershgorin(d, e, n, gl, gu, tnorm);
+  const double ortol = 1.0e-7 * tnorm;
+  for (int k = threadIdx.x; k < ne; k += blockDim.x) {   // first member of each value's cluster
+    int f = k;
+    while (f > 0 && !(lam[f] - lam[f - 1] > ortol)) --f;
+    cl_first[k] = f;
   }
   __syncthreads();
-  const double tnorm = s_norm;
-  const int k0 = blockIdx.x * blockDim.x + threadIdx.x;
+  const int k0 = blockIdx.x * per + threadIdx.x;
+  if (int(threadIdx.x) >= per) return;
   if (k0 < nev) w[k0] = lam[k0];
   if (k0 >= nev || cl_first[k0] != k0) return;
   const double tiny = DBL_EPSILON * tnorm;
@@ -246,14 +289,14 @@ __global__ void __launch_bounds__(kVectorThreads) tridiag_vectors_kernel(
   unsigned char* piv;
   int st;
   if (gscratch) {
-    st = gridDim.x * blockDim.x;
+    st = gridDim.x * per;
     ai = gscratch + k0;
     piv = reinterpret_cast<unsigned char*>(gscratch + 5 * size_t(n) * st) + k0;
   } else {
     size_t off = (2 * size_t(n) + ne) * sizeof(double) + size_t(ne) * sizeof(int);
     off = (off + 15) & ~size_t(15);
     double* sbase = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(sm) + off);
-    st = blockDim.x;
+    st = per;
     ai = sbase + threadIdx.x;
     piv = reinterpret_cast<unsigned char*>(sbase + 5 * size_t(n) * st) + threadIdx.x;
   }
@@ -309,62 +352,144 @@ __global__ void __launch_bounds__(kVectorThreads) tridiag_vectors_kernel(
   }
 }
 
-constexpr int kBackWarps = 8;   // eigenvectors per CTA of the back-transformation, one warp each
+constexpr int kBackWarps = 4;      // eigenvectors per CTA of the back-transformation, one warp each
+constexpr int kBackBlock = 4;      // reflectors applied together
 
-// V[:, j] = H(1) H(2) ... applied as Q z_j with Q = H(n-1) ... H(1)
-// (LAPACK zhetrd, UPLO = 'U': v(i) = 1, v(1:i-1) = A(1:i-1, i+1), tau(i)).
-// The CTA's warps share the reflectors, staged in shared memory `chunk` at a
-// time (v with its unit entry and zeros below, so the inner loops have no
-// branch); each warp applies them to its eigenvector in order.
+__device__ __forceinline__ void copy16_async(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+
+// Sums over the warp of eight values per lane at once: afterwards `v[0]` of
+// lane l holds the sum of value l >> 2 (9 exchanges instead of 40).
+__device__ __forceinline__ double warp_sum8(double (&v)[8]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int half = 4, bit = 16; half >= 1; half >>= 1, bit >>= 1) {
+    const bool up = lane & bit;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const double send = up ? v[i] : v[i + half], keep = up ? v[i + half] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+    }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  return v[0];
+}
+
+// V[:, j] = Q z_j with Q = H(n-1) ... H(1) (LAPACK zhetrd, UPLO = 'U':
+// v(i) = 1, v(1:i-1) = A(1:i-1, i+1), tau(i)).  One warp per eigenvector, the
+// vector in registers (row lane + 32 t in slot t < RX); the CTA's warps share
+// the reflectors, staged in shared memory `chunk` at a time (v with its unit
+// entry and zeros below).  A reflector by itself is a dot product, a
+// five-step shuffle reduction and an update, all dependent; four at a time
+// share one reduction: with d_i = v_i^H x and the Gram g_ij = v_i^H v_j
+// (j < i),  w_i = tau_i (d_i - sum_j g_ij w_j)  and  x -= sum_i w_i v_i.
+template <int RX>
 __global__ void __launch_bounds__(32 * kBackWarps) back_transform_kernel(const double2* __restrict__ A,
                                                                          const double2* __restrict__ tau,
                                                                          const double* __restrict__ Z, int n, int nev,
                                                                          int chunk, double2* __restrict__ V) {
-  extern __shared__ double2 sv[];
+  extern __shared__ __align__(16) double2 vs[];     // chunk x n
+  double2* ts = vs + (size_t)chunk * n;             // chunk
+  double2* gram = ts + chunk;                       // chunk / 4 x 8: g10, g20, g21, g30, g31, g32
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int j = blockIdx.x * kBackWarps + warp;
   const bool active = j < nev;
-  double2* x = sv + (size_t)warp * n;
-  double2* vs = sv + (size_t)kBackWarps * n;   // chunk x n
-  double2* ts = vs + (size_t)chunk * n;        // chunk
-  if (active)
-    for (int r = lane; r < n; r += 32) x[r] = make_double2(Z[(size_t)j * n + r], 0.0);
+  double2 x[RX];
+#pragma unroll
+  for (int t = 0; t < RX; ++t) {
+    const int r = lane + 32 * t;
+    x[t] = make_double2(active && r < n ? Z[(size_t)j * n + r] : 0.0, 0.0);
+  }
   for (int c0 = 0; c0 <= n - 2; c0 += chunk) {
     const int cnt = min(chunk, n - 1 - c0);
+    const int blocks = (cnt + kBackBlock - 1) / kBackBlock;
     __syncthreads();   // the previous chunk is consumed
-    for (int t = threadIdx.x; t < cnt * n; t += blockDim.x) {
-      const int q = t / n, row = t - q * n, i0 = c0 + q;
-      vs[t] = row < i0 ? A[(size_t)(i0 + 1) * n + row] : make_double2(row == i0 ? 1.0 : 0.0, 0.0);
+    for (int q = warp; q < blocks * kBackBlock; q += kBackWarps) {   // reflectors beyond the last: zero
+      const int i0 = c0 + q;
+      for (int r = lane; r < n; r += 32) {
+        if (q < cnt && r < i0) copy16_async(vs + (size_t)q * n + r, A + (size_t)(i0 + 1) * n + r);
+        else vs[(size_t)q * n + r] = make_double2(q < cnt && r == i0 ? 1.0 : 0.0, 0.0);
+      }
+      if (lane == 0) ts[q] = q < cnt ? tau[i0] : make_double2(0.0, 0.0);
     }
-    for (int t = threadIdx.x; t < cnt; t += blockDim.x) ts[t] = tau[c0 + t];
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    for (int b = warp; b < blocks; b += kBackWarps) {
+      const double2* v0 = vs + (size_t)b * kBackBlock * n;
+      double g[2][8] = {};
+      for (int r = lane; r < min(n, c0 + (b + 1) * kBackBlock); r += 32) {
+        const double2 a0 = v0[r], a1 = v0[n + r], a2 = v0[2 * n + r], a3 = v0[3 * n + r];
+        auto dot = [](double* o, double2 p, double2 q) {   // conj(p) q
+          o[0] += p.x * q.x + p.y * q.y;
+          o[1] += p.x * q.y - p.y * q.x;
+        };
+        dot(g[0], a1, a0);
+        dot(g[0] + 2, a2, a0);
+        dot(g[0] + 4, a2, a1);
+        dot(g[0] + 6, a3, a0);
+        dot(g[1], a3, a1);
+        dot(g[1] + 2, a3, a2);
+      }
+      double* out = reinterpret_cast<double*>(gram + b * 8);
+      const double s0 = warp_sum8(g[0]), s1 = warp_sum8(g[1]);
+      if ((lane & 3) == 0) {
+        out[lane >> 2] = s0;
+        if ((lane >> 2) < 4) out[8 + (lane >> 2)] = s1;
+      }
+    }
     __syncthreads();
     if (!active) continue;
-    for (int q = 0; q < cnt; ++q) {
-      const int i0 = c0 + q;
-      const double2* v = vs + (size_t)q * n;
-      const double2 t = ts[q];
-      double wr = 0, wi = 0;
-      for (int r = lane; r <= i0; r += 32) {
-        const double2 vr = v[r], xr = x[r];
-        wr += vr.x * xr.x + vr.y * xr.y;   // conj(v) . x
-        wi += vr.x * xr.y - vr.y * xr.x;
+    for (int b = 0; b < blocks; ++b) {
+      const double2* v = vs + (size_t)b * kBackBlock * n;
+      const int rows = min(n, c0 + (b + 1) * kBackBlock);   // rows 0 .. i0 of the block's last reflector
+      double d[8] = {};
+#pragma unroll
+      for (int t = 0; t < RX; ++t) {
+        const int r = lane + 32 * t;
+        if (r < rows) {
+#pragma unroll
+          for (int i = 0; i < kBackBlock; ++i) {
+            const double2 a = v[i * n + r];
+            d[2 * i] += a.x * x[t].x + a.y * x[t].y;
+            d[2 * i + 1] += a.x * x[t].y - a.y * x[t].x;
+          }
+        }
       }
-      for (int off = 16; off > 0; off >>= 1) {
-        wr += __shfl_xor_sync(0xffffffffu, wr, off);
-        wi += __shfl_xor_sync(0xffffffffu, wi, off);
+      const double mine = warp_sum8(d);
+      double2 w[kBackBlock];
+#pragma unroll
+      for (int i = 0; i < kBackBlock; ++i) {
+        w[i].x = __shfl_sync(0xffffffffu, mine, 8 * i);
+        w[i].y = __shfl_sync(0xffffffffu, mine, 8 * i + 4);
       }
-      // x -= tau * w * v
-      const double cr = t.x * wr - t.y * wi, ci = t.x * wi + t.y * wr;
-      for (int r = lane; r <= i0; r += 32) {
-        const double2 vr = v[r];
-        x[r].x -= cr * vr.x - ci * vr.y;
-        x[r].y -= cr * vr.y + ci * vr.x;
+      const double2* g = gram + b * 8;
+#pragma unroll
+      for (int i = 0; i < kBackBlock; ++i) {
+#pragma unroll
+        for (int k = 0; k < i; ++k) w[i] = csub(w[i], cmul(g[i * (i - 1) / 2 + k], w[k]));
+        w[i] = cmul(ts[b * kBackBlock + i], w[i]);
       }
-      __syncwarp();
+#pragma unroll
+      for (int t = 0; t < RX; ++t) {
+        const int r = lane + 32 * t;
+        if (r < rows) {
+#pragma unroll
+          for (int i = 0; i < kBackBlock; ++i) x[t] = csub(x[t], cmul(v[i * n + r], w[i]));
+        }
+      }
     }
   }
-  if (active)
-    for (int r = lane; r < n; r += 32) V[(size_t)j * n + r] = x[r];
+  if (active) {
+#pragma unroll
+    for (int t = 0; t < RX; ++t) {
+      const int r = lane + 32 * t;
+      if (r < n) V[(size_t)j * n + r] = x[t];
+    }
+  }
 }
 
 // lower triangle from the upper one (Hermitian)
@@ -393,118 +518,143 @@ __global__ void hermitian_fill_kernel(double2* A, int n) {
 // the direction stays in the span without being eliminated from later
 // columns.
 //
-// One CTA, the packed upper triangle in shared memory (m <= kMetricMax), and
-// ONE right-looking sweep that builds R^-1 together with R.  With
-// T(i,j) = sum_{l<j} X(i,l) R(l,j) for i < j (X = R^-1), step k is
+// One cluster of CTAs keeps the matrix in its shared memory, column j on CTA
+// j mod P, and makes ONE right-looking sweep that builds R^-1 together with R.
+// With T(i,j) = sum_{l<j} X(i,l) R(l,j) for i < j (X = R^-1), step k is
 //   W(i,j) -= conj(W(k,i)) W(k,j) / p_k    k < i <= j   (trailing Schur complement)
 //   T(i,j) -= T(i,k) W(k,j) / p_k          i < k < j
 //   T(k,j)  = W(k,j) / p_k                 j > k         (row k becomes X(k,k) R(k,j))
-// with p_k = W(k,k): a rank-1 update of every stored column right of k.  The
-// two index ranges occupy disjoint slots of one packed triangle (rows <= k
-// hold T, rows > k hold W), and at the end X(i,j) = -T(i,j) / R(j,j),
-// X(j,j) = 1 / R(j,j).  Two CTA barriers per step; the update's row factors
-// are held in registers (lane-owned rows), its column factors broadcast from
-// shared memory.  *status = 1 if a pivot was not finite.
-constexpr int kFactorThreads = 1024;
-constexpr int kFactorRows = (kMetricMax + 31) / 32;   // lane-owned rows per thread
+// with p_k = W(k,k): a rank-1 update of every column right of k.  The two
+// index ranges occupy disjoint rows of a column (rows <= k hold T, rows > k
+// hold W), and at the end X(i,j) = -T(i,j) / R(j,j), X(j,j) = 1 / R(j,j).
+// What a step needs from other CTAs is row k of W, which every CTA pushes to
+// all of them as it updates its columns in the step before, and column k of
+// T, which its owner no longer changes: one cluster barrier per step.
+// *status = 1 if a pivot was not finite.
+//
+// Bound by the chain of barriers and shared-memory round trips, about 1 us a
+// step: one CTA with the packed triangle in its own shared memory (orders up
+// to 164) took 2.0 us a step at order 140 from its rank-1 updates alone.
+constexpr int kClThreads = 256;
+constexpr int kClWarps = kClThreads / 32;
+constexpr int kClCols = 4;                        // columns a warp carries at once
 
-__global__ void __launch_bounds__(kFactorThreads) metric_factor_kernel(double2* __restrict__ M, int m,
-                                                                      int* __restrict__ status) {
-  extern __shared__ double2 pk[];                  // packed upper triangle, (i, j) at j (j + 1) / 2 + i
-  double2* av = pk + size_t(m) * (m + 1) / 2;      // row factors of the step (T(i,k) or conj W(k,i))
-  double2* cv = av + m;                            // column factors W(k,j) / p_k
-  double* dsc = reinterpret_cast<double*>(cv + m);   // D
-  double* ir = dsc + m;                              // 1 / R(k,k)
-  __shared__ int s_bad;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
-  if (tid == 0) s_bad = 0;
-  for (int j = tid; j < m; j += nt) dsc[j] = 1.0 / sqrt(fmax(M[size_t(j) * m + j].x, DBL_MIN));
-  __syncthreads();
-  for (int j = warp; j < m; j += nw) {
+__host__ __device__ inline size_t factor_smem(int m, int p) {
+  return (size_t((m + p - 1) / p) * m + 3 * size_t(m)) * sizeof(double2) + 2 * size_t(m) * sizeof(double);
+}
+
+__global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __restrict__ M, int m,
+                                                                   int* __restrict__ status) {
+  cg::cluster_group cl = cg::this_cluster();
+  const int P = int(cl.num_blocks()), rank = int(cl.block_rank());
+  const int nc = (m + P - 1) / P;
+  extern __shared__ __align__(16) double2 cols[];   // nc x m: column jl P + rank at cols + jl m
+  double2* gbuf = cols + size_t(nc) * m;            // 2 x m: row k of W, by parity of k
+  double2* av = gbuf + 2 * m;                       // row factors of the step (T(i,k) or conj W(k,i))
+  double* dsc = reinterpret_cast<double*>(av + m);  // D
+  double* ir = dsc + m;                             // 1 / R(k,k)
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int j = tid; j < m; j += kClThreads) dsc[j] = 1.0 / sqrt(fmax(M[size_t(j) * m + j].x, DBL_MIN));
+  cl.sync();   // every CTA's buffers exist, dsc is filled
+  for (int jl = warp; jl * P + rank < m; jl += kClWarps) {
+    const int j = jl * P + rank;
     const double dj = dsc[j];
-    double2* col = pk + size_t(j) * (j + 1) / 2;
     for (int i = lane; i <= j; i += 32) {
       double2 v = M[size_t(j) * m + i];
       if (i == j) v.y = 0.0;
-      col[i] = cscale(v, dsc[i] * dj);
+      cols[size_t(jl) * m + i] = cscale(v, dsc[i] * dj);
     }
+    __syncwarp();
+    if (lane < P) cl.map_shared_rank(gbuf, lane)[j] = cols[size_t(jl) * m];
   }
-  __syncthreads();
+  cl.sync();
+  int bad = 0;
   for (int k = 0; k < m; ++k) {
-    // phase A: pivot (every thread, same value) and the step's factor vectors
-    const double p = pk[size_t(k) * (k + 1) / 2 + k].x;
+    const double2* g = gbuf + (k & 1) * m;
+    double2* gn = gbuf + ((k + 1) & 1) * m;
+    const double p = g[k].x;
     const bool dep = !(p > 1.0e-14);   // also true for NaN
     const double invp = dep ? 0.0 : 1.0 / p;
-    if (tid == 0) {
-      if (!isfinite(p)) s_bad = 1;
-      ir[k] = dep ? 1.0e7 : 1.0 / sqrt(p);
-    }
-    const double2* colk = pk + size_t(k) * (k + 1) / 2;
-    for (int i = tid; i < m; i += nt) {
-      if (i < k) {
-        av[i] = colk[i];                                     // T(i, k)
-      } else if (i > k) {
-        const double2 w = pk[size_t(i) * (i + 1) / 2 + k];   // W(k, i)
-        av[i] = make_double2(w.x, -w.y);
-        cv[i] = cscale(w, invp);
-      }
+    if (!isfinite(p)) bad = 1;
+    if (tid == 0) ir[k] = dep ? 1.0e7 : 1.0 / sqrt(p);
+    const double2* tk = cl.map_shared_rank(cols, k % P) + size_t(k / P) * m;
+    for (int i = tid; i < m; i += kClThreads) {
+      double2 a = make_double2(0.0, 0.0);
+      if (i < k) a = tk[i];
+      else if (i > k) a = make_double2(g[i].x, -g[i].y);
+      av[i] = a;
     }
     __syncthreads();
-    // phase B: columns j > k, one warp per column, lane-owned rows i = lane + 32 t
-    double2 a[kFactorRows];
+    int jl0 = k + 1 > rank ? (k + 1 - rank + P - 1) / P : 0;   // first owned column right of k
+    for (jl0 += warp; jl0 * P + rank < m; jl0 += kClWarps * kClCols) {
+      double2 c[kClCols];
+      int jj[kClCols];
 #pragma unroll
-    for (int t = 0; t < kFactorRows; ++t) {
-      const int i = lane + 32 * t;
-      a[t] = i < m && i != k ? av[i] : make_double2(0.0, 0.0);
-    }
-    for (int j = k + 1 + warp; j < m; j += nw) {
-      const double2 c = cv[j];
-      double2* col = pk + size_t(j) * (j + 1) / 2;
+      for (int q = 0; q < kClCols; ++q) {
+        jj[q] = (jl0 + q * kClWarps) * P + rank;
+        c[q] = jj[q] < m ? cscale(g[jj[q]], invp) : make_double2(0.0, 0.0);
+      }
+      const int jmax = min(m - 1, jj[kClCols - 1]);
+      for (int i = lane; i <= jmax; i += 32) {
+        const double2 a = av[i];
 #pragma unroll
-      for (int t = 0; t < kFactorRows; ++t) {
-        const int i = lane + 32 * t;
-        if (i <= j) {
-          if (i == k) {
-            col[i] = c;
-          } else if (!dep) {
-            double2 x = col[i];
-            x.x -= a[t].x * c.x - a[t].y * c.y;
-            x.y -= a[t].x * c.y + a[t].y * c.x;
-            col[i] = x;
+        for (int q = 0; q < kClCols; ++q) {
+          if (i <= jj[q] && jj[q] < m) {
+            double2* e = cols + size_t(jl0 + q * kClWarps) * m + i;
+            if (i == k) {
+              *e = c[q];
+            } else if (!dep) {
+              double2 x = *e;
+              x.x -= a.x * c[q].x - a.y * c[q].y;
+              x.y -= a.x * c[q].y + a.y * c[q].x;
+              *e = x;
+            }
           }
         }
       }
+      __syncwarp();
+      // row k + 1 of these columns to every CTA: eight lanes per column
+      {
+        const int q = lane >> 3, j = (jl0 + q * kClWarps) * P + rank;
+        if (j < m) {
+          const double2 v = cols[size_t(jl0 + q * kClWarps) * m + k + 1];
+          for (int r = lane & 7; r < P; r += 8) cl.map_shared_rank(gn, r)[j] = v;
+        }
+      }
     }
-    __syncthreads();
+    cl.sync();
   }
   // U = D X with X(i,j) = -T(i,j) / R(j,j), X(j,j) = 1 / R(j,j); lower triangle zero
-  for (int j = warp; j < m; j += nw) {
-    const double2* col = pk + size_t(j) * (j + 1) / 2;
+  for (int jl = warp; jl * P + rank < m; jl += kClWarps) {
+    const int j = jl * P + rank;
     const double irj = ir[j];
     for (int i = lane; i < m; i += 32) {
       double2 u = make_double2(0.0, 0.0);
-      if (i < j) u = cscale(col[i], -irj * dsc[i]);
+      if (i < j) u = cscale(cols[size_t(jl) * m + i], -irj * dsc[i]);
       else if (i == j) u = make_double2(irj * dsc[i], 0.0);
       M[size_t(j) * m + i] = u;
     }
   }
-  if (tid == 0) *status = s_bad;
+  if (rank == 0 && tid == 0) *status = bad;
 }
 
-// Block-wide sum of a (real, imaginary) pair; every thread gets the result.
-__device__ double2 block_sum2(double a, double b, double* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// Block-wide sum of a (real, imaginary) pair through red (one slot per warp,
+// not reused before another barrier); every thread gets the result.
+__device__ __forceinline__ double2 block_sum2(double a, double b, double2* red) {
   for (int off = 16; off > 0; off >>= 1) {
     a += __shfl_xor_sync(0xffffffffu, a, off);
     b += __shfl_xor_sync(0xffffffffu, b, off);
   }
-  __syncthreads();   // red may still be read by a previous call
-  if (lane == 0) { red[2 * warp] = a; red[2 * warp + 1] = b; }
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_double2(a, b);
   __syncthreads();
-  double sa = 0, sb = 0;
-  for (int w = 0; w < nw; ++w) { sa += red[2 * w]; sb += red[2 * w + 1]; }
-  return make_double2(sa, sb);
+  double2 s = red[0];
+#pragma unroll
+  for (int w = 1; w < kClWarps; ++w) s = cadd(s, red[w]);
+  return s;
+}
+
+__host__ __device__ inline size_t hetrd_smem(int n, int p) {
+  return (size_t((n + p - 1) / p) * n + 5 * size_t(n)) * sizeof(double2);
 }
 
 // Householder reduction of a Hermitian A (n x n, upper triangle read) to the
@@ -512,130 +662,197 @@ __device__ double2 block_sum2(double a, double b, double* red) {
 // with UPLO = 'U' (the published zhetd2 algorithm): for i = n-2 .. 0 the
 // reflector H(i) = I - tau_i v v^H with v(i) = 1 and v(0:i-1) left in
 // A(0:i-1, i+1) annihilates A(0:i-1, i+1); d = diag(T), e = superdiagonal.
-// One CTA; the packed upper triangle stays in shared memory for the whole
-// reduction (n <= kMetricMax), replacing a launch pair per reflector.
-__global__ void __launch_bounds__(512) hetrd_kernel(double2* __restrict__ A, int n, double* __restrict__ dout,
-                                                    double* __restrict__ eout, double2* __restrict__ tauout) {
-  extern __shared__ double2 pk[];
-  double2* v = pk + size_t(n) * (n + 1) / 2;
-  double2* y = v + n;
-  __shared__ double red[64];
-  __shared__ double2 s_tau, s_scale, s_alpha2;
-  __shared__ double s_beta;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
-  auto at = [](int i, int j) { return j * (j + 1) / 2 + i; };
-  for (int q = tid; q < n * n; q += nt) {
-    const int i = q % n, j = q / n;
-    if (i <= j) {
-      double2 a = A[q];
-      if (i == j) a.y = 0.0;
-      pk[at(i, j)] = a;
+//
+// One cluster of CTAs holds the whole (both triangles) matrix in its shared
+// memory, column j on CTA j mod P, so y = A v is one local dot product per
+// column.  Per step: every CTA forms the reflector from its copy of the pivot
+// column; one pass over its columns applies the previous step's rank-2 update
+// and the product with v together; it pushes its entries of y to every CTA;
+// one cluster barrier; then every CTA forms w = y - (tau y^H v / 2) v and the
+// next pivot column (pulled from its owner, updated locally).  All CTAs do
+// the same arithmetic in the same order, so their copies agree bit for bit.
+//
+// Bound by the chain of three block barriers, one cluster barrier and the
+// exchange per step; the shared-memory traffic of the pass (32 bytes per
+// element, the vectors read once per four columns) shows above order 300.
+// One CTA with the packed triangle took 6.1 us a step at order 144.
+constexpr int kTrdRows = 2;                        // rows of a vector per thread
+static_assert(SmallEigen::kOwnMaxOrder <= kTrdRows * kClThreads, "rows of a vector per thread");
+
+__global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__ A, int n, double* __restrict__ dout,
+                                                           double* __restrict__ eout, double2* __restrict__ tauout) {
+  cg::cluster_group cl = cg::this_cluster();
+  const int P = int(cl.num_blocks()), rank = int(cl.block_rank());
+  const int nc = (n + P - 1) / P;
+  extern __shared__ __align__(16) double2 cols[];   // nc x n: column jl P + rank at cols + jl n
+  double2* ybuf = cols + size_t(nc) * n;            // 2 x n: tau A v, by parity of the step
+  double2* vbuf = ybuf + 2 * n;                     // 2 x n: this and the previous step's v
+  double2* wbuf = vbuf + 2 * n;                     // n: the previous step's w
+  __shared__ double2 red[2][kClWarps];
+  __shared__ double2 s_alpha[2];
+  __shared__ double s_diag[2];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int jl = warp; jl * P + rank < n; jl += kClWarps) {
+    const int j = jl * P + rank;
+    for (int r = lane; r < n; r += 32) {
+      double2 a = r <= j ? A[size_t(j) * n + r] : A[size_t(r) * n + j];
+      if (r == j) a.y = 0.0;
+      if (r > j) a.y = -a.y;
+      cols[size_t(jl) * n + r] = a;
     }
   }
-  __syncthreads();
-  for (int i0 = n - 2; i0 >= 0; --i0) {
-    const int L = i0 + 1, c = i0 + 1;
-    // zlarfg on (alpha = A(i0, c), x = A(0:i0-1, c))
+  for (int r = tid; r < n; r += kClThreads) {
+    vbuf[r] = vbuf[n + r] = wbuf[r] = make_double2(0.0, 0.0);
+  }
+  cl.sync();
+  double2 x[kTrdRows];   // the pivot column, rows tid + kClThreads t
+  {
+    const double2* c = cl.map_shared_rank(cols, (n - 1) % P) + size_t((n - 1) / P) * n;
+#pragma unroll
+    for (int t = 0; t < kTrdRows; ++t) {
+      const int r = tid + kClThreads * t;
+      x[t] = r < n ? c[r] : make_double2(0.0, 0.0);
+    }
+  }
+  int par = 0;
+  for (int i0 = n - 2; i0 >= 0; --i0, par ^= 1) {
+    const int c = i0 + 1, L = i0 + 1;
+    // zlarfg on (alpha = x(i0), x(0:i0-1))
     double part = 0;
-    for (int r = tid; r < i0; r += nt) {
-      const double2 x = pk[at(r, c)];
-      part += x.x * x.x + x.y * x.y;
+#pragma unroll
+    for (int t = 0; t < kTrdRows; ++t) {
+      const int r = tid + kClThreads * t;
+      if (r < i0) part += x[t].x * x[t].x + x[t].y * x[t].y;
+      if (r == i0) s_alpha[par] = x[t];
+      if (r == c) s_diag[par] = x[t].x;
     }
-    const double xn2 = block_sum2(part, 0.0, red).x;
-    if (tid == 0) {
-      const double2 al = pk[at(i0, c)];
-      if (xn2 == 0.0 && al.y == 0.0) {
-        s_tau = make_double2(0.0, 0.0);
-        s_beta = al.x;
-        s_scale = make_double2(1.0, 0.0);
-      } else {
-        const double beta = -copysign(sqrt(al.x * al.x + al.y * al.y + xn2), al.x);
-        s_tau = make_double2((beta - al.x) / beta, -al.y / beta);
-        const double dr = al.x - beta, di = al.y, den = dr * dr + di * di;
-        s_scale = make_double2(dr / den, -di / den);   // 1 / (alpha - beta)
-        s_beta = beta;
-      }
+    const double xn2 = block_sum2(part, 0.0, red[0]).x;   // its barrier also covers s_alpha and s_diag
+    const double2 al = s_alpha[par];
+    double2 tau = make_double2(0.0, 0.0), sc = make_double2(1.0, 0.0);
+    double beta = al.x;
+    if (!(xn2 == 0.0 && al.y == 0.0)) {
+      beta = -copysign(sqrt(al.x * al.x + al.y * al.y + xn2), al.x);
+      tau = make_double2((beta - al.x) / beta, -al.y / beta);
+      const double dr = al.x - beta, di = al.y, den = dr * dr + di * di;
+      sc = make_double2(dr / den, -di / den);   // 1 / (alpha - beta)
     }
-    __syncthreads();
-    const double2 tau = s_tau, sc = s_scale;
-    for (int r = tid; r < L; r += nt) {
-      double2 vr = make_double2(1.0, 0.0);
+    double2* v = vbuf + par * n;
+    const double2* vp = vbuf + (par ^ 1) * n;
+    double2 vr[kTrdRows];
+#pragma unroll
+    for (int t = 0; t < kTrdRows; ++t) {
+      const int r = tid + kClThreads * t;
+      vr[t] = make_double2(0.0, 0.0);
       if (r < i0) {
-        const double2 x = pk[at(r, c)];
-        vr = make_double2(x.x * sc.x - x.y * sc.y, x.x * sc.y + x.y * sc.x);
-        pk[at(r, c)] = vr;
+        vr[t] = cmul(x[t], sc);
+        if (rank == c % P) A[size_t(c) * n + r] = vr[t];
+      } else if (r == i0) {
+        vr[t] = make_double2(1.0, 0.0);
       }
-      v[r] = vr;
+      if (r <= i0) v[r] = vr[t];
     }
-    __syncthreads();
-    if (tau.x != 0.0 || tau.y != 0.0) {
-      // y = tau A(0:i0, 0:i0) v: g = 2^k threads per row, partial sums over
-      // s = p, p + g, ... combined by shuffles (deterministic order)
-      {
-        int lg = 0;
-        while (lg < 5 && (2 << lg) * L <= nt) ++lg;
-        const int g = 1 << lg, r = tid >> lg, p = tid & (g - 1);
-        double sr = 0, si = 0;
-        if (r < L) {
-          const double2* cr = pk + r * (r + 1) / 2;   // column r: A(s, r), s <= r
-          for (int s2 = p; s2 < L; s2 += g) {
-            double2 a;
-            if (r <= s2) a = pk[s2 * (s2 + 1) / 2 + r];
-            else { a = cr[s2]; a.y = -a.y; }
-            const double2 vv = v[s2];
-            sr += a.x * vv.x - a.y * vv.y;
-            si += a.x * vv.y + a.y * vv.x;
-          }
-        }
-        for (int off = g >> 1; off > 0; off >>= 1) {
-          sr += __shfl_xor_sync(0xffffffffu, sr, off);
-          si += __shfl_xor_sync(0xffffffffu, si, off);
-        }
-        if (r < L && p == 0) y[r] = make_double2(tau.x * sr - tau.y * si, tau.x * si + tau.y * sr);
-      }
-      __syncthreads();
-      // alpha2 = -tau (y^H v) / 2; w = y + alpha2 v
-      double pr = 0, pi = 0;
-      for (int r = tid; r < L; r += nt) {
-        const double2 yy = y[r], vv = v[r];
-        pr += yy.x * vv.x + yy.y * vv.y;   // conj(y) v
-        pi += yy.x * vv.y - yy.y * vv.x;
-      }
-      const double2 dot = block_sum2(pr, pi, red);
-      if (tid == 0) s_alpha2 = make_double2(-0.5 * (tau.x * dot.x - tau.y * dot.y), -0.5 * (tau.x * dot.y + tau.y * dot.x));
-      __syncthreads();
-      const double2 a2 = s_alpha2;
-      for (int r = tid; r < L; r += nt) {
-        const double2 vv = v[r];
-        y[r].x += a2.x * vv.x - a2.y * vv.y;
-        y[r].y += a2.x * vv.y + a2.y * vv.x;
-      }
-      __syncthreads();
-      // A(0:i0, 0:i0) -= v w^H + w v^H (upper triangle), one warp per column
-      for (int s2 = warp; s2 < L; s2 += nw) {
-        const double2 ws = y[s2], vs = v[s2];
-        double2* cs = pk + s2 * (s2 + 1) / 2;
-        for (int r = lane; r <= s2; r += 32) {
-          const double2 vr = v[r], wr = y[r];
-          cs[r].x -= (vr.x * ws.x + vr.y * ws.y) + (wr.x * vs.x + wr.y * vs.y);
-          cs[r].y -= (vr.y * ws.x - vr.x * ws.y) + (wr.y * vs.x - wr.x * vs.y);
-        }
-      }
-      __syncthreads();
-    }
-    if (tid == 0) {
-      eout[i0] = s_beta;
-      dout[i0 + 1] = pk[at(i0 + 1, i0 + 1)].x;
+    if (rank == 0 && tid == 0) {
+      eout[i0] = beta;
+      dout[c] = s_diag[par];
       tauout[i0] = tau;
     }
+    __syncthreads();
+    // columns s < L: the previous rank-2 update, then y(s) = tau sum_r conj(A(r, s)) v(r)
+    double2* y = ybuf + par * n;
+    for (int jl0 = warp; jl0 * P + rank < L; jl0 += kClWarps * kClCols) {
+      double2 ws[kClCols], vs[kClCols];
+      double acc[2 * kClCols] = {};
+      bool on[kClCols];
+#pragma unroll
+      for (int q = 0; q < kClCols; ++q) {
+        const int s = (jl0 + q * kClWarps) * P + rank;
+        on[q] = s < L;
+        ws[q] = on[q] ? wbuf[s] : make_double2(0.0, 0.0);
+        vs[q] = on[q] ? vp[s] : make_double2(0.0, 0.0);
+      }
+      for (int r = lane; r < L; r += 32) {
+        const double2 pv = vp[r], pw = wbuf[r], vv = v[r];
+#pragma unroll
+        for (int q = 0; q < kClCols; ++q) {
+          if (on[q]) {
+            double2* e = cols + size_t(jl0 + q * kClWarps) * n + r;
+            double2 a = *e;
+            a.x -= (pv.x * ws[q].x + pv.y * ws[q].y) + (pw.x * vs[q].x + pw.y * vs[q].y);
+            a.y -= (pv.y * ws[q].x - pv.x * ws[q].y) + (pw.y * vs[q].x - pw.x * vs[q].y);
+            *e = a;
+            acc[2 * q] += a.x * vv.x + a.y * vv.y;
+            acc[2 * q + 1] += a.x * vv.y - a.y * vv.x;
+          }
+        }
+      }
+      const double own = warp_sum8(acc);                                // value lane >> 2
+      const double other = __shfl_xor_sync(0xffffffffu, own, 4);
+      const bool im = lane & 4;
+      const double re = im ? other : own, imv = im ? own : other;
+      const int q = lane >> 3, s = (jl0 + q * kClWarps) * P + rank;   // eight lanes per column push
+      if (s < L) {
+        const double2 ys = make_double2(tau.x * re - tau.y * imv, tau.x * imv + tau.y * re);
+        for (int r = lane & 7; r < P; r += 8) cl.map_shared_rank(y, r)[s] = ys;
+      }
+    }
+    cl.sync();
+    // w = y + alpha2 v, alpha2 = -tau (y^H v) / 2; next pivot column i0, updated
+    const double2* next = cl.map_shared_rank(cols, i0 % P) + size_t(i0 / P) * n;
+    const double2 yi = y[i0];
+    double2 yr[kTrdRows], cr[kTrdRows];
+    double pr = 0, pi = 0;
+#pragma unroll
+    for (int t = 0; t < kTrdRows; ++t) {
+      const int r = tid + kClThreads * t;
+      yr[t] = r <= i0 ? y[r] : make_double2(0.0, 0.0);
+      cr[t] = r <= i0 ? next[r] : make_double2(0.0, 0.0);
+      pr += yr[t].x * vr[t].x + yr[t].y * vr[t].y;   // conj(y) v
+      pi += yr[t].x * vr[t].y - yr[t].y * vr[t].x;
+    }
+    const double2 dot = block_sum2(pr, pi, red[1]);
+    const double2 a2 = make_double2(-0.5 * (tau.x * dot.x - tau.y * dot.y), -0.5 * (tau.x * dot.y + tau.y * dot.x));
+    const double2 wi = cadd(yi, a2);   // w(i0), v(i0) = 1
+#pragma unroll
+    for (int t = 0; t < kTrdRows; ++t) {
+      const int r = tid + kClThreads * t;
+      if (r <= i0) {
+        const double2 w = cadd(yr[t], cmul(a2, vr[t]));
+        wbuf[r] = w;
+        x[t].x = cr[t].x - (vr[t].x * wi.x + vr[t].y * wi.y) - w.x;
+        x[t].y = cr[t].y - (vr[t].y * wi.x - vr[t].x * wi.y) - w.y;
+      }
+    }
   }
-  __syncthreads();
-  if (tid == 0) dout[0] = pk[at(0, 0)].x;
-  for (int q = tid; q < n * n; q += nt) {   // reflector vectors back to A (strict upper triangle)
-    const int i = q % n, j = q / n;
-    if (i < j) A[q] = pk[at(i, j)];
-  }
+  if (rank == 0 && tid == 0) dout[0] = x[0].x;
+  cl.sync();   // no CTA leaves while another may still read its columns
+}
+
+// CTAs of the cluster for an order-n reduction: the fewest that hold it, but
+// at least enough for about 12 columns each (below that the barrier costs
+// more than the pass saves), up to 16; 0 when it does not fit.
+int cluster_ctas(int n) {
+  for (int p = n <= 40 ? 1 : n <= 80 ? 4 : n <= 176 ? 8 : 16; p <= 16; p *= 2)
+    if (std::max(hetrd_smem(n, p), factor_smem(n, p)) <= kSmemMax) return p;
+  return 0;
+}
+
+template <typename... KArgs, typename... Args>
+void launch_cluster(void (*kernel)(KArgs...), int ctas, size_t smem, cudaStream_t s, Args... args) {
+  raise_smem_limit(kernel, smem);
+  if (ctas > 8) HALF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(kClThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ctas;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  HALF_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
 __global__ void real_to_complex_block_kernel(const double* __restrict__ z, long long count, double2* __restrict__ out) {
@@ -643,13 +860,31 @@ __global__ void real_to_complex_block_kernel(const double* __restrict__ z, long 
   if (t < count) out[t] = make_double2(z[t], 0.0);
 }
 
-// Large orders (the dense solves): T stays in global memory, read through
-// L1 with all lanes of a warp at the same index.  e2[i] = e[i]^2 and the
-// Gershgorin bounds (lo, hi, norm) are formed once by the first kernel.
-__global__ void tridiag_bounds_kernel(const double* __restrict__ d, const double* __restrict__ e, int n,
+// Large orders (the dense solves): the scaled T stays in global memory, read
+// through L1 with all lanes of a warp at the same index.  This kernel scales
+// d in place, squares e into e2 and leaves the scaled Gershgorin bounds
+// (lo, hi, norm) and the scale in bounds.
+__global__ void tridiag_bounds_kernel(double* __restrict__ d, const double* __restrict__ e, int n,
                                       double* __restrict__ e2, double* __restrict__ bounds) {
-  for (int i = threadIdx.x; i < n; i += blockDim.x) e2[i] = i < n - 1 ? e[i] * e[i] : 0.0;
-  if (threadIdx.x == 0) gershgorin(d, e, n, bounds[0], bounds[1], bounds[2]);
+  __shared__ double s_norm;
+  if (threadIdx.x < 32) {
+    double gl, gu, nrm;
+    gershgorin(d, e, n, gl, gu, nrm);
+    if (threadIdx.x == 0) {
+      const double sc = norm_scale(nrm);
+      s_norm = nrm;
+      bounds[0] = gl * sc;
+      bounds[1] = gu * sc;
+      bounds[2] = nrm * sc;
+      bounds[3] = sc;
+    }
+  }
+  __syncthreads();
+  const double sc = norm_scale(s_norm);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    d[i] *= sc;
+    e2[i] = scaled_e2(i < n - 1 ? e[i] : 0.0, sc);
+  }
 }
 
 // Eigenvalues k0 .. k0 + ne - 1 of T (ascending), one warp each, by the same
@@ -659,25 +894,10 @@ __global__ void __launch_bounds__(32 * kValueWarps) tridiag_values_global_kernel
                                                                                  int k0, int ne,
                                                                                  const double* __restrict__ bounds,
                                                                                  double* __restrict__ lam) {
-  const int lane = threadIdx.x & 31;
   const int j = blockIdx.x * kValueWarps + (threadIdx.x >> 5);
   if (j >= ne) return;
-  const int k = k0 + j;
-  const double tnorm = bounds[2];
-  double lo = bounds[0], hi = bounds[1];
-  for (int round = 0; round < 200; ++round) {
-    if (hi - lo <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + DBL_EPSILON * tnorm) break;
-    const double x = lo + (hi - lo) * double(lane + 1) / 33.0;
-    const unsigned b = __ballot_sync(0xffffffffu, sturm_count(d, e2, n, x) > k);
-    const int first = b ? __ffs(b) - 1 : 32;
-    const double xlo = __shfl_sync(0xffffffffu, x, first > 0 ? first - 1 : 0);
-    const double xhi = __shfl_sync(0xffffffffu, x, first < 32 ? first : 31);
-    const double nlo = first > 0 ? xlo : lo, nhi = first < 32 ? xhi : hi;
-    if (!(nlo > lo || nhi < hi)) break;
-    lo = nlo;
-    hi = nhi;
-  }
-  if (lane == 0) lam[j] = 0.5 * (lo + hi);
+  const double v = multisect(d, e2, n, k0 + j, bounds[0], bounds[1], bounds[2]);
+  if ((threadIdx.x & 31) == 0) lam[j] = v / bounds[3];
 }
 
 }  // namespace
@@ -718,11 +938,9 @@ void SmallEigen::reserve(Runtime& rt, int nmax) {
 void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* status) {
   reserve(rt, n);
   cudaStream_t s = rt.stream;
-  if (n <= kMetricMax) {   // whole reduction in one CTA
-    const size_t tsm = (size_t(n) * (n + 1) / 2 + 2 * size_t(n)) * sizeof(double2);
-    raise_smem_limit(hetrd_kernel, tsm);
-    hetrd_kernel<<<1, 512, tsm, s>>>(A, n, d.get(), e.get(), tau.get());
-    HALF_LAUNCH("Householder tridiagonalisation");
+  if (n <= kOwnMaxOrder) {   // whole reduction in one cluster
+    const int p = cluster_ctas(n);
+    launch_cluster(hetrd_kernel, p, hetrd_smem(n, p), s, A, n, d.get(), e.get(), tau.get());
     rt.prof.launches += 1;
   } else {
     cusolver_check(cusolverDnZhetrd(rt.solver, CUBLAS_FILL_MODE_UPPER, n, reinterpret_cast<cuDoubleComplex*>(A), n,
@@ -742,15 +960,21 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
   size_t tsm = (2 * size_t(n) + ne) * sizeof(double) + size_t(ne) * sizeof(int);
   if (tsm > kSmemMax) fail(kCapacity, "subspace eigenproblem too large for the tridiagonal solver: n=" + std::to_string(n));
   tsm = (tsm + 15) & ~size_t(15);
-  const size_t slots_sm = size_t(kVectorThreads) * (5 * size_t(n) * sizeof(double) + size_t(n));
+  const size_t slot = 5 * size_t(n) * sizeof(double) + size_t(n);
+  int per = kVectorThreads;
+  while (per > 4 && tsm + per * slot > kSmemMax) per /= 2;
   double* gs = nullptr;
-  if (tsm + slots_sm <= kSmemMax) tsm += slots_sm;
-  else gs = scratch.get();
+  if (tsm + per * slot <= kSmemMax) {
+    tsm += per * slot;
+  } else {
+    gs = scratch.get();
+    per = kVectorThreads;
+  }
   raise_smem_limit(tridiag_vectors_kernel, tsm);
-  tridiag_vectors_kernel<<<ceil_div(nev, kVectorThreads), kVectorThreads, tsm, s>>>(d.get(), e.get(), n, nev, ne,
-                                                                                     lam.get(), w, Z.get(), gs, status);
+  tridiag_vectors_kernel<<<ceil_div(nev, per), kVectorThreads, tsm, s>>>(d.get(), e.get(), n, nev, ne, per, lam.get(), w,
+                                                                          Z.get(), gs, status);
   HALF_LAUNCH("tridiagonal eigenvectors");
-  if (n > kMetricMax) {
+  if (n > kOwnMaxOrder) {
     // large orders: cuSOLVER's blocked back-transformation (zunmtr, Q Z with
     // zhetrd's reflectors) on the complex copy of Z
     real_to_complex_block_kernel<<<ceil_div((long long)n * nev, 256), 256, 0, s>>>(Z.get(), (long long)n * nev,
@@ -766,16 +990,19 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
     rt.prof.launches += 3;
     return;
   }
-  // back-transformation: the reflectors in chunks that fit next to the warps' vectors
-  const size_t vec_bytes = size_t(kBackWarps) * n * sizeof(double2);
-  if (vec_bytes + (size_t(n) + 1) * sizeof(double2) > kSmemMax)
-    fail(kCapacity, "subspace eigenproblem too large for the back-transformation: n=" + std::to_string(n));
-  const int chunk = int(std::max<size_t>(1, std::min<size_t>(size_t(std::max(n - 1, 1)),
-                                                             (kSmemMax - vec_bytes) / ((size_t(n) + 1) * sizeof(double2)))));
-  const size_t bsm = vec_bytes + size_t(chunk) * (n + 1) * sizeof(double2);
-  raise_smem_limit(back_transform_kernel, bsm);
-  back_transform_kernel<<<ceil_div(nev, kBackWarps), 32 * kBackWarps, bsm, s>>>(A, tau.get(), Z.get(), n, nev, chunk,
-                                                                                 V.get());
+  // back-transformation: as many reflectors at a time as fit, in blocks of four
+  const size_t per_block = kBackBlock * (size_t(n) + 1) * sizeof(double2) + 8 * sizeof(double2);
+  const int blocks = int(std::min<size_t>(ceil_div(std::max(n - 1, 1), kBackBlock), kSmemMax / per_block));
+  const size_t bsm = size_t(blocks) * per_block;
+  auto back = [&](auto kernel) {
+    raise_smem_limit(kernel, bsm);
+    kernel<<<ceil_div(nev, kBackWarps), 32 * kBackWarps, bsm, s>>>(A, tau.get(), Z.get(), n, nev, blocks * kBackBlock,
+                                                                   V.get());
+  };
+  if (n <= 64) back(back_transform_kernel<2>);
+  else if (n <= 160) back(back_transform_kernel<5>);
+  else if (n <= 288) back(back_transform_kernel<9>);
+  else back(back_transform_kernel<14>);
   HALF_LAUNCH("back transformation");
   HALF_CUDA(cudaMemcpyAsync(A, V.get(), size_t(n) * nev * sizeof(double2), cudaMemcpyDeviceToDevice, s));
   rt.prof.launches += 3;
@@ -786,7 +1013,7 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
 void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, double* w, int* status, int* chol_status) {
   reserve(rt, n);
   cudaStream_t s = rt.stream;
-  if (n <= kMetricMax) {
+  if (n <= kOwnMaxOrder) {
     // B -> X = D R^-1 with X^H B X = I (metric_factor_kernel), C = X^H A X,
     // C V = V Lambda, Y = X V: the same pencil reduction as zhegvd's
     // Cholesky / two triangular solves, with the factor inverted in shared
@@ -823,13 +1050,11 @@ void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, doubl
 }
 
 // U with (P U)^H S (P U) = I from M = P^H S P, overwriting M (see
-// metric_factor_kernel); false when m is beyond the shared-memory kernel.
+// metric_factor_kernel); false when m is beyond the cluster's shared memory.
 bool SmallEigen::metric_normalize(Runtime& rt, double2* M, int m, int* status) {
-  if (m > kMetricMax) return false;
-  const size_t sm = (size_t(m) * (m + 1) / 2 + 2 * size_t(m)) * sizeof(double2) + 2 * size_t(m) * sizeof(double);
-  raise_smem_limit(metric_factor_kernel, sm);
-  metric_factor_kernel<<<1, kFactorThreads, sm, rt.stream>>>(M, m, status);
-  HALF_LAUNCH("metric factor");
+  if (m > kOwnMaxOrder) return false;
+  const int p = cluster_ctas(m);
+  launch_cluster(metric_factor_kernel, p, factor_smem(m, p), rt.stream, M, m, status);
   rt.prof.launches += 1;
   return true;
 }
@@ -839,7 +1064,7 @@ void hermitian_eigenvalues_large(Runtime& rt, double2* A, long long n, const std
   if (n > INT32_MAX / 2) fail(kUnavailable, "dense order beyond the tridiagonalisation's range");
   cudaStream_t s = rt.stream;
   const int ni = int(n);
-  DeviceBuffer<double> d(ni), e(ni), e2(ni), bounds(3);
+  DeviceBuffer<double> d(ni), e(ni), e2(ni), bounds(4);
   DeviceBuffer<double2> tau(ni);
   DeviceBuffer<int> info(1);
   int lwork = 0;

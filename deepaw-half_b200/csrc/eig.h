@@ -8,9 +8,9 @@
 namespace hb {
 
 struct SmallEigen {
-  // Orders the one-CTA kernels serve; above it cuSOLVER's zhegvd is faster
-  // (order 320: 4.7 against 5.9 ms; order 1080: 20 against 37 ms).
-  static constexpr int kOwnMaxOrder = 164;
+  // Orders the cluster kernels serve: the matrix fits the shared memory of 16
+  // CTAs (432 x 432 x 16 bytes and the vectors).  Above it cuSOLVER.
+  static constexpr int kOwnMaxOrder = 432;
   int cap = 0;
   DeviceBuffer<double> d, e, Z, scratch, lam;
   DeviceBuffer<double2> tau, V, work;

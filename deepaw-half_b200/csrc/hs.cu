@@ -759,21 +759,22 @@ void apply_hs(Context& ctx, KOperatorSet& ks, const cplx_t<R>* x, long long ld, 
   if (nb <= 0) return;
   // chunk <= 0: bands per chunk chosen by the autotuner (tune.h) per box,
   // sphere extent and precision; every choice gives bit-identical results
-  int tune_token = 0;
+  int tune_token = 0, tune_index = 0;
+  std::string tune_key;
   if (chunk <= 0) {
     static const std::vector<int> cand = {16, 8, 32, 64};
-    const std::string key = "local " + std::to_string(op.n1) + "x" + std::to_string(op.n2) + "x" +
+    tune_key = "local " + std::to_string(op.n1) + "x" + std::to_string(op.n2) + "x" +
                             std::to_string(op.n3) + " planes " + std::to_string(op.nplanes) + " fp" +
                             std::to_string(8 * sizeof(R));
-    const int idx = Tuner::pick(key, cand);
-    chunk = cand[idx];
-    tune_token = Tuner::begin(key, idx, s);
+    tune_index = Tuner::pick(tune_key, cand);
+    chunk = cand[tune_index];
   }
   chunk = std::max(1, std::min(chunk, nb));
   if (op.work_chunk < chunk) {
     op.work.resize((size_t)chunk * op.nplanes * op.n2 * op.n3);
     op.work_chunk = chunk;
   }
+  if (!tune_key.empty()) tune_token = Tuner::begin(tune_key, tune_index, s);   // the kernels alone, no allocation
   const size_t psm = plane_smem<R>(op.n2, op.n3), xsm = xline_smem<R>(op.n1);
   const int pth = plane_threads<R>(psm);
   const int tiles = (op.n3 + kXTile - 1) / kXTile;

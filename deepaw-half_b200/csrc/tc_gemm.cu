@@ -128,8 +128,9 @@ __device__ __forceinline__ float2 projector_value(const TcOperand& op, int col, 
 // matrix, r < rows_pad, k < 16 nkb) goes to the four bf16 planes, plane p at
 // out + p plane_bytes, in the layout described at the top of this file.
 // One thread per (row, 8 consecutive k): consecutive threads take consecutive
-// rows, so row-contiguous operands load coalesced and each group of 8 rows
-// stores 128 contiguous bytes per plane.  Projector operands generate their
+// rows, so row-contiguous operands (kDenseMN) load coalesced and each group of
+// 8 rows stores 128 contiguous bytes per plane; k-contiguous operands go
+// through presplit_k_kernel below.  Projector operands generate their
 // elements from the tables (kProj: row = plane wave, k = projector column;
 // kProjConj: row = projector column, k = plane wave).
 __global__ void presplit_kernel(TcOperand op, int rows_pad, int nkb, unsigned char* __restrict__ out,
@@ -168,13 +169,7 @@ __global__ void presplit_kernel(TcOperand op, int rows_pad, int nkb, unsigned ch
       for (int i = 0; i < 8; ++i) {
         const int k = k0 + i;
         if (k < op.kdim) {
-          float2 x;
-          if (op.kind == TcOperand::kDenseK) {
-            const float2* src = r < op.split ? op.p + (long long)r * op.ld : op.p2 + (long long)(r - op.split) * op.ld;
-            x = __ldg(src + k);
-          } else {
-            x = __ldg(op.p + r + (long long)k * op.ld);
-          }
+          float2 x = __ldg(op.p + r + (long long)k * op.ld);
           if (op.conj) x.y = -x.y;
           v[i] = x;
         }
@@ -186,6 +181,52 @@ __global__ void presplit_kernel(TcOperand op, int rows_pad, int nkb, unsigned ch
   for (int i = 0; i < 4; ++i) {
     split_pair(v[2 * i].x, v[2 * i + 1].x, w[0][i], w[1][i]);
     split_pair(v[2 * i].y, v[2 * i + 1].y, w[2][i], w[3][i]);
+  }
+  const long long off = (long long)kb * rows_pad * 32 + (long long)(r >> 3) * 256 + half * 128 + (r & 7) * 16;
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+    *reinterpret_cast<uint4*>(out + p * plane_bytes + off) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+}
+
+// The same planes from a dense operand whose k index is contiguous (kDenseK).
+// One CTA takes a tile of kSplitRows rows x kSplitK k through shared memory:
+// the loads run along k (256 contiguous bytes per warp and row), then one
+// thread packs 8 consecutive k of a row.  With a thread loading its own 8 k
+// every load instruction of a warp touches 32 rows, one cache line each, and
+// the L1 lookups (32 per instruction) held the pass to half the copy rate:
+// 600 + 600 rows x 38,089 (366 MB read, 366 MB written) took 191 us.
+constexpr int kSplitRows = 32, kSplitK = 64, kSplitPitch = kSplitK + 1;   // odd pitch: conflict-free column reads
+
+__global__ void __launch_bounds__(256) presplit_k_kernel(TcOperand op, int rows_pad, int nkb,
+                                                         unsigned char* __restrict__ out, long long plane_bytes) {
+  __shared__ float2 tile[kSplitRows * kSplitPitch];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rtiles = (rows_pad + kSplitRows - 1) / kSplitRows;
+  const int r0 = int(blockIdx.x % unsigned(rtiles)) * kSplitRows, k0 = int(blockIdx.x / unsigned(rtiles)) * kSplitK;
+#pragma unroll
+  for (int i = 0; i < kSplitRows / 8; ++i) {
+    const int rl = warp + 8 * i, r = r0 + rl;
+    const float2* src = r < op.split ? op.p + (long long)r * op.ld : op.p2 + (long long)(r - op.split) * op.ld;
+#pragma unroll
+    for (int h = 0; h < kSplitK / 32; ++h) {
+      const int kl = lane + 32 * h, k = k0 + kl;
+      float2 x = make_float2(0.f, 0.f);
+      if (r < op.rows && k < op.kdim) x = __ldg(src + k);
+      if (op.conj) x.y = -x.y;
+      tile[rl * kSplitPitch + kl] = x;
+    }
+  }
+  __syncthreads();
+  // thread = (row lane, group of 8 k warp); 8 warps cover the tile's 64 k
+  const int r = r0 + lane, kb = k0 / 16 + (warp >> 1), half = warp & 1;
+  if (kb >= nkb || r >= rows_pad) return;
+  const float2* v = tile + lane * kSplitPitch + warp * 8;
+  uint32_t w[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 a = v[2 * i], b = v[2 * i + 1];
+    split_pair(a.x, b.x, w[0][i], w[1][i]);
+    split_pair(a.y, b.y, w[2][i], w[3][i]);
   }
   const long long off = (long long)kb * rows_pad * 32 + (long long)(r >> 3) * 256 + half * 128 + (r & 7) * 16;
 #pragma unroll
@@ -354,6 +395,47 @@ __global__ void splitk_reduce_kernel(const float2* __restrict__ W, int S, int M,
   write_out(dst, sr, si, o);
 }
 
+// The bf16 planes of `op` into out (rows_pad rows, a multiple of 16; zeros outside the operand).
+void launch_presplit(const TcOperand& op, int rows_pad, int nkb, unsigned char* out, long long plane_bytes,
+                     cudaStream_t st) {
+  if (op.kind == TcOperand::kDenseK) {
+    const long long ctas = (long long)ceil_div(rows_pad, kSplitRows) * ceil_div((long long)nkb * kBK, kSplitK);
+    presplit_k_kernel<<<unsigned(ctas), 256, 0, st>>>(op, rows_pad, nkb, out, plane_bytes);
+  } else {
+    presplit_kernel<<<ceil_div((long long)rows_pad * nkb * 2, 256), 256, 0, st>>>(op, rows_pad, nkb, out, plane_bytes);
+  }
+  HALF_LAUNCH("tensor-core operand split");
+}
+
+// Split-K count of a product of `tiles` 128 x bn tiles over nkb k blocks on
+// `sms` SMs (one CTA each): the count with the least estimated time
+//   waves x (k blocks per CTA x time per block + time per CTA) + reduction.
+// Per k block 3 ns per tile column (measured 0.78 us at bn 208, 12 MMAs);
+// per CTA 6 us for the launch, the pipeline's fill and the epilogue
+// (measured 9 us with partial-sum stores); the reduction re-reads the
+// partial sums at about 4 TB/s.  One split too many costs a whole second
+// wave: 600 x 600 x 38,089 (15 tiles) as 10 splits is 150 CTAs on 148 SMs
+// and took 375 us.  The fewest splits considered fill one wave, as short
+// chains also keep the error down: the FP32 accumulation of the tensor core
+// truncates, which costs about 1e-7 of the sum per k block.
+int pick_splits(long long tiles, int nkb, int bn, long long mn, int sms) {
+  const int most = std::max(1, std::min(nkb / 4, 256));
+  const int least = tiles < sms ? int(std::min<long long>((sms + tiles - 1) / tiles, std::max(1, nkb / 4))) : 1;
+  int best = least;
+  double best_t = 0;
+  for (int s = least; s <= std::max(least, most); ++s) {
+    const int per = (nkb + s - 1) / s, used = (nkb + per - 1) / per;
+    const long long waves = (tiles * used + sms - 1) / sms;
+    double tm = double(waves) * (per * 0.003 * bn + 6.0);
+    if (used > 1) tm += 3.0 + double(mn) * 8.0 * (used + 1) / 4.0e6;
+    if (best_t == 0 || tm < best_t) {
+      best_t = tm;
+      best = used;
+    }
+  }
+  return best;
+}
+
 int pick_bn(int N) {
   const int nt = (N + 255) / 256;
   int bn = (N + nt - 1) / nt;
@@ -403,11 +485,7 @@ void tc_cgemm(Runtime& rt, const TcOperand& A, const TcOperand& B, int M, int N,
   HALF_CUDA(cudaGetDevice(&dev));
   HALF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const long long tiles = (long long)mt * nt0;
-  int splits = 1;
-  if (tiles < sms && nkb > 0) {
-    splits = int(std::min<long long>((sms + tiles - 1) / tiles, std::max(1, nkb / 4)));
-    splits = std::max(1, splits);
-  }
+  int splits = nkb > 0 ? pick_splits(tiles, nkb, bn0, (long long)M * N, sms) : 1;
   const int kbps = nkb > 0 ? (nkb + splits - 1) / splits : 0;
   if (nkb > 0) splits = (nkb + kbps - 1) / kbps;
   // tile width: 0, 1 or 2 more N tiles than the fewest are the candidates
@@ -416,13 +494,13 @@ void tc_cgemm(Runtime& rt, const TcOperand& A, const TcOperand& B, int M, int N,
     const int t = nt0 + extra, w = ((N + t - 1) / t + 15) / 16 * 16;
     if (w >= 16 && (cand.empty() || w < cand.back())) cand.push_back(w);
   }
-  int tune_token = 0, bn = bn0;
+  int tune_token = 0, tune_index = 0, bn = bn0;
+  std::string key;
   if (nkb > 0 && cand.size() > 1) {
-    const std::string key = "gemm " + std::to_string(A.kind) + std::to_string(B.kind) + " " + std::to_string(M) +
+    key = "gemm " + std::to_string(A.kind) + std::to_string(B.kind) + " " + std::to_string(M) +
                             "x" + std::to_string(N) + "x" + std::to_string(K) + " s" + std::to_string(splits);
-    const int idx = Tuner::pick(key, cand);
-    bn = cand[idx];
-    tune_token = Tuner::begin(key, idx, st);
+    tune_index = Tuner::pick(key, cand);
+    bn = cand[tune_index];
   }
   const int nt = (N + bn - 1) / bn;
   // Operands not given as planes are split into bf16 planes in global memory
@@ -448,8 +526,7 @@ void tc_cgemm(Runtime& rt, const TcOperand& A, const TcOperand& B, int M, int N,
       unsigned char* planes = rt.tc_planes.get();
       span0 = pf.record(st);
       if (pa > 0) {
-        const long long th = (long long)rpa * nkb * 2;
-        presplit_kernel<<<ceil_div(th, 256), 256, 0, st>>>(A, rpa, nkb, planes, pa);
+        launch_presplit(A, rpa, nkb, planes, pa, st);
         Ak = TcOperand();
         Ak.kind = TcOperand::kPlanes;
         Ak.rows = A.rows;
@@ -460,8 +537,7 @@ void tc_cgemm(Runtime& rt, const TcOperand& A, const TcOperand& B, int M, int N,
         ++pf.launches;
       }
       if (pb > 0) {
-        const long long th = (long long)rpb * nkb * 2;
-        presplit_kernel<<<ceil_div(th, 256), 256, 0, st>>>(B, rpb, nkb, planes + 4 * pa, pb);
+        launch_presplit(B, rpb, nkb, planes + 4 * pa, pb, st);
         Bk = TcOperand();
         Bk.kind = TcOperand::kPlanes;
         Bk.rows = B.rows;
@@ -471,11 +547,14 @@ void tc_cgemm(Runtime& rt, const TcOperand& A, const TcOperand& B, int M, int N,
         Bk.rows_pad = rpb;
         ++pf.launches;
       }
-      HALF_LAUNCH("tensor-core operand split");
     }
   }
   const size_t sbytes = stage_bytes(bn);
-  const int nst = int(std::min<size_t>(kMaxPipe, (kSmemBudget - kSmemSlack) / sbytes));
+  // Short chains leave half the shared memory to a second CTA where their
+  // accumulators fit Tensor Memory twice (bn <= 128), so that one CTA's
+  // epilogue runs beside the other's copies and MMAs.
+  const size_t budget = bn <= 128 && kbps <= 16 ? kSmemBudget / 2 : kSmemBudget;
+  const int nst = int(std::min<size_t>(kMaxPipe, (budget - kSmemSlack) / sbytes));
   if (nst < 2) fail(kInternal, "tensor-core GEMM stage does not fit shared memory twice");
   const size_t smem = size_t(nst) * sbytes + kSmemSlack;
   raise_smem_limit(tc_cgemm_kernel, smem);
@@ -499,6 +578,7 @@ void tc_cgemm(Runtime& rt, const TcOperand& A, const TcOperand& B, int M, int N,
   }
   if (nkb > 0) {
     const int e0 = span0 >= 0 ? span0 : pf.record(st);
+    if (!key.empty()) tune_token = Tuner::begin(key, tune_index, st);   // the product alone, no allocation or split pass
     tc_cgemm_kernel<<<dim3(mt, nt, splits), kThreads, smem, st>>>(Ak, Bk, bn, nst, kbps, nkb, o, rt.tc_err.get());
     HALF_LAUNCH("tensor-core cgemm");
     Tuner::finish(tune_token, st, 1.0);
@@ -536,9 +616,7 @@ TcOperand tc_presplit_a(Runtime& rt, const TcOperand& op, DeviceBuffer<unsigned 
   o.plane_bytes = pbytes;
   if (pbytes == 0) return o;
   if (store.size() < size_t(4 * pbytes)) store.resize(size_t(4 * pbytes));
-  presplit_kernel<<<ceil_div((long long)rows_pad * nkb * 2, 256), 256, 0, rt.stream>>>(op, rows_pad, nkb, store.get(),
-                                                                                       pbytes);
-  HALF_LAUNCH("tensor-core operand split (kept)");
+  launch_presplit(op, rows_pad, nkb, store.get(), pbytes, rt.stream);
   ++rt.prof.launches;
   o.planes = store.get();
   return o;

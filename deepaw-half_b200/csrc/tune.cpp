@@ -22,9 +22,16 @@ struct Timing {
 struct Entry {
   std::vector<int> cand;
   std::vector<double> ms_per_unit;   // best completed timing per candidate, < 0 while unmeasured
+  std::vector<int> samples;          // completed timings per candidate
   int next = 0;
   int decided = -1;
 };
+
+// Timings per candidate before a decision; the best counts.  The first one of
+// a shape can hold a kernel's lazy load or a cold L2 (the 600 x 600 x 38,089
+// product used to settle on a tile width 1.7x slower than the best because
+// the candidate that went first had paid for both).
+constexpr int kSamples = 2;
 
 std::mutex g_mu;
 std::map<std::string, Entry> g_table;
@@ -51,7 +58,7 @@ void decide(const std::string& key, Entry& e) {
   if (e.decided >= 0) return;
   int best = -1;
   for (size_t i = 0; i < e.cand.size(); ++i) {
-    if (e.ms_per_unit[i] < 0) return;
+    if (e.samples[i] < kSamples) return;
     if (best < 0 || e.ms_per_unit[i] < e.ms_per_unit[best]) best = int(i);
   }
   e.decided = best;
@@ -78,6 +85,7 @@ void harvest() {
           const double v = double(ms) / t.units;
           double& cur = e.ms_per_unit[t.index];
           if (cur < 0 || v < cur) cur = v;
+          ++e.samples[t.index];
           decide(t.key, e);
         }
       } else {
@@ -103,6 +111,7 @@ int Tuner::pick(const std::string& key, const std::vector<int>& candidates) {
   if (e.cand != candidates) {
     e.cand = candidates;
     e.ms_per_unit.assign(candidates.size(), -1.0);
+    e.samples.assign(candidates.size(), 0);
     e.next = 0;
     e.decided = -1;
   }
@@ -110,7 +119,7 @@ int Tuner::pick(const std::string& key, const std::vector<int>& candidates) {
   const int n = int(e.cand.size());
   for (int t = 0; t < n; ++t) {
     const int i = (e.next + t) % n;
-    if (e.ms_per_unit[i] < 0) {
+    if (e.samples[i] < kSamples) {
       e.next = i + 1;
       return i;
     }

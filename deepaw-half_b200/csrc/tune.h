@@ -4,7 +4,7 @@
 // GEMM's tile width) is chosen per shape signature by measurement on the
 // caller's own work: successive calls with the same signature try the
 // candidates in turn, each timed with a pair of CUDA events on the call's
-// stream, and once every candidate has a completed timing the fastest per
+// stream, and once every candidate has two completed timings the fastest per
 // unit of work is used from then on.  Events are read without waiting (a
 // timing whose events have not completed yet is picked up by a later call),
 // so tuning adds no synchronisation.  Every candidate produces bit-identical
