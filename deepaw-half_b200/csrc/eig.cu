@@ -527,20 +527,24 @@ __global__ void hermitian_fill_kernel(double2* A, int n) {
 // with p_k = W(k,k): a rank-1 update of every column right of k.  The two
 // index ranges occupy disjoint rows of a column (rows <= k hold T, rows > k
 // hold W), and at the end X(i,j) = -T(i,j) / R(j,j), X(j,j) = 1 / R(j,j).
-// What a step needs from other CTAs is row k of W, which every CTA pushes to
-// all of them as it updates its columns in the step before, and column k of
-// T, which its owner no longer changes: one cluster barrier per step.
+// What a step needs from other CTAs is row k of W and column k of T; both are
+// pushed to every CTA in the step before, the row by each column's owner as it
+// updates the column, the column by its owner, whose threads update it
+// together first.  One cluster barrier per step and no other.
 // *status = 1 if a pivot was not finite.
 //
-// Bound by the chain of barriers and shared-memory round trips, about 1 us a
-// step: one CTA with the packed triangle in its own shared memory (orders up
-// to 164) took 2.0 us a step at order 140 from its rank-1 updates alone.
+// Bound by the chain of cluster barriers and shared-memory round trips.
+// Measured per solve at orders around 120 (12-atom cell, B200): one CTA with
+// the packed triangle 281 us; this kernel 235 us.
 constexpr int kClThreads = 256;
 constexpr int kClWarps = kClThreads / 32;
 constexpr int kClCols = 4;                        // columns a warp carries at once
 
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
 __host__ __device__ inline size_t factor_smem(int m, int p) {
-  return (size_t((m + p - 1) / p) * m + 3 * size_t(m)) * sizeof(double2) + 2 * size_t(m) * sizeof(double);
+  return (size_t((m + p - 1) / p) * m + 4 * size_t(m)) * sizeof(double2) + 2 * size_t(m) * sizeof(double);
 }
 
 __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __restrict__ M, int m,
@@ -550,9 +554,9 @@ __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __re
   const int nc = (m + P - 1) / P;
   extern __shared__ __align__(16) double2 cols[];   // nc x m: column jl P + rank at cols + jl m
   double2* gbuf = cols + size_t(nc) * m;            // 2 x m: row k of W, by parity of k
-  double2* av = gbuf + 2 * m;                       // row factors of the step (T(i,k) or conj W(k,i))
-  double* dsc = reinterpret_cast<double*>(av + m);  // D
-  double* ir = dsc + m;                             // 1 / R(k,k)
+  double2* tbuf = gbuf + 2 * m;                     // 2 x m: column k of T, by parity of k
+  double* dsc = reinterpret_cast<double*>(tbuf + 2 * m);   // D
+  double* ir = dsc + m;                                    // 1 / R(k,k)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int j = tid; j < m; j += kClThreads) dsc[j] = 1.0 / sqrt(fmax(M[size_t(j) * m + j].x, DBL_MIN));
   cl.sync();   // every CTA's buffers exist, dsc is filled
@@ -571,21 +575,39 @@ __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __re
   int bad = 0;
   for (int k = 0; k < m; ++k) {
     const double2* g = gbuf + (k & 1) * m;
+    const double2* tk = tbuf + (k & 1) * m;
     double2* gn = gbuf + ((k + 1) & 1) * m;
+    double2* tn = tbuf + ((k + 1) & 1) * m;
     const double p = g[k].x;
     const bool dep = !(p > 1.0e-14);   // also true for NaN
     const double invp = dep ? 0.0 : 1.0 / p;
     if (!isfinite(p)) bad = 1;
     if (tid == 0) ir[k] = dep ? 1.0e7 : 1.0 / sqrt(p);
-    const double2* tk = cl.map_shared_rank(cols, k % P) + size_t(k / P) * m;
-    for (int i = tid; i < m; i += kClThreads) {
-      double2 a = make_double2(0.0, 0.0);
-      if (i < k) a = tk[i];
-      else if (i > k) a = make_double2(g[i].x, -g[i].y);
-      av[i] = a;
+    // the step's update of element (i, column factor c): row k becomes c, the others lose a_i c
+    auto updated = [&](int i, double2 a, double2 x, double2 c) {
+      if (i == k) return c;
+      if (!dep) {
+        x.x -= a.x * c.x - a.y * c.y;
+        x.y -= a.x * c.y + a.y * c.x;
+      }
+      return x;
+    };
+    auto row_factor = [&](int i) {
+      if (i < k) return tk[i];                    // T(i, k)
+      const double2 w = g[i];
+      return make_double2(w.x, -w.y);             // conj W(k, i)
+    };
+    if (k + 1 < m && (k + 1) % P == rank) {   // the next pivot column, by the whole CTA
+      double2* col = cols + size_t((k + 1) / P) * m;
+      const double2 c = cscale(g[k + 1], invp);
+      for (int i = tid; i <= k + 1; i += kClThreads) {
+        const double2 x = updated(i, row_factor(i), col[i], c);
+        col[i] = x;
+        double2* dst = i <= k ? tn : gn;
+        for (int r = 0; r < P; ++r) cl.map_shared_rank(dst, r)[i] = x;
+      }
     }
-    __syncthreads();
-    int jl0 = k + 1 > rank ? (k + 1 - rank + P - 1) / P : 0;   // first owned column right of k
+    int jl0 = k + 2 > rank ? (k + 2 - rank + P - 1) / P : 0;   // first owned column right of k + 1
     for (jl0 += warp; jl0 * P + rank < m; jl0 += kClWarps * kClCols) {
       double2 c[kClCols];
       int jj[kClCols];
@@ -596,19 +618,12 @@ __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __re
       }
       const int jmax = min(m - 1, jj[kClCols - 1]);
       for (int i = lane; i <= jmax; i += 32) {
-        const double2 a = av[i];
+        const double2 a = row_factor(i);
 #pragma unroll
         for (int q = 0; q < kClCols; ++q) {
           if (i <= jj[q] && jj[q] < m) {
             double2* e = cols + size_t(jl0 + q * kClWarps) * m + i;
-            if (i == k) {
-              *e = c[q];
-            } else if (!dep) {
-              double2 x = *e;
-              x.x -= a.x * c[q].x - a.y * c[q].y;
-              x.y -= a.x * c[q].y + a.y * c[q].x;
-              *e = x;
-            }
+            *e = updated(i, a, *e, c[q]);
           }
         }
       }
@@ -622,7 +637,8 @@ __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __re
         }
       }
     }
-    cl.sync();
+    cluster_arrive();
+    cluster_wait();
   }
   // U = D X with X(i,j) = -T(i,j) / R(j,j), X(j,j) = 1 / R(j,j); lower triangle zero
   for (int jl = warp; jl * P + rank < m; jl += kClWarps) {
@@ -638,23 +654,8 @@ __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __re
   if (rank == 0 && tid == 0) *status = bad;
 }
 
-// Block-wide sum of a (real, imaginary) pair through red (one slot per warp,
-// not reused before another barrier); every thread gets the result.
-__device__ __forceinline__ double2 block_sum2(double a, double b, double2* red) {
-  for (int off = 16; off > 0; off >>= 1) {
-    a += __shfl_xor_sync(0xffffffffu, a, off);
-    b += __shfl_xor_sync(0xffffffffu, b, off);
-  }
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_double2(a, b);
-  __syncthreads();
-  double2 s = red[0];
-#pragma unroll
-  for (int w = 1; w < kClWarps; ++w) s = cadd(s, red[w]);
-  return s;
-}
-
 __host__ __device__ inline size_t hetrd_smem(int n, int p) {
-  return (size_t((n + p - 1) / p) * n + 5 * size_t(n)) * sizeof(double2);
+  return (size_t((n + p - 1) / p) * n + 5 * size_t(n)) * sizeof(double2) + 2 * size_t(p) * kClWarps * sizeof(double);
 }
 
 // Householder reduction of a Hermitian A (n x n, upper triangle read) to the
@@ -664,18 +665,23 @@ __host__ __device__ inline size_t hetrd_smem(int n, int p) {
 // A(0:i-1, i+1) annihilates A(0:i-1, i+1); d = diag(T), e = superdiagonal.
 //
 // One cluster of CTAs holds the whole (both triangles) matrix in its shared
-// memory, column j on CTA j mod P, so y = A v is one local dot product per
-// column.  Per step: every CTA forms the reflector from its copy of the pivot
-// column; one pass over its columns applies the previous step's rank-2 update
-// and the product with v together; it pushes its entries of y to every CTA;
-// one cluster barrier; then every CTA forms w = y - (tau y^H v / 2) v and the
-// next pivot column (pulled from its owner, updated locally).  All CTAs do
-// the same arithmetic in the same order, so their copies agree bit for bit.
-//
-// Bound by the chain of three block barriers, one cluster barrier and the
-// exchange per step; the shared-memory traffic of the pass (32 bytes per
-// element, the vectors read once per four columns) shows above order 300.
-// One CTA with the packed triangle took 6.1 us a step at order 144.
+// memory, column j on CTA j mod P, so a product with A is one local dot
+// product per column.  The step is bound by its chain of barriers and
+// reductions, so it is arranged around one block and one cluster barrier:
+// * the pass over the columns applies the previous step's rank-2 update and
+//   forms u = A x with the unnormalised pivot column x, whose norm every warp
+//   sums on the way; with v = sc x + kappa e(i), kappa = 1 - sc x(i), the
+//   product the method needs is  A v = sc u + kappa A(:, i);
+// * each warp pushes its entries of u, and its share of q = x^H u, to every
+//   CTA, and forms tau, sc and kappa while the cluster barrier completes;
+// * then every CTA pulls column i from its owner and has all it needs:
+//   y = tau A v,  v^H A v = |sc|^2 q + 2 Re(conj(sc) kappa conj(u(i))) +
+//   |kappa|^2 A(i,i),  w = y - (|tau|^2 v^H A v / 2) v  and the next pivot
+//   column A(:, i) - v conj(w(i)) - w.
+// All CTAs do the same arithmetic in the same order, so their copies agree
+// bit for bit.  Measured per solve at orders around 120 (12-atom cell, B200):
+// one CTA with the packed triangle 689 us; this kernel with three more block
+// barriers per step (norm, v and y^H v) 307 us; as it stands 297 us.
 constexpr int kTrdRows = 2;                        // rows of a vector per thread
 static_assert(SmallEigen::kOwnMaxOrder <= kTrdRows * kClThreads, "rows of a vector per thread");
 
@@ -685,12 +691,11 @@ __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__
   const int P = int(cl.num_blocks()), rank = int(cl.block_rank());
   const int nc = (n + P - 1) / P;
   extern __shared__ __align__(16) double2 cols[];   // nc x n: column jl P + rank at cols + jl n
-  double2* ybuf = cols + size_t(nc) * n;            // 2 x n: tau A v, by parity of the step
-  double2* vbuf = ybuf + 2 * n;                     // 2 x n: this and the previous step's v
-  double2* wbuf = vbuf + 2 * n;                     // n: the previous step's w
-  __shared__ double2 red[2][kClWarps];
-  __shared__ double2 s_alpha[2];
-  __shared__ double s_diag[2];
+  double2* ubuf = cols + size_t(nc) * n;            // 2 x n: A x, by parity of the step
+  double2* xbuf = ubuf + 2 * n;                     // n: the pivot column
+  double2* vbuf = xbuf + n;                         // n: the previous step's v and w
+  double2* wbuf = vbuf + n;
+  double* qbuf = reinterpret_cast<double*>(wbuf + n);   // 2 x P kClWarps: shares of x^H A x
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int jl = warp; jl * P + rank < n; jl += kClWarps) {
     const int j = jl * P + rank;
@@ -701,9 +706,7 @@ __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__
       cols[size_t(jl) * n + r] = a;
     }
   }
-  for (int r = tid; r < n; r += kClThreads) {
-    vbuf[r] = vbuf[n + r] = wbuf[r] = make_double2(0.0, 0.0);
-  }
+  for (int r = tid; r < n; r += kClThreads) vbuf[r] = wbuf[r] = make_double2(0.0, 0.0);
   cl.sync();
   double2 x[kTrdRows];   // the pivot column, rows tid + kClThreads t
   {
@@ -717,109 +720,112 @@ __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__
   int par = 0;
   for (int i0 = n - 2; i0 >= 0; --i0, par ^= 1) {
     const int c = i0 + 1, L = i0 + 1;
-    // zlarfg on (alpha = x(i0), x(0:i0-1))
-    double part = 0;
 #pragma unroll
     for (int t = 0; t < kTrdRows; ++t) {
       const int r = tid + kClThreads * t;
-      if (r < i0) part += x[t].x * x[t].x + x[t].y * x[t].y;
-      if (r == i0) s_alpha[par] = x[t];
-      if (r == c) s_diag[par] = x[t].x;
+      if (r < L) xbuf[r] = x[t];
+      if (r == c && rank == 0) dout[c] = x[t].x;
     }
-    const double xn2 = block_sum2(part, 0.0, red[0]).x;   // its barrier also covers s_alpha and s_diag
-    const double2 al = s_alpha[par];
-    double2 tau = make_double2(0.0, 0.0), sc = make_double2(1.0, 0.0);
-    double beta = al.x;
-    if (!(xn2 == 0.0 && al.y == 0.0)) {
-      beta = -copysign(sqrt(al.x * al.x + al.y * al.y + xn2), al.x);
-      tau = make_double2((beta - al.x) / beta, -al.y / beta);
-      const double dr = al.x - beta, di = al.y, den = dr * dr + di * di;
-      sc = make_double2(dr / den, -di / den);   // 1 / (alpha - beta)
-    }
-    double2* v = vbuf + par * n;
-    const double2* vp = vbuf + (par ^ 1) * n;
-    double2 vr[kTrdRows];
-#pragma unroll
-    for (int t = 0; t < kTrdRows; ++t) {
-      const int r = tid + kClThreads * t;
-      vr[t] = make_double2(0.0, 0.0);
-      if (r < i0) {
-        vr[t] = cmul(x[t], sc);
-        if (rank == c % P) A[size_t(c) * n + r] = vr[t];
-      } else if (r == i0) {
-        vr[t] = make_double2(1.0, 0.0);
-      }
-      if (r <= i0) v[r] = vr[t];
-    }
-    if (rank == 0 && tid == 0) {
-      eout[i0] = beta;
-      dout[c] = s_diag[par];
-      tauout[i0] = tau;
-    }
-    __syncthreads();
-    // columns s < L: the previous rank-2 update, then y(s) = tau sum_r conj(A(r, s)) v(r)
-    double2* y = ybuf + par * n;
-    for (int jl0 = warp; jl0 * P + rank < L; jl0 += kClWarps * kClCols) {
+    __syncthreads();   // xbuf, vbuf, wbuf
+    // columns s < L: the previous rank-2 update, then u(s) = sum_r conj(A(r, s)) x(r)
+    double2* u = ubuf + par * n;
+    double* qp = qbuf + par * P * kClWarps;
+    double norm = 0, q = 0;
+    bool first = true;
+    int jl0 = warp;
+    do {   // at least once: every warp needs the norm
       double2 ws[kClCols], vs[kClCols];
       double acc[2 * kClCols] = {};
       bool on[kClCols];
 #pragma unroll
-      for (int q = 0; q < kClCols; ++q) {
-        const int s = (jl0 + q * kClWarps) * P + rank;
-        on[q] = s < L;
-        ws[q] = on[q] ? wbuf[s] : make_double2(0.0, 0.0);
-        vs[q] = on[q] ? vp[s] : make_double2(0.0, 0.0);
+      for (int k = 0; k < kClCols; ++k) {
+        const int s = (jl0 + k * kClWarps) * P + rank;
+        on[k] = s < L;
+        ws[k] = on[k] ? wbuf[s] : make_double2(0.0, 0.0);
+        vs[k] = on[k] ? vbuf[s] : make_double2(0.0, 0.0);
       }
       for (int r = lane; r < L; r += 32) {
-        const double2 pv = vp[r], pw = wbuf[r], vv = v[r];
+        const double2 pv = vbuf[r], pw = wbuf[r], xx = xbuf[r];
+        if (first && r < i0) norm += xx.x * xx.x + xx.y * xx.y;
 #pragma unroll
-        for (int q = 0; q < kClCols; ++q) {
-          if (on[q]) {
-            double2* e = cols + size_t(jl0 + q * kClWarps) * n + r;
+        for (int k = 0; k < kClCols; ++k) {
+          if (on[k]) {
+            double2* e = cols + size_t(jl0 + k * kClWarps) * n + r;
             double2 a = *e;
-            a.x -= (pv.x * ws[q].x + pv.y * ws[q].y) + (pw.x * vs[q].x + pw.y * vs[q].y);
-            a.y -= (pv.y * ws[q].x - pv.x * ws[q].y) + (pw.y * vs[q].x - pw.x * vs[q].y);
+            a.x -= (pv.x * ws[k].x + pv.y * ws[k].y) + (pw.x * vs[k].x + pw.y * vs[k].y);
+            a.y -= (pv.y * ws[k].x - pv.x * ws[k].y) + (pw.y * vs[k].x - pw.x * vs[k].y);
             *e = a;
-            acc[2 * q] += a.x * vv.x + a.y * vv.y;
-            acc[2 * q + 1] += a.x * vv.y - a.y * vv.x;
+            acc[2 * k] += a.x * xx.x + a.y * xx.y;
+            acc[2 * k + 1] += a.x * xx.y - a.y * xx.x;
           }
         }
       }
+      first = false;
       const double own = warp_sum8(acc);                                // value lane >> 2
       const double other = __shfl_xor_sync(0xffffffffu, own, 4);
       const bool im = lane & 4;
-      const double re = im ? other : own, imv = im ? own : other;
-      const int q = lane >> 3, s = (jl0 + q * kClWarps) * P + rank;   // eight lanes per column push
+      const double2 us = make_double2(im ? other : own, im ? own : other);
+      const int s = (jl0 + (lane >> 3) * kClWarps) * P + rank;          // eight lanes per column push
       if (s < L) {
-        const double2 ys = make_double2(tau.x * re - tau.y * imv, tau.x * imv + tau.y * re);
-        for (int r = lane & 7; r < P; r += 8) cl.map_shared_rank(y, r)[s] = ys;
+        for (int r = lane & 7; r < P; r += 8) cl.map_shared_rank(u, r)[s] = us;
+        const double2 xs = xbuf[s];
+        q += xs.x * us.x + xs.y * us.y;   // Re(conj(x) u)
       }
+      jl0 += kClWarps * kClCols;
+    } while (jl0 * P + rank < L);
+    q += __shfl_xor_sync(0xffffffffu, q, 8);
+    q += __shfl_xor_sync(0xffffffffu, q, 16);
+    if (lane < P) cl.map_shared_rank(qp, lane)[rank * kClWarps + warp] = q;
+    const double2 al = xbuf[i0];
+    cluster_arrive();   // this thread is done with x, v and w in shared memory
+    for (int off = 16; off > 0; off >>= 1) norm += __shfl_xor_sync(0xffffffffu, norm, off);
+    double2 tau = make_double2(0.0, 0.0), sc = make_double2(1.0, 0.0);
+    double beta = al.x;
+    if (!(norm == 0.0 && al.y == 0.0)) {   // zlarfg on (alpha = x(i0), x(0:i0-1))
+      beta = -copysign(sqrt(al.x * al.x + al.y * al.y + norm), al.x);
+      const double ib = 1.0 / beta;
+      tau = make_double2((beta - al.x) * ib, -al.y * ib);
+      const double dr = al.x - beta, di = al.y, iden = 1.0 / (dr * dr + di * di);
+      sc = make_double2(dr * iden, -di * iden);   // 1 / (alpha - beta)
     }
-    cl.sync();
-    // w = y + alpha2 v, alpha2 = -tau (y^H v) / 2; next pivot column i0, updated
+    const double2 kap = csub(make_double2(1.0, 0.0), cmul(sc, al));
+    const double tau2 = tau.x * tau.x + tau.y * tau.y, sc2 = sc.x * sc.x + sc.y * sc.y;
+    const double2 tsc = cmul(tau, sc), tkap = cmul(tau, kap);
+    if (rank == 0 && tid == 0) {
+      eout[i0] = beta;
+      tauout[i0] = tau;
+    }
+    cluster_wait();
     const double2* next = cl.map_shared_rank(cols, i0 % P) + size_t(i0 / P) * n;
-    const double2 yi = y[i0];
-    double2 yr[kTrdRows], cr[kTrdRows];
-    double pr = 0, pi = 0;
+    double2 ur[kTrdRows], ar[kTrdRows];
 #pragma unroll
     for (int t = 0; t < kTrdRows; ++t) {
       const int r = tid + kClThreads * t;
-      yr[t] = r <= i0 ? y[r] : make_double2(0.0, 0.0);
-      cr[t] = r <= i0 ? next[r] : make_double2(0.0, 0.0);
-      pr += yr[t].x * vr[t].x + yr[t].y * vr[t].y;   // conj(y) v
-      pi += yr[t].x * vr[t].y - yr[t].y * vr[t].x;
+      ar[t] = r <= i0 ? next[r] : make_double2(0.0, 0.0);
+      ur[t] = r <= i0 ? u[r] : make_double2(0.0, 0.0);
     }
-    const double2 dot = block_sum2(pr, pi, red[1]);
-    const double2 a2 = make_double2(-0.5 * (tau.x * dot.x - tau.y * dot.y), -0.5 * (tau.x * dot.y + tau.y * dot.x));
-    const double2 wi = cadd(yi, a2);   // w(i0), v(i0) = 1
+    const double2 ai = next[i0], ui = u[i0];
+    double qs = 0;
+    for (int k = lane; k < P * kClWarps; k += 32) qs += qp[k];
+    for (int off = 16; off > 0; off >>= 1) qs += __shfl_xor_sync(0xffffffffu, qs, off);
+    const double2 sk = cconjmul(sc, kap);   // conj(sc) kappa
+    const double vav = sc2 * qs + 2.0 * (sk.x * ui.x + sk.y * ui.y) + (kap.x * kap.x + kap.y * kap.y) * ai.x;
+    const double a2 = -0.5 * tau2 * vav;
+    double2 wi = cadd(cmul(tsc, ui), cmul(tkap, ai));
+    wi.x += a2;   // w(i0), v(i0) = 1
 #pragma unroll
     for (int t = 0; t < kTrdRows; ++t) {
       const int r = tid + kClThreads * t;
       if (r <= i0) {
-        const double2 w = cadd(yr[t], cmul(a2, vr[t]));
+        const double2 v = r < i0 ? cmul(x[t], sc) : make_double2(1.0, 0.0);
+        if (r < i0 && rank == c % P) A[size_t(c) * n + r] = v;
+        double2 w = cadd(cmul(tsc, ur[t]), cmul(tkap, ar[t]));
+        w.x += a2 * v.x;
+        w.y += a2 * v.y;
+        vbuf[r] = v;
         wbuf[r] = w;
-        x[t].x = cr[t].x - (vr[t].x * wi.x + vr[t].y * wi.y) - w.x;
-        x[t].y = cr[t].y - (vr[t].y * wi.x - vr[t].x * wi.y) - w.y;
+        x[t].x = ar[t].x - (v.x * wi.x + v.y * wi.y) - w.x;
+        x[t].y = ar[t].y - (v.y * wi.x - v.x * wi.y) - w.y;
       }
     }
   }
