@@ -6,20 +6,27 @@
 // atom and band, then
 //   F_I,alpha -= 2 w f_n Re[((D_I - eps_n Q) c)^H dc_alpha] + w f_n Re[c^H dD_I/dR_alpha c].
 //
-// B200 design: one kernel, one CTA per (atom, tile of 128 bands; 64 or 32
-// for atoms with more than 8 or 16 channels), 8 warps.  Per
-// chunk of 32 plane waves the CTA stages psi (coalesced along g), the plane
-// waves' q vectors, the atom's phase exp(+i q.R) (from the packed G indices and
-// the atom's b_j.R / 2 pi, reduced to one turn in FP64) and the chunk of
+// B200 design: one kernel accumulates, one contracts.  force_adjoint_kernel
+// runs one CTA per (atom, tile of 128 bands; 64 or 32 for atoms with more
+// than 8 or 16 channels, slice of the plane waves), 8 warps.  Per chunk of 32
+// plane waves the CTA stages psi (coalesced along g), the plane waves' q
+// vectors, the atom's phase exp(+i q.R) (from the packed G indices and the
+// atom's b_j.R / 2 pi, reduced to one turn in FP64) and the chunk of
 // conj(B) = Omega^-1/2 beta_l(|q|) Y_lm(q^) i^l exp(+i q.R) generated from the
 // k point's radial-angular table: B is never stored, and neither is the
 // [psi | i q psi] block.  Thread = (band, group of up to four projector
 // channels): every thread accumulates c and u_alpha = sum_g q_alpha conj(B)
-// psi for its channels in FP64 registers (dc_alpha = i u_alpha).  The
-// epilogue contracts them with D, Q and dD/dR per band and reduces the
-// tile's bands with warp shuffles and one ordered sum; a second kernel
-// adds the band tiles of each atom in order, so the result does not depend on
-// scheduling.  Bands with zero occupation are skipped as in the reference.
+// psi for its channels in FP64 registers (dc_alpha = i u_alpha) and leaves
+// its slice's sums in memory.  force_contract_kernel adds the slices in
+// order, contracts c and dc with D, Q and dD/dR per band and sums the bands
+// of a tile; a third kernel adds the tiles of each atom in order, so the
+// result does not depend on scheduling.  Bands with zero occupation are
+// skipped as in the reference.
+//
+// The accumulation is bound by the FP64 pipe (12 operations per plane wave,
+// channel and band), so what matters is that every SM has work: without
+// slices the 64-atom cell's 160 bands were 128 CTAs of which half carried 32
+// bands, 3.57 ms (16 % of the FP64 rate); 1.85 ms with slices.
 #include <algorithm>
 
 #include "context.h"
@@ -41,18 +48,12 @@ struct AtomInfo {
   int qofs;    // offset of the species Q
 };
 
-// Shared memory of the kernel variant with BT bands per CTA (256 / BT
-// channel groups): the chunk staging, or the epilogue's c and dc of every
-// band of the tile, whichever is larger.
+// Shared memory of the kernel variant with BT bands per CTA: the chunk staging.
 size_t adjoint_smem(int bt) {
-  const int groups = kAdjThreads / bt;
-  const size_t chunk = (size_t(kAdjG) * kMaxNlm + size_t(kAdjG) * (bt + 1)) * sizeof(double2) +
-                       size_t(kAdjG) * 4 * sizeof(double);
-  const size_t epilogue = size_t(4) * bt * groups * kAdjPer * sizeof(double2) + 8 * 3 * sizeof(double);
-  return std::max(chunk, epilogue);
+  return (size_t(kAdjG) * kMaxNlm + size_t(kAdjG) * (bt + 1)) * sizeof(double2) + size_t(kAdjG) * 4 * sizeof(double);
 }
 
-// One CTA per (atom, BT-band tile).  Thread = (band b = tid % BT, channel
+// One CTA per (atom, BT-band tile, slice of gper plane waves).  Thread = (band b = tid % BT, channel
 // group grp = tid / BT); it owns channels grp, grp + G, ... (up to kAdjPer of
 // them, G = 256 / BT groups, so atoms of up to 4 G channels).  A warp is 32
 // consecutive bands of one group: psi loads from shared memory are
@@ -62,12 +63,8 @@ __global__ void __launch_bounds__(kAdjThreads)
     force_adjoint_kernel(const double2* __restrict__ psi, long long ld, int npw, int nb, const double* __restrict__ qv,
                          const double* __restrict__ ftab, const int* __restrict__ gpack, const int* __restrict__ pcol,
                          const double* __restrict__ afrac, double kf0, double kf1, double kf2,
-                         const AtomInfo* __restrict__ atoms, const double* __restrict__ dall,
-                         const double* __restrict__ ddall, const double* __restrict__ qall,
-                         const double* __restrict__ eig, const double* __restrict__ occ, double kweight,
-                         double* __restrict__ partial) {
+                         const AtomInfo* __restrict__ atoms, int gper, int nlm_max, double2* __restrict__ sums) {
   constexpr int G = kAdjThreads / BT;
-  constexpr int NL = G * kAdjPer;   // channel slots of a band in the epilogue
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* sB = reinterpret_cast<double2*>(smem_raw);      // [kAdjG][kMaxNlm]  conj(B)
   // [kAdjG][BT + 1]: the row pad keeps the g-major staging stores and the
@@ -95,12 +92,13 @@ __global__ void __launch_bounds__(kAdjThreads)
 #pragma unroll
     for (int j = 0; j < kAdjPer; ++j) acc[q][j] = make_double2(0.0, 0.0);
 
-  for (int g0 = 0; g0 < npw; g0 += kAdjG) {
+  const int gend = min(npw, (int(blockIdx.z) + 1) * gper);
+  for (int g0 = blockIdx.z * gper; g0 < gend; g0 += kAdjG) {
     __syncthreads();   // the previous chunk has been consumed
     if (tid < kAdjG) {
       const int g = g0 + tid;
       double2 ph = make_double2(0.0, 0.0);
-      if (g < npw) {
+      if (g < gend) {
         const int gp = gpack[g];
         const double t = (double((gp << 22) >> 22) + kf0) * f0 + (double((gp << 12) >> 22) + kf1) * f1 +
                          (double((gp << 2) >> 22) + kf2) * f2;
@@ -112,17 +110,17 @@ __global__ void __launch_bounds__(kAdjThreads)
     }
     for (int t = tid; t < kAdjG * BT; t += kAdjThreads) {
       const int gl = t % kAdjG, b = t / kAdjG, g = g0 + gl, nn = bt * BT + b;
-      spsi[gl * BP + b] = (g < npw && nn < nb) ? psi[(long long)nn * ld + g] : make_double2(0.0, 0.0);
+      spsi[gl * BP + b] = (g < gend && nn < nb) ? psi[(long long)nn * ld + g] : make_double2(0.0, 0.0);
     }
     for (int t = tid; t < kAdjG * 3; t += kAdjThreads) {
       const int gl = t / 3, a = t - 3 * gl, g = g0 + gl;
-      sq[4 * gl + a] = g < npw ? qv[3 * (long long)g + a] : 0.0;
+      sq[4 * gl + a] = g < gend ? qv[3 * (long long)g + a] : 0.0;
     }
     __syncthreads();
     for (int t = tid; t < kAdjG * nlm; t += kAdjThreads) {
       const int gl = t / nlm, a = t - gl * nlm, g = g0 + gl;
       double2 v = make_double2(0.0, 0.0);
-      if (g < npw) {
+      if (g < gend) {
         const double f = ftab[(long long)sfrow[a] * npw + g];
         const double2 p = sph[gl];
         double re, im;   // i^l (c + i s)
@@ -161,67 +159,70 @@ __global__ void __launch_bounds__(kAdjThreads)
       }
     }
   }
-  __syncthreads();
-  // c and dc_alpha = i u_alpha of every band of the tile -> shared memory
-  double2* sc = reinterpret_cast<double2*>(smem_raw);   // [4][BT][NL]
+  // sums: [slice][atom][c, u_x, u_y, u_z][channel][band]
+  if (n < nb) {
+    double2* out = sums + ((long long)blockIdx.z * gridDim.x + ion) * 4 * nlm_max * nb + n;
 #pragma unroll
-  for (int j = 0; j < kAdjPer; ++j) {
-    const int a = grp + j * G;
-    if (a < nlm) {
-      sc[(0 * BT + bl) * NL + a] = acc[0][j];
-      for (int al = 0; al < 3; ++al)
-        sc[((1 + al) * BT + bl) * NL + a] = make_double2(-acc[1 + al][j].y, acc[1 + al][j].x);
+    for (int j = 0; j < kAdjPer; ++j) {
+      const int a = grp + j * G;
+      if (a < nlm)
+        for (int q = 0; q < 4; ++q) out[((long long)q * nlm_max + a) * nb] = acc[q][j];
     }
+  }
+}
+
+constexpr int kConBands = 32;   // bands per CTA of the contraction, one lane each; warp = Cartesian component
+
+// partial[atom][tile][alpha] = the force of one tile of bands.
+__global__ void __launch_bounds__(3 * kConBands)
+    force_contract_kernel(const double2* __restrict__ sums, int slices, int nb, int nlm_max,
+                          const AtomInfo* __restrict__ atoms, const double* __restrict__ dall,
+                          const double* __restrict__ ddall, const double* __restrict__ qall,
+                          const double* __restrict__ eig, const double* __restrict__ occ, double kweight,
+                          double* __restrict__ partial) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* sc = reinterpret_cast<double2*>(smem_raw);   // [4][nlm][kConBands]
+  const int ion = blockIdx.x, tile = blockIdx.y, nions = gridDim.x;
+  const AtomInfo A = atoms[ion];
+  const int nlm = A.nlm;
+  for (int t = threadIdx.x; t < 4 * nlm * kConBands; t += blockDim.x) {
+    const int b = t % kConBands, qa = t / kConBands, q = qa / nlm, a = qa - q * nlm, n = tile * kConBands + b;
+    double2 s = make_double2(0.0, 0.0);
+    if (n < nb)
+      for (int z = 0; z < slices; ++z)
+        s = cadd(s, sums[(((long long)z * nions + ion) * 4 * nlm_max + (long long)q * nlm_max + a) * nb + n]);
+    sc[t] = s;
   }
   __syncthreads();
-  double* wsum = reinterpret_cast<double*>(sc + 4 * BT * NL);   // [BT / 32][3]
-  if (tid < BT) {
-    double fsum[3] = {0.0, 0.0, 0.0};
-    const double fo = n < nb ? occ[n] : 0.0;
-    if (fo != 0.0) {
-      const double e = eig[n];
-      const double* D = dall + A.dofs;
-      const double* Q = qall + A.qofs;
-      const double2* c = sc + bl * NL;
-      double2 mc[NL];
-      for (int a = 0; a < nlm; ++a) {
-        double2 s = make_double2(0.0, 0.0);
-        for (int k = 0; k < nlm; ++k) {
-          const double w = D[a * nlm + k] - e * Q[a * nlm + k];
-          s.x += w * c[k].x;
-          s.y += w * c[k].y;
-        }
-        mc[a] = s;
+  const int al = threadIdx.x / kConBands, lane = threadIdx.x % kConBands, n = tile * kConBands + lane;
+  double v = 0.0;
+  const double fo = n < nb ? occ[n] : 0.0;
+  if (fo != 0.0) {
+    const double e = eig[n];
+    const double* D = dall + A.dofs;
+    const double* Q = qall + A.qofs;
+    const double* dD = ddall + A.ddofs + al * nlm * nlm;
+    const double2* c = sc + lane;                                       // c[a] at c[a kConBands]
+    const double2* u = sc + (size_t)(1 + al) * nlm * kConBands + lane;   // dc = i u
+    double re = 0.0, q = 0.0;
+    for (int a = 0; a < nlm; ++a) {
+      double2 m = make_double2(0.0, 0.0), s = make_double2(0.0, 0.0);
+      for (int k = 0; k < nlm; ++k) {
+        const double w = D[a * nlm + k] - e * Q[a * nlm + k], d = dD[a * nlm + k];
+        const double2 ck = c[k * kConBands];
+        m.x += w * ck.x;
+        m.y += w * ck.y;
+        s.x += d * ck.x;
+        s.y += d * ck.y;
       }
-      for (int al = 0; al < 3; ++al) {
-        const double2* dc = sc + ((1 + al) * BT + bl) * NL;
-        double re = 0.0;
-        for (int a = 0; a < nlm; ++a) re += mc[a].x * dc[a].x + mc[a].y * dc[a].y;   // Re(conj(mc) . dc)
-        const double* dD = ddall + A.ddofs + al * nlm * nlm;
-        double q = 0.0;
-        for (int a = 0; a < nlm; ++a) {
-          double2 s = make_double2(0.0, 0.0);
-          for (int k = 0; k < nlm; ++k) {
-            s.x += dD[a * nlm + k] * c[k].x;
-            s.y += dD[a * nlm + k] * c[k].y;
-          }
-          q += c[a].x * s.x + c[a].y * s.y;   // Re(conj(c) . dD c)
-        }
-        fsum[al] = -2.0 * kweight * fo * re - kweight * fo * q;
-      }
+      const double2 ua = u[a * kConBands], ca = c[a * kConBands];
+      re += m.y * ua.x - m.x * ua.y;      // Re(conj(m) . i u)
+      q += ca.x * s.x + ca.y * s.y;       // Re(conj(c) . dD c)
     }
-    for (int al = 0; al < 3; ++al) {
-      double v = fsum[al];
-      for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-      if ((tid & 31) == 0) wsum[(tid >> 5) * 3 + al] = v;
-    }
+    v = -2.0 * kweight * fo * re - kweight * fo * q;
   }
-  __syncthreads();
-  if (tid < 3) {   // the tile's warps in order
-    double v = 0.0;
-    for (int w = 0; w < BT / 32; ++w) v += wsum[w * 3 + tid];
-    partial[((long long)ion * gridDim.y + bt) * 3 + tid] = v;
-  }
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+  if (lane == 0) partial[((long long)ion * gridDim.y + tile) * 3 + al] = v;
 }
 
 // out[ion][alpha] = sum over band tiles, in tile order.
@@ -268,32 +269,48 @@ void nonlocal_forces_device(Context& ctx, KOperatorSet& ks, const double2* dvec,
   for (auto& sp : ctx.species) nlm_max = std::max(nlm_max, sp.nlm);
   // bands per CTA: 128 for atoms of up to 8 channels, 64 up to 16, 32 up to 32
   const int bt = nlm_max <= 2 * kAdjPer ? 128 : nlm_max <= 4 * kAdjPer ? 64 : 32;
-  const int ntiles = (nb + bt - 1) / bt;
+  const int btiles = (nb + bt - 1) / bt, ntiles = (nb + kConBands - 1) / kConBands;
+  // Slices of the plane waves: enough for about six CTAs per SM (two are
+  // resident, so uneven tiles even out), each of at least four chunks, and
+  // sums of at most 256 MB.
+  const long long slice_bytes = (long long)nions * 4 * nlm_max * nb * (long long)sizeof(double2);
+  const int chunks = (npw + kAdjG - 1) / kAdjG;
+  long long slices = (6LL * 148 + (long long)nions * btiles - 1) / ((long long)nions * btiles);
+  slices = std::min(slices, (long long)std::max(1, chunks / 4));
+  slices = std::max(1LL, std::min(slices, (256LL << 20) / slice_bytes));
+  const int gper = ceil_div(chunks, slices) * kAdjG;
+  const int nsl = ceil_div(npw, gper);
   DeviceBuffer<AtomInfo> datoms;
   datoms.upload(atoms, st);
   DeviceBuffer<double> dd, ddd, dq, deig, docc, dpart(size_t(nions) * ntiles * 3), dout(size_t(nions) * 3);
+  DeviceBuffer<double2> dsums(size_t(nsl) * nions * 4 * nlm_max * nb);
   dd.upload(dall, st);
   ddd.upload(ddall, st);
   dq.upload(qall, st);
   deig.upload(eig, nb, st);
   docc.upload(occ, nb, st);
-  const size_t smem = adjoint_smem(bt);
+  const size_t smem = adjoint_smem(bt), csmem = size_t(4) * nlm_max * kConBands * sizeof(double2);
   Profile& pf = rt.prof;
   const int ev0 = pf.record(st);
   auto launch = [&](auto kernel) {
     raise_smem_limit(kernel, smem);
-    kernel<<<dim3(nions, ntiles), kAdjThreads, smem, st>>>(
+    kernel<<<dim3(nions, btiles, nsl), kAdjThreads, smem, st>>>(
         dvec, ld, npw, nb, ks.qvec.get(), ks.ftab64.get(), ks.gpack.get(), ks.pcol.get(), ks.afrac.get(), ks.kf[0],
-        ks.kf[1], ks.kf[2], datoms.get(), dd.get(), ddd.get(), dq.get(), deig.get(), docc.get(), kweight, dpart.get());
+        ks.kf[1], ks.kf[2], datoms.get(), gper, nlm_max, dsums.get());
   };
   if (bt == 128) launch(force_adjoint_kernel<128>);
   else if (bt == 64) launch(force_adjoint_kernel<64>);
   else launch(force_adjoint_kernel<32>);
   HALF_LAUNCH("force adjoint");
+  raise_smem_limit(force_contract_kernel, csmem);
+  force_contract_kernel<<<dim3(nions, ntiles), 3 * kConBands, csmem, st>>>(
+      dsums.get(), nsl, nb, nlm_max, datoms.get(), dd.get(), ddd.get(), dq.get(), deig.get(), docc.get(), kweight,
+      dpart.get());
+  HALF_LAUNCH("force contraction");
   sum_tiles_kernel<<<ceil_div(nions * 3, 128), 128, 0, st>>>(dpart.get(), nions, ntiles, dout.get());
   HALF_LAUNCH("force tiles");
   pf.span(Profile::kAdjoint, ev0, pf.record(st));
-  pf.launches += 2;
+  pf.launches += 3;
   auto f = dout.download(st);
   for (int i = 0; i < nions * 3; ++i) forces_host[i] += f[i];
 }
