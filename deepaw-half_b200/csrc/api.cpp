@@ -20,6 +20,7 @@
 #include "../../include/half_b200.h"
 #include "context.h"
 #include "devmem.h"
+#include "staging.h"
 #include "tc_gemm.h"
 
 using namespace hb;
@@ -285,7 +286,10 @@ int half_destroy(half_handle handle, char* error, int cap) {
     g_slots[s].used = false;
     bool any = false;
     for (const auto& sl : g_slots) any = any || sl.used;
-    if (!any) device_cache_release();   // last context gone: cached device blocks back to the driver
+    if (!any) {   // last context gone: cached device blocks and pinned buffers back to the driver
+      device_cache_release();
+      staging_release();
+    }
     return HALF_SUCCESS;
   });
 }
@@ -411,11 +415,8 @@ int half_assemble_hs(half_handle handle, const double kpoint[3], int64_t ld, HAL
     DeviceBuffer<double2> dh((size_t)n * n), ds((size_t)n * n);
     assemble_dense(*ctx, *ks, dh.get(), ds.get());
     cudaStream_t st = ctx->rt->stream;
-    HALF_CUDA(cudaMemcpy2DAsync(h, ld * sizeof(double2), dh.get(), n * sizeof(double2), n * sizeof(double2), n,
-                                cudaMemcpyDeviceToHost, st));
-    HALF_CUDA(cudaMemcpy2DAsync(s, ld * sizeof(double2), ds.get(), n * sizeof(double2), n * sizeof(double2), n,
-                                cudaMemcpyDeviceToHost, st));
-    HALF_CUDA(cudaStreamSynchronize(st));
+    block_to_host(h, ld, dh.get(), n, n, st);
+    block_to_host(s, ld, ds.get(), n, n, st);
     return HALF_SUCCESS;
   });
 }
@@ -434,8 +435,7 @@ int half_apply_hs(half_handle handle, const double kpoint[3], int nstates, int64
     if (ld < n) fail(kCapacity, "state leading dimension is too small");
     cudaStream_t st = ctx->rt->stream;
     DeviceBuffer<double2> x((size_t)n * nstates), hx((size_t)n * nstates), sx((size_t)n * nstates);
-    HALF_CUDA(cudaMemcpy2DAsync(x.get(), n * sizeof(double2), psi, ld * sizeof(double2), n * sizeof(double2), nstates,
-                                cudaMemcpyHostToDevice, st));
+    block_to_device(x.get(), psi, ld, n, nstates, st);
     ctx->last = SolveInfo();
     begin_call(*ctx->rt);
     if (fp32) {
@@ -445,11 +445,8 @@ int half_apply_hs(half_handle handle, const double kpoint[3], int nstates, int64
       apply_hs<double>(*ctx, *ks, x.get(), n, nstates, hx.get(), sx.get(), ctx->acc.block);
     }
     end_call(*ctx->rt, ctx->last);
-    HALF_CUDA(cudaMemcpy2DAsync(hpsi, ld * sizeof(double2), hx.get(), n * sizeof(double2), n * sizeof(double2), nstates,
-                                cudaMemcpyDeviceToHost, st));
-    HALF_CUDA(cudaMemcpy2DAsync(spsi, ld * sizeof(double2), sx.get(), n * sizeof(double2), n * sizeof(double2), nstates,
-                                cudaMemcpyDeviceToHost, st));
-    HALF_CUDA(cudaStreamSynchronize(st));
+    block_to_host(hpsi, ld, hx.get(), n, nstates, st);
+    block_to_host(spsi, ld, sx.get(), n, nstates, st);
     return HALF_SUCCESS;
   });
 }
@@ -470,12 +467,7 @@ int half_solve_kpoint(half_handle handle, const double kpoint[3], int nbands, do
     if (eigenvalues) std::copy(out.eigenvalues.begin(), out.eigenvalues.end(), eigenvalues);
     if (overlap_min) *overlap_min = out.overlap_min;
     if (overlap_max) *overlap_max = out.overlap_max;
-    if (vectors) {
-      cudaStream_t st = ctx->rt->stream;
-      HALF_CUDA(cudaMemcpy2DAsync(vectors, ld * sizeof(double2), out.dvectors.get(), n * sizeof(double2),
-                                  n * sizeof(double2), nbands, cudaMemcpyDeviceToHost, st));
-      HALF_CUDA(cudaStreamSynchronize(st));
-    }
+    if (vectors) block_to_host(vectors, ld, out.dvectors.get(), n, nbands, ctx->rt->stream);
     return HALF_SUCCESS;
   });
 }
@@ -780,8 +772,7 @@ int half_nonlocal_forces(half_handle handle, const double kpoint[3], int nbands,
     if (ld < n) fail(kCapacity, "eigenvector leading dimension is too small");
     cudaStream_t st = ctx->rt->stream;
     DeviceBuffer<double2> dv((size_t)n * nbands);
-    HALF_CUDA(cudaMemcpy2DAsync(dv.get(), n * sizeof(double2), vectors, ld * sizeof(double2), n * sizeof(double2),
-                                nbands, cudaMemcpyHostToDevice, st));
+    block_to_device(dv.get(), vectors, ld, n, nbands, st);
     ctx->last = SolveInfo();
     begin_call(*ctx->rt);
     nonlocal_forces_device(*ctx, *ks, dv.get(), n, nbands, eigenvalues, occupations, kweight, forces);
@@ -901,8 +892,7 @@ extern "C" int half_output_density(half_handle handle, int nk, const double* kpo
         continue;
       }
       dv[ik].resize((size_t)npw * nbands);
-      HALF_CUDA(cudaMemcpy2DAsync(dv[ik].get(), npw * sizeof(double2), src, ld * sizeof(double2),
-                                  npw * sizeof(double2), nbands, cudaMemcpyHostToDevice, st));
+      block_to_device(dv[ik].get(), src, ld, npw, nbands, st);
       ptr[ik] = dv[ik].get();
       lds[ik] = npw;
     }
@@ -1021,8 +1011,7 @@ extern "C" int half_pack_vasp_waves(half_handle handle, int nk, const double* kp
       long long sld = ld;
       if (!vec_dev) {
         dv.resize((size_t)npw * nbands);
-        HALF_CUDA(cudaMemcpy2DAsync(dv.get(), npw * sizeof(double2), src, ld * sizeof(double2), npw * sizeof(double2),
-                                    nbands, cudaMemcpyHostToDevice, st));
+        block_to_device(dv.get(), src, ld, npw, nbands, st);
         src = dv.get();
         sld = npw;
       }

@@ -500,14 +500,18 @@ HostGeom plane_geometry(const Basis& b, const AxisPlan& ax, const AxisPlan& ay, 
   h.row_start.push_back(int(h.row_list.size()));
   // z passes: threads run over a plane's rows, so neighbours in the list get
   // different shared-memory banks where the occupied rows allow it
+  std::vector<int> by_bank;
   for (int j = 0; j < h.nplanes; ++j) {
     const int a = h.row_start[j], e = h.row_start[j + 1];
-    std::vector<std::vector<int>> by_bank(16);
-    for (int r = a; r < e; ++r) by_bank[h.row_list[r] % 16].push_back(h.row_list[r]);
-    int o = a;
-    for (size_t i = 0; o < e; ++i)
-      for (auto& v : by_bank)
-        if (i < v.size()) h.row_list[o++] = v[i];
+    by_bank.assign(h.row_list.begin() + a, h.row_list.begin() + e);
+    std::sort(by_bank.begin(), by_bank.end(), [](int x, int y) { return x % 16 != y % 16 ? x % 16 < y % 16 : x < y; });
+    // deal the banks' rows out in turn: the i-th row of every bank, then the next
+    int start[17] = {};
+    for (int r : by_bank) ++start[r % 16 + 1];
+    for (int i = 0; i < 16; ++i) start[i + 1] += start[i];
+    for (int i = 0, o = a; o < e; ++i)
+      for (int bk = 0; bk < 16; ++bk)
+        if (start[bk] + i < start[bk + 1]) h.row_list[o++] = by_bank[start[bk] + i];
     h.max_rows = std::max(h.max_rows, e - a);
   }
   if (p != npw) fail(kInternal, "basis is not ordered by g1");
@@ -528,7 +532,7 @@ struct ProjGen {
 };
 
 template <typename R>
-void fill_operator(Context& ctx, Runtime& rt, const Basis& basis, const HostGeom& hg, const DeviceBuffer<double2>& B64, int np,
+void fill_operator(Context& ctx, Runtime& rt, const Basis& basis, const HostGeom& hg, DeviceBuffer<double2>& B64, int np,
                    const std::vector<int>& cb, const std::vector<int>& ca, const std::vector<int>& cn,
                    const std::vector<int>& cd, const std::vector<int>& cq, const ProjGen& gen, KOperator<R>& op) {
   using C = cplx_t<R>;
@@ -559,8 +563,7 @@ void fill_operator(Context& ctx, Runtime& rt, const Basis& basis, const HostGeom
   op.kinetic.resize(basis.npw());
   scale_copy_kernel<R><<<ceil_div(basis.npw(), 256), 256, 0, s>>>(kin.get(), op.kinetic.get(), basis.npw(), 1.0);
   if constexpr (sizeof(R) == 8) {
-    op.B.resize(B64.size());
-    HALF_CUDA(cudaMemcpyAsync(op.B.get(), B64.get(), B64.size() * sizeof(double2), cudaMemcpyDeviceToDevice, s));
+    op.B = std::move(B64);   // only the FP64 operator reads the stored matrix
   } else if (np > 0) {
     const long long nt = (long long)gen.frows.size() * basis.npw();
     op.ftab.resize(size_t(nt));

@@ -281,8 +281,8 @@ class Context:
             psi = psi[:, None]
         n, nb = psi.shape
         x = np.ascontiguousarray(psi.T)           # column-major (n x nb)
-        h = np.zeros_like(x)
-        s = np.zeros_like(x)
+        h = np.zeros(x.shape, dtype=x.dtype)   # untouched zero pages, unlike zeros_like's explicit fill
+        s = np.zeros(x.shape, dtype=x.dtype)
         _check(self.lib.half_apply_hs(self.handle, _ptr(kk), nb, n, _ptr(x), _ptr(h), _ptr(s), err, 512), err)
         return h.T, s.T
 
