@@ -58,6 +58,13 @@ __host__ __device__ inline uint32_t stage_bytes(int bn) {
   return ((s + 1023u) / 1024u) * 1024u;
 }
 
+// TMEM columns between two accumulators of a bn-wide tile.
+__host__ __device__ inline uint32_t accumulator_columns(int bn) {
+  uint32_t c = 16;
+  while (c < uint32_t(bn)) c <<= 1;
+  return c;
+}
+
 struct Out {
   int mode;          // 0: complex FP32 C, 1: complex FP64 C, 2: split-K partial sums
   void* c;
@@ -254,22 +261,24 @@ __device__ __forceinline__ void write_out(T* dst, double re, double im, const Ou
 
 // A and B are pre-split planes (TcOperand::kPlanes); A.rows_pad >= gridDim.x
 // 128 and B.rows_pad >= gridDim.y bn, both with nkb_total k blocks.
-__global__ void __launch_bounds__(kThreads, 1)
-    tc_cgemm_kernel(TcOperand A, TcOperand B, int bn, int nst, int kb_per_split, int nkb_total, Out out, int* err) {
+__global__ void __launch_bounds__(kThreads, 2)
+    tc_cgemm_kernel(TcOperand A, TcOperand B, int bn, int nst, int kb_per_split, int groups, int nkb_total, Out out,
+                    int* err) {
   extern __shared__ __align__(1024) unsigned char smem_dyn[];
   __shared__ uint64_t full_bar[kMaxPipe], empty_bar[kMaxPipe], accum_bar;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * bn, split = blockIdx.z;
-  const int kb0 = split * kb_per_split;
-  const int nkb = min(nkb_total, kb0 + kb_per_split) - kb0;
+  // a CTA runs `groups` consecutive splits, each into its own accumulators
+  const int kb0 = split * kb_per_split * groups;
+  const int nkb = min(nkb_total, kb0 + kb_per_split * groups) - kb0;
   const uint32_t sbase = (smem_addr(smem_dyn) + uint32_t(kSmemSlack - 1)) & ~uint32_t(kSmemSlack - 1);
   const uint32_t a_ps = uint32_t(kBM) * 32u, b_ps = uint32_t(bn) * 32u;
   const uint32_t sbytes = stage_bytes(bn);
+  const uint32_t ci_off = accumulator_columns(bn);   // (group, Re / Im) at (2 group + c) ci_off
   uint32_t tcols = 32;
-  while (tcols < uint32_t(2 * bn)) tcols <<= 1;
-  const uint32_t ci_off = tcols >> 1;
+  while (tcols < 2u * uint32_t(groups) * ci_off) tcols <<= 1;
   volatile int* abort = &abort_flag;
 
   if (warp == kMmaWarp) tmem_alloc(&tmem_slot, tcols);
@@ -318,12 +327,15 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (!mbar_wait(&full_bar[s], (i / nst) & 1, abort)) break;
         tcgen05_fence_after();
         const uint32_t abase = sbase + uint32_t(s) * sbytes, bbase = abase + 4u * a_ps;
+        const int grp = groups == 1 ? 0 : i / kb_per_split;
+        const bool first = i == grp * kb_per_split;
+        const uint32_t acc = tmem + 2u * uint32_t(grp) * ci_off;
 #pragma unroll
         for (int c = 0; c < 12; ++c) {
           const uint64_t ad = smem_desc(abase + uint32_t(kCombo[c][0]) * a_ps, 128u, 256u);
           const uint64_t bd = smem_desc(bbase + uint32_t(kCombo[c][1]) * b_ps, 128u, 256u);
-          mma_bf16(tmem + (kCombo[c][2] ? ci_off : 0u), ad, bd, kCombo[c][3] ? id_neg : id_pos,
-                   i > 0 || (c != 0 && c != 6));
+          mma_bf16(acc + (kCombo[c][2] ? ci_off : 0u), ad, bd, kCombo[c][3] ? id_neg : id_pos,
+                   !first || (c != 0 && c != 6));
         }
         mma_commit(&empty_bar[s]);
       }
@@ -337,8 +349,38 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int q = warp & 3, half = warp >> 2;
       const int row = m0 + q * 32 + lane;
       for (int c = half; c < bn / 16; c += 2) {
-        float cr[16], ci[16];
         const uint32_t ta = tmem + (uint32_t(q * 32) << 16) + uint32_t(c * 16);
+        if (groups > 1) {   // the splits' sums in order, in FP64, as the split-K reduction adds them
+          for (int h = 0; h < 2; ++h) {
+            double dr[8], di[8];
+            for (int g = 0; g < groups; ++g) {
+              float cr[8], ci[8];
+              tmem_ld8(ta + 8u * uint32_t(h) + 2u * uint32_t(g) * ci_off, cr);
+              tmem_ld8(ta + 8u * uint32_t(h) + (2u * uint32_t(g) + 1u) * ci_off, ci);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                dr[j] = g ? dr[j] + cr[j] : double(cr[j]);
+                di[j] = g ? di[j] + ci[j] : double(ci[j]);
+              }
+            }
+            if (row < out.M) {
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                const int col = n0 + c * 16 + h * 8 + j;
+                if (col >= out.N) break;
+                const bool second = col >= out.split_col;
+                const long long o = row + (long long)(second ? col - out.split_col : col) * out.ldc;
+                if (out.mode == 0)
+                  write_out(reinterpret_cast<float2*>(second ? out.c2 : out.c) + o, dr[j], di[j], out);
+                else
+                  write_out(reinterpret_cast<double2*>(second ? out.c2 : out.c) + o, dr[j], di[j], out);
+              }
+            }
+          }
+          continue;
+        }
+        float cr[16], ci[16];
         tmem_ld16(ta, cr);
         tmem_ld16(ta + ci_off, ci);
         tmem_ld_wait();
@@ -488,13 +530,20 @@ void tc_cgemm(Runtime& rt, const TcOperand& A, const TcOperand& B, int M, int N,
   int splits = nkb > 0 ? pick_splits(tiles, nkb, bn0, (long long)M * N, sms) : 1;
   const int kbps = nkb > 0 ? (nkb + splits - 1) / splits : 0;
   if (nkb > 0) splits = (nkb + kbps - 1) / kbps;
+  // Few splits of a short K run in one CTA, each into accumulators of its own
+  // (2 x splits x bn TMEM columns), and are added in the epilogue: the same
+  // sums without partial sums in memory and a reduction pass (11,023 x 187 x
+  // 193, 2 splits: the call 85 -> 70 us).
+  const int groups = splits >= 2 && splits <= 4 && nkb <= 64 ? splits : 1;
+  const int most_bn = groups == 1 ? 256 : groups == 2 ? 128 : 64;
   // tile width: 0, 1 or 2 more N tiles than the fewest are the candidates
   std::vector<int> cand;
+  const int ntf = (N + most_bn - 1) / most_bn;
   for (int extra = 0; extra < 3; ++extra) {
-    const int t = nt0 + extra, w = ((N + t - 1) / t + 15) / 16 * 16;
+    const int t = (groups == 1 ? nt0 : ntf) + extra, w = ((N + t - 1) / t + 15) / 16 * 16;
     if (w >= 16 && (cand.empty() || w < cand.back())) cand.push_back(w);
   }
-  int tune_token = 0, tune_index = 0, bn = bn0;
+  int tune_token = 0, tune_index = 0, bn = groups == 1 ? bn0 : std::min(most_bn, cand.empty() ? 16 : cand[0]);
   std::string key;
   if (nkb > 0 && cand.size() > 1) {
     key = "gemm " + std::to_string(A.kind) + std::to_string(B.kind) + " " + std::to_string(M) +
@@ -551,9 +600,9 @@ void tc_cgemm(Runtime& rt, const TcOperand& A, const TcOperand& B, int M, int N,
   }
   const size_t sbytes = stage_bytes(bn);
   // Short chains leave half the shared memory to a second CTA where their
-  // accumulators fit Tensor Memory twice (bn <= 128), so that one CTA's
+  // accumulators fit Tensor Memory twice, so that one CTA's
   // epilogue runs beside the other's copies and MMAs.
-  const size_t budget = bn <= 128 && kbps <= 16 ? kSmemBudget / 2 : kSmemBudget;
+  const size_t budget = groups * 2 * accumulator_columns(bn) <= 256 && kbps * groups <= 16 ? kSmemBudget / 2 : kSmemBudget;
   const int nst = int(std::min<size_t>(kMaxPipe, (budget - kSmemSlack) / sbytes));
   if (nst < 2) fail(kInternal, "tensor-core GEMM stage does not fit shared memory twice");
   const size_t smem = size_t(nst) * sbytes + kSmemSlack;
@@ -563,7 +612,7 @@ void tc_cgemm(Runtime& rt, const TcOperand& A, const TcOperand& B, int M, int N,
   o.beta = beta;
   o.M = M;
   o.N = N;
-  const bool direct = splits == 1 && nkb > 0;
+  const bool direct = splits == groups && nkb > 0;
   if (direct) {
     o.mode = c_fp64 ? 1 : 0;
     o.c = C;
@@ -579,7 +628,8 @@ void tc_cgemm(Runtime& rt, const TcOperand& A, const TcOperand& B, int M, int N,
   if (nkb > 0) {
     const int e0 = span0 >= 0 ? span0 : pf.record(st);
     if (!key.empty()) tune_token = Tuner::begin(key, tune_index, st);   // the product alone, no allocation or split pass
-    tc_cgemm_kernel<<<dim3(mt, nt, splits), kThreads, smem, st>>>(Ak, Bk, bn, nst, kbps, nkb, o, rt.tc_err.get());
+    tc_cgemm_kernel<<<dim3(mt, nt, splits / groups), kThreads, smem, st>>>(Ak, Bk, bn, nst, kbps, groups, nkb, o,
+                                                                           rt.tc_err.get());
     HALF_LAUNCH("tensor-core cgemm");
     Tuner::finish(tune_token, st, 1.0);
     pf.span(Profile::kTensor, e0, pf.record(st));
