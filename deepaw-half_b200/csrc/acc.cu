@@ -38,6 +38,7 @@
 #include <string>
 
 #include "blas.h"
+#include "blockops.h"
 #include "context.h"
 #include "eig.h"
 
@@ -421,6 +422,11 @@ struct AccRun {
   long long op_cols = 0;
   Tracer* tr = nullptr;
   void mark(const char* s) { if (tr) tr->mark(s); }
+  // FP64 blocks of the small cells: the iteration's products through the fused block kernels
+  bool fused(int order) const {
+    if constexpr (sizeof(R) == 8) return zblock_fused(n, order);
+    return false;
+  }
 
   void apply(const C* x, C* hx, C* sx, int nb) {
     auto t0 = std::chrono::steady_clock::now();
@@ -447,7 +453,19 @@ struct AccRun {
     const auto one = cval<R>(1.0), zero = cval<R>(0.0);
     double2* hs = sc.hsub.get();
     double2* ssb = sc.ssub.get();
+    int nx = blk.cur ^ 1;
     if constexpr (sizeof(R) == 8) {
+      if (fused(m)) {
+        const ZBlock b[2] = {{blk.hx(), m}, {blk.sx(), m}};
+        double2* const c[2] = {hs, ssb};
+        zgram(rt, n, {blk.x(), m}, b, c, 2, m, true);
+        ss.hegvd(hs, ssb, m, sc.w.get(), m);
+        const ZBlock z[3] = {{blk.x(), m}, {blk.hx(), m}, {blk.sx(), m}};
+        double2* const out[3] = {blk.X[nx].get(), blk.HX[nx].get(), blk.SX[nx].get()};
+        zupdate(rt, n, z, hs, m, out, m, 3, 1.0, 0.0);
+        blk.cur = nx;
+        return;
+      }
       gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, m, n, one, blk.x(), n, blk.hx(), n, zero, hs, m);
       gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, m, n, one, blk.x(), n, blk.sx(), n, zero, ssb, m);
     } else {
@@ -456,7 +474,6 @@ struct AccRun {
     }
     ss.hegvd(hs, ssb, m, sc.w.get(), m);
     to_r(hs, m, blk.Y.get(), m, m, m);
-    int nx = blk.cur ^ 1;
     gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, m, m, one, blk.x(), n, blk.Y.get(), m, zero, blk.X[nx].get(), n);
     gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, m, m, one, blk.hx(), n, blk.Y.get(), m, zero, blk.HX[nx].get(), n);
     gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, m, m, one, blk.sx(), n, blk.Y.get(), m, zero, blk.SX[nx].get(), n);
@@ -566,11 +583,24 @@ struct AccRun {
     mark("precondition");
     apply(blk.P.get(), blk.HP.get(), blk.SP.get(), np);
     mark("apply");
+    const bool fuse = fused(m + np);
     // S-orthogonalise against X
-    gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, np, n, one, blk.x(), n, blk.SP.get(), n, zero, blk.small.get(), m);
-    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, m, mone, blk.x(), n, blk.small.get(), m, one, blk.P.get(), n);
-    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, m, mone, blk.hx(), n, blk.small.get(), m, one, blk.HP.get(), n);
-    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, m, mone, blk.sx(), n, blk.small.get(), m, one, blk.SP.get(), n);
+    if constexpr (sizeof(R) == 8) {
+      if (fuse) {
+        const ZBlock b = {blk.SP.get(), np};
+        double2* const c = blk.small.get();
+        zgram(rt, n, {blk.x(), m}, &b, &c, 1, m, false);
+        const ZBlock z[3] = {{blk.x(), m}, {blk.hx(), m}, {blk.sx(), m}};
+        double2* const out[3] = {blk.P.get(), blk.HP.get(), blk.SP.get()};
+        zupdate(rt, n, z, blk.small.get(), m, out, np, 3, -1.0, 1.0);
+      }
+    }
+    if (!fuse) {
+      gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, np, n, one, blk.x(), n, blk.SP.get(), n, zero, blk.small.get(), m);
+      gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, m, mone, blk.x(), n, blk.small.get(), m, one, blk.P.get(), n);
+      gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, m, mone, blk.hx(), n, blk.small.get(), m, one, blk.HP.get(), n);
+      gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, m, mone, blk.sx(), n, blk.small.get(), m, one, blk.SP.get(), n);
+    }
     mark("orth_gemm");
     // In the guard-band modes the separate S-metric normalisation is
     // skipped.  The library's own pencil solver (small orders) Jacobi-scales
@@ -601,6 +631,14 @@ struct AccRun {
     };
     if (!skip_metric) use_metric();
     auto project = [&]() {
+      if constexpr (sizeof(R) == 8) {
+        if (fuse) {
+          const ZBlock b[2] = {{blk.hx() + off, mu, hpu, np}, {blk.sx() + off, mu, spu, np}};
+          double2* const c[2] = {hs, ssb};
+          zgram(rt, n, {blk.x() + off, mu, pu, np}, b, c, 2, ord, true);
+          return;
+        }
+      }
       project_upper<R>(rt, n, mu, np, blk.x() + off, pu, blk.hx() + off, hpu, hs);
       project_upper<R>(rt, n, mu, np, blk.x() + off, pu, blk.sx() + off, spu, ssb);
     };
@@ -628,16 +666,15 @@ struct AccRun {
       ss.hegvd(hs, ssb, ord, wu, mu);
     }
     mark("hegvd");
-    to_r(hs, ord, blk.Y.get(), ord, ord, mu);
-    const C* ytop = blk.Y.get();
-    const C* ybot = blk.Y.get() + mu;
     int nx = blk.cur ^ 1;
-    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, mu, mu, one, blk.x() + off, n, ytop, ord, zero, blk.X[nx].get() + off, n);
-    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, mu, np, one, pu, n, ybot, ord, one, blk.X[nx].get() + off, n);
-    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, mu, mu, one, blk.hx() + off, n, ytop, ord, zero, blk.HX[nx].get() + off, n);
-    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, mu, np, one, hpu, n, ybot, ord, one, blk.HX[nx].get() + off, n);
-    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, mu, mu, one, blk.sx() + off, n, ytop, ord, zero, blk.SX[nx].get() + off, n);
-    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, mu, np, one, spu, n, ybot, ord, one, blk.SX[nx].get() + off, n);
+    if constexpr (sizeof(R) == 8) {
+      if (fuse) {
+        const ZBlock z[3] = {{blk.x() + off, mu, pu, np}, {blk.hx() + off, mu, hpu, np}, {blk.sx() + off, mu, spu, np}};
+        double2* const out[3] = {blk.X[nx].get() + off, blk.HX[nx].get() + off, blk.SX[nx].get() + off};
+        zupdate(rt, n, z, hs, ord, out, mu, 3, 1.0, 0.0);
+      }
+    }
+    if (!fuse) rotate(ord, mu, np, off, pu, hpu, spu, hs, nx);
     if (nl > 0) {   // locked columns go along unchanged
       const size_t bytes = size_t(off) * sizeof(C);
       HALF_CUDA(cudaMemcpyAsync(blk.X[nx].get(), blk.x(), bytes, cudaMemcpyDeviceToDevice, rt.stream));
@@ -648,12 +685,30 @@ struct AccRun {
     mark("rr_rot");
   }
 
+  // X[nx], HX[nx], SX[nx] from column offset off on = [X_U pu] Y and the same of H and S, Y = hs (ord x mu, FP64)
+  void rotate(int ord, int mu, int np, long long off, const C* pu, const C* hpu, const C* spu, const double2* hs,
+              int nx) {
+    const auto one = cval<R>(1.0), zero = cval<R>(0.0);
+    to_r(hs, ord, blk.Y.get(), ord, ord, mu);
+    const C* ytop = blk.Y.get();
+    const C* ybot = blk.Y.get() + mu;
+    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, mu, mu, one, blk.x() + off, n, ytop, ord, zero, blk.X[nx].get() + off, n);
+    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, mu, np, one, pu, n, ybot, ord, one, blk.X[nx].get() + off, n);
+    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, mu, mu, one, blk.hx() + off, n, ytop, ord, zero, blk.HX[nx].get() + off, n);
+    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, mu, np, one, hpu, n, ybot, ord, one, blk.HX[nx].get() + off, n);
+    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, mu, mu, one, blk.sx() + off, n, ytop, ord, zero, blk.SX[nx].get() + off, n);
+    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, mu, np, one, spu, n, ybot, ord, one, blk.SX[nx].get() + off, n);
+  }
+
   // S-metric normalisation of the np columns of P, HP, SP into PU, HPU, SPU
   // (src/half_cuda_iterative_solver.cuf:166-176)
   void normalise_metric(cplx_t<R> one, cplx_t<R> zero, int np) {
     double2* metric = sc.metric.get();
+    const bool fuse = fused(m + np);
     if constexpr (sizeof(R) == 8) {
-      gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, np, np, n, one, blk.P.get(), n, blk.SP.get(), n, zero, metric, np);
+      const ZBlock b = {blk.SP.get(), np};
+      if (fuse) zgram(rt, n, {blk.P.get(), np}, &b, &metric, 1, np, true);
+      else gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, np, np, n, one, blk.P.get(), n, blk.SP.get(), n, zero, metric, np);
     } else {
       gemm_to64(rt, CUBLAS_OP_C, CUBLAS_OP_N, np, np, n, blk.P.get(), n, blk.SP.get(), n, metric, np);
     }
@@ -664,6 +719,15 @@ struct AccRun {
       ++rt.prof.launches;
     }
     mark("heevd");
+    if constexpr (sizeof(R) == 8) {
+      if (fuse) {
+        const ZBlock z[3] = {{blk.P.get(), np}, {blk.HP.get(), np}, {blk.SP.get(), np}};
+        double2* const out[3] = {blk.PU.get(), blk.HPU.get(), blk.SPU.get()};
+        zupdate(rt, n, z, metric, np, out, np, 3, 1.0, 0.0);
+        mark("metric_rot");
+        return;
+      }
+    }
     to_r(metric, np, blk.small.get(), np, np, np);
     gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, np, one, blk.P.get(), n, blk.small.get(), np, zero, blk.PU.get(), n);
     gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, np, one, blk.HP.get(), n, blk.small.get(), np, zero, blk.HPU.get(), n);
