@@ -518,144 +518,288 @@ __global__ void hermitian_fill_kernel(double2* A, int n) {
 // the direction stays in the span without being eliminated from later
 // columns.
 //
-// One cluster of CTAs keeps the matrix in its shared memory, column j on CTA
-// j mod P, and makes ONE right-looking sweep that builds R^-1 together with R.
-// With T(i,j) = sum_{l<j} X(i,l) R(l,j) for i < j (X = R^-1), step k is
+// One right-looking sweep builds R^-1 together with R.  With
+// T(i,j) = sum_{l<j} X(i,l) R(l,j) for i < j (X = R^-1), step k is
 //   W(i,j) -= conj(W(k,i)) W(k,j) / p_k    k < i <= j   (trailing Schur complement)
 //   T(i,j) -= T(i,k) W(k,j) / p_k          i < k < j
 //   T(k,j)  = W(k,j) / p_k                 j > k         (row k becomes X(k,k) R(k,j))
 // with p_k = W(k,k): a rank-1 update of every column right of k.  The two
 // index ranges occupy disjoint rows of a column (rows <= k hold T, rows > k
 // hold W), and at the end X(i,j) = -T(i,j) / R(j,j), X(j,j) = 1 / R(j,j).
-// What a step needs from other CTAs is row k of W and column k of T; both are
-// pushed to every CTA in the step before, the row by each column's owner as it
-// updates the column, the column by its owner, whose threads update it
-// together first.  One cluster barrier per step and no other.
+//
+// Eight steps go together, so that the chain of barriers is one eighth as
+// long: column block K (8 columns, on CTA K mod P of a cluster that keeps
+// the packed upper triangle in its shared memory)
+//   1. its owner eliminates inside the block: one warp the 8 x 8 diagonal
+//      block, then one thread per row the rows above it;
+//   2. one thread per remaining column runs the eight pivot rows through the
+//      diagonal block (forward substitution), which gives the column's eight
+//      factors c_l and its entries of the block's rows;
+//   3. with F(l,i) = T(i, k0+l) above the block and conj W(k0+l, i) right of
+//      it, every remaining element loses sum_l F(l,i) c_l(j).
+// The panel F and the diagonal block travel through global memory (L2): one
+// writer and many readers, where pushes through distributed shared memory
+// cost 6-8 cycles per 16 bytes and target.  Two cluster barriers per block.
 // *status = 1 if a pivot was not finite.
 //
-// Bound by the chain of cluster barriers and shared-memory round trips.
-// Measured per solve at orders around 120 (12-atom cell, B200): one CTA with
-// the packed triangle 281 us; this kernel 235 us.
+// Bound by the chain: about 4 us a block.  Measured per solve at orders
+// around 120 (12-atom cell, B200): one CTA with the packed triangle, one
+// column per step, 281 us; a cluster with one column per step 235 us; this
+// kernel 135 us.
 constexpr int kClThreads = 256;
 constexpr int kClWarps = kClThreads / 32;
 constexpr int kClCols = 4;                        // columns a warp carries at once
+constexpr int kFB = 8;                            // columns per block of the metric factor
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
-__host__ __device__ inline size_t factor_smem(int m, int p) {
-  return (size_t((m + p - 1) / p) * m + 4 * size_t(m)) * sizeof(double2) + 2 * size_t(m) * sizeof(double);
-}
-
-__global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __restrict__ M, int m,
-                                                                   int* __restrict__ status) {
-  cg::cluster_group cl = cg::this_cluster();
-  const int P = int(cl.num_blocks()), rank = int(cl.block_rank());
-  const int nc = (m + P - 1) / P;
-  extern __shared__ __align__(16) double2 cols[];   // nc x m: column jl P + rank at cols + jl m
-  double2* gbuf = cols + size_t(nc) * m;            // 2 x m: row k of W, by parity of k
-  double2* tbuf = gbuf + 2 * m;                     // 2 x m: column k of T, by parity of k
-  double* dsc = reinterpret_cast<double*>(tbuf + 2 * m);   // D
-  double* ir = dsc + m;                                    // 1 / R(k,k)
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int j = tid; j < m; j += kClThreads) dsc[j] = 1.0 / sqrt(fmax(M[size_t(j) * m + j].x, DBL_MIN));
-  cl.sync();   // every CTA's buffers exist, dsc is filled
-  for (int jl = warp; jl * P + rank < m; jl += kClWarps) {
-    const int j = jl * P + rank;
-    const double dj = dsc[j];
-    for (int i = lane; i <= j; i += 32) {
-      double2 v = M[size_t(j) * m + i];
-      if (i == j) v.y = 0.0;
-      cols[size_t(jl) * m + i] = cscale(v, dsc[i] * dj);
-    }
-    __syncwarp();
-    if (lane < P) cl.map_shared_rank(gbuf, lane)[j] = cols[size_t(jl) * m];
-  }
-  cl.sync();
-  int bad = 0;
-  for (int k = 0; k < m; ++k) {
-    const double2* g = gbuf + (k & 1) * m;
-    const double2* tk = tbuf + (k & 1) * m;
-    double2* gn = gbuf + ((k + 1) & 1) * m;
-    double2* tn = tbuf + ((k + 1) & 1) * m;
-    const double p = g[k].x;
-    const bool dep = !(p > 1.0e-14);   // also true for NaN
-    const double invp = dep ? 0.0 : 1.0 / p;
-    if (!isfinite(p)) bad = 1;
-    if (tid == 0) ir[k] = dep ? 1.0e7 : 1.0 / sqrt(p);
-    // the step's update of element (i, column factor c): row k becomes c, the others lose a_i c
-    auto updated = [&](int i, double2 a, double2 x, double2 c) {
-      if (i == k) return c;
-      if (!dep) {
-        x.x -= a.x * c.x - a.y * c.y;
-        x.y -= a.x * c.y + a.y * c.x;
-      }
-      return x;
-    };
-    auto row_factor = [&](int i) {
-      if (i < k) return tk[i];                    // T(i, k)
-      const double2 w = g[i];
-      return make_double2(w.x, -w.y);             // conj W(k, i)
-    };
-    if (k + 1 < m && (k + 1) % P == rank) {   // the next pivot column, by the whole CTA
-      double2* col = cols + size_t((k + 1) / P) * m;
-      const double2 c = cscale(g[k + 1], invp);
-      for (int i = tid; i <= k + 1; i += kClThreads) {
-        const double2 x = updated(i, row_factor(i), col[i], c);
-        col[i] = x;
-        double2* dst = i <= k ? tn : gn;
-        for (int r = 0; r < P; ++r) cl.map_shared_rank(dst, r)[i] = x;
-      }
-    }
-    int jl0 = k + 2 > rank ? (k + 2 - rank + P - 1) / P : 0;   // first owned column right of k + 1
-    for (jl0 += warp; jl0 * P + rank < m; jl0 += kClWarps * kClCols) {
-      double2 c[kClCols];
-      int jj[kClCols];
-#pragma unroll
-      for (int q = 0; q < kClCols; ++q) {
-        jj[q] = (jl0 + q * kClWarps) * P + rank;
-        c[q] = jj[q] < m ? cscale(g[jj[q]], invp) : make_double2(0.0, 0.0);
-      }
-      const int jmax = min(m - 1, jj[kClCols - 1]);
-      for (int i = lane; i <= jmax; i += 32) {
-        const double2 a = row_factor(i);
-#pragma unroll
-        for (int q = 0; q < kClCols; ++q) {
-          if (i <= jj[q] && jj[q] < m) {
-            double2* e = cols + size_t(jl0 + q * kClWarps) * m + i;
-            *e = updated(i, a, *e, c[q]);
-          }
-        }
-      }
-      __syncwarp();
-      // row k + 1 of these columns to every CTA: eight lanes per column
-      {
-        const int q = lane >> 3, j = (jl0 + q * kClWarps) * P + rank;
-        if (j < m) {
-          const double2 v = cols[size_t(jl0 + q * kClWarps) * m + k + 1];
-          for (int r = lane & 7; r < P; r += 8) cl.map_shared_rank(gn, r)[j] = v;
-        }
-      }
-    }
+// Barrier of the P CTAs working on one matrix.
+__device__ __forceinline__ void group_barrier(int P) {
+  if (P == 1) {
+    __syncthreads();
+  } else {
     cluster_arrive();
     cluster_wait();
   }
+}
+
+// Packed column storage of CTA `rank`: its t-th block (block t P + rank of
+// the matrix) starts at this element and keeps 8 columns of 8 (t P + rank + 1) rows.
+__host__ __device__ inline size_t factor_base(int t, int P, int rank) {
+  return size_t(kFB) * kFB * (size_t(P) * t * (t - 1) / 2 + size_t(t) * (rank + 1));
+}
+
+__host__ inline size_t factor_smem(int m, int P) {
+  const int nblk = (m + kFB - 1) / kFB;
+  size_t most = 0;
+  for (int r = 0; r < P && r < nblk; ++r) most = std::max(most, factor_base((nblk - r + P - 1) / P, P, r));
+  const size_t cols = size_t((nblk + P - 1) / P) * kFB;
+  return (most + size_t(kFB) * m + kFB * cols + 3 * kFB * kFB) * sizeof(double2) + (2 * size_t(m) + kFB) * sizeof(double);
+}
+
+// Global scratch of the factor, in double2: the panel and the diagonal block, by parity of K.
+__host__ __device__ inline size_t factor_panel(int m) { return size_t(kFB) * m + 2 * kFB * kFB + kFB; }
+
+__global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __restrict__ M, int m, int P,
+                                                                   double2* __restrict__ panels,
+                                                                   int* __restrict__ status) {
+  const int rank = blockIdx.x;   // the grid is one cluster of P CTAs
+  const int nblk = (m + kFB - 1) / kFB, nown = nblk > rank ? (nblk - rank + P - 1) / P : 0;
+  const int maxown = (nblk + P - 1) / P * kFB;
+  extern __shared__ __align__(16) double2 cols[];
+  size_t most = 0;
+  for (int r = 0; r < P && r < nblk; ++r) {
+    const size_t s = factor_base((nblk - r + P - 1) / P, P, r);
+    if (s > most) most = s;
+  }
+  double2* F = cols + most;                                   // [kFB][m]
+  double2* sc = F + size_t(kFB) * m;                          // [kFB][maxown]: c_l of the owned columns
+  double2* sW = sc + size_t(kFB) * maxown;                    // [kFB][kFB]: W(k0+l, k0+c) before its scaling
+  double2* sC = sW + kFB * kFB;                               // [kFB][kFB]: c(l, c) inside the block
+  double2* sD = sC + kFB * kFB;                               // [kFB][kFB]: the block; at the end T inside it
+  double* dsc = reinterpret_cast<double*>(sD + kFB * kFB);    // D
+  double* ir = dsc + m;                                       // 1 / R(k,k) of the owned columns
+  double* sinv = ir + m;                                      // [kFB] 1 / p
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (rank == 0 && tid == 0) *status = 0;   // at least one group barrier lies before another CTA's flag
+  for (int j = tid; j < m; j += kClThreads) dsc[j] = 1.0 / sqrt(fmax(M[size_t(j) * m + j].x, DBL_MIN));
+  __syncthreads();
+  auto column_of = [&](int t, int c) {   // owned column c of block t P + rank
+    return cols + factor_base(t, P, rank) + size_t(c) * (size_t(kFB) * (t * P + rank + 1));
+  };
+  for (int q = warp; q < nown * kFB; q += kClWarps) {
+    const int t = q / kFB, c = q - t * kFB, j = (t * P + rank) * kFB + c;
+    if (j >= m) continue;
+    const double dj = dsc[j];
+    double2* col = column_of(t, c);
+    for (int i = lane; i <= j; i += 32) {
+      double2 v = M[size_t(j) * m + i];
+      if (i == j) v.y = 0.0;
+      col[i] = cscale(v, dsc[i] * dj);
+    }
+  }
+  __syncthreads();
+  int bad = 0;
+  for (int K = 0; K < nblk; ++K) {
+    const int k0 = K * kFB, kb = min(kFB, m - k0), k1 = k0 + kb, owner = K % P;
+    double2* panel = panels + (K & 1) * factor_panel(m);
+    double2* pdiag = panel + size_t(kFB) * m;   // sW, then T inside the block, then 1 / p
+    if (rank == owner) {
+      const int t = K / P;
+      if (warp == 0) {   // the diagonal block: element (r, c), r <= c, two per lane
+        for (int e = lane; e < kFB * kFB; e += 32) {
+          const int r = e >> 3, c = e & 7;
+          sD[e] = r <= c && c < kb ? column_of(t, c)[k0 + r] : make_double2(0.0, 0.0);
+          sW[e] = sC[e] = make_double2(0.0, 0.0);
+        }
+        __syncwarp();
+        for (int l = 0; l < kb; ++l) {
+          const double p = sD[l * kFB + l].x;
+          const bool dep = !(p > 1.0e-14);   // also true for NaN
+          const double invp = dep ? 0.0 : 1.0 / p;
+          double2 out[2];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int e = lane + 32 * h, r = e >> 3, c = e & 7;
+            double2 x = sD[e];
+            if (c > l && r <= c && c < kb) {
+              const double2 w = sD[l * kFB + c], f = cscale(w, invp);
+              if (r == l) {
+                x = f;
+              } else {
+                const double2 a = r < l ? sD[r * kFB + l] : make_double2(sD[l * kFB + r].x, -sD[l * kFB + r].y);
+                x = csub(x, cmul(a, f));
+              }
+            }
+            out[h] = x;
+          }
+          if (lane < kFB && lane > l) {
+            sW[l * kFB + lane] = sD[l * kFB + lane];
+            sC[l * kFB + lane] = cscale(sD[l * kFB + lane], invp);
+          }
+          if (lane == 0) {
+            if (!isfinite(p)) bad = 1;
+            sinv[l] = invp;
+            ir[k0 + l] = p;   // 1 / R(k,k) below
+          }
+          __syncwarp();
+          sD[lane] = out[0];
+          sD[lane + 32] = out[1];
+          __syncwarp();
+        }
+        if (lane < kb) {
+          const double p = ir[k0 + lane];
+          ir[k0 + lane] = !(p > 1.0e-14) ? 1.0e7 : 1.0 / sqrt(p);
+        }
+        for (int e = lane; e < kFB * kFB; e += 32) {
+          const int r = e >> 3, c = e & 7;
+          if (r < c && c < kb) column_of(t, c)[k0 + r] = sD[e];
+          if (P > 1) {
+            pdiag[e] = sW[e];
+            pdiag[kFB * kFB + e] = sD[e];
+          }
+        }
+        if (P > 1 && lane < kb) pdiag[2 * kFB * kFB + lane] = make_double2(sinv[lane], 0.0);
+      }
+      __syncthreads();
+      {
+        for (int i = tid; i < k0; i += kClThreads) {   // rows above the block
+          double2 tv[kFB];
+#pragma unroll
+          for (int l = 0; l < kFB; ++l) tv[l] = l < kb ? column_of(t, l)[i] : make_double2(0.0, 0.0);
+#pragma unroll
+          for (int l = 0; l < kFB; ++l)
+#pragma unroll
+            for (int c = l + 1; c < kFB; ++c) tv[c] = csub(tv[c], cmul(tv[l], sC[l * kFB + c]));
+#pragma unroll
+          for (int l = 0; l < kFB; ++l)
+            if (l < kb) {
+              column_of(t, l)[i] = tv[l];
+              if (P > 1) panel[size_t(l) * m + i] = tv[l];
+              else F[size_t(l) * m + i] = tv[l];
+            }
+        }
+      }
+    }
+    if (k1 >= m) break;   // the last block has no columns to its right
+    group_barrier(P);
+    if (rank != owner) {
+      for (int e = tid; e < kFB * kFB; e += kClThreads) {
+        sW[e] = __ldcg(pdiag + e);
+        sD[e] = __ldcg(pdiag + kFB * kFB + e);
+      }
+      if (tid < kFB) sinv[tid] = __ldcg(pdiag + 2 * kFB * kFB + tid).x;
+      __syncthreads();
+    }
+    // owned columns right of the block, one thread each (a full block: kb = kFB)
+    const int t0 = K + 1 > rank ? (K + 1 - rank + P - 1) / P : 0;   // first owned block right of K
+    for (int q = t0 * kFB + tid; q < nown * kFB; q += kClThreads) {
+      const int t = q / kFB, c = q - t * kFB, j = (t * P + rank) * kFB + c;
+      if (j >= m) continue;
+      double2* col = column_of(t, c) + k0;
+      double2 y[kFB], f[kFB];
+#pragma unroll
+      for (int l = 0; l < kFB; ++l) y[l] = col[l];
+#pragma unroll
+      for (int l = 0; l < kFB; ++l) {
+        f[l] = cscale(y[l], sinv[l]);
+#pragma unroll
+        for (int r = l + 1; r < kFB; ++r) y[r] = csub(y[r], cconjmul(sW[l * kFB + r], f[l]));
+      }
+#pragma unroll
+      for (int l = 0; l < kFB; ++l) {
+        sc[size_t(l) * maxown + q] = f[l];
+        const double2 w = make_double2(y[l].x, -y[l].y);
+        if (P > 1) panel[size_t(l) * m + j] = w;
+        else F[size_t(l) * m + j] = w;
+        double2 tv = f[l];
+#pragma unroll
+        for (int r = l + 1; r < kFB; ++r) tv = csub(tv, cmul(sD[l * kFB + r], f[r]));
+        col[l] = tv;
+      }
+    }
+    group_barrier(P);
+    if (P > 1) {
+      for (int e = tid; e < kFB * m; e += kClThreads) {
+        const int i = e % m;
+        if (i < k0 || i >= k1) F[e] = __ldcg(panel + e);
+      }
+      __syncthreads();
+    }
+    for (int q0 = t0 * kFB + warp; q0 < nown * kFB; q0 += kClWarps * kClCols) {
+      int jj[kClCols];
+      double2* col[kClCols];
+      int jmax = -1;
+#pragma unroll
+      for (int u = 0; u < kClCols; ++u) {
+        const int q = q0 + u * kClWarps, t = q / kFB, c = q - t * kFB;
+        const int j = (t * P + rank) * kFB + c;
+        jj[u] = q < nown * kFB && j < m ? j : -1;
+        col[u] = jj[u] >= 0 ? column_of(t, c) : cols;
+        jmax = max(jmax, jj[u]);
+      }
+      for (int i = lane; i <= jmax; i += 32) {
+        if (i >= k0 && i < k1) continue;
+        double2 f[kFB];
+#pragma unroll
+        for (int l = 0; l < kFB; ++l) f[l] = F[size_t(l) * m + i];
+#pragma unroll
+        for (int u = 0; u < kClCols; ++u) {
+          if (i <= jj[u]) {
+            double2 x = col[u][i];
+#pragma unroll
+            for (int l = 0; l < kFB; ++l) {
+              const double2 c = sc[size_t(l) * maxown + q0 + u * kClWarps];
+              x.x -= f[l].x * c.x - f[l].y * c.y;
+              x.y -= f[l].x * c.y + f[l].y * c.x;
+            }
+            col[u][i] = x;
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  __syncthreads();
   // U = D X with X(i,j) = -T(i,j) / R(j,j), X(j,j) = 1 / R(j,j); lower triangle zero
-  for (int jl = warp; jl * P + rank < m; jl += kClWarps) {
-    const int j = jl * P + rank;
+  for (int q = warp; q < nown * kFB; q += kClWarps) {
+    const int t = q / kFB, c = q - t * kFB, j = (t * P + rank) * kFB + c;
+    if (j >= m) continue;
     const double irj = ir[j];
+    const double2* col = column_of(t, c);
     for (int i = lane; i < m; i += 32) {
       double2 u = make_double2(0.0, 0.0);
-      if (i < j) u = cscale(cols[size_t(jl) * m + i], -irj * dsc[i]);
+      if (i < j) u = cscale(col[i], -irj * dsc[i]);
       else if (i == j) u = make_double2(irj * dsc[i], 0.0);
       M[size_t(j) * m + i] = u;
     }
   }
-  if (rank == 0 && tid == 0) *status = bad;
+  if (bad) atomicExch(status, 1);
 }
 
 __host__ __device__ inline size_t hetrd_smem(int n, int p) {
-  return (size_t((n + p - 1) / p) * n + 5 * size_t(n)) * sizeof(double2) + 2 * size_t(p) * kClWarps * sizeof(double);
+  return (size_t((n + p - 1) / p) * n + 6 * size_t(n)) * sizeof(double2);
 }
 
 // Householder reduction of a Hermitian A (n x n, upper triangle read) to the
@@ -672,30 +816,30 @@ __host__ __device__ inline size_t hetrd_smem(int n, int p) {
 //   forms u = A x with the unnormalised pivot column x, whose norm every warp
 //   sums on the way; with v = sc x + kappa e(i), kappa = 1 - sc x(i), the
 //   product the method needs is  A v = sc u + kappa A(:, i);
-// * each warp pushes its entries of u, and its share of q = x^H u, to every
-//   CTA, and forms tau, sc and kappa while the cluster barrier completes;
+// * each warp pushes its entries of u to every CTA, and forms tau, sc and
+//   kappa while the cluster barrier completes;
 // * then every CTA pulls column i from its owner and has all it needs:
-//   y = tau A v,  v^H A v = |sc|^2 q + 2 Re(conj(sc) kappa conj(u(i))) +
+//   q = x^H u,  y = tau A v,  v^H A v = |sc|^2 q + 2 Re(conj(sc) kappa conj(u(i))) +
 //   |kappa|^2 A(i,i),  w = y - (|tau|^2 v^H A v / 2) v  and the next pivot
 //   column A(:, i) - v conj(w(i)) - w.
 // All CTAs do the same arithmetic in the same order, so their copies agree
 // bit for bit.  Measured per solve at orders around 120 (12-atom cell, B200):
 // one CTA with the packed triangle 689 us; this kernel with three more block
-// barriers per step (norm, v and y^H v) 307 us; as it stands 297 us.
+// barriers per step (norm, v and y^H v) 307 us; as it stands 270 us.
 constexpr int kTrdRows = 2;                        // rows of a vector per thread
 static_assert(SmallEigen::kOwnMaxOrder <= kTrdRows * kClThreads, "rows of a vector per thread");
 
 __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__ A, int n, double* __restrict__ dout,
                                                            double* __restrict__ eout, double2* __restrict__ tauout) {
   cg::cluster_group cl = cg::this_cluster();
-  const int P = int(cl.num_blocks()), rank = int(cl.block_rank());
+  const int P = int(cl.num_blocks()), rank = int(cl.block_rank());   // P is a power of two
+  const int lg = 31 - __clz(P);
   const int nc = (n + P - 1) / P;
   extern __shared__ __align__(16) double2 cols[];   // nc x n: column jl P + rank at cols + jl n
   double2* ubuf = cols + size_t(nc) * n;            // 2 x n: A x, by parity of the step
-  double2* xbuf = ubuf + 2 * n;                     // n: the pivot column
-  double2* vbuf = xbuf + n;                         // n: the previous step's v and w
+  double2* xbufs = ubuf + 2 * n;                    // 2 x n: the pivot column
+  double2* vbuf = xbufs + 2 * n;                    // n: the previous step's v and w
   double2* wbuf = vbuf + n;
-  double* qbuf = reinterpret_cast<double*>(wbuf + n);   // 2 x P kClWarps: shares of x^H A x
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int jl = warp; jl * P + rank < n; jl += kClWarps) {
     const int j = jl * P + rank;
@@ -710,7 +854,7 @@ __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__
   cl.sync();
   double2 x[kTrdRows];   // the pivot column, rows tid + kClThreads t
   {
-    const double2* c = cl.map_shared_rank(cols, (n - 1) % P) + size_t((n - 1) / P) * n;
+    const double2* c = cl.map_shared_rank(cols, (n - 1) & (P - 1)) + size_t((n - 1) >> lg) * n;
 #pragma unroll
     for (int t = 0; t < kTrdRows; ++t) {
       const int r = tid + kClThreads * t;
@@ -720,6 +864,7 @@ __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__
   int par = 0;
   for (int i0 = n - 2; i0 >= 0; --i0, par ^= 1) {
     const int c = i0 + 1, L = i0 + 1;
+    double2* xbuf = xbufs + par * n;
 #pragma unroll
     for (int t = 0; t < kTrdRows; ++t) {
       const int r = tid + kClThreads * t;
@@ -729,8 +874,7 @@ __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__
     __syncthreads();   // xbuf, vbuf, wbuf
     // columns s < L: the previous rank-2 update, then u(s) = sum_r conj(A(r, s)) x(r)
     double2* u = ubuf + par * n;
-    double* qp = qbuf + par * P * kClWarps;
-    double norm = 0, q = 0;
+    double norm = 0;
     bool first = true;
     int jl0 = warp;
     do {   // at least once: every warp needs the norm
@@ -768,16 +912,11 @@ __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__
       const int s = (jl0 + (lane >> 3) * kClWarps) * P + rank;          // eight lanes per column push
       if (s < L) {
         for (int r = lane & 7; r < P; r += 8) cl.map_shared_rank(u, r)[s] = us;
-        const double2 xs = xbuf[s];
-        q += xs.x * us.x + xs.y * us.y;   // Re(conj(x) u)
       }
       jl0 += kClWarps * kClCols;
     } while (jl0 * P + rank < L);
-    q += __shfl_xor_sync(0xffffffffu, q, 8);
-    q += __shfl_xor_sync(0xffffffffu, q, 16);
-    if (lane < P) cl.map_shared_rank(qp, lane)[rank * kClWarps + warp] = q;
     const double2 al = xbuf[i0];
-    cluster_arrive();   // this thread is done with x, v and w in shared memory
+    cluster_arrive();   // this thread is done with v and w in shared memory
     for (int off = 16; off > 0; off >>= 1) norm += __shfl_xor_sync(0xffffffffu, norm, off);
     double2 tau = make_double2(0.0, 0.0), sc = make_double2(1.0, 0.0);
     double beta = al.x;
@@ -796,7 +935,7 @@ __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__
       tauout[i0] = tau;
     }
     cluster_wait();
-    const double2* next = cl.map_shared_rank(cols, i0 % P) + size_t(i0 / P) * n;
+    const double2* next = cl.map_shared_rank(cols, i0 & (P - 1)) + size_t(i0 >> lg) * n;
     double2 ur[kTrdRows], ar[kTrdRows];
 #pragma unroll
     for (int t = 0; t < kTrdRows; ++t) {
@@ -806,7 +945,10 @@ __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__
     }
     const double2 ai = next[i0], ui = u[i0];
     double qs = 0;
-    for (int k = lane; k < P * kClWarps; k += 32) qs += qp[k];
+    for (int r = lane; r < L; r += 32) {
+      const double2 a = xbuf[r], b = u[r];
+      qs += a.x * b.x + a.y * b.y;   // Re(conj(x) u)
+    }
     for (int off = 16; off > 0; off >>= 1) qs += __shfl_xor_sync(0xffffffffu, qs, off);
     const double2 sk = cconjmul(sc, kap);   // conj(sc) kappa
     const double vav = sc2 * qs + 2.0 * (sk.x * ui.x + sk.y * ui.y) + (kap.x * kap.x + kap.y * kap.y) * ai.x;
@@ -818,7 +960,7 @@ __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__
       const int r = tid + kClThreads * t;
       if (r <= i0) {
         const double2 v = r < i0 ? cmul(x[t], sc) : make_double2(1.0, 0.0);
-        if (r < i0 && rank == c % P) A[size_t(c) * n + r] = v;
+        if (r < i0 && rank == (c & (P - 1))) A[size_t(c) * n + r] = v;
         double2 w = cadd(cmul(tsc, ur[t]), cmul(tkap, ar[t]));
         w.x += a2 * v.x;
         w.y += a2 * v.y;
@@ -833,14 +975,13 @@ __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__
   cl.sync();   // no CTA leaves while another may still read its columns
 }
 
-// CTAs of the cluster for an order-n reduction: the fewest that hold it, but
-// at least enough for about 12 columns each (below that the barrier costs
-// more than the pass saves), up to 16; 0 when it does not fit.
-int cluster_ctas(int n) {
-  for (int p = n <= 40 ? 1 : n <= 80 ? 4 : n <= 176 ? 8 : 16; p <= 16; p *= 2)
-    if (std::max(hetrd_smem(n, p), factor_smem(n, p)) <= kSmemMax) return p;
-  return 0;
-}
+// CTAs of the cluster for an order-n tridiagonalisation: measured best at 8
+// from order 40 to 176 (order 80: 1, 2, 4, 8 and 16 CTAs 283, 218, 192, 183
+// and 191 us); beyond, the shared memory of 16.
+int hetrd_ctas(int n) { return n <= 40 ? 4 : n <= 176 ? 8 : 16; }
+
+// CTAs for an order-m metric factor: one while its panel update is short.
+int factor_ctas(int m) { return m <= 64 ? 1 : m <= 176 ? 8 : 16; }
 
 template <typename... KArgs, typename... Args>
 void launch_cluster(void (*kernel)(KArgs...), int ctas, size_t smem, cudaStream_t s, Args... args) {
@@ -945,7 +1086,7 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
   reserve(rt, n);
   cudaStream_t s = rt.stream;
   if (n <= kOwnMaxOrder) {   // whole reduction in one cluster
-    const int p = cluster_ctas(n);
+    const int p = hetrd_ctas(n);
     launch_cluster(hetrd_kernel, p, hetrd_smem(n, p), s, A, n, d.get(), e.get(), tau.get());
     rt.prof.launches += 1;
   } else {
@@ -1059,8 +1200,9 @@ void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, doubl
 // metric_factor_kernel); false when m is beyond the cluster's shared memory.
 bool SmallEigen::metric_normalize(Runtime& rt, double2* M, int m, int* status) {
   if (m > kOwnMaxOrder) return false;
-  const int p = cluster_ctas(m);
-  launch_cluster(metric_factor_kernel, p, factor_smem(m, p), rt.stream, M, m, status);
+  const int p = factor_ctas(m);
+  if (panels.size() < 2 * factor_panel(m)) panels.resize(2 * factor_panel(kOwnMaxOrder));
+  launch_cluster(metric_factor_kernel, p, factor_smem(m, p), rt.stream, M, m, p, panels.get(), status);
   rt.prof.launches += 1;
   return true;
 }

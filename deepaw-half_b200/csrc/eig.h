@@ -14,6 +14,7 @@ struct SmallEigen {
   int cap = 0;
   DeviceBuffer<double> d, e, Z, scratch, lam;
   DeviceBuffer<double2> tau, V, work;
+  DeviceBuffer<double2> panels;   // exchange buffer of the metric factor's CTAs
   DeviceBuffer<int> info;   // zhetrd status (reports illegal arguments only)
   void reserve(Runtime& rt, int nmax);
   // A (n x n, upper triangle) -> nev lowest eigenpairs; vectors overwrite
