@@ -422,9 +422,9 @@ struct AccRun {
   long long op_cols = 0;
   Tracer* tr = nullptr;
   void mark(const char* s) { if (tr) tr->mark(s); }
-  // FP64 blocks of the small cells: the iteration's products through the fused block kernels
-  bool fused(int order) const {
-    if constexpr (sizeof(R) == 8) return zblock_fused(n, order);
+  // the FP64 iteration's products through the block kernels (blockops.h)
+  bool fused(int order, int cols) const {
+    if constexpr (sizeof(R) == 8) return zblock_fused(n, order, cols);
     return false;
   }
 
@@ -455,7 +455,7 @@ struct AccRun {
     double2* ssb = sc.ssub.get();
     int nx = blk.cur ^ 1;
     if constexpr (sizeof(R) == 8) {
-      if (fused(m)) {
+      if (fused(m, m)) {
         const ZBlock b[2] = {{blk.hx(), m}, {blk.sx(), m}};
         double2* const c[2] = {hs, ssb};
         zgram(rt, n, {blk.x(), m}, b, c, 2, m, true);
@@ -493,7 +493,7 @@ struct AccRun {
     HALF_CUDA(cudaMemcpyAsync(wh.data(), sc.w.get(), m * sizeof(double), cudaMemcpyDeviceToHost, rt.stream));
     ss.status_async(infos);
     HALF_CUDA(cudaStreamSynchronize(rt.stream));
-    if constexpr (sizeof(R) == 4) tc_check(rt);
+    if (sizeof(R) == 4 || rt.crt_pending) tc_check(rt);
     mark("residual");
     if (infos[0] != 0) fail(kInternal, "ACC correction metric eigensolve failed (info " + std::to_string(infos[0]) + ")");
     if (infos[1] != 0) fail(kInternal, "ACC small generalized eigensolve failed (info " + std::to_string(infos[1]) + ")");
@@ -583,7 +583,7 @@ struct AccRun {
     mark("precondition");
     apply(blk.P.get(), blk.HP.get(), blk.SP.get(), np);
     mark("apply");
-    const bool fuse = fused(m + np);
+    const bool fuse = fused(m - nl + np, m - nl);
     // S-orthogonalise against X
     if constexpr (sizeof(R) == 8) {
       if (fuse) {
@@ -704,7 +704,7 @@ struct AccRun {
   // (src/half_cuda_iterative_solver.cuf:166-176)
   void normalise_metric(cplx_t<R> one, cplx_t<R> zero, int np) {
     double2* metric = sc.metric.get();
-    const bool fuse = fused(m + np);
+    const bool fuse = fused(m + np, np);
     if constexpr (sizeof(R) == 8) {
       const ZBlock b = {blk.SP.get(), np};
       if (fuse) zgram(rt, n, {blk.P.get(), np}, &b, &metric, 1, np, true);

@@ -151,6 +151,10 @@ void end_call(Runtime& rt, SolveInfo& info) {
   Profile& pf = rt.prof;
   HALF_CUDA(cudaEventRecord(pf.b, rt.stream));
   HALF_CUDA(cudaEventSynchronize(pf.b));
+  if (rt.crt_pending) tc_check(rt);
+  // The residue planes go back to the thread's cache (the call's work is
+  // done): gigabytes that the next context's first call finds there.
+  for (auto* b : {&rt.crt_a, &rt.crt_b, &rt.crt_res}) b->release();
   float ms = 0;
   HALF_CUDA(cudaEventElapsedTime(&ms, pf.a, pf.b));
   pf.collect();
@@ -414,6 +418,7 @@ int half_assemble_hs(half_handle handle, const double kpoint[3], int64_t ld, HAL
     if (ld < n) fail(kCapacity, "matrix leading dimension is too small");
     DeviceBuffer<double2> dh((size_t)n * n), ds((size_t)n * n);
     assemble_dense(*ctx, *ks, dh.get(), ds.get());
+    if (ctx->rt->crt_pending) tc_check(*ctx->rt);
     cudaStream_t st = ctx->rt->stream;
     block_to_host(h, ld, dh.get(), n, n, st);
     block_to_host(s, ld, ds.get(), n, n, st);

@@ -20,6 +20,7 @@
 #include <algorithm>
 
 #include "blockops.h"
+#include "zcrt.h"
 
 namespace hb {
 
@@ -263,9 +264,28 @@ __global__ void __launch_bounds__(kUpThreads) zupdate_kernel(UpdateArgs u) {
 // FP64 solves (cuBLAS / fused, ms): 2-atom cell, order 32: 144 / 133; 12-atom
 // cell, orders 80, 160 and 300: 16.8 / 14.8, 19.8 / 19.3, 31.3 / 32.3; 64-atom
 // cell, orders 150 and 400: 60.5 / 60.6, 121 / 135.
-bool zblock_fused(int n, int order) {
-  return double(n) * order * order < 2.0e8;
+bool zblock_small(int n, int order) { return double(n) * order * order < 2.0e8; }
+
+bool zblock_fused(int n, int order, int cols) {
+  return zblock_small(n, order) || (zcrt_serves(order, order, n) && zcrt_serves(n, cols, order));
 }
+
+namespace {
+
+CrtSide side_of(const ZBlock& b, int n, bool k_is_rows, bool conj) {
+  CrtSide s;
+  s.p = b.p1;
+  s.p2 = b.p2;
+  s.split = b.c2 > 0 ? b.c1 : INT32_MAX;
+  s.ld = n;
+  s.rows = k_is_rows ? b.cols() : n;
+  s.k = k_is_rows ? n : b.cols();
+  s.kcontig = k_is_rows;
+  s.conj = conj;
+  return s;
+}
+
+}  // namespace
 
 void zgram(Runtime& rt, int n, const ZBlock& a, const ZBlock* b, double2* const* c, int count, int ldc, bool upper) {
   GramArgs g{};
@@ -276,6 +296,14 @@ void zgram(Runtime& rt, int n, const ZBlock& a, const ZBlock* b, double2* const*
   g.cols = b[0].cols();
   g.upper = upper;
   if (g.rows <= 0 || g.cols <= 0) return;
+  if (!zblock_small(n, std::max(g.rows, g.cols)) && zcrt_serves(g.rows, g.cols, n)) {
+    const CrtPlanes pa = crt_prepare(rt, side_of(a, n, true, true), false, rt.crt_a);   // shared by the products
+    for (int i = 0; i < count; ++i) {
+      const CrtPlanes pb = crt_prepare(rt, side_of(b[i], n, true, false), true, rt.crt_b);
+      crt_product(rt, pa, pb, make_double2(1, 0), make_double2(0, 0), c[i], ldc, upper);
+    }
+    return;
+  }
   for (int i = 0; i < count; ++i) {
     g.b[i] = b[i];
     g.c[i] = c[i];
@@ -305,6 +333,20 @@ void zgram(Runtime& rt, int n, const ZBlock& a, const ZBlock* b, double2* const*
 void zupdate(Runtime& rt, int n, const ZBlock* z, const double2* y, int ldy, double2* const* c, int cols, int count,
              double alpha, double beta) {
   if (n <= 0 || cols <= 0) return;
+  if (!zblock_small(n, std::max(cols, z[0].cols())) && zcrt_serves(n, cols, z[0].cols())) {
+    CrtSide ys;
+    ys.p = y;
+    ys.ld = ldy;
+    ys.rows = cols;
+    ys.k = z[0].cols();
+    ys.kcontig = true;
+    const CrtPlanes py = crt_prepare(rt, ys, true, rt.crt_b);   // shared by the blocks
+    for (int i = 0; i < count; ++i) {
+      const CrtPlanes pz = crt_prepare(rt, side_of(z[i], n, false, false), false, rt.crt_a);
+      crt_product(rt, pz, py, make_double2(alpha, 0), make_double2(beta, 0), c[i], n);
+    }
+    return;
+  }
   UpdateArgs u{};
   for (int i = 0; i < count; ++i) {
     u.z[i] = z[i];

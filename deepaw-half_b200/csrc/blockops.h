@@ -28,7 +28,9 @@ void zupdate(Runtime& rt, int n, const ZBlock* z, const double2* y, int ldy, dou
              double alpha, double beta);
 
 // Whether the products of an n-row iteration with pencils of order `order`
-// go through these kernels rather than cuBLAS.
-bool zblock_fused(int n, int order);
+// (blocks of up to `cols` columns) go through zgram and zupdate rather than
+// ZGEMM calls: small ones on their FP64 kernels, large ones on the integer
+// tensor cores (zcrt.cu).
+bool zblock_fused(int n, int order, int cols);
 
 }  // namespace hb

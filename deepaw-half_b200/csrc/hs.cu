@@ -34,6 +34,7 @@
 #include "blas.h"
 #include "context.h"
 #include "tune.h"
+#include "zcrt.h"
 
 namespace hb {
 
@@ -49,6 +50,10 @@ struct KOperator {
   DeviceBuffer<C> work;      // chunk x nplanes x n2 x n3
   int work_chunk = 0;
   DeviceBuffer<C> B;         // FP64: npw x np, column-major
+  // FP64: B^H and B in the residue planes of the integer product, made by the
+  // first application large enough to use them
+  DeviceBuffer<unsigned char> crt_bh_store, crt_b_store;
+  CrtPlanes crt_bh, crt_b;
   // FP32: the projector matrix is generated from these tables straight into
   // the bf16 planes of the tensor-core GEMM (tc_gemm.cu), once per k point,
   // in the two orientations the products use
@@ -855,6 +860,39 @@ void apply_nonlocal(Runtime& rt, KOperator<R>& op, const cplx_t<R>* x, long long
     y.split = nb;
     tc_cgemm(rt, op.b_planes, y, op.npw, 2 * nb, op.np, make_double2(1, 0), make_double2(1, 0), hx, false, ld, sx, nb);
   } else {
+    const bool kept = op.crt_bh.planes != nullptr;
+    if (zcrt_serves(op.np, nb, op.npw, kept) && zcrt_serves(op.npw, 2 * nb, op.np, kept)) {
+      // coeff = B^H X, [H X | S X] += B [DY | QY] on the integer tensor cores
+      CrtSide s;
+      s.ld = op.npw;
+      if (!kept) {
+        s.p = op.B.get();
+        s.rows = op.np;
+        s.k = op.npw;
+        s.kcontig = s.conj = true;
+        op.crt_bh = crt_prepare(rt, s, false, op.crt_bh_store);
+        s.rows = op.npw;
+        s.k = op.np;
+        s.kcontig = s.conj = false;
+        op.crt_b = crt_prepare(rt, s, false, op.crt_b_store);
+      }
+      s.p = x;
+      s.ld = ld;
+      s.rows = nb;
+      s.k = op.npw;
+      s.kcontig = true;
+      s.conj = false;
+      crt_product(rt, op.crt_bh, crt_prepare(rt, s, true, rt.crt_b), one, zero, op.coeff.get(), op.np);
+      mix();
+      s.p = op.dy.get();
+      s.p2 = op.qy.get();
+      s.split = nb;
+      s.ld = op.np;
+      s.rows = 2 * nb;
+      s.k = op.np;
+      crt_product(rt, op.crt_b, crt_prepare(rt, s, true, rt.crt_b), one, one, hx, ld, false, sx, nb);
+      return;
+    }
     gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, op.np, nb, op.npw, one, op.B.get(), op.npw, x, ld, zero, op.coeff.get(), op.np);
     mix();
     gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, op.npw, nb, op.np, one, op.B.get(), op.npw, op.dy.get(), op.np, one, hx, ld);

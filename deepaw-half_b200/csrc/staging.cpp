@@ -29,7 +29,7 @@ namespace {
 
 constexpr size_t kPiece = size_t(2) << 20;      // bytes of a pinned buffer
 constexpr size_t kMinPiece = size_t(256) << 10; // smallest piece worth a thread
-constexpr size_t kMinBytes = size_t(1) << 20;   // below this the driver's path is as fast
+constexpr size_t kMinBytes = size_t(8) << 20;    // below this the driver's path is faster (2 MB blocks: 165 against 310 us)
 constexpr int kThreads = 8;                     // pieces in flight per copy
 constexpr int kMaxSlots = 4 * kThreads;         // 64 MB of pinned memory: four copies at once
 

@@ -673,6 +673,7 @@ TcOperand tc_presplit_a(Runtime& rt, const TcOperand& op, DeviceBuffer<unsigned 
 }
 
 void tc_check(Runtime& rt) {
+  rt.crt_pending = false;
   if (rt.tc_err.size() == 0) return;
   int flag = 0;
   HALF_CUDA(cudaMemcpyAsync(&flag, rt.tc_err.get(), sizeof(int), cudaMemcpyDeviceToHost, rt.stream));
