@@ -89,10 +89,17 @@ __global__ void init_states_kernel(C* x, long long ld, int n, int m, const int* 
   x[(long long)j * ld + i] = v;
 }
 
-// norms[j] = || H x_j - eps_j S x_j ||  (one block per band, FP64 accumulation)
+// norms[j] = || H x_j - eps_j S x_j ||  (one block per band, FP64 accumulation).
+// report: what the host reads once per iteration, in one copy: the norms, the
+// Ritz values, the three solver status words and the tensor-core error flag.
 template <typename C>
 __global__ void residual_norm_kernel(const C* __restrict__ hx, const C* __restrict__ sx, long long ld, int n,
-                                     const double* __restrict__ eps, double* __restrict__ norms) {
+                                     const double* __restrict__ eps, const int* __restrict__ info,
+                                     const int* __restrict__ tc_err, double* __restrict__ norms,
+                                     double* __restrict__ report) {
+  if (blockIdx.x == 0 && threadIdx.x < 4)
+    report[2 * gridDim.x + threadIdx.x] =
+        threadIdx.x < 3 ? double(info[threadIdx.x]) : tc_err ? double(*tc_err) : 0.0;
   const int j = blockIdx.x;
   const double e = eps[j];
   const C* h = hx + (long long)j * ld;
@@ -110,7 +117,12 @@ __global__ void residual_norm_kernel(const C* __restrict__ hx, const C* __restri
     int nw = blockDim.x >> 5;
     acc = threadIdx.x < nw ? red[threadIdx.x] : 0.0;
     for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
-    if (threadIdx.x == 0) norms[j] = sqrt(fmax(0.0, acc));
+    if (threadIdx.x == 0) {
+      const double v = sqrt(fmax(0.0, acc));
+      norms[j] = v;
+      report[j] = v;
+      report[gridDim.x + j] = e;
+    }
   }
 }
 
@@ -345,10 +357,6 @@ struct SmallSolver {
                                     info.get() + 1),
                    "zhegvd");
   }
-  // status words of the last solves -> host (three ints: metric, Rayleigh-Ritz, its Cholesky factor)
-  void status_async(int* host) {
-    HALF_CUDA(cudaMemcpyAsync(host, info.get(), 3 * sizeof(int), cudaMemcpyDeviceToHost, rt.stream));
-  }
 };
 
 // Block state of one precision.
@@ -376,7 +384,7 @@ struct Blocks {
 
 struct Scratch64 {
   DeviceBuffer<double2> metric, hsub, ssub;   // m x m, 2m x 2m, 2m x 2m
-  DeviceBuffer<double> w, mu, norms, kinetic, jacobi;
+  DeviceBuffer<double> w, mu, norms, kinetic, jacobi, report;
   DeviceBuffer<int> idx, active, perm;
 };
 
@@ -418,7 +426,6 @@ struct AccRun {
   int nl = 0;                  // hard-locked columns, at the front of X, H X, S X
   std::vector<double> wh;      // Ritz values (host copy, physical column order)
   std::vector<int> req;        // requested bands: physical columns of the mcheck lowest Ritz values
-  double op_ms = 0;
   long long op_cols = 0;
   Tracer* tr = nullptr;
   void mark(const char* s) { if (tr) tr->mark(s); }
@@ -428,12 +435,10 @@ struct AccRun {
     return false;
   }
 
+  // (timed by the sweep's events: no host synchronisation)
   void apply(const C* x, C* hx, C* sx, int nb) {
-    auto t0 = std::chrono::steady_clock::now();
     apply_hs<R>(ctx, ks, x, n, nb, hx, sx, chunk);
     op_cols += nb;
-    HALF_CUDA(cudaStreamSynchronize(rt.stream));
-    op_ms += ms_since(t0);
   }
 
   // small FP64 matrices -> this precision
@@ -484,16 +489,19 @@ struct AccRun {
   // requested bands, which are the mcheck lowest Ritz values (req, physical
   // column indices in ascending order of their values; host sync)
   double residuals(std::vector<double>& norms, int* infos) {
-    residual_norm_kernel<C><<<m, 256, 0, rt.stream>>>(blk.hx(), blk.sx(), n, n, sc.w.get(), sc.norms.get());
+    residual_norm_kernel<C><<<m, 256, 0, rt.stream>>>(blk.hx(), blk.sx(), n, n, sc.w.get(), ss.info.get(),
+                                                      rt.tc_err.get(), sc.norms.get(), sc.report.get());
     ++rt.prof.launches;
     HALF_LAUNCH("residual norms");
-    norms.resize(m);
-    wh.resize(m);
-    HALF_CUDA(cudaMemcpyAsync(norms.data(), sc.norms.get(), m * sizeof(double), cudaMemcpyDeviceToHost, rt.stream));
-    HALF_CUDA(cudaMemcpyAsync(wh.data(), sc.w.get(), m * sizeof(double), cudaMemcpyDeviceToHost, rt.stream));
-    ss.status_async(infos);
+    const size_t words = size_t(2) * m + 4;
+    double* host = rt.pinned(words);
+    HALF_CUDA(cudaMemcpyAsync(host, sc.report.get(), words * sizeof(double), cudaMemcpyDeviceToHost, rt.stream));
     HALF_CUDA(cudaStreamSynchronize(rt.stream));
-    if (sizeof(R) == 4 || rt.crt_pending) tc_check(rt);
+    norms.assign(host, host + m);
+    wh.assign(host + m, host + 2 * m);
+    for (int i = 0; i < 3; ++i) infos[i] = int(host[2 * m + i]);
+    if (host[2 * m + 3] != 0.0) tc_check(rt);   // raises
+    rt.crt_pending = false;
     mark("residual");
     if (infos[0] != 0) fail(kInternal, "ACC correction metric eigensolve failed (info " + std::to_string(infos[0]) + ")");
     if (infos[1] != 0) fail(kInternal, "ACC small generalized eigensolve failed (info " + std::to_string(infos[1]) + ")");
@@ -771,6 +779,7 @@ void solve_acc(Context& ctx, KOperatorSet& ks, int nbands, bool want_vectors, So
   sc.jacobi.resize(2 * m);
   sc.mu.resize(m);
   sc.norms.resize(m);
+  sc.report.resize(2 * size_t(m) + 4);
   sc.kinetic.upload(ks.basis.kinetic, rt.stream);
   auto order = kinetic_order(ks.basis.kinetic);
   order.resize(m);
@@ -833,7 +842,6 @@ void solve_acc(Context& ctx, KOperatorSet& ks, int nbands, bool want_vectors, So
   int iter = 0, fp64_iter = 0;
   bool converged = false;
   double max_res = HUGE_VAL;
-  double op_ms = 0;
   long long op_cols = 0;
 
   int fallbacks = 0;
@@ -875,7 +883,6 @@ void solve_acc(Context& ctx, KOperatorSet& ks, int nbands, bool want_vectors, So
       advance(run32, lock_frac * switch_tol);
     }
     if (iter > cfg.max_iter) iter = cfg.max_iter;
-    op_ms += run32.op_ms;
     op_cols += run32.op_cols;
     fallbacks += run32.metric_fallbacks;
     // promote X, recreate H X and S X in FP64, Rayleigh-Ritz
@@ -905,7 +912,6 @@ void solve_acc(Context& ctx, KOperatorSet& ks, int nbands, bool want_vectors, So
     iter = std::min(iter, cfg.max_iter);
     fp64_iter = iter;
   }
-  op_ms += run64.op_ms;
   op_cols += run64.op_cols;
   fallbacks += run64.metric_fallbacks;
   // the requested eigenpairs in ascending order (req: physical columns, from
@@ -937,7 +943,6 @@ void solve_acc(Context& ctx, KOperatorSet& ks, int nbands, bool want_vectors, So
   info.max_residual = max_res;
   info.npw = n;
   info.operator_columns = op_cols;
-  info.operator_ms = op_ms;
   info.solve_ms = ms_since(t_start);
   if (!converged && max_res > std::max(100.0 * cfg.tol, 1e-2))
     std::fprintf(stderr, "HALF ACC warning: stopped after %d iterations; max residual=%12.4E\n", cfg.max_iter, max_res);

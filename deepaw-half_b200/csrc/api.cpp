@@ -191,6 +191,7 @@ void solve_one(Context& ctx, Runtime& rt, const double k[3], int nbands, bool wa
   info.setup_ms = setup_ms;
   info.npw = ks->basis.npw();
   end_call(rt, info);
+  info.operator_ms = info.sweep_ms;
   if (keep) *keep = std::move(ks);
 }
 

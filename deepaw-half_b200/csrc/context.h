@@ -72,6 +72,7 @@ struct Runtime {
   cudaStream_t stream = nullptr;
   cublasHandle_t blas = nullptr;
   cusolverDnHandle_t solver = nullptr;
+  int sms = 148;         // multiprocessors of the stream's device
   bool bf16x9 = false;   // cuBLAS offers FP32 emulation on BF16 tensor cores
   bool tc_gemm = true;   // complex FP32 GEMMs on the library's tcgen05 kernel (tc_gemm.cu)
   DeviceBuffer<unsigned char> tc_work;   // its split-K partial sums, grow-only
@@ -81,10 +82,15 @@ struct Runtime {
   bool crt_pending = false;              // such products ran since the last tc_check
   DeviceBuffer<int> tc_err;              // raised when one of its pipeline waits gave up
   Profile prof;
+  double* pinned(size_t words);          // host staging of small results, grow-only, page-locked
   Runtime();
   ~Runtime();
   Runtime(const Runtime&) = delete;
   Runtime& operator=(const Runtime&) = delete;
+
+ private:
+  double* pinned_ = nullptr;
+  size_t pinned_words_ = 0;
 };
 
 // Plane-wave basis (src/half_basis.F90:9-55); fft_index is 0-based C order.

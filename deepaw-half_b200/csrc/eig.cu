@@ -32,6 +32,7 @@
 #include <string>
 
 #include "blas.h"
+#include "blockops.h"
 #include "context.h"
 #include "eig.h"
 
@@ -975,6 +976,11 @@ __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__
   cl.sync();   // no CTA leaves while another may still read its columns
 }
 
+// Orders whose congruence and final rotation go through the block kernels
+// (blockops.h) instead of ZGEMM with its split-K reductions: two to four
+// launches fewer, while one product does not fill the GPU.
+constexpr int kSmallProducts = 176;
+
 // CTAs of the cluster for an order-n tridiagonalisation: measured best at 8
 // from order 40 to 176 (order 80: 1, 2, 4, 8 and 16 CTAs 283, 218, 192, 183
 // and 191 us); beyond, the shared memory of 16.
@@ -1080,8 +1086,8 @@ void SmallEigen::reserve(Runtime& rt, int nmax) {
   work.resize(size_t(std::max({l1, l2, l3, 1})));
 }
 
-// Hermitian eigenproblem of A (n x n, upper triangle used); the nev lowest
-// eigenvectors overwrite A[:, :nev], eigenvalues go to w.
+// Hermitian eigenproblem of A (n x n, upper triangle used, destroyed); the nev
+// lowest eigenvectors go to V[:, :nev] (leading dimension n), eigenvalues to w.
 void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* status) {
   reserve(rt, n);
   cudaStream_t s = rt.stream;
@@ -1133,7 +1139,6 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
                                     reinterpret_cast<cuDoubleComplex*>(V.get()), n,
                                     reinterpret_cast<cuDoubleComplex*>(work.get()), int(work.size()), info.get()),
                    "zunmtr");
-    HALF_CUDA(cudaMemcpyAsync(A, V.get(), size_t(n) * nev * sizeof(double2), cudaMemcpyDeviceToDevice, s));
     rt.prof.launches += 3;
     return;
   }
@@ -1151,7 +1156,6 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
   else if (n <= 288) back(back_transform_kernel<9>);
   else back(back_transform_kernel<14>);
   HALF_LAUNCH("back transformation");
-  HALF_CUDA(cudaMemcpyAsync(A, V.get(), size_t(n) * nev * sizeof(double2), cudaMemcpyDeviceToDevice, s));
   rt.prof.launches += 3;
 }
 
@@ -1169,11 +1173,19 @@ void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, doubl
     hermitian_fill_kernel<<<ceil_div((long long)n * n, 256), 256, 0, s>>>(A, n);
     rt.prof.launches += 1;
     const double2 one = make_double2(1.0, 0.0), zero = make_double2(0.0, 0.0);
+    if (n <= kSmallProducts) {
+      double2* const v = V.get();
+      const ZBlock ba = {A, n}, bb = {B, n}, bv = {v, n};
+      zupdate(rt, n, &ba, B, n, &v, n, 1, 1.0, 0.0);
+      zgram(rt, n, bb, &bv, &A, 1, n, true);
+      heev(rt, A, n, nev, w, status);
+      zupdate(rt, n, &bb, v, n, &A, nev, 1, 1.0, 0.0);
+      return;
+    }
     gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, n, n, one, A, n, B, n, zero, V.get(), n);
     gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, n, n, n, one, B, n, V.get(), n, zero, A, n);
     heev(rt, A, n, nev, w, status);
-    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, nev, n, one, B, n, A, n, zero, V.get(), n);
-    HALF_CUDA(cudaMemcpyAsync(A, V.get(), size_t(n) * nev * sizeof(double2), cudaMemcpyDeviceToDevice, s));
+    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, nev, n, one, B, n, V.get(), n, zero, A, n);
     return;
   }
   auto* Bc = reinterpret_cast<cuDoubleComplex*>(B);
@@ -1191,6 +1203,7 @@ void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, doubl
                            &one, Bc, n, Ac, n),
                "ztrsm");
   heev(rt, A, n, nev, w, status);
+  HALF_CUDA(cudaMemcpyAsync(A, V.get(), size_t(n) * nev * sizeof(double2), cudaMemcpyDeviceToDevice, s));
   cublas_check(cublasZtrsm(rt.blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N, CUBLAS_DIAG_NON_UNIT, n, nev,
                            &one, Bc, n, Ac, n),
                "ztrsm");

@@ -17,8 +17,8 @@ struct SmallEigen {
   DeviceBuffer<double2> panels;   // exchange buffer of the metric factor's CTAs
   DeviceBuffer<int> info;   // zhetrd status (reports illegal arguments only)
   void reserve(Runtime& rt, int nmax);
-  // A (n x n, upper triangle) -> nev lowest eigenpairs; vectors overwrite
-  // A[:, :nev].  *status (device) becomes nonzero if inverse iteration failed.
+  // A (n x n, upper triangle, destroyed) -> nev lowest eigenpairs; vectors in
+  // V[:, :nev].  *status (device) becomes nonzero if inverse iteration failed.
   void heev(Runtime& rt, double2* A, int n, int nev, double* w, int* status);
   // A y = lambda B y, B Hermitian positive definite; Y^H B Y = I.
   // *chol_status (device) is zpotrf's info (> 0: B not positive definite).

@@ -7,8 +7,8 @@
 //   F_I,alpha -= 2 w f_n Re[((D_I - eps_n Q) c)^H dc_alpha] + w f_n Re[c^H dD_I/dR_alpha c].
 //
 // B200 design: one kernel accumulates, one contracts.  force_adjoint_kernel
-// runs one CTA per (atom, tile of 128 bands; 64 or 32 for atoms with more
-// than 8 or 16 channels, slice of the plane waves), 8 warps.  Per chunk of 32
+// runs one CTA per (atom, tile of 64 bands; 32 for atoms with more than 16
+// channels, slice of the plane waves), 8 warps.  Per chunk of 32
 // plane waves the CTA stages psi (coalesced along g), the plane waves' q
 // vectors, the atom's phase exp(+i q.R) (from the packed G indices and the
 // atom's b_j.R / 2 pi, reduced to one turn in FP64) and the chunk of
@@ -26,7 +26,7 @@
 // The accumulation is bound by the FP64 pipe (12 operations per plane wave,
 // channel and band), so what matters is that every SM has work: without
 // slices the 64-atom cell's 160 bands were 128 CTAs of which half carried 32
-// bands, 3.57 ms (16 % of the FP64 rate); 1.85 ms with slices.
+// bands, 3.57 ms (16 % of the FP64 rate); 1.55 ms with slices and 64-band tiles.
 #include <algorithm>
 
 #include "context.h"
@@ -54,11 +54,11 @@ size_t adjoint_smem(int bt) {
 }
 
 // One CTA per (atom, BT-band tile, slice of gper plane waves).  Thread = (band b = tid % BT, channel
-// group grp = tid / BT); it owns channels grp, grp + G, ... (up to kAdjPer of
-// them, G = 256 / BT groups, so atoms of up to 4 G channels).  A warp is 32
+// group grp = tid / BT); it owns channels grp, grp + G, ... (up to PER of
+// them, G = 256 / BT groups, so atoms of up to PER G channels).  A warp is 32
 // consecutive bands of one group: psi loads from shared memory are
 // conflict-free and the conj(B), q and phase loads are broadcasts.
-template <int BT>
+template <int BT, int PER>
 __global__ void __launch_bounds__(kAdjThreads)
     force_adjoint_kernel(const double2* __restrict__ psi, long long ld, int npw, int nb, const double* __restrict__ qv,
                          const double* __restrict__ ftab, const int* __restrict__ gpack, const int* __restrict__ pcol,
@@ -86,11 +86,11 @@ __global__ void __launch_bounds__(kAdjThreads)
   }
   const int atom = pcol[A.col] >> 16;
   const double f0 = afrac[3 * atom], f1 = afrac[3 * atom + 1], f2 = afrac[3 * atom + 2];
-  double2 acc[4][kAdjPer];
+  double2 acc[4][PER];
 #pragma unroll
   for (int q = 0; q < 4; ++q)
 #pragma unroll
-    for (int j = 0; j < kAdjPer; ++j) acc[q][j] = make_double2(0.0, 0.0);
+    for (int j = 0; j < PER; ++j) acc[q][j] = make_double2(0.0, 0.0);
 
   const int gend = min(npw, (int(blockIdx.z) + 1) * gper);
   for (int g0 = blockIdx.z * gper; g0 < gend; g0 += kAdjG) {
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kAdjThreads)
         const double2 x = spsi[gl * BP + bl];
         const double qx = sq[4 * gl], qy = sq[4 * gl + 1], qz = sq[4 * gl + 2];
 #pragma unroll
-        for (int j = 0; j < kAdjPer; ++j) {
+        for (int j = 0; j < PER; ++j) {
           const int a = grp + j * G;
           if (a < nlm) {
             const double2 b = sB[gl * kMaxNlm + a];
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kAdjThreads)
   if (n < nb) {
     double2* out = sums + ((long long)blockIdx.z * gridDim.x + ion) * 4 * nlm_max * nb + n;
 #pragma unroll
-    for (int j = 0; j < kAdjPer; ++j) {
+    for (int j = 0; j < PER; ++j) {
       const int a = grp + j * G;
       if (a < nlm)
         for (int q = 0; q < 4; ++q) out[((long long)q * nlm_max + a) * nb] = acc[q][j];
@@ -267,8 +267,11 @@ void nonlocal_forces_device(Context& ctx, KOperatorSet& ks, const double2* dvec,
   }
   int nlm_max = 1;
   for (auto& sp : ctx.species) nlm_max = std::max(nlm_max, sp.nlm);
-  // bands per CTA: 128 for atoms of up to 8 channels, 64 up to 16, 32 up to 32
-  const int bt = nlm_max <= 2 * kAdjPer ? 128 : nlm_max <= 4 * kAdjPer ? 64 : 32;
+  // Bands per CTA: 64 for atoms of up to 16 channels, 32 up to 32.  (128 bands
+  // with four channels a thread need half the registers' occupancy: 64-atom
+  // cell, 160, 97 and 60 bands, 128 / 64: 1.89 / 1.55, 1.16 / 1.12, 1.07 / 0.61
+  // ms; 216-atom cell, 480 bands: 46.4 / 39.6 ms.)
+  const int bt = nlm_max <= 4 * kAdjPer ? 64 : 32;
   const int btiles = (nb + bt - 1) / bt, ntiles = (nb + kConBands - 1) / kConBands;
   // Slices of the plane waves: enough for about six CTAs per SM (two are
   // resident, so uneven tiles even out), each of at least four chunks, and
@@ -298,9 +301,9 @@ void nonlocal_forces_device(Context& ctx, KOperatorSet& ks, const double2* dvec,
         dvec, ld, npw, nb, ks.qvec.get(), ks.ftab64.get(), ks.gpack.get(), ks.pcol.get(), ks.afrac.get(), ks.kf[0],
         ks.kf[1], ks.kf[2], datoms.get(), gper, nlm_max, dsums.get());
   };
-  if (bt == 128) launch(force_adjoint_kernel<128>);
-  else if (bt == 64) launch(force_adjoint_kernel<64>);
-  else launch(force_adjoint_kernel<32>);
+  if (bt == 64 && nlm_max <= 8) launch(force_adjoint_kernel<64, 2>);
+  else if (bt == 64) launch(force_adjoint_kernel<64, kAdjPer>);
+  else launch(force_adjoint_kernel<32, kAdjPer>);
   HALF_LAUNCH("force adjoint");
   raise_smem_limit(force_contract_kernel, csmem);
   force_contract_kernel<<<dim3(nions, ntiles), 3 * kConBands, csmem, st>>>(

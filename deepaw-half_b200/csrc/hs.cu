@@ -786,9 +786,7 @@ void apply_hs(Context& ctx, KOperatorSet& ks, const cplx_t<R>* x, long long ld, 
   const size_t psm = plane_smem<R>(op.n2, op.n3), xsm = xline_smem<R>(op.n1);
   const int pth = plane_threads<R>(psm);
   const int tiles = (op.n3 + kXTile - 1) / kXTile;
-  int sms = 148, dev = 0;
-  HALF_CUDA(cudaGetDevice(&dev));
-  HALF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int sms = rt.sms;
   Profile& pf = rt.prof;
   const int ev_sweep = pf.record(s);
   const int ev_local = ev_sweep;

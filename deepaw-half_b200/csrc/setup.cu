@@ -33,6 +33,7 @@ Runtime::Runtime() {
   cudaGetDevice(&dev);
   cudaDeviceProp prop;
   cudaGetDeviceProperties(&prop, dev);
+  sms = prop.multiProcessorCount;
   // FP32 emulation on BF16 tensor cores: cuBLAS >= 12.9 on compute capability 10.x.
   // The math mode only affects FP32 routines, i.e. the mixed-precision GEMMs.
   bf16x9 = (v >= 120900) && prop.major == 10;
@@ -74,7 +75,20 @@ void Profile::destroy() {
   a = b = nullptr;
 }
 
+double* Runtime::pinned(size_t words) {
+  if (words > pinned_words_) {
+    if (pinned_) cudaFreeHost(pinned_);
+    pinned_ = nullptr;
+    pinned_words_ = 0;
+    const size_t want = std::max<size_t>(words, 4096);
+    HALF_CUDA(cudaMallocHost(&pinned_, want * sizeof(double)));
+    pinned_words_ = want;
+  }
+  return pinned_;
+}
+
 Runtime::~Runtime() {
+  if (pinned_) cudaFreeHost(pinned_);
   prof.destroy();
   if (solver) cusolverDnDestroy(solver);
   if (blas) cublasDestroy(blas);

@@ -523,9 +523,7 @@ void tc_cgemm(Runtime& rt, const TcOperand& A, const TcOperand& B, int M, int N,
   const int bn0 = pick_bn(N);
   const int mt = (M + kBM - 1) / kBM, nt0 = (N + bn0 - 1) / bn0;
   const int nkb = (K + kBK - 1) / kBK;
-  int dev = 0, sms = 148;
-  HALF_CUDA(cudaGetDevice(&dev));
-  HALF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int sms = rt.sms;
   const long long tiles = (long long)mt * nt0;
   int splits = nkb > 0 ? pick_splits(tiles, nkb, bn0, (long long)M * N, sms) : 1;
   const int kbps = nkb > 0 ? (nkb + splits - 1) / splits : 0;
@@ -675,10 +673,10 @@ TcOperand tc_presplit_a(Runtime& rt, const TcOperand& op, DeviceBuffer<unsigned 
 void tc_check(Runtime& rt) {
   rt.crt_pending = false;
   if (rt.tc_err.size() == 0) return;
-  int flag = 0;
-  HALF_CUDA(cudaMemcpyAsync(&flag, rt.tc_err.get(), sizeof(int), cudaMemcpyDeviceToHost, rt.stream));
+  int* flag = reinterpret_cast<int*>(rt.pinned(1));
+  HALF_CUDA(cudaMemcpyAsync(flag, rt.tc_err.get(), sizeof(int), cudaMemcpyDeviceToHost, rt.stream));
   HALF_CUDA(cudaStreamSynchronize(rt.stream));
-  if (flag) {
+  if (*flag) {
     rt.tc_err.zero(rt.stream);
     fail(kInternal, "tensor-core GEMM pipeline wait timed out");
   }
