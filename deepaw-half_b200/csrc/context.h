@@ -194,6 +194,7 @@ struct KOperator;   // hs.cu
 
 struct KOperatorSet {
   Runtime* rt = nullptr;                      // stream and handles the operator runs on
+  DeviceBuffer<unsigned char> arena;          // the small tables of the operators below (UploadBatch)
   Basis basis;
   int np = 0;                                 // projector columns (all species)
   std::unique_ptr<KOperator<double>> op64;

@@ -58,10 +58,6 @@ struct KOperator {
   // the bf16 planes of the tensor-core GEMM (tc_gemm.cu), once per k point,
   // in the two orientations the products use
   DeviceBuffer<float> ftab;  // [frow][npw] Omega^-1/2 beta_l(|q|) Y_lm(q^), frow = (species, channel, m)
-  DeviceBuffer<int> gpack;   // npw packed (n1, n2, n3)
-  DeviceBuffer<int> pcol;    // np: (ion << 16) | (frow << 2) | l
-  DeviceBuffer<double> afrac;   // nions x 3: b_j . R / 2 pi
-  double kf[3] = {0, 0, 0};
   DeviceBuffer<unsigned char> bh_store, b_store;
   TcOperand bh_planes;       // conj(B)^T: np x npw
   TcOperand b_planes;        // B: npw x np
@@ -429,27 +425,33 @@ __device__ __forceinline__ double radial_angular(const ProjCol& col, double qx, 
 }
 
 // B[g, p] = Omega^-1/2 (-i)^l beta_l(|q|) Y_lm(q^) exp(-i q.R)   (src/half_paw.F90:52-65)
+// One thread per (plane wave, atom): the phase once, the radial-angular
+// factors from the table that the atoms of a species share.  Evaluating
+// spline, harmonics and phase per element took 151 us for the 64-atom cell
+// (512 projectors, 11,000 plane waves, 90 MB written).
 __global__ void projector_kernel(double2* __restrict__ B, int npw, const double* __restrict__ q,
-                                 const ProjCol* __restrict__ cols, const double* __restrict__ ry,
-                                 const double* __restrict__ rm2, const double* __restrict__ pos, double pref) {
-  int g = blockIdx.x * blockDim.x + threadIdx.x;
-  int p = blockIdx.y;
+                                 const double* __restrict__ ftab, const int* __restrict__ pcol,
+                                 const int2* __restrict__ atom_cols, const double* __restrict__ pos) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x, ion = blockIdx.y;
   if (g >= npw) return;
-  const ProjCol col = cols[p];
-  double qx = q[3 * g], qy = q[3 * g + 1], qz = q[3 * g + 2];
-  double ph = qx * pos[3 * col.ion] + qy * pos[3 * col.ion + 1] + qz * pos[3 * col.ion + 2];
+  const int2 cols = atom_cols[ion];   // first column, columns
+  const double ph = q[3 * g] * pos[3 * ion] + q[3 * g + 1] * pos[3 * ion + 1] + q[3 * g + 2] * pos[3 * ion + 2];
   double s, c;
   sincos(ph, &s, &c);
-  double amp = pref * radial_angular(col, qx, qy, qz, ry, rm2);
-  // (-i)^l * (cos - i sin)
-  double re = amp * c, im = -amp * s, tr, ti;
-  switch (col.l & 3) {
-    case 0: tr = re; ti = im; break;
-    case 1: tr = im; ti = -re; break;
-    case 2: tr = -re; ti = -im; break;
-    default: tr = -im; ti = re; break;
+  for (int p = cols.x; p < cols.x + cols.y; ++p) {
+    const int d = pcol[p];
+    const double amp = ftab[(long long)((d >> 2) & 0x3FFF) * npw + g];
+    // (-i)^l * (cos - i sin)
+    const double re = amp * c, im = -amp * s;
+    double tr, ti;
+    switch (d & 3) {
+      case 0: tr = re; ti = im; break;
+      case 1: tr = im; ti = -re; break;
+      case 2: tr = -re; ti = -im; break;
+      default: tr = -im; ti = re; break;
+    }
+    B[(long long)p * npw + g] = make_double2(tr, ti);
   }
-  B[(long long)p * npw + g] = make_double2(tr, ti);
 }
 
 // ftab[r][g] = Omega^-1/2 beta_l(|q|) Y_lm(q^) for the channel rows of the
@@ -523,25 +525,27 @@ HostGeom plane_geometry(const Basis& b, const AxisPlan& ax, const AxisPlan& ay, 
   return h;
 }
 
-// What the FP32 operator needs to generate projector tiles: one radial-angular
-// row per (species, channel, m), the column descriptors, and the ions' b_j.R / 2 pi.
+// What generates projector elements: one radial-angular row per (species,
+// channel, m), the column descriptors, the packed plane-wave indices and the
+// ions' b_j.R / 2 pi.
 struct ProjGen {
   std::vector<ProjCol> frows;
   std::vector<int> pcol, gpack;
   std::vector<double> afrac;
-  const double* ftab64 = nullptr;   // device [frow][npw], built by prepare_operator
-  const double* qvec = nullptr;   // device npw x 3
-  const double* ry = nullptr;     // device radial tables
-  const double* rm2 = nullptr;
-  double pref = 0;
 };
 
+// The projector columns' tables: first column of a column's atom, its place
+// in the atom, the atom's column count, offsets of D and Q.
+struct ProjTables {
+  std::vector<int> base, a, nlm, dofs, qofs;
+};
+
+// Sizes and small tables of one precision's operator; the tables are on the
+// device once the batch is flushed.
 template <typename R>
-void fill_operator(Context& ctx, Runtime& rt, const Basis& basis, const HostGeom& hg, DeviceBuffer<double2>& B64, int np,
-                   const std::vector<int>& cb, const std::vector<int>& ca, const std::vector<int>& cn,
-                   const std::vector<int>& cd, const std::vector<int>& cq, const ProjGen& gen, KOperator<R>& op) {
+void stage_operator(Context& ctx, const Basis& basis, const HostGeom& hg, int np, const ProjTables& pt,
+                    UploadBatch& batch, KOperator<R>& op) {
   using C = cplx_t<R>;
-  cudaStream_t s = rt.stream;
   op.npw = int(basis.npw());
   op.n1 = basis.shape[0]; op.n2 = basis.shape[1]; op.n3 = basis.shape[2];
   op.ax = make_axis_plan(op.n1); op.ay = make_axis_plan(op.n2); op.az = make_axis_plan(op.n3);
@@ -549,72 +553,66 @@ void fill_operator(Context& ctx, Runtime& rt, const Basis& basis, const HostGeom
   if (plane_smem<R>(op.n2, op.n3) > 227 * 1024)
     fail(kUnavailable, "FFT plane " + std::to_string(op.n2) + "x" + std::to_string(op.n3) +
                            " exceeds the shared-memory capacity of one CTA at this precision");
-  op.plane_start.upload(hg.plane_start, s);
-  op.spos.upload(hg.spos, s);
-  op.row_start.upload(hg.row_start, s);
-  op.row_list.upload(hg.row_list, s);
-  op.slot_plane.upload(hg.slot_plane, s);
+  batch.add(op.plane_start, hg.plane_start);
+  batch.add(op.spos, hg.spos);
+  batch.add(op.row_start, hg.row_start);
+  batch.add(op.row_list, hg.row_list);
+  batch.add(op.slot_plane, hg.slot_plane);
   std::vector<C> tw;
   const int axes[3] = {op.n1, op.n2, op.n3};
   for (int a = 0; a < 3; ++a)
     for (int t = 0; t < axes[a]; ++t)
       tw.push_back(cmake(R(std::cos(2.0 * kPi * t / axes[a])), R(-std::sin(2.0 * kPi * t / axes[a]))));
-  op.tw.upload(tw, s);
-  const long long nr = ctx.nr();
-  op.veff.resize(nr);
-  scale_copy_kernel<R><<<ceil_div(nr, 256), 256, 0, s>>>(ctx.veff.get(), op.veff.get(), nr, 1.0 / double(nr));
-  DeviceBuffer<double> kin;
-  kin.upload(basis.kinetic, s);
-  op.kinetic.resize(basis.npw());
-  scale_copy_kernel<R><<<ceil_div(basis.npw(), 256), 256, 0, s>>>(kin.get(), op.kinetic.get(), basis.npw(), 1.0);
-  if constexpr (sizeof(R) == 8) {
-    op.B = std::move(B64);   // only the FP64 operator reads the stored matrix
-  } else if (np > 0) {
-    const long long nt = (long long)gen.frows.size() * basis.npw();
-    op.ftab.resize(size_t(nt));
-    scale_copy_kernel<float><<<ceil_div(nt, 256), 256, 0, s>>>(gen.ftab64, op.ftab.get(), nt, 1.0);
-    HALF_LAUNCH("radial-angular table (FP32)");
-    op.gpack.upload(gen.gpack, s);
-    op.pcol.upload(gen.pcol, s);
-    op.afrac.upload(gen.afrac, s);
-    for (int j = 0; j < 3; ++j) op.kf[j] = basis.kpoint[j];
-    TcOperand g;
-    g.kind = TcOperand::kProjConj;
-    g.rows = np;
-    g.kdim = op.npw;
-    g.ftab = op.ftab.get();
-    g.gpack = op.gpack.get();
-    g.pcol = op.pcol.get();
-    g.afrac = op.afrac.get();
-    g.kf0 = op.kf[0];
-    g.kf1 = op.kf[1];
-    g.kf2 = op.kf[2];
-    g.npw = op.npw;
-    op.bh_planes = tc_presplit_a(rt, g, op.bh_store);
-    g.kind = TcOperand::kProj;
-    g.rows = op.npw;
-    g.kdim = np;
-    op.b_planes = tc_presplit_a(rt, g, op.b_store);
-  }
-  std::vector<double> dall, qall;
+  batch.add(op.tw, tw);
+  batch.add(op.kinetic, std::vector<R>(basis.kinetic.begin(), basis.kinetic.end()));
+  std::vector<R> dall, qall;
   for (auto& sp : ctx.species) {
     dall.insert(dall.end(), sp.dij_host.begin(), sp.dij_host.end());
     qall.insert(qall.end(), sp.qij_host.begin(), sp.qij_host.end());
   }
-  DeviceBuffer<double> dd, dq;
-  dd.upload(dall, s);
-  dq.upload(qall, s);
-  op.dall.resize(dall.size());
-  op.qall.resize(qall.size());
-  scale_copy_kernel<R><<<ceil_div((long long)dall.size(), 256), 256, 0, s>>>(dd.get(), op.dall.get(), (long long)dall.size(), 1.0);
-  scale_copy_kernel<R><<<ceil_div((long long)qall.size(), 256), 256, 0, s>>>(dq.get(), op.qall.get(), (long long)qall.size(), 1.0);
-  op.col_base.upload(cb, s);
-  op.col_a.upload(ca, s);
-  op.col_nlm.upload(cn, s);
-  op.col_dofs.upload(cd, s);
-  op.col_qofs.upload(cq, s);
+  batch.add(op.dall, dall);
+  batch.add(op.qall, qall);
+  batch.add(op.col_base, pt.base);
+  batch.add(op.col_a, pt.a);
+  batch.add(op.col_nlm, pt.nlm);
+  batch.add(op.col_dofs, pt.dofs);
+  batch.add(op.col_qofs, pt.qofs);
+}
+
+// The operator's large tables, on the device.
+template <typename R>
+void fill_operator(Context& ctx, Runtime& rt, KOperatorSet& ks, int nfrows, DeviceBuffer<double2>& B64,
+                   KOperator<R>& op) {
+  cudaStream_t s = rt.stream;
+  const long long nr = ctx.nr();
+  op.veff.resize(nr);
+  scale_copy_kernel<R><<<ceil_div(nr, 256), 256, 0, s>>>(ctx.veff.get(), op.veff.get(), nr, 1.0 / double(nr));
+  if constexpr (sizeof(R) == 8) {
+    op.B = std::move(B64);   // only the FP64 operator reads the stored matrix
+  } else if (op.np > 0) {
+    const long long nt = (long long)nfrows * op.npw;
+    op.ftab.resize(size_t(nt));
+    scale_copy_kernel<float><<<ceil_div(nt, 256), 256, 0, s>>>(ks.ftab64.get(), op.ftab.get(), nt, 1.0);
+    HALF_LAUNCH("radial-angular table (FP32)");
+    TcOperand g;
+    g.kind = TcOperand::kProjConj;
+    g.rows = op.np;
+    g.kdim = op.npw;
+    g.ftab = op.ftab.get();
+    g.gpack = ks.gpack.get();
+    g.pcol = ks.pcol.get();
+    g.afrac = ks.afrac.get();
+    g.kf0 = ks.kf[0];
+    g.kf1 = ks.kf[1];
+    g.kf2 = ks.kf[2];
+    g.npw = op.npw;
+    op.bh_planes = tc_presplit_a(rt, g, op.bh_store);
+    g.kind = TcOperand::kProj;
+    g.rows = op.npw;
+    g.kdim = op.np;
+    op.b_planes = tc_presplit_a(rt, g, op.b_store);
+  }
   HALF_LAUNCH("operator tables");
-  HALF_CUDA(cudaStreamSynchronize(s));
   raise_smem_limit(k1_sphere_to_planes<R>, plane_smem<R>(op.n2, op.n3));
   raise_smem_limit(k3_planes_to_sphere<R>, plane_smem<R>(op.n2, op.n3));
   raise_smem_limit(k2_xlines<R>, xline_smem<R>(op.n1));
@@ -634,21 +632,23 @@ std::unique_ptr<KOperatorSet> prepare_operator(Context& ctx, Runtime& rt, const 
   HostGeom hg = plane_geometry(basis, ax, ay, az);
   // projector columns: species-major, atom-major, then (channel, m)
   std::vector<ProjCol> cols;
-  std::vector<int> cb, ca, cn, cd, cq;
+  ProjTables pt;
+  std::vector<int2> atom_cols(ctx.crystal.nions(), make_int2(0, 0));   // first column and columns per ion
   std::vector<double> ry, rm2, pos;
   int chan0 = 0, dofs = 0, qofs = 0, col0 = 0;
   for (auto& sp : ctx.species) {
     for (int a = 0; a < sp.natoms; ++a) {
       int ilm = 0;
+      atom_cols[sp.first_ion + a] = make_int2(col0 + a * sp.nlm, sp.nlm);
       for (int c = 0; c < sp.nchan; ++c) {
         int l = sp.lps[c];
         for (int m = -l; m <= l; ++m, ++ilm) {
           cols.push_back({chan0 + c, l, m, sp.first_ion + a, sp.pspnl_gmax});
-          cb.push_back(col0 + a * sp.nlm);
-          ca.push_back(ilm);
-          cn.push_back(sp.nlm);
-          cd.push_back(dofs + a * sp.nlm * sp.nlm);
-          cq.push_back(qofs);
+          pt.base.push_back(col0 + a * sp.nlm);
+          pt.a.push_back(ilm);
+          pt.nlm.push_back(sp.nlm);
+          pt.dofs.push_back(dofs + a * sp.nlm * sp.nlm);
+          pt.qofs.push_back(qofs);
         }
       }
     }
@@ -693,49 +693,49 @@ std::unique_ptr<KOperatorSet> prepare_operator(Context& ctx, Runtime& rt, const 
   }
   for (size_t g = 0; g < basis.gvec.size(); ++g)
     if (basis.gvec[g] < -512 || basis.gvec[g] > 511) fail(kUnavailable, "plane-wave index beyond the packed range");
-  ks->qvec.upload(basis.qvec, s);
-  DeviceBuffer<ProjCol> dcols;
-  dcols.upload(cols, s);
+  gen.gpack.resize(npw);
+  for (int g = 0; g < npw; ++g)
+    gen.gpack[g] = (basis.gvec[3 * g] & 1023) | ((basis.gvec[3 * g + 1] & 1023) << 10) |
+                   ((basis.gvec[3 * g + 2] & 1023) << 20);
+  for (int j = 0; j < 3; ++j) ks->kf[j] = basis.kpoint[j];
+  // every small table in one copy
+  UploadBatch batch;
   DeviceBuffer<double> dry, drm2, dpos;
-  dry.upload(ry, s);
-  drm2.upload(rm2, s);
-  dpos.upload(pos, s);
-  DeviceBuffer<double2> B64((size_t)npw * np);
-  gen.qvec = ks->qvec.get();
-  gen.ry = dry.get();
-  gen.rm2 = drm2.get();
-  gen.pref = 1.0 / std::sqrt(ctx.crystal.volume());
   DeviceBuffer<ProjCol> drows;
-  if (np > 0) {   // projector generation tables, shared by the FP32 operator's planes and the force adjoint
-    const int nf = int(gen.frows.size());
-    drows.upload(gen.frows, s);
-    ks->ftab64.resize(size_t(nf) * npw);
-    radial_angular_table_kernel<<<dim3(ceil_div(npw, 256), nf), 256, 0, s>>>(ks->ftab64.get(), npw, ks->qvec.get(),
-                                                                            drows.get(), dry.get(), drm2.get(), gen.pref);
-    HALF_LAUNCH("radial-angular table");
-    gen.gpack.resize(npw);
-    for (int g = 0; g < npw; ++g)
-      gen.gpack[g] = (basis.gvec[3 * g] & 1023) | ((basis.gvec[3 * g + 1] & 1023) << 10) |
-                     ((basis.gvec[3 * g + 2] & 1023) << 20);
-    ks->gpack.upload(gen.gpack, s);
-    ks->pcol.upload(gen.pcol, s);
-    ks->afrac.upload(gen.afrac, s);
-    for (int j = 0; j < 3; ++j) ks->kf[j] = basis.kpoint[j];
-    gen.ftab64 = ks->ftab64.get();
-  }
-  if (np > 0) {
-    projector_kernel<<<dim3(ceil_div(npw, 256), np), 256, 0, s>>>(B64.get(), npw, ks->qvec.get(), dcols.get(), dry.get(),
-                                                                   drm2.get(), dpos.get(), 1.0 / std::sqrt(ctx.crystal.volume()));
-    HALF_LAUNCH("projectors");
-  }
+  DeviceBuffer<int2> datom;
+  batch.add(ks->qvec, basis.qvec);
+  batch.add(ks->gpack, gen.gpack);
+  batch.add(ks->pcol, gen.pcol);
+  batch.add(ks->afrac, gen.afrac);
+  batch.add(dry, ry);
+  batch.add(drm2, rm2);
+  batch.add(dpos, pos);
+  batch.add(drows, gen.frows);
+  batch.add(datom, atom_cols);
   if (fp64) {
     ks->op64 = std::make_unique<KOperator<double>>();
-    fill_operator<double>(ctx, rt, basis, hg, B64, np, cb, ca, cn, cd, cq, gen, *ks->op64);
+    stage_operator<double>(ctx, basis, hg, np, pt, batch, *ks->op64);
   }
   if (fp32) {
     ks->op32 = std::make_unique<KOperator<float>>();
-    fill_operator<float>(ctx, rt, basis, hg, B64, np, cb, ca, cn, cd, cq, gen, *ks->op32);
+    stage_operator<float>(ctx, basis, hg, np, pt, batch, *ks->op32);
   }
+  batch.flush(ks->arena, s);
+  DeviceBuffer<double2> B64(fp64 ? (size_t)npw * np : 0);
+  const int nf = int(gen.frows.size());
+  if (np > 0) {   // projector generation tables, shared by the FP32 operator's planes and the force adjoint
+    ks->ftab64.resize(size_t(nf) * npw);
+    radial_angular_table_kernel<<<dim3(ceil_div(npw, 256), nf), 256, 0, s>>>(
+        ks->ftab64.get(), npw, ks->qvec.get(), drows.get(), dry.get(), drm2.get(), 1.0 / std::sqrt(ctx.crystal.volume()));
+    HALF_LAUNCH("radial-angular table");
+    if (fp64) {
+      projector_kernel<<<dim3(ceil_div(npw, 256), ctx.crystal.nions()), 256, 0, s>>>(
+          B64.get(), npw, ks->qvec.get(), ks->ftab64.get(), ks->pcol.get(), datom.get(), dpos.get());
+      HALF_LAUNCH("projectors");
+    }
+  }
+  if (fp64) fill_operator<double>(ctx, rt, *ks, nf, B64, *ks->op64);
+  if (fp32) fill_operator<float>(ctx, rt, *ks, nf, B64, *ks->op32);
   HALF_CUDA(cudaStreamSynchronize(s));
   return ks;
 }
