@@ -298,7 +298,7 @@ struct SmallSolver {
     if (const char* po = std::getenv("HALF_PENCIL_OWN")) own_large = own && std::string(po) != "0";
     info.resize(3);
     info.zero(rt.stream);
-    if (own) eig.reserve(rt, own_large ? 2 * m : std::min(2 * m, SmallEigen::kOwnMaxOrder));   // locking shrinks pencils below it
+    if (own) eig.reserve(rt, own_large ? 2 * m : std::min(2 * m, SmallEigen::kGridMaxOrder));   // locking shrinks pencils below it
     int l1 = 0, l2 = 0, l3 = 0;
     cusolver_check(cusolverDnZheevd_bufferSize(rt.solver, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, m,
                                                reinterpret_cast<cuDoubleComplex*>(a), m, w, &l1),
@@ -335,9 +335,14 @@ struct SmallSolver {
                                     reinterpret_cast<cuDoubleComplex*>(work.get()), int(work.size()), info.get()),
                    "zheevd");
   }
+  // orders of the own solver; those of the grid-wide tridiagonalisation in the
+  // guard-band modes only (the FP64 mode keeps zhegvd there)
+  bool own_order(int n) const {
+    return own && (n <= SmallEigen::kOwnMaxOrder || (range && n <= SmallEigen::kGridMaxOrder) || own_large);
+  }
   // generalized problem of order n; the nev lowest eigenvectors are wanted
   void hegvd(double2* a, double2* b, int n, double* w, int nev) {
-    if (own && (n <= SmallEigen::kOwnMaxOrder || own_large)) {
+    if (own_order(n)) {
       eig.hegv(rt, a, b, n, nev, w, info.get() + 1, info.get() + 2);
       return;
     }

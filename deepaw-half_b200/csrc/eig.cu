@@ -207,18 +207,20 @@ __device__ double multisect(const double* d, const double* e2, int n, int k, dou
   return 0.5 * (lo + hi);
 }
 
-// Eigenvalues 0..ne-1 of T (ascending), one warp each.  Also clears *status
-// for the vector kernel that follows on the stream.
+// Eigenvalues 0..ne-1 of T (ascending), one warp each.  Also sets *status for
+// the vector kernel that follows on the stream: 0, or 2 when a grid barrier of
+// the tridiagonalisation gave up.
 __global__ void __launch_bounds__(32 * kValueWarps) tridiag_values_kernel(const double* __restrict__ d_in,
                                                                           const double* __restrict__ e_in, int n,
                                                                           int ne, double* __restrict__ lam,
+                                                                          const int* __restrict__ grid_err,
                                                                           int* __restrict__ status) {
   extern __shared__ double sm[];
   double* d = sm;
   double* e = d + n;
   double* e2 = e + n;
   __shared__ double s_gl, s_gu, s_norm;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *status = grid_err && *grid_err ? 2 : 0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     d[i] = d_in[i];
     e[i] = i < n - 1 ? e_in[i] : 0.0;
@@ -976,10 +978,218 @@ __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__
   cl.sync();   // no CTA leaves while another may still read its columns
 }
 
+// The same reduction for orders beyond one cluster: a cooperative launch of
+// one CTA per SM, column j on CTA j mod G, u and the pivot column exchanged
+// through global memory (L2), one grid barrier per step.  Waits are bounded:
+// a barrier that is not reached in two seconds raises *err, and every CTA
+// leaves.  Needs ceil(n / G) n + 3 n elements of shared memory per CTA.
+//
+// Bound by the chain per step (grid barrier, L2 round trip, reductions) and,
+// near the upper end, by the pass over shared memory.  480-band solve of the
+// 216-atom cell, its 25 pencils: 84.5 ms here for the 17 of orders 434 to
+// 1,200 and 10.4 ms in the cluster kernel for the rest (cuSOLVER's zhetrd for
+// all of them 187 ms); the solve 723 -> 601 ms.
+constexpr int kGridRows = (SmallEigen::kGridMaxOrder + kClThreads - 1) / kClThreads;
+constexpr unsigned long long kGridWaitNs = 2000000000ull;
+
+inline size_t hetrd_grid_smem(int n, int ctas) {
+  return (size_t((n + ctas - 1) / ctas) * n + 3 * size_t(n)) * sizeof(double2);
+}
+
+__device__ __forceinline__ int load_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Waits until `counter` reaches `target`; false when it does not in time or another CTA gave up.
+__device__ bool grid_wait(const int* counter, int target, int* err) {
+  unsigned long long t0 = 0;
+  for (unsigned spin = 0;; ++spin) {
+    if (load_acquire(counter) >= target) return true;
+    if ((spin & 255u) == 255u) {
+      unsigned long long t;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+      if (t0 == 0) t0 = t;
+      if (t - t0 > kGridWaitNs || *reinterpret_cast<volatile int*>(err) != 0) {
+        atomicExch(err, 1);
+        return false;
+      }
+    }
+  }
+}
+
+// exchange: u and the pivot column, 2 x 2 x n by parity of the step; counter
+// zero at launch.
+__global__ void __launch_bounds__(kClThreads) hetrd_grid_kernel(double2* __restrict__ A, int n,
+                                                                double* __restrict__ dout, double* __restrict__ eout,
+                                                                double2* __restrict__ tauout, double2* exchange,
+                                                                int* counter, int* err) {
+  const int G = gridDim.x, rank = blockIdx.x;
+  const int nc = (n + G - 1) / G;
+  extern __shared__ __align__(16) double2 cols[];   // nc x n: column jl G + rank at cols + jl n
+  double2* xbuf = cols + size_t(nc) * n;            // the pivot column
+  double2* vbuf = xbuf + n;                         // the previous step's v and w
+  double2* wbuf = vbuf + n;
+  __shared__ double red[kClWarps];
+  __shared__ int s_ok;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int jl = warp; jl * G + rank < n; jl += kClWarps) {
+    const int j = jl * G + rank;
+    for (int r = lane; r < n; r += 32) {
+      double2 a = r <= j ? A[size_t(j) * n + r] : A[size_t(r) * n + j];
+      if (r == j) a.y = 0.0;
+      if (r > j) a.y = -a.y;
+      cols[size_t(jl) * n + r] = a;
+    }
+  }
+  for (int r = tid; r < n; r += kClThreads) vbuf[r] = wbuf[r] = make_double2(0.0, 0.0);
+  double2 x[kGridRows];   // the pivot column, rows tid + kClThreads t
+#pragma unroll
+  for (int t = 0; t < kGridRows; ++t) {
+    const int r = tid + kClThreads * t;
+    x[t] = r < n ? A[size_t(n - 1) * n + r] : make_double2(0.0, 0.0);
+    if (r == n - 1) x[t].y = 0.0;
+  }
+  // A is overwritten with the reflectors from the first step on: wait until
+  // every CTA has read its columns
+  int target = G;
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    atomicAdd(counter, 1);
+    s_ok = grid_wait(counter, target, err);
+  }
+  __syncthreads();
+  if (!s_ok) return;
+  int par = 0;
+  for (int i0 = n - 2; i0 >= 0; --i0, par ^= 1) {
+    const int c = i0 + 1, L = i0 + 1;
+#pragma unroll
+    for (int t = 0; t < kGridRows; ++t) {
+      const int r = tid + kClThreads * t;
+      if (r < L) xbuf[r] = x[t];
+      if (r == c && rank == 0) dout[c] = x[t].x;
+    }
+    __syncthreads();   // xbuf, vbuf, wbuf
+    double2* gu = exchange + size_t(2 * par) * n;
+    double2* ga = gu + n;
+    double norm = 0;
+    bool first = true;
+    int jl0 = warp;
+    do {   // at least once: every warp needs the norm
+      double2 ws[kClCols], vs[kClCols];
+      double acc[2 * kClCols] = {};
+      bool on[kClCols];
+      int pivot = -1;   // the slot that holds column i0
+#pragma unroll
+      for (int k = 0; k < kClCols; ++k) {
+        const int s = (jl0 + k * kClWarps) * G + rank;
+        on[k] = s < L;
+        if (s == i0) pivot = k;
+        ws[k] = on[k] ? wbuf[s] : make_double2(0.0, 0.0);
+        vs[k] = on[k] ? vbuf[s] : make_double2(0.0, 0.0);
+      }
+      for (int r = lane; r < L; r += 32) {
+        const double2 pv = vbuf[r], pw = wbuf[r], xx = xbuf[r];
+        if (first && r < i0) norm += xx.x * xx.x + xx.y * xx.y;
+#pragma unroll
+        for (int k = 0; k < kClCols; ++k) {
+          if (on[k]) {
+            double2* e = cols + size_t(jl0 + k * kClWarps) * n + r;
+            double2 a = *e;
+            a.x -= (pv.x * ws[k].x + pv.y * ws[k].y) + (pw.x * vs[k].x + pw.y * vs[k].y);
+            a.y -= (pv.y * ws[k].x - pv.x * ws[k].y) + (pw.y * vs[k].x - pw.x * vs[k].y);
+            *e = a;
+            if (k == pivot) ga[r] = a;
+            acc[2 * k] += a.x * xx.x + a.y * xx.y;
+            acc[2 * k + 1] += a.x * xx.y - a.y * xx.x;
+          }
+        }
+      }
+      first = false;
+      const double own = warp_sum8(acc);                                // value lane >> 2
+      const double other = __shfl_xor_sync(0xffffffffu, own, 4);
+      const int s = (jl0 + (lane >> 3) * kClWarps) * G + rank;
+      if (s < L && (lane & 7) == 0) gu[s] = make_double2(own, other);
+      jl0 += kClWarps * kClCols;
+    } while (jl0 * G + rank < L);
+    const double2 al = xbuf[i0];
+    target += G;
+    __syncthreads();   // this CTA's part of u and of the pivot column is written
+    if (tid == 0) {
+      __threadfence();
+      atomicAdd(counter, 1);
+    }
+    for (int off = 16; off > 0; off >>= 1) norm += __shfl_xor_sync(0xffffffffu, norm, off);
+    double2 tau = make_double2(0.0, 0.0), sc = make_double2(1.0, 0.0);
+    double beta = al.x;
+    if (!(norm == 0.0 && al.y == 0.0)) {   // zlarfg on (alpha = x(i0), x(0:i0-1))
+      beta = -copysign(sqrt(al.x * al.x + al.y * al.y + norm), al.x);
+      const double ib = 1.0 / beta;
+      tau = make_double2((beta - al.x) * ib, -al.y * ib);
+      const double dr = al.x - beta, di = al.y, iden = 1.0 / (dr * dr + di * di);
+      sc = make_double2(dr * iden, -di * iden);   // 1 / (alpha - beta)
+    }
+    const double2 kap = csub(make_double2(1.0, 0.0), cmul(sc, al));
+    const double tau2 = tau.x * tau.x + tau.y * tau.y, sc2 = sc.x * sc.x + sc.y * sc.y;
+    const double2 tsc = cmul(tau, sc), tkap = cmul(tau, kap);
+    if (rank == 0 && tid == 0) {
+      eout[i0] = beta;
+      tauout[i0] = tau;
+    }
+    if (tid == 0) s_ok = grid_wait(counter, target, err);
+    __syncthreads();
+    if (!s_ok) return;
+    double2 ur[kGridRows], ar[kGridRows];
+    double qs = 0;
+#pragma unroll
+    for (int t = 0; t < kGridRows; ++t) {
+      const int r = tid + kClThreads * t;
+      ur[t] = ar[t] = make_double2(0.0, 0.0);
+      if (r <= i0) {
+        ur[t] = __ldcg(gu + r);
+        ar[t] = __ldcg(ga + r);
+        qs += x[t].x * ur[t].x + x[t].y * ur[t].y;   // Re(conj(x) u)
+      }
+    }
+    const double2 ui = __ldcg(gu + i0), ai = __ldcg(ga + i0);
+    for (int off = 16; off > 0; off >>= 1) qs += __shfl_xor_sync(0xffffffffu, qs, off);
+    if (lane == 0) red[warp] = qs;
+    __syncthreads();
+    qs = red[0];
+#pragma unroll
+    for (int w = 1; w < kClWarps; ++w) qs += red[w];
+    const double2 sk = cconjmul(sc, kap);   // conj(sc) kappa
+    const double vav = sc2 * qs + 2.0 * (sk.x * ui.x + sk.y * ui.y) + (kap.x * kap.x + kap.y * kap.y) * ai.x;
+    const double a2 = -0.5 * tau2 * vav;
+    double2 wi = cadd(cmul(tsc, ui), cmul(tkap, ai));
+    wi.x += a2;   // w(i0), v(i0) = 1
+#pragma unroll
+    for (int t = 0; t < kGridRows; ++t) {
+      const int r = tid + kClThreads * t;
+      if (r <= i0) {
+        const double2 v = r < i0 ? cmul(x[t], sc) : make_double2(1.0, 0.0);
+        if (r < i0 && rank == c % G) A[size_t(c) * n + r] = v;
+        double2 w = cadd(cmul(tsc, ur[t]), cmul(tkap, ar[t]));
+        w.x += a2 * v.x;
+        w.y += a2 * v.y;
+        vbuf[r] = v;
+        wbuf[r] = w;
+        x[t].x = ar[t].x - (v.x * wi.x + v.y * wi.y) - w.x;
+        x[t].y = ar[t].y - (v.y * wi.x - v.x * wi.y) - w.y;
+      }
+    }
+  }
+  if (rank == 0 && tid == 0) dout[0] = x[0].x;
+}
+
 // Orders whose congruence and final rotation go through the block kernels
 // (blockops.h) instead of ZGEMM with its split-K reductions: two to four
 // launches fewer, while one product does not fill the GPU.
 constexpr int kSmallProducts = 176;
+
+constexpr size_t kGridSmem = 227 * 1024 - 256;   // leaves room for the kernel's static shared memory
 
 // CTAs of the cluster for an order-n tridiagonalisation: measured best at 8
 // from order 40 to 176 (order 80: 1, 2, 4, 8 and 16 CTAs 283, 218, 192, 183
@@ -1091,9 +1301,23 @@ void SmallEigen::reserve(Runtime& rt, int nmax) {
 void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* status) {
   reserve(rt, n);
   cudaStream_t s = rt.stream;
+  const int* gave_up = nullptr;
   if (n <= kOwnMaxOrder) {   // whole reduction in one cluster
     const int p = hetrd_ctas(n);
     launch_cluster(hetrd_kernel, p, hetrd_smem(n, p), s, A, n, d.get(), e.get(), tau.get());
+    rt.prof.launches += 1;
+  } else if (const size_t gsm = hetrd_grid_smem(n, rt.sms); n <= kGridMaxOrder && gsm <= kGridSmem) {
+    if (exchange.size() < 4 * size_t(n)) exchange.resize(4 * size_t(kGridMaxOrder));
+    if (grid_state.size() == 0) grid_state.resize(2);   // barrier counter, error flag
+    grid_state.zero(s);
+    gave_up = grid_state.get() + 1;
+    raise_smem_limit(hetrd_grid_kernel, gsm);
+    double *dp = d.get(), *ep = e.get();
+    double2 *tp = tau.get(), *xp = exchange.get();
+    int *cp = grid_state.get(), *gp = cp + 1;
+    void* args[] = {&A, &n, &dp, &ep, &tp, &xp, &cp, &gp};
+    HALF_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(hetrd_grid_kernel), dim3(rt.sms),
+                                          dim3(kClThreads), args, gsm, s));
     rt.prof.launches += 1;
   } else {
     cusolver_check(cusolverDnZhetrd(rt.solver, CUBLAS_FILL_MODE_UPPER, n, reinterpret_cast<cuDoubleComplex*>(A), n,
@@ -1108,7 +1332,7 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
   const size_t vsm = 3 * size_t(n) * sizeof(double);
   raise_smem_limit(tridiag_values_kernel, vsm);
   tridiag_values_kernel<<<ceil_div(ne, kValueWarps), 32 * kValueWarps, vsm, s>>>(d.get(), e.get(), n, ne, lam.get(),
-                                                                                  status);
+                                                                                  gave_up, status);
   HALF_LAUNCH("tridiagonal eigenvalues");
   size_t tsm = (2 * size_t(n) + ne) * sizeof(double) + size_t(ne) * sizeof(int);
   if (tsm > kSmemMax) fail(kCapacity, "subspace eigenproblem too large for the tridiagonal solver: n=" + std::to_string(n));

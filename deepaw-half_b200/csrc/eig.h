@@ -9,12 +9,17 @@ namespace hb {
 
 struct SmallEigen {
   // Orders the cluster kernels serve: the matrix fits the shared memory of 16
-  // CTAs (432 x 432 x 16 bytes and the vectors).  Above it cuSOLVER.
+  // CTAs (432 x 432 x 16 bytes and the vectors).
   static constexpr int kOwnMaxOrder = 432;
+  // Orders whose tridiagonalisation the whole GPU's shared memory holds (148
+  // SMs: ceil(n / 148) n + 3 n elements of 16 bytes).  Above it cuSOLVER.
+  static constexpr int kGridMaxOrder = 1208;
   int cap = 0;
   DeviceBuffer<double> d, e, Z, scratch, lam;
   DeviceBuffer<double2> tau, V, work;
   DeviceBuffer<double2> panels;   // exchange buffer of the metric factor's CTAs
+  DeviceBuffer<double2> exchange; // and of the grid-wide tridiagonalisation's
+  DeviceBuffer<int> grid_state;   // its barrier counter and error flag
   DeviceBuffer<int> info;   // zhetrd status (reports illegal arguments only)
   void reserve(Runtime& rt, int nmax);
   // A (n x n, upper triangle, destroyed) -> nev lowest eigenpairs; vectors in
