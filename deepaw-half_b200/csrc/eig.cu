@@ -982,18 +982,22 @@ __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__
 // one CTA per SM, column j on CTA j mod G, u and the pivot column exchanged
 // through global memory (L2), one grid barrier per step.  Waits are bounded:
 // a barrier that is not reached in two seconds raises *err, and every CTA
-// leaves.  Needs ceil(n / G) n + 3 n elements of shared memory per CTA.
+// leaves.  Needs ceil(n / G) n elements of shared memory per CTA.
 //
-// Bound by the chain per step (grid barrier, L2 round trip, reductions) and,
-// near the upper end, by the pass over shared memory.  480-band solve of the
-// 216-atom cell, its 25 pencils: 84.5 ms here for the 17 of orders 434 to
-// 1,200 and 10.4 ms in the cluster kernel for the rest (cuSOLVER's zhetrd for
-// all of them 187 ms); the solve 723 -> 601 ms.
+// Bound by the chain per step (grid barrier, L2 round trips, reductions) and,
+// near the upper end, by the pass over shared memory.  A thread owns rows
+// tid + 256 t of all the CTA's columns, so that x, v and w of its rows stay in
+// registers and the pass reads and writes each element once and nothing else;
+// with a warp per column the three vectors came from shared memory for every
+// column (84.5 ms for the 17 pencils of orders 434 to 1,200 of a 480-band
+// solve, 63.3 ms like this; cuSOLVER's zhetrd 187 ms for these and the eight
+// smaller ones, which take 10.4 ms in the cluster kernel).
 constexpr int kGridRows = (SmallEigen::kGridMaxOrder + kClThreads - 1) / kClThreads;
+constexpr int kGridCols = 12;   // columns a CTA can own, a multiple of kClCols
 constexpr unsigned long long kGridWaitNs = 2000000000ull;
 
 inline size_t hetrd_grid_smem(int n, int ctas) {
-  return (size_t((n + ctas - 1) / ctas) * n + 3 * size_t(n)) * sizeof(double2);
+  return size_t((n + ctas - 1) / ctas) * n * sizeof(double2);
 }
 
 __device__ __forceinline__ int load_acquire(const int* p) {
@@ -1028,10 +1032,10 @@ __global__ void __launch_bounds__(kClThreads) hetrd_grid_kernel(double2* __restr
   const int G = gridDim.x, rank = blockIdx.x;
   const int nc = (n + G - 1) / G;
   extern __shared__ __align__(16) double2 cols[];   // nc x n: column jl G + rank at cols + jl n
-  double2* xbuf = cols + size_t(nc) * n;            // the pivot column
-  double2* vbuf = xbuf + n;                         // the previous step's v and w
-  double2* wbuf = vbuf + n;
-  __shared__ double red[kClWarps];
+  __shared__ double red[kClWarps][2 * kGridCols];   // the warps' shares of u
+  __shared__ double rnorm[kClWarps], rqs[kClWarps];
+  __shared__ double2 vcol[kGridCols], wcol[kGridCols];   // the previous step's v and w at this CTA's columns
+  __shared__ double2 s_al;
   __shared__ int s_ok;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int jl = warp; jl * G + rank < n; jl += kClWarps) {
@@ -1043,13 +1047,17 @@ __global__ void __launch_bounds__(kClThreads) hetrd_grid_kernel(double2* __restr
       cols[size_t(jl) * n + r] = a;
     }
   }
-  for (int r = tid; r < n; r += kClThreads) vbuf[r] = wbuf[r] = make_double2(0.0, 0.0);
-  double2 x[kGridRows];   // the pivot column, rows tid + kClThreads t
+  if (tid < kGridCols) vcol[tid] = wcol[tid] = make_double2(0.0, 0.0);
+  // rows tid + kClThreads t: the pivot column, the previous step's v and w
+  double2 x[kGridRows], v[kGridRows], w[kGridRows];
+  int slot[kGridRows];   // row r is this CTA's column slot, or -1
 #pragma unroll
   for (int t = 0; t < kGridRows; ++t) {
     const int r = tid + kClThreads * t;
     x[t] = r < n ? A[size_t(n - 1) * n + r] : make_double2(0.0, 0.0);
     if (r == n - 1) x[t].y = 0.0;
+    v[t] = w[t] = make_double2(0.0, 0.0);
+    slot[t] = r < n && r % G == rank ? r / G : -1;
   }
   // A is overwritten with the reflectors from the first step on: wait until
   // every CTA has read its columns
@@ -1065,63 +1073,67 @@ __global__ void __launch_bounds__(kClThreads) hetrd_grid_kernel(double2* __restr
   int par = 0;
   for (int i0 = n - 2; i0 >= 0; --i0, par ^= 1) {
     const int c = i0 + 1, L = i0 + 1;
-#pragma unroll
-    for (int t = 0; t < kGridRows; ++t) {
-      const int r = tid + kClThreads * t;
-      if (r < L) xbuf[r] = x[t];
-      if (r == c && rank == 0) dout[c] = x[t].x;
-    }
-    __syncthreads();   // xbuf, vbuf, wbuf
     double2* gu = exchange + size_t(2 * par) * n;
     double2* ga = gu + n;
     double norm = 0;
-    bool first = true;
-    int jl0 = warp;
-    do {   // at least once: every warp needs the norm
-      double2 ws[kClCols], vs[kClCols];
+#pragma unroll
+    for (int t = 0; t < kGridRows; ++t) {
+      const int r = tid + kClThreads * t;
+      if (r < i0) norm += x[t].x * x[t].x + x[t].y * x[t].y;
+      if (r == i0) s_al = x[t];
+      if (r == c && rank == 0) dout[c] = x[t].x;
+    }
+    __syncthreads();   // vcol, wcol
+    // columns s < L: the previous rank-2 update, then u(s) = sum_r conj(A(r, s)) x(r)
+    for (int jl0 = 0; jl0 * G + rank < L; jl0 += kClCols) {
       double acc[2 * kClCols] = {};
-      bool on[kClCols];
-      int pivot = -1;   // the slot that holds column i0
 #pragma unroll
       for (int k = 0; k < kClCols; ++k) {
-        const int s = (jl0 + k * kClWarps) * G + rank;
-        on[k] = s < L;
-        if (s == i0) pivot = k;
-        ws[k] = on[k] ? wbuf[s] : make_double2(0.0, 0.0);
-        vs[k] = on[k] ? vbuf[s] : make_double2(0.0, 0.0);
-      }
-      for (int r = lane; r < L; r += 32) {
-        const double2 pv = vbuf[r], pw = wbuf[r], xx = xbuf[r];
-        if (first && r < i0) norm += xx.x * xx.x + xx.y * xx.y;
+        const int s = (jl0 + k) * G + rank;
+        if (s < L) {
+          const double2 ws = wcol[jl0 + k], vs = vcol[jl0 + k];
+          double2* col = cols + size_t(jl0 + k) * n;
 #pragma unroll
-        for (int k = 0; k < kClCols; ++k) {
-          if (on[k]) {
-            double2* e = cols + size_t(jl0 + k * kClWarps) * n + r;
-            double2 a = *e;
-            a.x -= (pv.x * ws[k].x + pv.y * ws[k].y) + (pw.x * vs[k].x + pw.y * vs[k].y);
-            a.y -= (pv.y * ws[k].x - pv.x * ws[k].y) + (pw.y * vs[k].x - pw.x * vs[k].y);
-            *e = a;
-            if (k == pivot) ga[r] = a;
-            acc[2 * k] += a.x * xx.x + a.y * xx.y;
-            acc[2 * k + 1] += a.x * xx.y - a.y * xx.x;
+          for (int t = 0; t < kGridRows; ++t) {
+            const int r = tid + kClThreads * t;
+            if (r < L) {
+              double2 a = col[r];
+              a.x -= (v[t].x * ws.x + v[t].y * ws.y) + (w[t].x * vs.x + w[t].y * vs.y);
+              a.y -= (v[t].y * ws.x - v[t].x * ws.y) + (w[t].y * vs.x - w[t].x * vs.y);
+              col[r] = a;
+              if (s == i0) ga[r] = a;
+              acc[2 * k] += a.x * x[t].x + a.y * x[t].y;
+              acc[2 * k + 1] += a.x * x[t].y - a.y * x[t].x;
+            }
           }
         }
       }
-      first = false;
-      const double own = warp_sum8(acc);                                // value lane >> 2
-      const double other = __shfl_xor_sync(0xffffffffu, own, 4);
-      const int s = (jl0 + (lane >> 3) * kClWarps) * G + rank;
-      if (s < L && (lane & 7) == 0) gu[s] = make_double2(own, other);
-      jl0 += kClWarps * kClCols;
-    } while (jl0 * G + rank < L);
-    const double2 al = xbuf[i0];
-    target += G;
-    __syncthreads();   // this CTA's part of u and of the pivot column is written
-    if (tid == 0) {
-      __threadfence();
-      atomicAdd(counter, 1);
+      const double sum = warp_sum8(acc);   // value lane >> 2
+      if ((lane & 3) == 0) red[warp][2 * jl0 + (lane >> 2)] = sum;
     }
     for (int off = 16; off > 0; off >>= 1) norm += __shfl_xor_sync(0xffffffffu, norm, off);
+    if (lane == 0) rnorm[warp] = norm;
+    const double2 own_al = s_al;   // written before the barrier above
+    target += G;
+    __syncthreads();   // red, rnorm; this CTA's part of the pivot column is written
+    if (warp == 0) {
+      const int s = (lane >> 1) * G + rank;
+      if (s < L) {   // at most 2 kGridCols <= 32 values
+        double sum = red[0][lane];
+#pragma unroll
+        for (int k = 1; k < kClWarps; ++k) sum += red[k][lane];
+        reinterpret_cast<double*>(gu + s)[lane & 1] = sum;
+      }
+      __syncwarp();
+      if (lane == 0) {
+        __threadfence();
+        atomicAdd(counter, 1);
+      }
+    }
+    norm = rnorm[0];
+#pragma unroll
+    for (int k = 1; k < kClWarps; ++k) norm += rnorm[k];
+    const double2 al = own_al;
     double2 tau = make_double2(0.0, 0.0), sc = make_double2(1.0, 0.0);
     double beta = al.x;
     if (!(norm == 0.0 && al.y == 0.0)) {   // zlarfg on (alpha = x(i0), x(0:i0-1))
@@ -1150,16 +1162,20 @@ __global__ void __launch_bounds__(kClThreads) hetrd_grid_kernel(double2* __restr
       if (r <= i0) {
         ur[t] = __ldcg(gu + r);
         ar[t] = __ldcg(ga + r);
-        qs += x[t].x * ur[t].x + x[t].y * ur[t].y;   // Re(conj(x) u)
       }
     }
     const double2 ui = __ldcg(gu + i0), ai = __ldcg(ga + i0);
-    for (int off = 16; off > 0; off >>= 1) qs += __shfl_xor_sync(0xffffffffu, qs, off);
-    if (lane == 0) red[warp] = qs;
-    __syncthreads();
-    qs = red[0];
 #pragma unroll
-    for (int w = 1; w < kClWarps; ++w) qs += red[w];
+    for (int t = 0; t < kGridRows; ++t) {
+      const int r = tid + kClThreads * t;
+      if (r <= i0) qs += x[t].x * ur[t].x + x[t].y * ur[t].y;   // Re(conj(x) u)
+    }
+    for (int off = 16; off > 0; off >>= 1) qs += __shfl_xor_sync(0xffffffffu, qs, off);
+    if (lane == 0) rqs[warp] = qs;
+    __syncthreads();
+    qs = rqs[0];
+#pragma unroll
+    for (int k = 1; k < kClWarps; ++k) qs += rqs[k];
     const double2 sk = cconjmul(sc, kap);   // conj(sc) kappa
     const double vav = sc2 * qs + 2.0 * (sk.x * ui.x + sk.y * ui.y) + (kap.x * kap.x + kap.y * kap.y) * ai.x;
     const double a2 = -0.5 * tau2 * vav;
@@ -1169,15 +1185,17 @@ __global__ void __launch_bounds__(kClThreads) hetrd_grid_kernel(double2* __restr
     for (int t = 0; t < kGridRows; ++t) {
       const int r = tid + kClThreads * t;
       if (r <= i0) {
-        const double2 v = r < i0 ? cmul(x[t], sc) : make_double2(1.0, 0.0);
-        if (r < i0 && rank == c % G) A[size_t(c) * n + r] = v;
-        double2 w = cadd(cmul(tsc, ur[t]), cmul(tkap, ar[t]));
-        w.x += a2 * v.x;
-        w.y += a2 * v.y;
-        vbuf[r] = v;
-        wbuf[r] = w;
-        x[t].x = ar[t].x - (v.x * wi.x + v.y * wi.y) - w.x;
-        x[t].y = ar[t].y - (v.y * wi.x - v.x * wi.y) - w.y;
+        v[t] = r < i0 ? cmul(x[t], sc) : make_double2(1.0, 0.0);
+        if (r < i0 && rank == c % G) A[size_t(c) * n + r] = v[t];
+        w[t] = cadd(cmul(tsc, ur[t]), cmul(tkap, ar[t]));
+        w[t].x += a2 * v[t].x;
+        w[t].y += a2 * v[t].y;
+        if (slot[t] >= 0) {
+          vcol[slot[t]] = v[t];
+          wcol[slot[t]] = w[t];
+        }
+        x[t].x = ar[t].x - (v[t].x * wi.x + v[t].y * wi.y) - w[t].x;
+        x[t].y = ar[t].y - (v[t].y * wi.x - v[t].x * wi.y) - w[t].y;
       }
     }
   }
@@ -1189,7 +1207,7 @@ __global__ void __launch_bounds__(kClThreads) hetrd_grid_kernel(double2* __restr
 // launches fewer, while one product does not fill the GPU.
 constexpr int kSmallProducts = 176;
 
-constexpr size_t kGridSmem = 227 * 1024 - 256;   // leaves room for the kernel's static shared memory
+constexpr size_t kGridSmem = 227 * 1024 - 2560;   // leaves room for the kernel's static shared memory
 
 // CTAs of the cluster for an order-n tridiagonalisation: measured best at 8
 // from order 40 to 176 (order 80: 1, 2, 4, 8 and 16 CTAs 283, 218, 192, 183
@@ -1306,12 +1324,12 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
     const int p = hetrd_ctas(n);
     launch_cluster(hetrd_kernel, p, hetrd_smem(n, p), s, A, n, d.get(), e.get(), tau.get());
     rt.prof.launches += 1;
-  } else if (const size_t gsm = hetrd_grid_smem(n, rt.sms); n <= kGridMaxOrder && gsm <= kGridSmem) {
+  } else if (const size_t gsm = hetrd_grid_smem(n, rt.sms); n <= kGridMaxOrder && n <= kGridCols * rt.sms && gsm <= kGridSmem) {
     if (exchange.size() < 4 * size_t(n)) exchange.resize(4 * size_t(kGridMaxOrder));
     if (grid_state.size() == 0) grid_state.resize(2);   // barrier counter, error flag
     grid_state.zero(s);
     gave_up = grid_state.get() + 1;
-    raise_smem_limit(hetrd_grid_kernel, gsm);
+    raise_smem_limit(hetrd_grid_kernel, kGridSmem);   // static and dynamic together may pass 48 KB before gsm does
     double *dp = d.get(), *ep = e.get();
     double2 *tp = tau.get(), *xp = exchange.get();
     int *cp = grid_state.get(), *gp = cp + 1;

@@ -11,9 +11,10 @@ struct SmallEigen {
   // Orders the cluster kernels serve: the matrix fits the shared memory of 16
   // CTAs (432 x 432 x 16 bytes and the vectors).
   static constexpr int kOwnMaxOrder = 432;
-  // Orders whose tridiagonalisation the whole GPU's shared memory holds (148
-  // SMs: ceil(n / 148) n + 3 n elements of 16 bytes).  Above it cuSOLVER.
-  static constexpr int kGridMaxOrder = 1208;
+  // Orders whose tridiagonalisation goes over the whole GPU's shared memory
+  // (five rows a thread; 148 SMs hold ceil(n / 148) n elements of 16 bytes
+  // each up to 1,436).  Above it cuSOLVER.
+  static constexpr int kGridMaxOrder = 1280;
   int cap = 0;
   DeviceBuffer<double> d, e, Z, scratch, lam;
   DeviceBuffer<double2> tau, V, work;
