@@ -59,15 +59,20 @@ HALF_HD inline double assoc_legendre(int l, int m, double x) {
   return pmmp1;
 }
 
+// Factor of P_l^m(x) cos(m phi) (or sin) in the real harmonic (l, +-m), m >= 0.
+HALF_HD inline double real_ylm_norm(int l, int m) {
+  double norm = sqrt((2 * l + 1) / (4 * kPi) * factorial_d(l - m) / factorial_d(l + m));
+  double sgn = (m % 2) ? -1.0 : 1.0;
+  return m > 0 ? sqrt(2.0) * sgn * norm : norm;
+}
+
 // Real harmonic of the reference from x = cos(theta) and phi.
 HALF_HD inline double real_ylm(int l, int m, double x, double phi) {
   int am = m < 0 ? -m : m;
-  double p = assoc_legendre(l, am, x);
-  double norm = sqrt((2 * l + 1) / (4 * kPi) * factorial_d(l - am) / factorial_d(l + am));
-  double sgn = (am % 2) ? -1.0 : 1.0;
-  if (m > 0) return sqrt(2.0) * sgn * norm * p * cos(am * phi);
-  if (m < 0) return sqrt(2.0) * sgn * norm * p * sin(am * phi);
-  return norm * p;
+  double p = real_ylm_norm(l, am) * assoc_legendre(l, am, x);
+  if (m > 0) return p * cos(am * phi);
+  if (m < 0) return p * sin(am * phi);
+  return p;
 }
 
 // Per-species QDEP tables (src/half_uspp.F90:137-200): radial weights,
