@@ -619,9 +619,9 @@ struct AccRun {
     // skipped.  The library's own pencil solver (small orders) Jacobi-scales
     // the overlap and floors dependent pivots exactly like the metric step,
     // so [X P] spans the same space and the Ritz pairs are the same.  Larger
-    // pencils go to cuSOLVER zhegvd Jacobi-scaled here, whose Cholesky of
-    // the overlap then does the metric step's work; if that Cholesky (or
-    // the solve) fails, the step is redone with the metric normalisation.
+    // pencils are Jacobi-scaled here and go through a plain Cholesky of the
+    // overlap (SmallEigen::hegv, or cuSOLVER beyond its orders), which then
+    // does the metric step's work; if that Cholesky (or the solve) fails, the step is redone with the metric normalisation.
     // The FP64 mode keeps the reference's metric step.
     // Rayleigh-Ritz on Z = [X_U PU], X_U = the unlocked columns [nl, m) of X
     // (all of them without hard locking)

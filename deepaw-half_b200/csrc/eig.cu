@@ -5,10 +5,14 @@
 // Rayleigh-Ritz) once per iteration (src/half_cuda_iterative_solver.cuf:
 // 242-275).  For the sizes the solver meets (m <= a few hundred) those calls
 // are dominated by per-reflector back-transformation launches and a host
-// round trip.  Here the same reduction is kept -- B = U^H U (Cholesky),
-// C = U^-H A U^-1, Householder tridiagonalisation (cuSOLVER zhetrd) -- and
-// the rest is done by two kernels of this file:
+// round trip.  Here the same reduction -- X with X^H B X = I, C = X^H A X,
+// Householder tridiagonalisation, Y = X V -- runs in kernels that keep the
+// matrix in the shared memory of a cluster of CTAs (orders to 432):
 //
+//   metric_factor_kernel   X = D R^-1 from a floored Cholesky factorisation;
+//   hetrd_kernel           tridiagonalisation (hetrd_grid_kernel: over the
+//                          whole GPU, orders 434 to 1,280, between cuSOLVER's
+//                          zpotrf / ztrsm and zunmtr / ztrsm);
 //   tridiag_values_kernel  eigenvalues of the real symmetric tridiagonal T by
 //                          multisection on Sturm counts (one warp per
 //                          eigenvalue, CTAs across the GPU);
@@ -18,12 +22,10 @@
 //                          whose members are iterated in order and
 //                          Gram-Schmidt orthogonalised against each other (the
 //                          strategy of LAPACK's dstebz/dstein);
-//   back_transform_kernel  V = Q Z with Q = H(n-1)...H(1) from zhetrd's
-//                          reflectors staged in shared memory, one warp per
-//                          eigenvector.
+//   back_transform_kernel  V = Q Z with Q = H(n-1)...H(1), the reflectors
+//                          staged in shared memory, one warp per eigenvector.
 //
-// The eigenvectors are finally Y = U^-1 V (trsm), giving Y^H B Y = I, the
-// same normalisation as zhegvd (itype 1, upper).
+// Y^H B Y = I, the same normalisation as zhegvd (itype 1, upper).
 #include <algorithm>
 #include <cooperative_groups.h>
 

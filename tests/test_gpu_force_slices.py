@@ -1,5 +1,5 @@
-"""The force adjoint over band counts at the edges of its band tiles (32, 64,
-128) and of the contraction's 32-band tiles, for atoms of up to 8 and of 18
+"""The force adjoint over band counts at the edges of its band tiles (32 and
+64) and of the contraction's 32-band tiles, for atoms of up to 8 and of 18
 channels, with several plane-wave slices (both cells are small enough to need
 them), and staged host copies with padded leading dimensions.  Against the
 oracle's restatement on random states: sums of products of order one over
