@@ -338,7 +338,7 @@ struct SmallSolver {
   // orders of the own solver; those of the grid-wide tridiagonalisation in the
   // guard-band modes only (the FP64 mode keeps zhegvd there)
   bool own_order(int n) const {
-    return own && (n <= SmallEigen::kOwnMaxOrder || (range && n <= SmallEigen::kGridMaxOrder) || own_large);
+    return own && (n <= SmallEigen::kOwnMaxOrder || (range && SmallEigen::grid_order(rt, n)) || own_large);
   }
   // generalized problem of order n; the nev lowest eigenvectors are wanted
   void hegvd(double2* a, double2* b, int n, double* w, int nev) {
@@ -616,7 +616,7 @@ struct AccRun {
     }
     mark("orth_gemm");
     // In the guard-band modes the separate S-metric normalisation is
-    // skipped.  The library's own pencil solver (small orders) Jacobi-scales
+    // skipped.  The library's own pencil solver (to order 1,280) Jacobi-scales
     // the overlap and floors dependent pivots exactly like the metric step,
     // so [X P] spans the same space and the Ritz pairs are the same.  Larger
     // pencils are Jacobi-scaled here and go through a plain Cholesky of the
@@ -628,7 +628,7 @@ struct AccRun {
     const int mu = m - nl;
     const long long off = (long long)nl * n;
     const int ord = mu + np;
-    const bool own_pencil = ss.own && ord <= SmallEigen::kOwnMaxOrder;
+    const bool own_pencil = ss.own && (ord <= SmallEigen::kOwnMaxOrder || (ss.range && SmallEigen::grid_order(rt, ord)));
     bool skip_metric = guarded && ss.own;
     double2* hs = sc.hsub.get();
     double2* ssb = sc.ssub.get();

@@ -10,9 +10,9 @@
 // matrix in the shared memory of a cluster of CTAs (orders to 432):
 //
 //   metric_factor_kernel   X = D R^-1 from a floored Cholesky factorisation;
-//   hetrd_kernel           tridiagonalisation (hetrd_grid_kernel: over the
-//                          whole GPU, orders 434 to 1,280, between cuSOLVER's
-//                          zpotrf / ztrsm and zunmtr / ztrsm);
+//   hetrd_kernel           tridiagonalisation (both also over the whole GPU's
+//                          shared memory, orders 434 to 1,280, with cuSOLVER's
+//                          zunmtr behind them);
 //   tridiag_values_kernel  eigenvalues of the real symmetric tridiagonal T by
 //                          multisection on Sturm counts (one warp per
 //                          eigenvalue, CTAs across the GPU);
@@ -551,6 +551,15 @@ __global__ void hermitian_fill_kernel(double2* A, int n) {
 // around 120 (12-atom cell, B200): one CTA with the packed triangle, one
 // column per step, 281 us; a cluster with one column per step 235 us; this
 // kernel 135 us.
+//
+// Orders beyond a cluster (kGrid, cooperative launch): the same sweep over the
+// CTAs of the whole GPU, column block K on CTA K mod P, bounded grid barriers.
+// The panel (8 m elements) does not fit beside the columns there: a thread
+// takes rows of all the CTA's columns and reads their eight panel elements
+// from L2 once.  The 17 pencils of orders 434 to 1,200 of a 480-band solve:
+// 26.6 ms (10 us a block: two grid barriers, the owner's elimination, the
+// update); the solve 561 ms, 577 with cuSOLVER's zpotrf and three ztrsm in
+// place of this kernel and three products.
 constexpr int kClThreads = 256;
 constexpr int kClWarps = kClThreads / 32;
 constexpr int kClCols = 4;                        // columns a warp carries at once
@@ -569,27 +578,69 @@ __device__ __forceinline__ void group_barrier(int P) {
   }
 }
 
+constexpr unsigned long long kGridWaitNs = 2000000000ull;
+
+__device__ __forceinline__ int load_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Waits until `counter` reaches `target`; false when it does not in time or another CTA gave up.
+__device__ bool grid_wait(const int* counter, int target, int* err) {
+  unsigned long long t0 = 0;
+  for (unsigned spin = 0;; ++spin) {
+    if (load_acquire(counter) >= target) return true;
+    if ((spin & 255u) == 255u) {
+      unsigned long long t;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+      if (t0 == 0) t0 = t;
+      if (t - t0 > kGridWaitNs || *reinterpret_cast<volatile int*>(err) != 0) {
+        atomicExch(err, 1);
+        return false;
+      }
+    }
+  }
+}
+
+// Barrier of a cooperative launch's CTAs; false when it gave up.
+__device__ bool grid_barrier(int* counter, int& target, int* err) {
+  __shared__ int ok;
+  target += gridDim.x;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(counter, 1);
+    ok = grid_wait(counter, target, err);
+  }
+  __syncthreads();
+  return ok;
+}
+
 // Packed column storage of CTA `rank`: its t-th block (block t P + rank of
 // the matrix) starts at this element and keeps 8 columns of 8 (t P + rank + 1) rows.
 __host__ __device__ inline size_t factor_base(int t, int P, int rank) {
   return size_t(kFB) * kFB * (size_t(P) * t * (t - 1) / 2 + size_t(t) * (rank + 1));
 }
 
-__host__ inline size_t factor_smem(int m, int P) {
+__host__ inline size_t factor_smem(int m, int P, bool grid = false) {
   const int nblk = (m + kFB - 1) / kFB;
   size_t most = 0;
   for (int r = 0; r < P && r < nblk; ++r) most = std::max(most, factor_base((nblk - r + P - 1) / P, P, r));
   const size_t cols = size_t((nblk + P - 1) / P) * kFB;
-  return (most + size_t(kFB) * m + kFB * cols + 3 * kFB * kFB) * sizeof(double2) + (2 * size_t(m) + kFB) * sizeof(double);
+  return (most + (grid ? 0 : size_t(kFB) * m) + kFB * cols + 3 * kFB * kFB) * sizeof(double2) +
+         (2 * size_t(m) + kFB) * sizeof(double);
 }
 
 // Global scratch of the factor, in double2: the panel and the diagonal block, by parity of K.
 __host__ __device__ inline size_t factor_panel(int m) { return size_t(kFB) * m + 2 * kFB * kFB + kFB; }
 
+// grid_state (kGrid): barrier counter and error flag, zero at launch.
+template <bool kGrid>
 __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __restrict__ M, int m, int P,
                                                                    double2* __restrict__ panels,
-                                                                   int* __restrict__ status) {
-  const int rank = blockIdx.x;   // the grid is one cluster of P CTAs
+                                                                   int* __restrict__ status, int* grid_state) {
+  const int rank = blockIdx.x;   // the grid is one cluster of P CTAs, or a cooperative launch of P
   const int nblk = (m + kFB - 1) / kFB, nown = nblk > rank ? (nblk - rank + P - 1) / P : 0;
   const int maxown = (nblk + P - 1) / P * kFB;
   extern __shared__ __align__(16) double2 cols[];
@@ -599,7 +650,7 @@ __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __re
     if (s > most) most = s;
   }
   double2* F = cols + most;                                   // [kFB][m]
-  double2* sc = F + size_t(kFB) * m;                          // [kFB][maxown]: c_l of the owned columns
+  double2* sc = F + (kGrid ? 0 : size_t(kFB) * m);            // [kFB][maxown]: c_l of the owned columns
   double2* sW = sc + size_t(kFB) * maxown;                    // [kFB][kFB]: W(k0+l, k0+c) before its scaling
   double2* sC = sW + kFB * kFB;                               // [kFB][kFB]: c(l, c) inside the block
   double2* sD = sC + kFB * kFB;                               // [kFB][kFB]: the block; at the end T inside it
@@ -625,7 +676,15 @@ __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __re
     }
   }
   __syncthreads();
-  int bad = 0;
+  int bad = 0, target = 0;
+  auto barrier = [&]() {
+    if constexpr (kGrid) {
+      return grid_barrier(grid_state, target, grid_state + 1);
+    } else {
+      group_barrier(P);
+      return true;
+    }
+  };
   for (int K = 0; K < nblk; ++K) {
     const int k0 = K * kFB, kb = min(kFB, m - k0), k1 = k0 + kb, owner = K % P;
     double2* panel = panels + (K & 1) * factor_panel(m);
@@ -708,7 +767,10 @@ __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __re
       }
     }
     if (k1 >= m) break;   // the last block has no columns to its right
-    group_barrier(P);
+    if (!barrier()) {
+      if (tid == 0) atomicExch(status, 2);
+      return;
+    }
     if (rank != owner) {
       for (int e = tid; e < kFB * kFB; e += kClThreads) {
         sW[e] = __ldcg(pdiag + e);
@@ -744,7 +806,39 @@ __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __re
         col[l] = tv;
       }
     }
-    group_barrier(P);
+    if (!barrier()) {
+      if (tid == 0) atomicExch(status, 2);
+      return;
+    }
+    if constexpr (kGrid) {
+      const int last = nown > t0 ? min(m, ((nown - 1) * P + rank + 1) * kFB) : 0;   // rows of the longest column
+      for (int i = tid; i < last; i += kClThreads) {
+        if (i >= k0 && i < k1) continue;
+        double2 f[kFB];
+#pragma unroll
+        for (int l = 0; l < kFB; ++l) f[l] = __ldcg(panel + size_t(l) * m + i);
+        for (int t = t0; t < nown; ++t) {
+          const int j0 = (t * P + rank) * kFB;
+          double2* col = column_of(t, 0) + i;
+          const int stride = kFB * (t * P + rank + 1);
+#pragma unroll 4
+          for (int c = 0; c < kFB; ++c) {
+            if (i <= j0 + c && j0 + c < m) {
+              double2 x = col[size_t(c) * stride];
+#pragma unroll
+              for (int l = 0; l < kFB; ++l) {
+                const double2 g = sc[size_t(l) * maxown + t * kFB + c];
+                x.x -= f[l].x * g.x - f[l].y * g.y;
+                x.y -= f[l].x * g.y + f[l].y * g.x;
+              }
+              col[size_t(c) * stride] = x;
+            }
+          }
+        }
+      }
+      __syncthreads();
+      continue;
+    }
     if (P > 1) {
       for (int e = tid; e < kFB * m; e += kClThreads) {
         const int i = e % m;
@@ -996,33 +1090,9 @@ __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__
 // smaller ones, which take 10.4 ms in the cluster kernel).
 constexpr int kGridRows = (SmallEigen::kGridMaxOrder + kClThreads - 1) / kClThreads;
 constexpr int kGridCols = 12;   // columns a CTA can own, a multiple of kClCols
-constexpr unsigned long long kGridWaitNs = 2000000000ull;
 
 inline size_t hetrd_grid_smem(int n, int ctas) {
   return size_t((n + ctas - 1) / ctas) * n * sizeof(double2);
-}
-
-__device__ __forceinline__ int load_acquire(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// Waits until `counter` reaches `target`; false when it does not in time or another CTA gave up.
-__device__ bool grid_wait(const int* counter, int target, int* err) {
-  unsigned long long t0 = 0;
-  for (unsigned spin = 0;; ++spin) {
-    if (load_acquire(counter) >= target) return true;
-    if ((spin & 255u) == 255u) {
-      unsigned long long t;
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-      if (t0 == 0) t0 = t;
-      if (t - t0 > kGridWaitNs || *reinterpret_cast<volatile int*>(err) != 0) {
-        atomicExch(err, 1);
-        return false;
-      }
-    }
-  }
 }
 
 // exchange: u and the pivot column, 2 x 2 x n by parity of the step; counter
@@ -1217,6 +1287,8 @@ constexpr size_t kGridSmem = 227 * 1024 - 2560;   // leaves room for the kernel'
 int hetrd_ctas(int n) { return n <= 40 ? 4 : n <= 176 ? 8 : 16; }
 
 // CTAs for an order-m metric factor: one while its panel update is short.
+int factor_grid_ctas(const Runtime& rt, int m) { return std::min(rt.sms, ceil_div(m, kFB)); }
+
 int factor_ctas(int m) { return m <= 64 ? 1 : m <= 176 ? 8 : 16; }
 
 template <typename... KArgs, typename... Args>
@@ -1316,6 +1388,17 @@ void SmallEigen::reserve(Runtime& rt, int nmax) {
   work.resize(size_t(std::max({l1, l2, l3, 1})));
 }
 
+// Whether order n goes through the grid-wide kernels.
+bool SmallEigen::grid_order(const Runtime& rt, int n) {
+  return n > kOwnMaxOrder && n <= kGridMaxOrder && n <= kGridCols * rt.sms && hetrd_grid_smem(n, rt.sms) <= kGridSmem &&
+         factor_smem(n, factor_grid_ctas(rt, n), true) <= kSmemMax;
+}
+
+void SmallEigen::clear_grid_state(cudaStream_t s) {
+  if (grid_state.size() == 0) grid_state.resize(2);   // barrier counter, error flag
+  grid_state.zero(s);
+}
+
 // Hermitian eigenproblem of A (n x n, upper triangle used, destroyed); the nev
 // lowest eigenvectors go to V[:, :nev] (leading dimension n), eigenvalues to w.
 void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* status) {
@@ -1326,10 +1409,10 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
     const int p = hetrd_ctas(n);
     launch_cluster(hetrd_kernel, p, hetrd_smem(n, p), s, A, n, d.get(), e.get(), tau.get());
     rt.prof.launches += 1;
-  } else if (const size_t gsm = hetrd_grid_smem(n, rt.sms); n <= kGridMaxOrder && n <= kGridCols * rt.sms && gsm <= kGridSmem) {
+  } else if (grid_order(rt, n)) {
+    const size_t gsm = hetrd_grid_smem(n, rt.sms);
     if (exchange.size() < 4 * size_t(n)) exchange.resize(4 * size_t(kGridMaxOrder));
-    if (grid_state.size() == 0) grid_state.resize(2);   // barrier counter, error flag
-    grid_state.zero(s);
+    clear_grid_state(s);
     gave_up = grid_state.get() + 1;
     raise_smem_limit(hetrd_grid_kernel, kGridSmem);   // static and dynamic together may pass 48 KB before gsm does
     double *dp = d.get(), *ep = e.get();
@@ -1408,12 +1491,26 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
 void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, double* w, int* status, int* chol_status) {
   reserve(rt, n);
   cudaStream_t s = rt.stream;
-  if (n <= kOwnMaxOrder) {
+  if (n <= kOwnMaxOrder || grid_order(rt, n)) {
     // B -> X = D R^-1 with X^H B X = I (metric_factor_kernel), C = X^H A X,
     // C V = V Lambda, Y = X V: the same pencil reduction as zhegvd's
     // Cholesky / two triangular solves, with the factor inverted in shared
-    // memory and the products done by three small GEMMs
-    metric_normalize(rt, B, n, chol_status);
+    // memory and the products done by three GEMMs
+    if (n <= kOwnMaxOrder) {
+      metric_normalize(rt, B, n, chol_status);
+    } else {
+      int p = factor_grid_ctas(rt, n);
+      const size_t fsm = factor_smem(n, p, true);
+      if (panels.size() < 2 * factor_panel(n)) panels.resize(2 * factor_panel(kGridMaxOrder));
+      clear_grid_state(s);
+      raise_smem_limit(metric_factor_kernel<true>, kSmemMax);
+      double2* pp = panels.get();
+      int* gp = grid_state.get();
+      void* args[] = {&B, &n, &p, &pp, &chol_status, &gp};
+      HALF_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(metric_factor_kernel<true>), dim3(p),
+                                            dim3(kClThreads), args, fsm, s));
+      rt.prof.launches += 1;
+    }
     hermitian_fill_kernel<<<ceil_div((long long)n * n, 256), 256, 0, s>>>(A, n);
     rt.prof.launches += 1;
     const double2 one = make_double2(1.0, 0.0), zero = make_double2(0.0, 0.0);
@@ -1459,7 +1556,8 @@ bool SmallEigen::metric_normalize(Runtime& rt, double2* M, int m, int* status) {
   if (m > kOwnMaxOrder) return false;
   const int p = factor_ctas(m);
   if (panels.size() < 2 * factor_panel(m)) panels.resize(2 * factor_panel(kOwnMaxOrder));
-  launch_cluster(metric_factor_kernel, p, factor_smem(m, p), rt.stream, M, m, p, panels.get(), status);
+  launch_cluster(metric_factor_kernel<false>, p, factor_smem(m, p), rt.stream, M, m, p, panels.get(), status,
+                 static_cast<int*>(nullptr));
   rt.prof.launches += 1;
   return true;
 }

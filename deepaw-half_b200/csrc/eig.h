@@ -11,27 +11,34 @@ struct SmallEigen {
   // Orders the cluster kernels serve: the matrix fits the shared memory of 16
   // CTAs (432 x 432 x 16 bytes and the vectors).
   static constexpr int kOwnMaxOrder = 432;
-  // Orders whose tridiagonalisation goes over the whole GPU's shared memory
-  // (five rows a thread; 148 SMs hold ceil(n / 148) n elements of 16 bytes
-  // each up to 1,436).  Above it cuSOLVER.
+  // Orders whose factor and tridiagonalisation go over the whole GPU's shared
+  // memory (five rows a thread; 148 SMs hold ceil(n / 148) n elements of 16
+  // bytes each up to 1,436).  Above it cuSOLVER.
   static constexpr int kGridMaxOrder = 1280;
   int cap = 0;
   DeviceBuffer<double> d, e, Z, scratch, lam;
   DeviceBuffer<double2> tau, V, work;
   DeviceBuffer<double2> panels;   // exchange buffer of the metric factor's CTAs
   DeviceBuffer<double2> exchange; // and of the grid-wide tridiagonalisation's
-  DeviceBuffer<int> grid_state;   // its barrier counter and error flag
+  DeviceBuffer<int> grid_state;   // barrier counter and error flag of the grid-wide kernels
   DeviceBuffer<int> info;   // zhetrd status (reports illegal arguments only)
   void reserve(Runtime& rt, int nmax);
   // A (n x n, upper triangle, destroyed) -> nev lowest eigenpairs; vectors in
   // V[:, :nev].  *status (device) becomes nonzero if inverse iteration failed.
   void heev(Runtime& rt, double2* A, int n, int nev, double* w, int* status);
   // A y = lambda B y, B Hermitian positive definite; Y^H B Y = I.
-  // *chol_status (device) is zpotrf's info (> 0: B not positive definite).
+  // *chol_status (device): nonzero when the factor saw a pivot that is not
+  // finite (beyond the grid-wide kernels' orders zpotrf's info)
   void hegv(Runtime& rt, double2* A, double2* B, int n, int nev, double* w, int* status, int* chol_status);
   // ACC correction metric: M = P^H S P (m x m) -> U, upper triangular, with
   // (P U)^H S (P U) = I; returns false (nothing launched) when m is too large.
   bool metric_normalize(Runtime& rt, double2* M, int m, int* status);
+  // Whether an order above kOwnMaxOrder goes through the grid-wide kernels,
+  // whose metric factor floors dependent pivots like the cluster kernel's.
+  static bool grid_order(const Runtime& rt, int n);
+
+ private:
+  void clear_grid_state(cudaStream_t s);
 };
 
 // Selected eigenvalues of a large Hermitian matrix A (n x n, column-major,

@@ -1,7 +1,7 @@
 """The Rayleigh-Ritz pencils over the orders where their solver changes: the
 CTA counts of the cluster kernels (1, 4, 8 and 16 CTAs up to orders 40, 80,
 176 and 432), orders that leave the last CTAs with a column less, the
-grid-wide reduction from 434 to 1,280 and the first order beyond, which goes
+grid-wide factor and reduction from 434 to 1,280 and the first order beyond, which goes
 to cuSOLVER.  The converged eigenvalues of the 12-atom cell against the FP64
 dense solve (1e-8 eV, the parity tests' bound for converged solves)."""
 import numpy as np
