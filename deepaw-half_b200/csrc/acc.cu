@@ -97,6 +97,7 @@ __global__ void residual_norm_kernel(const C* __restrict__ hx, const C* __restri
                                      const double* __restrict__ eps, const int* __restrict__ info,
                                      const int* __restrict__ tc_err, double* __restrict__ norms,
                                      double* __restrict__ report) {
+  after_previous();
   if (blockIdx.x == 0 && threadIdx.x < 4)
     report[2 * gridDim.x + threadIdx.x] =
         threadIdx.x < 3 ? double(info[threadIdx.x]) : tc_err ? double(*tc_err) : 0.0;
@@ -134,6 +135,7 @@ __global__ void precondition_kernel(const C* __restrict__ hx, const C* __restric
                                     int np, const int* __restrict__ cols, const double* __restrict__ eps,
                                     const double* __restrict__ norms, double seed_threshold,
                                     const double* __restrict__ kinetic, CO* __restrict__ p) {
+  after_previous();
   long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= (long long)n * np) return;
   const int a = int(t / n), i = int(t - (long long)a * n);
@@ -195,6 +197,7 @@ __global__ void scale_rows_kernel(double2* __restrict__ y, int ld, int rows, int
 template <typename C>
 __global__ void gather_columns_kernel(const C* __restrict__ in, C* __restrict__ out, int n, int m,
                                       const int* __restrict__ perm) {
+  after_previous();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= (long long)n * m) return;
   const int j = int(t / n), i = int(t - (long long)j * n);
@@ -203,6 +206,7 @@ __global__ void gather_columns_kernel(const C* __restrict__ in, C* __restrict__ 
 
 __global__ void gather_values_kernel(const double* __restrict__ in, double* __restrict__ out, int m,
                                      const int* __restrict__ perm) {
+  after_previous();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j < m) out[j] = in[perm[j]];
 }
@@ -494,8 +498,8 @@ struct AccRun {
   // requested bands, which are the mcheck lowest Ritz values (req, physical
   // column indices in ascending order of their values; host sync)
   double residuals(std::vector<double>& norms, int* infos) {
-    residual_norm_kernel<C><<<m, 256, 0, rt.stream>>>(blk.hx(), blk.sx(), n, n, sc.w.get(), ss.info.get(),
-                                                      rt.tc_err.get(), sc.norms.get(), sc.report.get());
+    launch_chained(m, 256, 0, rt.stream, residual_norm_kernel<C>,
+        blk.hx(), blk.sx(), n, n, sc.w.get(), ss.info.get(), rt.tc_err.get(), sc.norms.get(), sc.report.get());
     ++rt.prof.launches;
     HALF_LAUNCH("residual norms");
     const size_t words = size_t(2) * m + 4;
@@ -556,12 +560,17 @@ struct AccRun {
     sc.perm.upload(perm, rt.stream);
     const int nx = blk.cur ^ 1;
     const long long cnt = (long long)n * m;
-    gather_columns_kernel<C><<<ceil_div(cnt, 256), 256, 0, rt.stream>>>(blk.x(), blk.X[nx].get(), n, m, sc.perm.get());
-    gather_columns_kernel<C><<<ceil_div(cnt, 256), 256, 0, rt.stream>>>(blk.hx(), blk.HX[nx].get(), n, m, sc.perm.get());
-    gather_columns_kernel<C><<<ceil_div(cnt, 256), 256, 0, rt.stream>>>(blk.sx(), blk.SX[nx].get(), n, m, sc.perm.get());
-    gather_values_kernel<<<ceil_div(m, 256), 256, 0, rt.stream>>>(sc.w.get(), sc.mu.get(), m, sc.perm.get());
+    launch_chained(ceil_div(cnt, 256), 256, 0, rt.stream, gather_columns_kernel<C>,
+        blk.x(), blk.X[nx].get(), n, m, sc.perm.get());
+    launch_chained(ceil_div(cnt, 256), 256, 0, rt.stream, gather_columns_kernel<C>,
+        blk.hx(), blk.HX[nx].get(), n, m, sc.perm.get());
+    launch_chained(ceil_div(cnt, 256), 256, 0, rt.stream, gather_columns_kernel<C>,
+        blk.sx(), blk.SX[nx].get(), n, m, sc.perm.get());
+    launch_chained(ceil_div(m, 256), 256, 0, rt.stream, gather_values_kernel,
+        sc.w.get(), sc.mu.get(), m, sc.perm.get());
     HALF_CUDA(cudaMemcpyAsync(sc.w.get(), sc.mu.get(), m * sizeof(double), cudaMemcpyDeviceToDevice, rt.stream));
-    gather_values_kernel<<<ceil_div(m, 256), 256, 0, rt.stream>>>(sc.norms.get(), sc.mu.get(), m, sc.perm.get());
+    launch_chained(ceil_div(m, 256), 256, 0, rt.stream, gather_values_kernel,
+        sc.norms.get(), sc.mu.get(), m, sc.perm.get());
     HALF_CUDA(cudaMemcpyAsync(sc.norms.get(), sc.mu.get(), m * sizeof(double), cudaMemcpyDeviceToDevice, rt.stream));
     HALF_LAUNCH("lock columns");
     rt.prof.launches += 5;
@@ -588,9 +597,9 @@ struct AccRun {
       cols = sc.active.get();
     }
     long long nm = (long long)n * np;
-    precondition_kernel<C><<<ceil_div(nm, 256), 256, 0, rt.stream>>>(blk.hx(), blk.sx(), n, n, m, np, cols, sc.w.get(),
-                                                                       sc.norms.get(), seed_threshold, sc.kinetic.get(),
-                                                                       blk.P.get());
+    launch_chained(ceil_div(nm, 256), 256, 0, rt.stream, precondition_kernel<C>,
+        blk.hx(), blk.sx(), n, n, m, np, cols, sc.w.get(), sc.norms.get(), seed_threshold, sc.kinetic.get(),
+        blk.P.get());
     ++rt.prof.launches;
     HALF_LAUNCH("precondition");
     mark("precondition");
@@ -930,7 +939,7 @@ void solve_acc(Context& ctx, KOperatorSet& ks, int nbands, bool want_vectors, So
   out.overlap_max = -1.0;
   out.dvectors.resize(size_t(n) * mreq);
   sc.perm.upload(req, rt.stream);
-  gather_columns_kernel<double2><<<ceil_div((long long)n * mreq, 256), 256, 0, rt.stream>>>(
+  launch_chained(ceil_div((long long)n * mreq, 256), 256, 0, rt.stream, gather_columns_kernel<double2>,
       b64.x(), out.dvectors.get(), n, mreq, sc.perm.get());
   HALF_LAUNCH("ACC output gather");
   ++rt.prof.launches;

@@ -87,6 +87,7 @@ __device__ __forceinline__ void gram_tile(const GramArgs& g, int t, int& p, int&
 // rows ti + 8 r and columns tj + 8 q of the 32 x 32 tile.
 __global__ void __launch_bounds__(kGramThreads) zgram_kernel(GramArgs g, int kper, int slices,
                                                              double2* __restrict__ partial) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* const sa = reinterpret_cast<double2*>(smem_raw);   // [2][kT][kGramPitch]
   double2* const sb = sa + 2 * kT * kGramPitch;
@@ -160,6 +161,7 @@ __global__ void __launch_bounds__(kGramThreads) zgram_kernel(GramArgs g, int kpe
 
 // C = the slices' tiles added in order; one CTA of 256 threads per quarter tile.
 __global__ void __launch_bounds__(256) zgram_reduce_kernel(GramArgs g, int slices, const double2* __restrict__ partial) {
+  after_previous();
   const int tile = blockIdx.x >> 2, e = (blockIdx.x & 3) * 256 + threadIdx.x, tiles = gridDim.x >> 2;
   int p, bi, bj;
   gram_tile(g, tile, p, bi, bj);
@@ -184,6 +186,7 @@ struct UpdateArgs {
 // One CTA per (64 rows, 32 columns, block): 128 threads, thread (ti, tj) owns
 // rows ti + 16 r and columns tj + 8 q.
 __global__ void __launch_bounds__(kUpThreads) zupdate_kernel(UpdateArgs u) {
+  after_previous();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double2* const sz = reinterpret_cast<double2*>(smem_raw);   // [2][kUpK][kUpRows]
   double2* const sy = sz + 2 * kUpK * kUpRows;                // [2][kT][kUpPitch]
@@ -320,11 +323,13 @@ void zgram(Runtime& rt, int n, const ZBlock& a, const ZBlock* b, double2* const*
   const size_t need = slices > 1 ? size_t(slices) * tiles * kT * kT : 0;
   if (rt.zwork.size() < need) rt.zwork.resize(need);
   raise_smem_limit(zgram_kernel, kGramSmem);
-  zgram_kernel<<<dim3(tiles, slices), kGramThreads, kGramSmem, rt.stream>>>(g, kper, slices, rt.zwork.get());
+  launch_chained(dim3(tiles, slices), kGramThreads, kGramSmem, rt.stream, zgram_kernel,
+      g, kper, slices, rt.zwork.get());
   HALF_LAUNCH("block Gram products");
   ++rt.prof.launches;
   if (slices > 1) {
-    zgram_reduce_kernel<<<4 * tiles, 256, 0, rt.stream>>>(g, slices, rt.zwork.get());
+    launch_chained(4 * tiles, 256, 0, rt.stream, zgram_reduce_kernel,
+        g, slices, rt.zwork.get());
     HALF_LAUNCH("block Gram reduction");
     ++rt.prof.launches;
   }
@@ -359,7 +364,8 @@ void zupdate(Runtime& rt, int n, const ZBlock* z, const double2* y, int ldy, dou
   u.alpha = alpha;
   u.beta = beta;
   raise_smem_limit(zupdate_kernel, kUpSmem);
-  zupdate_kernel<<<dim3(ceil_div(n, kUpRows), ceil_div(cols, kT), count), kUpThreads, kUpSmem, rt.stream>>>(u);
+  launch_chained(dim3(ceil_div(n, kUpRows), ceil_div(cols, kT), count), kUpThreads, kUpSmem, rt.stream, zupdate_kernel,
+      u);
   HALF_LAUNCH("block update");
   ++rt.prof.launches;
 }

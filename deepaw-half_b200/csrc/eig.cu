@@ -217,6 +217,7 @@ __global__ void __launch_bounds__(32 * kValueWarps) tridiag_values_kernel(const 
                                                                           int ne, double* __restrict__ lam,
                                                                           const int* __restrict__ grid_err,
                                                                           int* __restrict__ status) {
+  wait_previous();
   extern __shared__ double sm[];
   double* d = sm;
   double* e = d + n;
@@ -265,6 +266,7 @@ __global__ void __launch_bounds__(kVectorThreads) tridiag_vectors_kernel(
     const double* __restrict__ d_in, const double* __restrict__ e_in, int n, int nev, int ne, int per,
     const double* __restrict__ lam_g, double* __restrict__ w, double* __restrict__ Z, double* __restrict__ gscratch,
     int* __restrict__ status) {
+  wait_previous();
   extern __shared__ double sm[];
   double* d = sm;
   double* e = d + n;
@@ -397,6 +399,7 @@ __global__ void __launch_bounds__(32 * kBackWarps) back_transform_kernel(const d
                                                                          const double2* __restrict__ tau,
                                                                          const double* __restrict__ Z, int n, int nev,
                                                                          int chunk, double2* __restrict__ V) {
+  wait_previous();
   extern __shared__ __align__(16) double2 vs[];     // chunk x n
   double2* ts = vs + (size_t)chunk * n;             // chunk
   double2* gram = ts + chunk;                       // chunk / 4 x 8: g10, g20, g21, g30, g31, g32
@@ -499,6 +502,7 @@ __global__ void __launch_bounds__(32 * kBackWarps) back_transform_kernel(const d
 
 // lower triangle from the upper one (Hermitian)
 __global__ void hermitian_fill_kernel(double2* A, int n) {
+  after_previous();
   long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= (long long)n * n) return;
   int j = int(t / n), i = int(t - (long long)j * n);
@@ -640,6 +644,7 @@ template <bool kGrid>
 __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __restrict__ M, int m, int P,
                                                                    double2* __restrict__ panels,
                                                                    int* __restrict__ status, int* grid_state) {
+  wait_previous();
   const int rank = blockIdx.x;   // the grid is one cluster of P CTAs, or a cooperative launch of P
   const int nblk = (m + kFB - 1) / kFB, nown = nblk > rank ? (nblk - rank + P - 1) / P : 0;
   const int maxown = (nblk + P - 1) / P * kFB;
@@ -930,6 +935,7 @@ static_assert(SmallEigen::kOwnMaxOrder <= kTrdRows * kClThreads, "rows of a vect
 
 __global__ void __launch_bounds__(kClThreads) hetrd_kernel(double2* __restrict__ A, int n, double* __restrict__ dout,
                                                            double* __restrict__ eout, double2* __restrict__ tauout) {
+  wait_previous();
   cg::cluster_group cl = cg::this_cluster();
   const int P = int(cl.num_blocks()), rank = int(cl.block_rank());   // P is a power of two
   const int lg = 31 - __clz(P);
@@ -1300,13 +1306,15 @@ void launch_cluster(void (*kernel)(KArgs...), int ctas, size_t smem, cudaStream_
   cfg.blockDim = dim3(kClThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = ctas;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // as launch_chained
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   HALF_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 
@@ -1434,8 +1442,8 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
   const int ne = std::min(n, nev + kExtraEig);
   const size_t vsm = 3 * size_t(n) * sizeof(double);
   raise_smem_limit(tridiag_values_kernel, vsm);
-  tridiag_values_kernel<<<ceil_div(ne, kValueWarps), 32 * kValueWarps, vsm, s>>>(d.get(), e.get(), n, ne, lam.get(),
-                                                                                  gave_up, status);
+  launch_chained(ceil_div(ne, kValueWarps), 32 * kValueWarps, vsm, s, tridiag_values_kernel,
+      d.get(), e.get(), n, ne, lam.get(), gave_up, status);
   HALF_LAUNCH("tridiagonal eigenvalues");
   size_t tsm = (2 * size_t(n) + ne) * sizeof(double) + size_t(ne) * sizeof(int);
   if (tsm > kSmemMax) fail(kCapacity, "subspace eigenproblem too large for the tridiagonal solver: n=" + std::to_string(n));
@@ -1451,8 +1459,8 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
     per = kVectorThreads;
   }
   raise_smem_limit(tridiag_vectors_kernel, tsm);
-  tridiag_vectors_kernel<<<ceil_div(nev, per), kVectorThreads, tsm, s>>>(d.get(), e.get(), n, nev, ne, per, lam.get(), w,
-                                                                          Z.get(), gs, status);
+  launch_chained(ceil_div(nev, per), kVectorThreads, tsm, s, tridiag_vectors_kernel,
+      d.get(), e.get(), n, nev, ne, per, lam.get(), w, Z.get(), gs, status);
   HALF_LAUNCH("tridiagonal eigenvectors");
   if (n > kOwnMaxOrder) {
     // large orders: cuSOLVER's blocked back-transformation (zunmtr, Q Z with
@@ -1475,8 +1483,8 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
   const size_t bsm = size_t(blocks) * per_block;
   auto back = [&](auto kernel) {
     raise_smem_limit(kernel, bsm);
-    kernel<<<ceil_div(nev, kBackWarps), 32 * kBackWarps, bsm, s>>>(A, tau.get(), Z.get(), n, nev, blocks * kBackBlock,
-                                                                   V.get());
+    launch_chained(ceil_div(nev, kBackWarps), 32 * kBackWarps, bsm, s, kernel, A, tau.get(), Z.get(), n, nev,
+                   blocks * kBackBlock, V.get());
   };
   if (n <= 64) back(back_transform_kernel<2>);
   else if (n <= 160) back(back_transform_kernel<5>);
@@ -1511,7 +1519,8 @@ void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, doubl
                                             dim3(kClThreads), args, fsm, s));
       rt.prof.launches += 1;
     }
-    hermitian_fill_kernel<<<ceil_div((long long)n * n, 256), 256, 0, s>>>(A, n);
+    launch_chained(ceil_div((long long)n * n, 256), 256, 0, s, hermitian_fill_kernel,
+        A, n);
     rt.prof.launches += 1;
     const double2 one = make_double2(1.0, 0.0), zero = make_double2(0.0, 0.0);
     if (n <= kSmallProducts) {
@@ -1534,7 +1543,8 @@ void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, doubl
   cusolver_check(cusolverDnZpotrf(rt.solver, CUBLAS_FILL_MODE_UPPER, n, Bc, n,
                                   reinterpret_cast<cuDoubleComplex*>(work.get()), int(work.size()), chol_status),
                  "zpotrf");
-  hermitian_fill_kernel<<<ceil_div((long long)n * n, 256), 256, 0, s>>>(A, n);
+  launch_chained(ceil_div((long long)n * n, 256), 256, 0, s, hermitian_fill_kernel,
+      A, n);
   rt.prof.launches += 1;
   const cuDoubleComplex one = make_cuDoubleComplex(1.0, 0.0);
   cublas_check(cublasZtrsm(rt.blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_C, CUBLAS_DIAG_NON_UNIT, n, n,

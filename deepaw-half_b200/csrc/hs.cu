@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(kPlaneThreads, sizeof(R) == 4 ? 2 : 1)
                         const int* __restrict__ plane_start, const int* __restrict__ spos,
                         const int* __restrict__ row_start, const int* __restrict__ row_list, FFTPlan py, FFTPlan pz,
                         const cplx_t<R>* __restrict__ tw_yz, cplx_t<R>* __restrict__ work) {
+  wait_previous();
   using C = cplx_t<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const PlaneSmem<R> sm(smem_raw, n2, n3);
@@ -201,6 +202,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 2) k2_xlines(cplx_t<
                                                  const int* __restrict__ slot_plane, FFTPlan px,
                                                  const cplx_t<R>* __restrict__ tw_x, const R* __restrict__ veff, int nb,
                                                  int bands_per_cta) {
+  wait_previous();
   using C = cplx_t<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* const tw = reinterpret_cast<C*>(smem_raw);
@@ -264,6 +266,7 @@ __global__ void __launch_bounds__(kPlaneThreads, sizeof(R) == 4 ? 2 : 1)
                         const int* __restrict__ row_start, const int* __restrict__ row_list, FFTPlan py, FFTPlan pz,
                         const cplx_t<R>* __restrict__ tw_yz, const cplx_t<R>* __restrict__ psi, long long ld, int b0,
                         const R* __restrict__ kinetic, cplx_t<R>* __restrict__ hpsi, cplx_t<R>* __restrict__ spsi) {
+  wait_previous();
   using C = cplx_t<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const PlaneSmem<R> sm(smem_raw, n2, n3);
@@ -383,6 +386,7 @@ __global__ void mix_kernel(const cplx_t<R>* __restrict__ coeff, int np, int nb, 
                            const int* __restrict__ col_dofs, const int* __restrict__ col_qofs,
                            const R* __restrict__ dall, const R* __restrict__ qall, cplx_t<R>* __restrict__ dy,
                            cplx_t<R>* __restrict__ qy) {
+  after_previous();
   using C = cplx_t<R>;
   long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (idx >= (long long)np * nb) return;
@@ -792,17 +796,17 @@ void apply_hs(Context& ctx, KOperatorSet& ks, const cplx_t<R>* x, long long ld, 
   const int ev_local = ev_sweep;
   for (int b0 = 0; b0 < nb; b0 += chunk) {
     int nbc = std::min(chunk, nb - b0);
-    k1_sphere_to_planes<R><<<dim3(op.nplanes, nbc), pth, psm, s>>>(
-        x, ld, b0, op.n2, op.n3, op.nplanes, op.plane_start.get(), op.spos.get(), op.row_start.get(), op.row_list.get(),
-        op.ay.plan, op.az.plan, op.tw.get() + op.n1, op.work.get());
+    launch_chained(dim3(op.nplanes, nbc), pth, psm, s, k1_sphere_to_planes<R>,
+        x, ld, b0, op.n2, op.n3, op.nplanes, op.plane_start.get(), op.spos.get(), op.row_start.get(),
+        op.row_list.get(), op.ay.plan, op.az.plan, op.tw.get() + op.n1, op.work.get());
     // bands per K2 CTA: as many as keep about eight CTAs per SM busy
     const int lines = op.n2 * tiles;
     const int groups = std::max(1, std::min(nbc, ceil_div(8 * sms, lines)));
     const int bpc = ceil_div(nbc, groups);
-    k2_xlines<R><<<dim3(lines, ceil_div(nbc, bpc)), xline_threads(op.ax.plan), xsm, s>>>(
-        op.work.get(), op.n1, op.n2, op.n3, op.nplanes, op.slot_plane.get(), op.ax.plan, op.tw.get(), op.veff.get(), nbc,
-        bpc);
-    k3_planes_to_sphere<R><<<dim3(op.nplanes, nbc), pth, psm, s>>>(
+    launch_chained(dim3(lines, ceil_div(nbc, bpc)), xline_threads(op.ax.plan), xsm, s, k2_xlines<R>,
+        op.work.get(), op.n1, op.n2, op.n3, op.nplanes, op.slot_plane.get(), op.ax.plan, op.tw.get(), op.veff.get(),
+        nbc, bpc);
+    launch_chained(dim3(op.nplanes, nbc), pth, psm, s, k3_planes_to_sphere<R>,
         op.work.get(), op.n2, op.n3, op.nplanes, op.plane_start.get(), op.spos.get(), op.row_start.get(),
         op.row_list.get(), op.ay.plan, op.az.plan, op.tw.get() + op.n1, x, ld, b0, op.kinetic.get(), hx, sx);
     pf.launches += 3;
@@ -839,10 +843,9 @@ void apply_nonlocal(Runtime& rt, KOperator<R>& op, const cplx_t<R>* x, long long
   }
   const C one = cval<R>(1.0), zero = cval<R>(0.0);
   auto mix = [&]() {
-    mix_kernel<R><<<ceil_div((long long)op.np * nb, 256), 256, 0, s>>>(op.coeff.get(), op.np, nb, op.col_base.get(),
-                                                                       op.col_a.get(), op.col_nlm.get(), op.col_dofs.get(),
-                                                                       op.col_qofs.get(), op.dall.get(), op.qall.get(),
-                                                                       op.dy.get(), op.qy.get());
+    launch_chained(ceil_div((long long)op.np * nb, 256), 256, 0, s, mix_kernel<R>,
+        op.coeff.get(), op.np, nb, op.col_base.get(), op.col_a.get(), op.col_nlm.get(), op.col_dofs.get(),
+        op.col_qofs.get(), op.dall.get(), op.qall.get(), op.dy.get(), op.qy.get());
     HALF_LAUNCH("mix");
     ++rt.prof.launches;
   };
@@ -946,7 +949,7 @@ void accumulate_band_density(KOperatorSet& ks, const double2* x, long long ld, i
   const int tiles = (op.n3 + kXTile - 1) / kXTile;
   for (int b0 = 0; b0 < nb; b0 += chunk) {
     const int nbc = std::min(chunk, nb - b0);
-    k1_sphere_to_planes<double><<<dim3(op.nplanes, nbc), pth, psm, s>>>(
+    launch_chained(dim3(op.nplanes, nbc), pth, psm, s, k1_sphere_to_planes<double>,
         x, ld, b0, op.n2, op.n3, op.nplanes, op.plane_start.get(), op.spos.get(), op.row_start.get(),
         op.row_list.get(), op.ay.plan, op.az.plan, op.tw.get() + op.n1, op.work.get());
     k2_density<<<op.n2 * tiles, xline_threads(op.ax.plan), dsm, s>>>(

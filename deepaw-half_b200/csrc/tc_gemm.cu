@@ -142,6 +142,7 @@ __device__ __forceinline__ float2 projector_value(const TcOperand& op, int col, 
 // kProjConj: row = projector column, k = plane wave).
 __global__ void presplit_kernel(TcOperand op, int rows_pad, int nkb, unsigned char* __restrict__ out,
                                 long long plane_bytes) {
+  wait_previous();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= (long long)rows_pad * nkb * 2) return;
   const int r = int(t % rows_pad);
@@ -206,6 +207,7 @@ constexpr int kSplitRows = 32, kSplitK = 64, kSplitPitch = kSplitK + 1;   // odd
 
 __global__ void __launch_bounds__(256) presplit_k_kernel(TcOperand op, int rows_pad, int nkb,
                                                          unsigned char* __restrict__ out, long long plane_bytes) {
+  wait_previous();
   __shared__ float2 tile[kSplitRows * kSplitPitch];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rtiles = (rows_pad + kSplitRows - 1) / kSplitRows;
@@ -420,6 +422,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 template <typename T>
 __global__ void splitk_reduce_kernel(const float2* __restrict__ W, int S, int M, int N, double2 alpha, double2 beta,
                                      T* C, T* C2, int split_col, long long ldc) {
+  wait_previous();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= (long long)M * N) return;
   const int i = int(t % M), j = int(t / M);
@@ -442,9 +445,11 @@ void launch_presplit(const TcOperand& op, int rows_pad, int nkb, unsigned char* 
                      cudaStream_t st) {
   if (op.kind == TcOperand::kDenseK) {
     const long long ctas = (long long)ceil_div(rows_pad, kSplitRows) * ceil_div((long long)nkb * kBK, kSplitK);
-    presplit_k_kernel<<<unsigned(ctas), 256, 0, st>>>(op, rows_pad, nkb, out, plane_bytes);
+    launch_chained(unsigned(ctas), 256, 0, st, presplit_k_kernel,
+        op, rows_pad, nkb, out, plane_bytes);
   } else {
-    presplit_kernel<<<ceil_div((long long)rows_pad * nkb * 2, 256), 256, 0, st>>>(op, rows_pad, nkb, out, plane_bytes);
+    launch_chained(ceil_div((long long)rows_pad * nkb * 2, 256), 256, 0, st, presplit_kernel,
+        op, rows_pad, nkb, out, plane_bytes);
   }
   HALF_LAUNCH("tensor-core operand split");
 }
@@ -626,6 +631,7 @@ void tc_cgemm(Runtime& rt, const TcOperand& A, const TcOperand& B, int M, int N,
   if (nkb > 0) {
     const int e0 = span0 >= 0 ? span0 : pf.record(st);
     if (!key.empty()) tune_token = Tuner::begin(key, tune_index, st);   // the product alone, no allocation or split pass
+    // a plain launch: set up early, its CTAs (as many as SMs) would share the SMs that drain first
     tc_cgemm_kernel<<<dim3(mt, nt, splits / groups), kThreads, smem, st>>>(Ak, Bk, bn, nst, kbps, groups, nkb, o,
                                                                            rt.tc_err.get());
     HALF_LAUNCH("tensor-core cgemm");
@@ -640,13 +646,11 @@ void tc_cgemm(Runtime& rt, const TcOperand& A, const TcOperand& B, int M, int N,
     const int S = nkb > 0 ? splits : 0;
     const float2* W = reinterpret_cast<const float2*>(rt.tc_work.get());
     if (c_fp64)
-      splitk_reduce_kernel<double2><<<ceil_div(mn, 256), 256, 0, st>>>(W, S, M, N, alpha, beta,
-                                                                       static_cast<double2*>(C),
-                                                                       static_cast<double2*>(C2), split_col, ldc);
+      launch_chained(ceil_div(mn, 256), 256, 0, st, splitk_reduce_kernel<double2>,
+          W, S, M, N, alpha, beta, static_cast<double2*>(C), static_cast<double2*>(C2), split_col, ldc);
     else
-      splitk_reduce_kernel<float2><<<ceil_div(mn, 256), 256, 0, st>>>(W, S, M, N, alpha, beta,
-                                                                      static_cast<float2*>(C),
-                                                                      static_cast<float2*>(C2), split_col, ldc);
+      launch_chained(ceil_div(mn, 256), 256, 0, st, splitk_reduce_kernel<float2>,
+          W, S, M, N, alpha, beta, static_cast<float2*>(C), static_cast<float2*>(C2), split_col, ldc);
     HALF_LAUNCH("split-K reduction");
     ++rt.prof.launches;
   }
