@@ -208,10 +208,10 @@ void raise_smem_limit(F* kernel, size_t bytes) {
 // wait_previous() before anything else, in every thread: what it reads and
 // writes is then ordered as in a plain launch, also with kernels further back,
 // since its predecessor did the same.  Takes 1-2 us of launch gap off each
-// link of the acc iteration's chain of short kernels: 2-atom FP64 solve (57
-// launches an iteration) 92.5 -> 88.3 ms on a slow host and 77.8 -> 76.0 ms on
-// a fast one, 12-atom relaxation step 16.3 -> 15.8 ms, one small tensor-core
-// product 67.3 -> 66.1 us.
+// link of the acc iteration's chain of short kernels: 2-atom FP64 solve (30
+// launches an iteration) 92.5 -> 86.3 ms on a slow host and 77.8 -> 76.0 ms on
+// a fast one, 12-atom relaxation step 16.3 -> 15.6 ms, one small tensor-core
+// product 67.3 -> 66.4 us.
 template <typename... K, typename... A>
 void launch_chained(dim3 grid, dim3 block, size_t smem, cudaStream_t stream, void (*kernel)(K...), A... args) {
   cudaLaunchAttribute at[1];
