@@ -1,8 +1,6 @@
 // Typed GEMM entry used by the solvers.  Complex FP64 (the FP64 mode and the
 // refinement phase) maps to cuBLAS ZGEMM, the reference's own call
-// (src/half_cuda_iterative_solver.cuf:163-194), or, where the product is
-// large enough to gain, to the library's exact integer product on the int8
-// tensor cores (zcrt.cu); complex FP32 (the mixed
+// (src/half_cuda_iterative_solver.cuf:163-194); complex FP32 (the mixed
 // mode's iterations) runs on the library's tcgen05 kernel with in-kernel
 // bf16 hi/lo splitting (tc_gemm.cu).  Environment HALF_TC_GEMM=0 sends the
 // FP32 products to cuBLAS CGEMM instead, for A/B measurements.
@@ -10,7 +8,6 @@
 
 #include "context.h"
 #include "tc_gemm.h"
-#include "zcrt.h"
 
 namespace hb {
 
@@ -18,10 +15,6 @@ inline void gemm(Runtime& rt, cublasOperation_t ta, cublasOperation_t tb, int m,
                  const double2* A, long long lda, const double2* B, long long ldb, double2 beta, double2* C,
                  long long ldc) {
   if (m <= 0 || n <= 0) return;
-  if (zcrt_serves(m, n, k)) {
-    zcrt_gemm(rt, ta, tb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-    return;
-  }
   cublas_check(cublasZgemm(rt.blas, ta, tb, m, n, k, reinterpret_cast<const cuDoubleComplex*>(&alpha),
                            reinterpret_cast<const cuDoubleComplex*>(A), int(lda),
                            reinterpret_cast<const cuDoubleComplex*>(B), int(ldb),

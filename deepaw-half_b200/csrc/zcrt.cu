@@ -535,24 +535,4 @@ void crt_product(Runtime& rt, const CrtPlanes& a, const CrtPlanes& b, double2 al
   rt.crt_pending = true;
 }
 
-void zcrt_gemm(Runtime& rt, cublasOperation_t ta, cublasOperation_t tb, int m, int n, int k, double2 alpha,
-               const double2* A, long long lda, const double2* B, long long ldb, double2 beta, double2* C,
-               long long ldc) {
-  CrtSide a, b;
-  a.p = A;
-  a.ld = lda;
-  a.rows = m;
-  a.k = k;
-  a.kcontig = ta != CUBLAS_OP_N;
-  a.conj = ta == CUBLAS_OP_C;
-  b.p = B;
-  b.ld = ldb;
-  b.rows = n;
-  b.k = k;
-  b.kcontig = tb == CUBLAS_OP_N;
-  b.conj = tb == CUBLAS_OP_C;
-  const CrtPlanes pa = crt_prepare(rt, a, false, rt.crt_a), pb = crt_prepare(rt, b, true, rt.crt_b);
-  crt_product(rt, pa, pb, alpha, beta, C, ldc);
-}
-
 }  // namespace hb

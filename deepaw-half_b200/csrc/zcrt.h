@@ -34,11 +34,6 @@ CrtPlanes crt_prepare(Runtime& rt, const CrtSide& s, bool as_b, DeviceBuffer<uns
 void crt_product(Runtime& rt, const CrtPlanes& a, const CrtPlanes& b, double2 alpha, double2 beta, double2* C,
                  long long ldc, bool upper = false, double2* C2 = nullptr, int split_col = INT32_MAX);
 
-// As cublasZgemm, for shapes that zcrt_serves accepts.
-void zcrt_gemm(Runtime& rt, cublasOperation_t ta, cublasOperation_t tb, int m, int n, int k, double2 alpha,
-               const double2* A, long long lda, const double2* B, long long ldb, double2 beta, double2* C,
-               long long ldc);
-
 // Whether an m x n product over k is large enough to gain over ZGEMM (a_kept:
 // the left operand's planes exist already) and within the method's range and
 // memory.
