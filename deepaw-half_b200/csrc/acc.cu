@@ -397,25 +397,16 @@ struct Scratch64 {
   DeviceBuffer<int> idx, active, perm;
 };
 
-// projected blocks into an ((m + np) x (m + np), ld m + np) FP64 matrix:
+// FP32 blocks projected into an ((m + np) x (m + np), ld m + np) FP64 matrix:
 // [0:m,0:m] = A^H B1, [0:m,m:] = A^H B2, [m:,m:] = P^H B2 (the upper triangle
-// is what zhegvd reads); np = m is the reference's 2m x 2m pencil.
-// (FP32 blocks: tensor-core products written straight into the FP64 pencil,
-// split-K partial sums reduced in FP64.)
-template <typename R>
-void project_upper(Runtime& rt, int n, int m, int np, const cplx_t<R>* x, const cplx_t<R>* p, const cplx_t<R>* bx,
-                   const cplx_t<R>* bp, double2* out) {
+// is what zhegvd reads); tensor-core products written straight into the FP64
+// pencil, split-K partial sums reduced in FP64.
+void project_upper(Runtime& rt, int n, int m, int np, const float2* x, const float2* p, const float2* bx,
+                   const float2* bp, double2* out) {
   const int ld = m + np;
-  if constexpr (sizeof(R) == 4) {
-    gemm_to64(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, m, n, x, n, bx, n, out, ld);
-    gemm_to64(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, np, n, x, n, bp, n, out + (long long)m * ld, ld);
-    gemm_to64(rt, CUBLAS_OP_C, CUBLAS_OP_N, np, np, n, p, n, bp, n, out + (long long)m * ld + m, ld);
-  } else {
-    const auto one = cval<R>(1.0), zero = cval<R>(0.0);
-    gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, m, n, one, x, n, bx, n, zero, out, ld);
-    gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, np, n, one, x, n, bp, n, zero, out + (long long)m * ld, ld);
-    gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, np, np, n, one, p, n, bp, n, zero, out + (long long)m * ld + m, ld);
-  }
+  gemm_to64(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, m, n, x, n, bx, n, out, ld);
+  gemm_to64(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, np, n, x, n, bp, n, out + (long long)m * ld, ld);
+  gemm_to64(rt, CUBLAS_OP_C, CUBLAS_OP_N, np, np, n, p, n, bp, n, out + (long long)m * ld + m, ld);
 }
 
 template <typename R>
@@ -438,11 +429,13 @@ struct AccRun {
   long long op_cols = 0;
   Tracer* tr = nullptr;
   void mark(const char* s) { if (tr) tr->mark(s); }
-  // the FP64 iteration's products through the block kernels (blockops.h)
-  bool fused(int order, int cols) const {
-    if constexpr (sizeof(R) == 8) return zblock_fused(n, order, cols);
-    return false;
-  }
+  // FP64 phase of a mixed solve: the projections and the S-orthogonalisation
+  // may run on the integer tensor cores.  They hold an operand in fixed point
+  // relative to its rows' norms (zcrt.cu has the errors, which there are below
+  // ZGEMM's).  The rotations never do: a row of [X P] holds X beside P entries
+  // as small as the residuals, and near convergence Y is close to the
+  // identity, where ZGEMM loses next to nothing.
+  bool integer = false;
 
   // (timed by the sweep's events: no host synchronisation)
   void apply(const C* x, C* hx, C* sx, int nb) {
@@ -450,47 +443,36 @@ struct AccRun {
     op_cols += nb;
   }
 
-  // small FP64 matrices -> this precision
-  void to_r(const double2* in, long long ldi, C* out, long long ldo, int rows, int cols) {
-    if constexpr (sizeof(R) == 8) {
-      HALF_CUDA(cudaMemcpy2DAsync(out, ldo * sizeof(C), in, ldi * sizeof(C), rows * sizeof(C), cols,
-                                  cudaMemcpyDeviceToDevice, rt.stream));
-    } else {
-      convert_block_kernel<double2, float2><<<ceil_div((long long)rows * cols, 256), 256, 0, rt.stream>>>(in, ldi, out, ldo,
-                                                                                                       rows, cols);
-      ++rt.prof.launches;
-    }
+  // small FP64 matrices -> FP32
+  void to_r(const double2* in, long long ldi, float2* out, long long ldo, int rows, int cols) {
+    convert_block_kernel<double2, float2><<<ceil_div((long long)rows * cols, 256), 256, 0, rt.stream>>>(in, ldi, out, ldo,
+                                                                                                     rows, cols);
+    ++rt.prof.launches;
   }
 
   // Rayleigh-Ritz on the current X only (m x m)
   void rayleigh_ritz_x() {
-    const auto one = cval<R>(1.0), zero = cval<R>(0.0);
     double2* hs = sc.hsub.get();
     double2* ssb = sc.ssub.get();
     int nx = blk.cur ^ 1;
     if constexpr (sizeof(R) == 8) {
-      if (fused(m, m)) {
-        const ZBlock b[2] = {{blk.hx(), m}, {blk.sx(), m}};
-        double2* const c[2] = {hs, ssb};
-        zgram(rt, n, {blk.x(), m}, b, c, 2, m, true);
-        ss.hegvd(hs, ssb, m, sc.w.get(), m);
-        const ZBlock z[3] = {{blk.x(), m}, {blk.hx(), m}, {blk.sx(), m}};
-        double2* const out[3] = {blk.X[nx].get(), blk.HX[nx].get(), blk.SX[nx].get()};
-        zupdate(rt, n, z, hs, m, out, m, 3, 1.0, 0.0);
-        blk.cur = nx;
-        return;
-      }
-      gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, m, n, one, blk.x(), n, blk.hx(), n, zero, hs, m);
-      gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, m, n, one, blk.x(), n, blk.sx(), n, zero, ssb, m);
+      const ZBlock b[2] = {{blk.hx(), m}, {blk.sx(), m}};
+      double2* const c[2] = {hs, ssb};
+      zgram(rt, n, {blk.x(), m}, b, c, 2, m, true, zgram_route(n, m, m, integer));
+      ss.hegvd(hs, ssb, m, sc.w.get(), m);
+      const ZBlock z[3] = {{blk.x(), m}, {blk.hx(), m}, {blk.sx(), m}};
+      double2* const out[3] = {blk.X[nx].get(), blk.HX[nx].get(), blk.SX[nx].get()};
+      zupdate(rt, n, z, hs, m, out, m, 3, 1.0, 0.0, zupdate_route(n, m, m, false));
     } else {
+      const auto one = cval<R>(1.0), zero = cval<R>(0.0);
       gemm_to64(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, m, n, blk.x(), n, blk.hx(), n, hs, m);
       gemm_to64(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, m, n, blk.x(), n, blk.sx(), n, ssb, m);
+      ss.hegvd(hs, ssb, m, sc.w.get(), m);
+      to_r(hs, m, blk.Y.get(), m, m, m);
+      gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, m, m, one, blk.x(), n, blk.Y.get(), m, zero, blk.X[nx].get(), n);
+      gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, m, m, one, blk.hx(), n, blk.Y.get(), m, zero, blk.HX[nx].get(), n);
+      gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, m, m, one, blk.sx(), n, blk.Y.get(), m, zero, blk.SX[nx].get(), n);
     }
-    ss.hegvd(hs, ssb, m, sc.w.get(), m);
-    to_r(hs, m, blk.Y.get(), m, m, m);
-    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, m, m, one, blk.x(), n, blk.Y.get(), m, zero, blk.X[nx].get(), n);
-    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, m, m, one, blk.hx(), n, blk.Y.get(), m, zero, blk.HX[nx].get(), n);
-    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, m, m, one, blk.sx(), n, blk.Y.get(), m, zero, blk.SX[nx].get(), n);
     blk.cur = nx;
   }
 
@@ -605,19 +587,15 @@ struct AccRun {
     mark("precondition");
     apply(blk.P.get(), blk.HP.get(), blk.SP.get(), np);
     mark("apply");
-    const bool fuse = fused(m - nl + np, m - nl);
     // S-orthogonalise against X
     if constexpr (sizeof(R) == 8) {
-      if (fuse) {
-        const ZBlock b = {blk.SP.get(), np};
-        double2* const c = blk.small.get();
-        zgram(rt, n, {blk.x(), m}, &b, &c, 1, m, false);
-        const ZBlock z[3] = {{blk.x(), m}, {blk.hx(), m}, {blk.sx(), m}};
-        double2* const out[3] = {blk.P.get(), blk.HP.get(), blk.SP.get()};
-        zupdate(rt, n, z, blk.small.get(), m, out, np, 3, -1.0, 1.0);
-      }
-    }
-    if (!fuse) {
+      const ZBlock b = {blk.SP.get(), np};
+      double2* const c = blk.small.get();
+      zgram(rt, n, {blk.x(), m}, &b, &c, 1, m, false, zgram_route(n, m, np, integer));
+      const ZBlock z[3] = {{blk.x(), m}, {blk.hx(), m}, {blk.sx(), m}};
+      double2* const out[3] = {blk.P.get(), blk.HP.get(), blk.SP.get()};
+      zupdate(rt, n, z, blk.small.get(), m, out, np, 3, -1.0, 1.0, zupdate_route(n, m, np, integer));
+    } else {
       gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, np, n, one, blk.x(), n, blk.SP.get(), n, zero, blk.small.get(), m);
       gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, m, mone, blk.x(), n, blk.small.get(), m, one, blk.P.get(), n);
       gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, m, mone, blk.hx(), n, blk.small.get(), m, one, blk.HP.get(), n);
@@ -654,15 +632,13 @@ struct AccRun {
     if (!skip_metric) use_metric();
     auto project = [&]() {
       if constexpr (sizeof(R) == 8) {
-        if (fuse) {
-          const ZBlock b[2] = {{blk.hx() + off, mu, hpu, np}, {blk.sx() + off, mu, spu, np}};
-          double2* const c[2] = {hs, ssb};
-          zgram(rt, n, {blk.x() + off, mu, pu, np}, b, c, 2, ord, true);
-          return;
-        }
+        const ZBlock b[2] = {{blk.hx() + off, mu, hpu, np}, {blk.sx() + off, mu, spu, np}};
+        double2* const c[2] = {hs, ssb};
+        zgram(rt, n, {blk.x() + off, mu, pu, np}, b, c, 2, ord, true, zgram_route(n, ord, ord, integer));
+      } else {
+        project_upper(rt, n, mu, np, blk.x() + off, pu, blk.hx() + off, hpu, hs);
+        project_upper(rt, n, mu, np, blk.x() + off, pu, blk.sx() + off, spu, ssb);
       }
-      project_upper<R>(rt, n, mu, np, blk.x() + off, pu, blk.hx() + off, hpu, hs);
-      project_upper<R>(rt, n, mu, np, blk.x() + off, pu, blk.sx() + off, spu, ssb);
     };
     project();
     mark("rr_gemm");
@@ -690,13 +666,12 @@ struct AccRun {
     mark("hegvd");
     int nx = blk.cur ^ 1;
     if constexpr (sizeof(R) == 8) {
-      if (fuse) {
-        const ZBlock z[3] = {{blk.x() + off, mu, pu, np}, {blk.hx() + off, mu, hpu, np}, {blk.sx() + off, mu, spu, np}};
-        double2* const out[3] = {blk.X[nx].get() + off, blk.HX[nx].get() + off, blk.SX[nx].get() + off};
-        zupdate(rt, n, z, hs, ord, out, mu, 3, 1.0, 0.0);
-      }
+      const ZBlock z[3] = {{blk.x() + off, mu, pu, np}, {blk.hx() + off, mu, hpu, np}, {blk.sx() + off, mu, spu, np}};
+      double2* const out[3] = {blk.X[nx].get() + off, blk.HX[nx].get() + off, blk.SX[nx].get() + off};
+      zupdate(rt, n, z, hs, ord, out, mu, 3, 1.0, 0.0, zupdate_route(n, ord, mu, false));
+    } else {
+      rotate(ord, mu, np, off, pu, hpu, spu, hs, nx);
     }
-    if (!fuse) rotate(ord, mu, np, off, pu, hpu, spu, hs, nx);
     if (nl > 0) {   // locked columns go along unchanged
       const size_t bytes = size_t(off) * sizeof(C);
       HALF_CUDA(cudaMemcpyAsync(blk.X[nx].get(), blk.x(), bytes, cudaMemcpyDeviceToDevice, rt.stream));
@@ -707,7 +682,7 @@ struct AccRun {
     mark("rr_rot");
   }
 
-  // X[nx], HX[nx], SX[nx] from column offset off on = [X_U pu] Y and the same of H and S, Y = hs (ord x mu, FP64)
+  // FP32: X[nx], HX[nx], SX[nx] from column offset off on = [X_U pu] Y and the same of H and S, Y = hs (ord x mu, FP64)
   void rotate(int ord, int mu, int np, long long off, const C* pu, const C* hpu, const C* spu, const double2* hs,
               int nx) {
     const auto one = cval<R>(1.0), zero = cval<R>(0.0);
@@ -726,11 +701,9 @@ struct AccRun {
   // (src/half_cuda_iterative_solver.cuf:166-176)
   void normalise_metric(cplx_t<R> one, cplx_t<R> zero, int np) {
     double2* metric = sc.metric.get();
-    const bool fuse = fused(m + np, np);
     if constexpr (sizeof(R) == 8) {
       const ZBlock b = {blk.SP.get(), np};
-      if (fuse) zgram(rt, n, {blk.P.get(), np}, &b, &metric, 1, np, true);
-      else gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, np, np, n, one, blk.P.get(), n, blk.SP.get(), n, zero, metric, np);
+      zgram(rt, n, {blk.P.get(), np}, &b, &metric, 1, np, true, zgram_route(n, np, np, integer));
     } else {
       gemm_to64(rt, CUBLAS_OP_C, CUBLAS_OP_N, np, np, n, blk.P.get(), n, blk.SP.get(), n, metric, np);
     }
@@ -742,18 +715,15 @@ struct AccRun {
     }
     mark("heevd");
     if constexpr (sizeof(R) == 8) {
-      if (fuse) {
-        const ZBlock z[3] = {{blk.P.get(), np}, {blk.HP.get(), np}, {blk.SP.get(), np}};
-        double2* const out[3] = {blk.PU.get(), blk.HPU.get(), blk.SPU.get()};
-        zupdate(rt, n, z, metric, np, out, np, 3, 1.0, 0.0);
-        mark("metric_rot");
-        return;
-      }
+      const ZBlock z[3] = {{blk.P.get(), np}, {blk.HP.get(), np}, {blk.SP.get(), np}};
+      double2* const out[3] = {blk.PU.get(), blk.HPU.get(), blk.SPU.get()};
+      zupdate(rt, n, z, metric, np, out, np, 3, 1.0, 0.0, zupdate_route(n, np, np, false));
+    } else {
+      to_r(metric, np, blk.small.get(), np, np, np);
+      gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, np, one, blk.P.get(), n, blk.small.get(), np, zero, blk.PU.get(), n);
+      gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, np, one, blk.HP.get(), n, blk.small.get(), np, zero, blk.HPU.get(), n);
+      gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, np, one, blk.SP.get(), n, blk.small.get(), np, zero, blk.SPU.get(), n);
     }
-    to_r(metric, np, blk.small.get(), np, np, np);
-    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, np, one, blk.P.get(), n, blk.small.get(), np, zero, blk.PU.get(), n);
-    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, np, one, blk.HP.get(), n, blk.small.get(), np, zero, blk.HPU.get(), n);
-    gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, np, one, blk.SP.get(), n, blk.small.get(), np, zero, blk.SPU.get(), n);
     mark("metric_rot");
   }
 };
@@ -868,6 +838,7 @@ void solve_acc(Context& ctx, KOperatorSet& ks, int nbands, bool want_vectors, So
   run64.tr = &tracer;
   run64.mcheck = mreq;
   run64.guarded = guarded;
+  run64.integer = mixed;
 
   if (mixed) {
     // ---------------- FP32 phase

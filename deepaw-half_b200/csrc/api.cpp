@@ -18,10 +18,12 @@
 #include <thread>
 
 #include "../../include/half_b200.h"
+#include "blockops.h"
 #include "context.h"
 #include "devmem.h"
 #include "staging.h"
 #include "tc_gemm.h"
+#include "zcrt.h"
 
 using namespace hb;
 
@@ -1112,6 +1114,60 @@ extern "C" int half_tc_cgemm(char op_a, char op_b, int m, int n, int k, const do
     tc_cgemm(rt, tc_dense_a(ta, A, lda, m, k), tc_dense_b(tb, B, ldb, k, n), m, n, k, make_double2(alpha[0], alpha[1]),
              make_double2(beta[0], beta[1]), c, c_fp64 != 0, ldc);
     tc_check(rt);
+    return HALF_SUCCESS;
+  });
+}
+
+// ---- test entries (exported, but not part of the ABI): the FP64 block products of the solver on device blocks
+extern "C" int hb_diag_gram_route(int n, int rows, int cols, int integer) {
+  return int(zgram_route(n, rows, cols, integer != 0));
+}
+
+extern "C" int hb_diag_update_route(int n, int k, int cols, int integer) {
+  return int(zupdate_route(n, k, cols, integer != 0));
+}
+
+// 'G': c (a1 + a2 x b1 + b2, leading dimension ldc) = [a | a_2]^H [b | b_2].  'U': c (n x b1) = beta c + alpha [a | a_2] b.
+// 'P': [c (n x b1) | c_2 (n x b2)] += a [b | b_2] on the integer tensor cores, as the projector product.
+// Blocks have n rows and no padding; b is (a1 + a2) x b1 (and x b2) in 'U' and 'P'.
+extern "C" int hb_diag_block_product(char kind, int route, int upper, int n, int a1, int a2, const void* a,
+                                     const void* a_2, int b1, int b2, const void* b, const void* b_2, double alpha,
+                                     double beta, void* c, void* c_2, int ldc, char* error, int cap) {
+  clear_error(error, cap);
+  return guarded(error, cap, [&]() -> int {
+    if (n < 1 || a1 < 1 || a2 < 0 || b1 < 1 || b2 < 0 || route < 1 || route > 3) fail(kInvalidArgument, "invalid block shapes");
+    if (ldc < (kind == 'G' ? a1 + a2 : n) || (upper && (a1 != b1 || a2 != b2))) fail(kInvalidArgument, "invalid output shape");
+    for (const void* p : {a, a2 ? a_2 : a, b, b2 ? b_2 : b, static_cast<const void*>(c)})
+      if (!device_pointer(p)) fail(kInvalidArgument, "operands must be device memory");
+    std::lock_guard<std::mutex> lock(g_diag_mutex);
+    Runtime& rt = diagnostic_runtime();
+    rt.prof.reset();
+    auto z = [](const void* p) { return static_cast<const double2*>(p); };
+    double2* out = static_cast<double2*>(c);
+    const ZBlock A = {z(a), a1, z(a_2), a2}, B = {z(b), b1, z(b_2), b2};
+    if (kind == 'G') {
+      zgram(rt, n, A, &B, &out, 1, ldc, upper != 0, ZRoute(route));
+    } else if (kind == 'U') {
+      zupdate(rt, n, &A, z(b), a1 + a2, &out, b1, 1, alpha, beta, ZRoute(route));
+    } else if (kind == 'P' && a2 == 0) {
+      CrtSide s;
+      s.p = z(a);
+      s.ld = s.rows = n;
+      s.k = a1;
+      const CrtPlanes pa = crt_prepare(rt, s, false, rt.crt_a);
+      s.p = z(b);
+      s.p2 = z(b_2);
+      s.split = b1;
+      s.ld = a1;
+      s.rows = b1 + b2;
+      s.kcontig = true;
+      crt_product(rt, pa, crt_prepare(rt, s, true, rt.crt_b), make_double2(1, 0), make_double2(1, 0), out, ldc, false,
+                  static_cast<double2*>(c_2), b1);
+    } else {
+      fail(kInvalidArgument, "unknown block product");
+    }
+    tc_check(rt);
+    HALF_CUDA(cudaStreamSynchronize(rt.stream));
     return HALF_SUCCESS;
   });
 }

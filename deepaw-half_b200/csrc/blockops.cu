@@ -15,10 +15,12 @@
 // Both kernels are register-tiled FP64 FMA (4 x 4 complex accumulators per
 // thread; 64 FMAs per 8 shared-memory loads), fed by cp.async two chunks deep.
 // On the FP64 pipe they are about as fast as cuBLAS's DMMA kernels (the B200's
-// FP64 vector and tensor rates are alike) but not faster, so the large cells,
-// whose products fill the GPU by themselves, stay on cuBLAS.
+// FP64 vector and tensor rates are alike) but not faster, so products that
+// fill the GPU by themselves go to cuBLAS or, in the FP64 phase of a mixed
+// solve, to the integer tensor cores (zcrt.cu).
 #include <algorithm>
 
+#include "blas.h"
 #include "blockops.h"
 #include "zcrt.h"
 
@@ -263,17 +265,13 @@ __global__ void __launch_bounds__(kUpThreads) zupdate_kernel(UpdateArgs u) {
 
 }  // namespace
 
+namespace {
+
 // The line lies where the fused kernels' time meets cuBLAS's, measured on whole
 // FP64 solves (cuBLAS / fused, ms): 2-atom cell, order 32: 144 / 133; 12-atom
 // cell, orders 80, 160 and 300: 16.8 / 14.8, 19.8 / 19.3, 31.3 / 32.3; 64-atom
 // cell, orders 150 and 400: 60.5 / 60.6, 121 / 135.
 bool zblock_small(int n, int order) { return double(n) * order * order < 2.0e8; }
-
-bool zblock_fused(int n, int order, int cols) {
-  return zblock_small(n, order) || (zcrt_serves(order, order, n) && zcrt_serves(n, cols, order));
-}
-
-namespace {
 
 CrtSide side_of(const ZBlock& b, int n, bool k_is_rows, bool conj) {
   CrtSide s;
@@ -290,7 +288,18 @@ CrtSide side_of(const ZBlock& b, int n, bool k_is_rows, bool conj) {
 
 }  // namespace
 
-void zgram(Runtime& rt, int n, const ZBlock& a, const ZBlock* b, double2* const* c, int count, int ldc, bool upper) {
+ZRoute zgram_route(int n, int rows, int cols, bool integer) {
+  if (zblock_small(n, std::max(rows, cols))) return ZRoute::kBlock;
+  return integer && zcrt_serves(rows, cols, n) ? ZRoute::kInteger : ZRoute::kLibrary;
+}
+
+ZRoute zupdate_route(int n, int k, int cols, bool integer) {
+  if (zblock_small(n, std::max(k, cols))) return ZRoute::kBlock;
+  return integer && zcrt_serves(n, cols, k) ? ZRoute::kInteger : ZRoute::kLibrary;
+}
+
+void zgram(Runtime& rt, int n, const ZBlock& a, const ZBlock* b, double2* const* c, int count, int ldc, bool upper,
+           ZRoute route) {
   GramArgs g{};
   g.a = a;
   g.n = n;
@@ -299,11 +308,22 @@ void zgram(Runtime& rt, int n, const ZBlock& a, const ZBlock* b, double2* const*
   g.cols = b[0].cols();
   g.upper = upper;
   if (g.rows <= 0 || g.cols <= 0) return;
-  if (!zblock_small(n, std::max(g.rows, g.cols)) && zcrt_serves(g.rows, g.cols, n)) {
+  const double2 one = make_double2(1, 0), zero = make_double2(0, 0);
+  if (route == ZRoute::kLibrary) {
+    for (int i = 0; i < count; ++i) {
+      double2* const right = c[i] + (long long)b[i].c1 * ldc;   // columns of the second buffer
+      gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, a.c1, b[i].c1, n, one, a.p1, n, b[i].p1, n, zero, c[i], ldc);
+      gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, a.c1, b[i].c2, n, one, a.p1, n, b[i].p2, n, zero, right, ldc);
+      if (!upper) gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, a.c2, b[i].c1, n, one, a.p2, n, b[i].p1, n, zero, c[i] + a.c1, ldc);
+      gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, a.c2, b[i].c2, n, one, a.p2, n, b[i].p2, n, zero, right + a.c1, ldc);
+    }
+    return;
+  }
+  if (route == ZRoute::kInteger) {
     const CrtPlanes pa = crt_prepare(rt, side_of(a, n, true, true), false, rt.crt_a);   // shared by the products
     for (int i = 0; i < count; ++i) {
       const CrtPlanes pb = crt_prepare(rt, side_of(b[i], n, true, false), true, rt.crt_b);
-      crt_product(rt, pa, pb, make_double2(1, 0), make_double2(0, 0), c[i], ldc, upper);
+      crt_product(rt, pa, pb, one, zero, c[i], ldc, upper);
     }
     return;
   }
@@ -336,9 +356,18 @@ void zgram(Runtime& rt, int n, const ZBlock& a, const ZBlock* b, double2* const*
 }
 
 void zupdate(Runtime& rt, int n, const ZBlock* z, const double2* y, int ldy, double2* const* c, int cols, int count,
-             double alpha, double beta) {
+             double alpha, double beta, ZRoute route) {
   if (n <= 0 || cols <= 0) return;
-  if (!zblock_small(n, std::max(cols, z[0].cols())) && zcrt_serves(n, cols, z[0].cols())) {
+  if (route == ZRoute::kLibrary) {
+    const double2 al = make_double2(alpha, 0), one = make_double2(1, 0);
+    for (int i = 0; i < count; ++i) {
+      const ZBlock& b = z[i];
+      gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, cols, b.c1, al, b.p1, n, y, ldy, make_double2(beta, 0), c[i], n);
+      if (b.c2 > 0) gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, cols, b.c2, al, b.p2, n, y + b.c1, ldy, one, c[i], n);
+    }
+    return;
+  }
+  if (route == ZRoute::kInteger) {
     CrtSide ys;
     ys.p = y;
     ys.ld = ldy;

@@ -16,21 +16,23 @@ struct ZBlock {
   int cols() const { return c1 + c2; }
 };
 
+// Where a product of blocks runs: small ones on the kernels of blockops.cu,
+// large ones on the integer tensor cores (zcrt.cu) where the caller allows
+// that, every other on ZGEMM.
+enum class ZRoute { kBlock = 1, kInteger = 2, kLibrary = 3 };
+ZRoute zgram_route(int n, int rows, int cols, bool integer);     // A^H B: rows x cols over n
+ZRoute zupdate_route(int n, int k, int cols, bool integer);      // Z Y: n x cols over k
+
 // C_i = A^H B_i for i < count (count 1 or 2, blocks of one shape), written
 // with leading dimension ldc.  upper: only the upper triangle is needed (A
-// and B_i of equal width); elements below it may or may not be written.
-void zgram(Runtime& rt, int n, const ZBlock& a, const ZBlock* b, double2* const* c, int count, int ldc, bool upper);
+// and B_i of equal width and split); elements below it may or may not be written.
+void zgram(Runtime& rt, int n, const ZBlock& a, const ZBlock* b, double2* const* c, int count, int ldc, bool upper,
+           ZRoute route);
 
 // C_i = beta C_i + alpha Z_i Y for i < count (up to 3 blocks of one shape):
 // Z_i n x K, Y K x cols (leading dimension ldy), C_i n x cols, beta 0 or 1.
 // C_i overlaps no Z_i.
 void zupdate(Runtime& rt, int n, const ZBlock* z, const double2* y, int ldy, double2* const* c, int cols, int count,
-             double alpha, double beta);
-
-// Whether the products of an n-row iteration with pencils of order `order`
-// (blocks of up to `cols` columns) go through zgram and zupdate rather than
-// ZGEMM calls: small ones on their FP64 kernels, large ones on the integer
-// tensor cores (zcrt.cu).
-bool zblock_fused(int n, int order, int cols);
+             double alpha, double beta, ZRoute route);
 
 }  // namespace hb

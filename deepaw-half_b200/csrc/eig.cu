@@ -1108,8 +1108,7 @@ __global__ void __launch_bounds__(kClThreads) hetrd_grid_kernel(double2* __restr
                                                                 double2* __restrict__ tauout, double2* exchange,
                                                                 int* counter, int* err) {
   const int G = gridDim.x, rank = blockIdx.x;
-  const int nc = (n + G - 1) / G;
-  extern __shared__ __align__(16) double2 cols[];   // nc x n: column jl G + rank at cols + jl n
+  extern __shared__ __align__(16) double2 cols[];   // ceil(n / G) x n: column jl G + rank at cols + jl n
   __shared__ double red[kClWarps][2 * kGridCols];   // the warps' shares of u
   __shared__ double rnorm[kClWarps], rqs[kClWarps];
   __shared__ double2 vcol[kGridCols], wcol[kGridCols];   // the previous step's v and w at this CTA's columns
@@ -1532,10 +1531,10 @@ void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, doubl
     if (n <= kSmallProducts) {
       double2* const v = V.get();
       const ZBlock ba = {A, n}, bb = {B, n}, bv = {v, n};
-      zupdate(rt, n, &ba, B, n, &v, n, 1, 1.0, 0.0);
-      zgram(rt, n, bb, &bv, &A, 1, n, true);
+      zupdate(rt, n, &ba, B, n, &v, n, 1, 1.0, 0.0, ZRoute::kBlock);
+      zgram(rt, n, bb, &bv, &A, 1, n, true, ZRoute::kBlock);
       heev(rt, A, n, nev, w, status);
-      zupdate(rt, n, &bb, v, n, &A, nev, 1, 1.0, 0.0);
+      zupdate(rt, n, &bb, v, n, &A, nev, 1, 1.0, 0.0, ZRoute::kBlock);
       return;
     }
     gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, n, n, one, A, n, B, n, zero, V.get(), n);

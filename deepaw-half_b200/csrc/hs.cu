@@ -50,8 +50,10 @@ struct KOperator {
   DeviceBuffer<C> work;      // chunk x nplanes x n2 x n3
   int work_chunk = 0;
   DeviceBuffer<C> B;         // FP64: npw x np, column-major
-  // FP64: B^H and B in the residue planes of the integer product, made by the
+  // FP64 operator of a mixed solve: its projector products may run on the
+  // integer tensor cores (zcrt.cu).  B^H and B in residue planes, made by the
   // first application large enough to use them
+  bool integer = false;
   DeviceBuffer<unsigned char> crt_bh_store, crt_b_store;
   CrtPlanes crt_bh, crt_b;
   // FP32: the projector matrix is generated from these tables straight into
@@ -719,6 +721,7 @@ std::unique_ptr<KOperatorSet> prepare_operator(Context& ctx, Runtime& rt, const 
   batch.add(datom, atom_cols);
   if (fp64) {
     ks->op64 = std::make_unique<KOperator<double>>();
+    ks->op64->integer = fp32;   // both precisions: a mixed solve
     stage_operator<double>(ctx, basis, hg, np, pt, batch, *ks->op64);
   }
   if (fp32) {
@@ -863,7 +866,7 @@ void apply_nonlocal(Runtime& rt, KOperator<R>& op, const cplx_t<R>* x, long long
     tc_cgemm(rt, op.b_planes, y, op.npw, 2 * nb, op.np, make_double2(1, 0), make_double2(1, 0), hx, false, ld, sx, nb);
   } else {
     const bool kept = op.crt_bh.planes != nullptr;
-    if (zcrt_serves(op.np, nb, op.npw, kept) && zcrt_serves(op.npw, 2 * nb, op.np, kept)) {
+    if (op.integer && zcrt_serves(op.np, nb, op.npw, kept) && zcrt_serves(op.npw, 2 * nb, op.np, kept)) {
       // coeff = B^H X, [H X | S X] += B [DY | QY] on the integer tensor cores
       CrtSide s;
       s.ld = op.npw;

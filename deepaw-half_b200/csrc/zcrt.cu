@@ -1,21 +1,38 @@
-// Complex FP64 GEMM on the int8 tensor cores (tcgen05 kind::i8) by the
-// Chinese remainder theorem, for the large products of the FP64 phase.
+// Complex FP64 products on the int8 tensor cores (tcgen05 kind::i8) by the
+// Chinese remainder theorem, for large products of a mixed solve's FP64 phase.
 //
 // The B200's FP64 pipes give about 37 TFLOP/s, vector or tensor, and ZGEMM
 // runs at that rate on the large cells, so a faster product has to leave
 // them.  Method (Ozaki, Uchino and Imamura, "Ozaki scheme II", 2025): every
 // row of op(A) and column of op(B) is scaled by a power of two to a norm
-// below 2^58 and rounded to integers; the integer product is formed modulo 15
+// below 2^62 and rounded to integers; the integer product is formed modulo 16
 // coprime moduli p_i <= 256, each an int8 product with exact int32
-// accumulation, and put together again.  By Cauchy-Schwarz the integer result
-// is below 2^108, inside the moduli's product of 2^110, so the result is
-// exact up to the rounding of the operands to 2^-55 of their row's norm:
-// |error| is at most 2^-54 |a| |b| and in practice sqrt(K) below that, which
-// is no more than the FP64 accumulation of ZGEMM loses (measured against
-// double-double sums over the tests' shapes: ERRORS).
+// accumulation, and put together again.  By Cauchy-Schwarz the integer sums
+// are below 2^124, inside half the moduli's product of 2^125.4, so the result
+// is exact up to the rounding of the operands: an element is held in units of
+// at most 2^-61 of its row's norm, full FP64 down to 2^-9 of that norm and
+// fewer bits below.  The error of an element of the product is at most
+// 2 sqrt(K) 2^-61.5 |a| |b| and a rounding of the result; measured, 2^-60 |a| |b|.
+//
+// That bound is relative to the norms, where ZGEMM's is relative to
+// sum |a_k| |b_k|.  So the product is for operands whose rows are not graded
+// against each other, and a caller has to allow it: the iteration does for its
+// projections, its S-orthogonalisation and the projector products, in the
+// FP64 phase of a mixed solve only, and not for its rotations and pencils.
+// Errors there against double-double sums, beside ZGEMM's on the same
+// operands (rms over 4,096 elements and every iteration; worst product):
+// relative to |a| |b|, 0.02 of ZGEMM's for the projectors' B^H X, 0.02 for
+// X^H S P, 0.09 for the projections, and equal (the rounding of the sum it is
+// added to) for the two that accumulate; relative to sum |a_k| |b_k|, 0.02,
+// 0.02, 0.1, 0.94 and 0.98 (216-atom cell, 480 bands, 2e-5 and 1e-7 eV), and
+// 0.2 to 0.7 on the 12-atom cell with 512 bands to 1e-9 eV.  (The rotations,
+// with the columns of [X P] scaled alike, would be at 0.07 and 900.)  Where
+// translational symmetry makes vectors' supports disjoint (64-atom cell, no
+// atom displaced), ZGEMM leaves the elements that vanish by it at zero, and
+// they are about 2^-61 |a| |b| here; relative to |a| |b| the worst is 0.12.
 //
 //   crt_norm_*      row norms -> power-of-two scales
-//   crt_split       residues of Re and Im, 30 bytes per element, in the
+//   crt_split       residues of Re and Im, 32 bytes per element, in the
 //                   K-major no-swizzle UMMA layout: 8 rows x 128 k are 1 KB
 //                   (8 core matrices of 8 rows x 16 bytes), so a stage's tile
 //                   of one plane is one contiguous bulk copy
@@ -27,11 +44,10 @@
 //                   times P and the scales
 //
 // Bound by the L2 traffic of the planes (54 bytes per cycle and SM at tensor
-// rate; the residues of one modulus are of no use to another) and, for the
-// rotations, by the split and join passes.  Measured with both operands
-// split, ZGEMM / this: 600 x 600 x 38,089 3.21 / 1.54 ms, 1,696 x 600 x 38,089
-// 8.90 / 3.20 ms, 38,089 x 600 x 1,200 6.12 / 3.22 ms; the 216-atom cell's mixed
-// solve 933 -> 728 ms.
+// rate; the residues of one modulus are of no use to another) and by the
+// split and join passes.  Both operands split, one product, ZGEMM / this:
+// X^H Y 600 x 600 x 38,089 3.22 / 1.61 ms, upper half of 1,200 x 1,200 x 38,089
+// 12.5 / 3.4 ms (ZGEMM of the whole matrix), 1,696 x 600 x 38,089 8.91 / 3.49 ms, X C 38,089 x 600 x 600 3.16 / 2.23 ms.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -46,9 +62,9 @@ namespace {
 
 using namespace tc;
 
-constexpr int kMods = 15;
-constexpr int kScaleBits = 58;     // row norms are scaled below 2^58; the products' sums stay below 2^116 < P / 2
-constexpr int kMod[kMods] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197};
+constexpr int kMods = 16;
+constexpr int kScaleBits = 62;     // row norms are scaled below 2^62; the products' sums stay below 2^124 < P / 2 = 2^124.4
+constexpr int kMod[kMods] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193};
 constexpr int kMaxK = 65000;       // |2 K 128 128| < 2^31
 constexpr int kBM = 128, kBN = 160;   // three int32 accumulators of kBN columns fit Tensor Memory
 constexpr int kKB = 128;           // k per stage
@@ -63,7 +79,7 @@ struct Modulus {
   int p;
   unsigned magic;        // floor(2^32 / p) + 1
   int wlo, whi;          // 2^(8 j) mod p, balanced, as packed signed bytes
-  int bias;              // makes the split's weighted byte sum positive and undoes its 2^60 offset
+  int bias;              // makes the split's weighted byte sum positive and undoes its 2^62 offset
   unsigned bias32;       // multiple of p just above 2^31
   unsigned long long fhi;   // y / p with y = (P / p)^-1 mod p, as a 96-bit fraction
   unsigned flo;
@@ -96,7 +112,7 @@ const Moduli& moduli() {
       }
       m.wlo = int(w[0]);
       m.whi = int(w[1]);
-      m.bias = p * ((8 * 255 * 128 + p - 1) / p) + (p - mod_pow2(60, p)) % p;
+      m.bias = p * ((8 * 255 * 128 + p - 1) / p) + (p - mod_pow2(62, p)) % p;
       m.bias32 = unsigned(((1ull << 31) + unsigned(p) - 1) / unsigned(p) * unsigned(p));
       const int q = int(P / unsigned(p) % unsigned(p));
       int y = 1 % p;
@@ -195,7 +211,7 @@ __device__ __forceinline__ int dot4_us(unsigned bytes, int weights, int acc) {
   return r;
 }
 
-// balanced residue (a signed byte) of the integer held as u = q + 2^60
+// balanced residue (a signed byte) of the integer held as u = q + 2^62
 __device__ __forceinline__ int residue(unsigned long long u, const Modulus& m) {
   const int v = dot4_us(unsigned(u), m.wlo, dot4_us(unsigned(u >> 32), m.whi, m.bias));
   int r = v - int(__umulhi(unsigned(v), m.magic)) * m.p;
@@ -203,7 +219,7 @@ __device__ __forceinline__ int residue(unsigned long long u, const Modulus& m) {
 }
 
 __device__ __forceinline__ unsigned long long to_integer(double x, double s1, double s2) {
-  return (unsigned long long)__double2ll_rn(x * s1 * s2) + (1ull << 60);
+  return (unsigned long long)__double2ll_rn(x * s1 * s2) + (1ull << 62);   // |x s1 s2| <= 2^62
 }
 
 // Planes of a side: part q of modulus i at out + (2 i + q) plane_bytes; element
@@ -400,7 +416,7 @@ __global__ void __launch_bounds__(256) crt_join(const unsigned char* __restrict_
   const unsigned char* src = res + (long long)col * m_pad + r0 + 4 * lane;
   const long long plane = (long long)N * m_pad;
   for (int s = 0; s < slices; ++s) {
-#pragma unroll 5
+#pragma unroll 4
     for (int i = 0; i < kMods; ++i) {
       const unsigned f2 = unsigned(mods.m[i].fhi >> 32), f1 = unsigned(mods.m[i].fhi), f0 = mods.m[i].flo;
 #pragma unroll
@@ -425,7 +441,8 @@ __global__ void __launch_bounds__(256) crt_join(const unsigned char* __restrict_
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       const unsigned long long f = ((unsigned long long)c32[2 * j + q] << 32) + b64[2 * j + q] + (a64[2 * j + q] >> 32);
-      const double s = double((long long)f);   // centred: |x| < P / 2
+      // centred: |x| < P / 2; the low digit keeps small sums at full precision
+      const double s = fma(double(unsigned(a64[2 * j + q])), 0x1p-32, double((long long)f));
       v[q] = fma(s, mods.phi, s * mods.plo);
       v[q] = e0 == kNaN || e1 == kNaN ? nan("") : scalbn(v[q], -(e0 + e1));
     }

@@ -1,7 +1,6 @@
 // Complex FP64 products on the integer tensor cores (zcrt.cu).
 #pragma once
 
-#include "blockops.h"
 #include "context.h"
 
 namespace hb {
