@@ -10,6 +10,7 @@
 #include <cstdlib>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <utility>
 
@@ -22,7 +23,10 @@ namespace {
 using Key = std::pair<int, size_t>;   // (device, bytes)
 using Pool = std::multimap<Key, void*>;
 
-constexpr size_t kThreadCap = size_t(32) << 30;   // cached bytes kept per thread (a 216-atom solve takes 17 GB in all)
+// Cached bytes kept by one thread (a 216-atom solve takes 17 GB in all) and by
+// the process: what four k-point workers and their caller need.
+constexpr size_t kThreadCap = size_t(32) << 30;
+constexpr size_t kProcessCap = size_t(80) << 30;
 
 size_t round_bytes(size_t b) {
   if (b <= (size_t(1) << 20)) return (b + 511) & ~size_t(511);
@@ -34,8 +38,12 @@ void timed_free(void* p, size_t bytes) {
   cudaFree(p);
 }
 
-std::mutex g_mu;
+struct ThreadCache;
+
+std::mutex g_mu;                       // guards g_pool and g_caches; taken before a cache's own mutex
 Pool g_pool;
+std::set<ThreadCache*> g_caches;       // of the live threads
+std::atomic<size_t> g_cached{0};       // bytes in all caches and the pool
 
 // Smallest block in [key.bytes, 2 key.bytes] on the same device, removed from pool.
 void* take(Pool& pool, const Key& key, size_t* granted) {
@@ -48,12 +56,18 @@ void* take(Pool& pool, const Key& key, size_t* granted) {
 }
 
 struct ThreadCache {
+  std::mutex mu;   // another thread takes it only to give everything back
   Pool pool;
   size_t bytes = 0;
-  ~ThreadCache() {
-    if (pool.empty()) return;
-    cudaDeviceSynchronize();   // every use of these blocks has finished
+  ThreadCache() {
     std::lock_guard<std::mutex> lock(g_mu);
+    g_caches.insert(this);
+  }
+  ~ThreadCache() {
+    if (!pool.empty()) cudaDeviceSynchronize();   // every use of these blocks has finished
+    std::lock_guard<std::mutex> lock(g_mu);
+    g_caches.erase(this);
+    std::lock_guard<std::mutex> own(mu);
     for (auto& kv : pool) g_pool.insert(kv);
     pool.clear();
   }
@@ -62,9 +76,12 @@ struct ThreadCache {
 thread_local ThreadCache t_cache;
 std::atomic<long long> g_requests{0}, g_driver_allocs{0};
 
-void release_all_locked() {
-  for (auto& kv : g_pool) timed_free(kv.second, kv.first.second);
-  g_pool.clear();
+void release_all_locked(Pool& pool) {
+  for (auto& kv : pool) {
+    timed_free(kv.second, kv.first.second);
+    g_cached.fetch_sub(kv.first.second);
+  }
+  pool.clear();
 }
 
 }  // namespace
@@ -74,13 +91,20 @@ void* device_alloc(size_t bytes, size_t* granted) {
   int dev = 0;
   cudaGetDevice(&dev);
   const Key key{dev, round_bytes(bytes)};
-  if (void* p = take(t_cache.pool, key, granted)) {
-    t_cache.bytes -= *granted;
-    return p;
+  {
+    std::lock_guard<std::mutex> own(t_cache.mu);
+    if (void* p = take(t_cache.pool, key, granted)) {
+      t_cache.bytes -= *granted;
+      g_cached.fetch_sub(*granted);
+      return p;
+    }
   }
   {
     std::lock_guard<std::mutex> lock(g_mu);
-    if (void* p = take(g_pool, key, granted)) return p;
+    if (void* p = take(g_pool, key, granted)) {
+      g_cached.fetch_sub(*granted);
+      return p;
+    }
   }
   void* p = nullptr;
   cudaError_t e;
@@ -106,14 +130,20 @@ void* device_alloc(size_t bytes, size_t* granted) {
 
 void device_free(void* p, size_t granted) {
   if (!p) return;
-  if (t_cache.bytes + granted > kThreadCap) {
-    timed_free(p, granted);
-    return;
-  }
   int dev = 0;
   cudaGetDevice(&dev);
-  t_cache.pool.insert({Key{dev, granted}, p});
-  t_cache.bytes += granted;
+  {
+    std::lock_guard<std::mutex> own(t_cache.mu);
+    if (t_cache.bytes + granted <= kThreadCap) {
+      if (g_cached.fetch_add(granted) + granted <= kProcessCap) {
+        t_cache.pool.insert({Key{dev, granted}, p});
+        t_cache.bytes += granted;
+        return;
+      }
+      g_cached.fetch_sub(granted);
+    }
+  }
+  timed_free(p, granted);
 }
 
 void device_alloc_counts(long long* requests, long long* driver_allocations) {
@@ -121,13 +151,17 @@ void device_alloc_counts(long long* requests, long long* driver_allocations) {
   if (driver_allocations) *driver_allocations = g_driver_allocs.load(std::memory_order_relaxed);
 }
 
+// Another thread's cached blocks may still be used by work on its stream:
+// cudaFree waits for that.
 void device_cache_release() {
   cudaDeviceSynchronize();
-  for (auto& kv : t_cache.pool) timed_free(kv.second, kv.first.second);
-  t_cache.pool.clear();
-  t_cache.bytes = 0;
   std::lock_guard<std::mutex> lock(g_mu);
-  release_all_locked();
+  for (ThreadCache* c : g_caches) {
+    std::lock_guard<std::mutex> own(c->mu);
+    release_all_locked(c->pool);
+    c->bytes = 0;
+  }
+  release_all_locked(g_pool);
 }
 
 }  // namespace hb

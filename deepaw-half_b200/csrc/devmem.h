@@ -12,7 +12,9 @@
 //     may take them;
 //   * a request takes the smallest cached block of at least its (rounded)
 //     size and at most twice it; on an allocation failure every cached block
-//     is released and the allocation retried once.
+//     of every thread is released and the allocation retried once;
+//   * a thread keeps at most 32 GB and the process at most 80 GB: beyond that
+//     a freed block goes back to the driver.
 #pragma once
 
 #include <cstddef>
@@ -21,7 +23,7 @@ namespace hb {
 
 void* device_alloc(size_t bytes, size_t* granted);   // throws hb::Error on failure
 void device_free(void* p, size_t granted);
-void device_cache_release();                          // return cached blocks to the driver
+void device_cache_release();                          // return the cached blocks of all threads to the driver
 // Process-wide counts since start: device_alloc calls (cached or not) and the
 // cudaMalloc calls among them.
 void device_alloc_counts(long long* requests, long long* driver_allocations);
