@@ -194,7 +194,10 @@ void solve_one(Context& ctx, Runtime& rt, const double k[3], int nbands, bool wa
   info.npw = ks->basis.npw();
   end_call(rt, info);
   info.operator_ms = info.sweep_ms;
-  if (keep) *keep = std::move(ks);
+  if (keep) {
+    release_solve_planes(*ks);   // 4 GB of a 216-atom cell's k point, of no use to the forces
+    *keep = std::move(ks);
+  }
 }
 
 void solve_one(Context& ctx, const double k[3], int nbands, bool want_vectors, SolveOutput& out,
@@ -1118,7 +1121,10 @@ extern "C" int half_tc_cgemm(char op_a, char op_b, int m, int n, int k, const do
   });
 }
 
-// ---- test entries (exported, but not part of the ABI): the FP64 block products of the solver on device blocks
+// ---- test entries (exported, but not part of the ABI): device memory that runs out, and the FP64 block products
+// of the solver on device blocks
+extern "C" long long hb_diag_refuse_allocations(size_t bytes) { return device_refuse_above(bytes); }
+
 extern "C" int hb_diag_gram_route(int n, int rows, int cols, int integer) {
   return int(zgram_route(n, rows, cols, integer != 0));
 }

@@ -309,6 +309,9 @@ void zgram(Runtime& rt, int n, const ZBlock& a, const ZBlock* b, double2* const*
   g.upper = upper;
   if (g.rows <= 0 || g.cols <= 0) return;
   const double2 one = make_double2(1, 0), zero = make_double2(0, 0);
+  if (route == ZRoute::kInteger && !crt_reserve(rt, crt_plane_bytes(g.rows, n, false), crt_plane_bytes(g.cols, n, true),
+                                                crt_result_bytes(g.rows, g.cols, n)))
+    route = ZRoute::kLibrary;
   if (route == ZRoute::kLibrary) {
     for (int i = 0; i < count; ++i) {
       double2* const right = c[i] + (long long)b[i].c1 * ldc;   // columns of the second buffer
@@ -358,6 +361,10 @@ void zgram(Runtime& rt, int n, const ZBlock& a, const ZBlock* b, double2* const*
 void zupdate(Runtime& rt, int n, const ZBlock* z, const double2* y, int ldy, double2* const* c, int cols, int count,
              double alpha, double beta, ZRoute route) {
   if (n <= 0 || cols <= 0) return;
+  const int k = z[0].cols();
+  if (route == ZRoute::kInteger && !crt_reserve(rt, crt_plane_bytes(n, k, false), crt_plane_bytes(cols, k, true),
+                                                crt_result_bytes(n, cols, k)))
+    route = ZRoute::kLibrary;
   if (route == ZRoute::kLibrary) {
     const double2 al = make_double2(alpha, 0), one = make_double2(1, 0);
     for (int i = 0; i < count; ++i) {

@@ -68,6 +68,7 @@ struct AllocTimer {
 };
 
 void* device_alloc(size_t bytes, size_t* granted);   // devmem.cpp: caching allocator
+void* device_try_alloc(size_t bytes, size_t* granted);
 void device_free(void* p, size_t granted);
 
 // Owning device allocation through the caching allocator (devmem.h).
@@ -94,6 +95,14 @@ class DeviceBuffer {
     release();
     if (n) p_ = static_cast<T*>(device_alloc(n * sizeof(T), &cap_));
     n_ = n;
+  }
+  // At least n elements; false, and empty, where memory does not suffice.
+  bool try_reserve(size_t n) {
+    if (n <= n_) return true;
+    release();
+    p_ = static_cast<T*>(device_try_alloc(n * sizeof(T), &cap_));
+    if (p_) n_ = n;
+    return p_ != nullptr;
   }
   // Non-owning: n elements at p, which somebody else keeps alive.
   void view(T* p, size_t n) {

@@ -212,6 +212,10 @@ struct KOperatorSet {
 
 std::unique_ptr<KOperatorSet> prepare_operator(Context& ctx, Runtime& rt, const double k[3], bool fp64, bool fp32);
 
+// Gives back what only the iteration of a mixed solve uses of its operator (the
+// residue planes of the projectors); call after its work has completed.
+void release_solve_planes(KOperatorSet& ks);
+
 // H/S application on device blocks (column-major, leading dimension ld).
 template <typename R>
 void apply_hs(Context& ctx, KOperatorSet& ks, const cplx_t<R>* x, long long ld, int nb, cplx_t<R>* hx,

@@ -74,7 +74,8 @@ struct ThreadCache {
 };
 
 thread_local ThreadCache t_cache;
-std::atomic<long long> g_requests{0}, g_driver_allocs{0};
+std::atomic<long long> g_requests{0}, g_driver_allocs{0}, g_refused{0};
+std::atomic<size_t> g_refuse_above{0};
 
 void release_all_locked(Pool& pool) {
   for (auto& kv : pool) {
@@ -86,8 +87,12 @@ void release_all_locked(Pool& pool) {
 
 }  // namespace
 
-void* device_alloc(size_t bytes, size_t* granted) {
+void* device_try_alloc(size_t bytes, size_t* granted) {
   g_requests.fetch_add(1, std::memory_order_relaxed);
+  if (const size_t most = g_refuse_above.load(std::memory_order_relaxed); most != 0 && bytes > most) {
+    g_refused.fetch_add(1);
+    return nullptr;
+  }
   int dev = 0;
   cudaGetDevice(&dev);
   const Key key{dev, round_bytes(bytes)};
@@ -122,9 +127,15 @@ void* device_alloc(size_t bytes, size_t* granted) {
   }
   if (e != cudaSuccess) {
     cudaGetLastError();
-    fail(kInternal, "device allocation of " + std::to_string(bytes) + " bytes failed: " + cudaGetErrorString(e));
+    return nullptr;
   }
   *granted = key.second;
+  return p;
+}
+
+void* device_alloc(size_t bytes, size_t* granted) {
+  void* p = device_try_alloc(bytes, granted);
+  if (!p) fail(kInternal, "device allocation of " + std::to_string(bytes) + " bytes failed: out of memory");
   return p;
 }
 
@@ -144,6 +155,11 @@ void device_free(void* p, size_t granted) {
     }
   }
   timed_free(p, granted);
+}
+
+long long device_refuse_above(size_t bytes) {
+  g_refuse_above.store(bytes);
+  return g_refused.exchange(0);
 }
 
 void device_alloc_counts(long long* requests, long long* driver_allocations) {

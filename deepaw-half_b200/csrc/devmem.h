@@ -21,11 +21,15 @@
 
 namespace hb {
 
-void* device_alloc(size_t bytes, size_t* granted);   // throws hb::Error on failure
+void* device_alloc(size_t bytes, size_t* granted);       // throws hb::Error on failure
+void* device_try_alloc(size_t bytes, size_t* granted);   // null on failure
 void device_free(void* p, size_t granted);
 void device_cache_release();                          // return the cached blocks of all threads to the driver
 // Process-wide counts since start: device_alloc calls (cached or not) and the
 // cudaMalloc calls among them.
 void device_alloc_counts(long long* requests, long long* driver_allocations);
+// For tests: requests of more than `bytes` fail as if the device were full (0:
+// none do).  Returns how many did since the last call.
+long long device_refuse_above(size_t bytes);
 
 }  // namespace hb

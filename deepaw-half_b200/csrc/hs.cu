@@ -833,6 +833,22 @@ void apply_hs(Context& ctx, KOperatorSet& ks, const cplx_t<R>* x, long long ld, 
   pf.sweep_columns += nb;
 }
 
+namespace {
+
+// The planes of B given back; the products go to ZGEMM from here on.
+void release_integer(KOperator<double>& op) {
+  op.integer = false;
+  op.crt_bh = op.crt_b = CrtPlanes();
+  op.crt_bh_store.release();
+  op.crt_b_store.release();
+}
+
+}  // namespace
+
+void release_solve_planes(KOperatorSet& ks) {
+  if (ks.op64) release_integer(*ks.op64);
+}
+
 // Projector part: H X += B blockdiag(D) B^H X, S X += B blockdiag(Q) B^H X
 template <typename R>
 void apply_nonlocal(Runtime& rt, KOperator<R>& op, const cplx_t<R>* x, long long ld, int nb, cplx_t<R>* hx,
@@ -866,7 +882,15 @@ void apply_nonlocal(Runtime& rt, KOperator<R>& op, const cplx_t<R>* x, long long
     tc_cgemm(rt, op.b_planes, y, op.npw, 2 * nb, op.np, make_double2(1, 0), make_double2(1, 0), hx, false, ld, sx, nb);
   } else {
     const bool kept = op.crt_bh.planes != nullptr;
-    if (op.integer && zcrt_serves(op.np, nb, op.npw, kept) && zcrt_serves(op.npw, 2 * nb, op.np, kept)) {
+    auto room = [&]() {   // for the planes of B and of the blocks, and the residues
+      const bool ok = crt_reserve(rt, 0, std::max(crt_plane_bytes(nb, op.npw, true), crt_plane_bytes(2 * nb, op.np, true)),
+                                  std::max(crt_result_bytes(op.np, nb, op.npw), crt_result_bytes(op.npw, 2 * nb, op.np))) &&
+                      op.crt_bh_store.try_reserve(crt_plane_bytes(op.np, op.npw, false)) &&
+                      op.crt_b_store.try_reserve(crt_plane_bytes(op.npw, op.np, false));
+      if (!ok) release_integer(op);
+      return ok;
+    };
+    if (op.integer && zcrt_serves(op.np, nb, op.npw, kept) && zcrt_serves(op.npw, 2 * nb, op.np, kept) && room()) {
       // coeff = B^H X, [H X | S X] += B [DY | QY] on the integer tensor cores
       CrtSide s;
       s.ld = op.npw;

@@ -491,14 +491,29 @@ constexpr double kMaxBytes = 8e9;   // planes of one operand, and residues of on
 bool zcrt_serves(int m, int n, int k, bool a_kept) {
   if (m < 1 || n < 1 || k < 1 || k > kMaxK) return false;
   const double M = m, N = n, K = k;
-  if (2.0 * kMods * (std::max(M, N) + 160) * (K + 128) > kMaxBytes || 2.0 * kMods * (M + 128) * N > kMaxBytes) return false;
-  const double native = 8.0 * M * N * K / 36.0e12;
   const long long tiles = (long long)ceil_div(m, kBM) * ceil_div(n, kBN) * kMods;
   const int steps = ceil_div(k, kKB), s = pick_slices(tiles, steps, M * N), per = ceil_div(steps, s);
+  if (double(std::max(crt_plane_bytes(m, k, false), crt_plane_bytes(n, k, true))) > kMaxBytes ||
+      double(crt_result_bytes(m, n, k)) > kMaxBytes)
+    return false;
+  const double native = 8.0 * M * N * K / 36.0e12;
   const double waves = std::ceil(double(tiles) * s / 148.0);
   const double crt = 40e-6 + ((a_kept ? 0.0 : M) + N) * K * (2 * 16 + 2 * kMods) / 4.0e12 +
                      waves * (per * 1.0e-6 + 4e-6) + M * N * (4.0 * kMods * s + 16) / 3.0e12;
   return crt < 0.85 * native;
+}
+
+size_t crt_plane_bytes(int rows, int k, bool as_b) {
+  return size_t(2 * kMods) * pad_to(rows, as_b ? kBN : kBM) * pad_to(k, kKB) + size_t(rows) * sizeof(int);
+}
+
+size_t crt_result_bytes(int m, int n, int k) {
+  const int mt = ceil_div(m, kBM), nt = ceil_div(n, kBN), steps = ceil_div(k, kKB);
+  return size_t(2 * kMods) * pick_slices((long long)mt * nt * kMods, steps, double(m) * n) * n * mt * kBM;
+}
+
+bool crt_reserve(Runtime& rt, size_t a, size_t b, size_t result) {
+  return rt.crt_a.try_reserve(a) && rt.crt_b.try_reserve(b) && rt.crt_res.try_reserve(result);
 }
 
 CrtPlanes crt_prepare(Runtime& rt, const CrtSide& s, bool as_b, DeviceBuffer<unsigned char>& store) {
@@ -508,8 +523,7 @@ CrtPlanes crt_prepare(Runtime& rt, const CrtSide& s, bool as_b, DeviceBuffer<uns
   o.rows_pad = pad_to(s.rows, as_b ? kBN : kBM);
   o.k = s.k;
   o.k_pad = pad_to(s.k, kKB);
-  const size_t bytes = size_t(2 * kMods) * o.rows_pad * o.k_pad;
-  const size_t need = bytes + size_t(s.rows) * sizeof(int);
+  const size_t bytes = size_t(2 * kMods) * o.rows_pad * o.k_pad, need = crt_plane_bytes(s.rows, s.k, as_b);
   if (store.size() < need) store.resize(need);
   unsigned char* planes = store.get();
   int* e = reinterpret_cast<int*>(planes + bytes);   // bytes is a multiple of 1,024
@@ -538,7 +552,7 @@ void crt_product(Runtime& rt, const CrtPlanes& a, const CrtPlanes& b, double2 al
   const int steps = a.k_pad / kKB;
   const int s = pick_slices((long long)mt * nt * kMods, steps, double(m) * n), per = ceil_div(steps, s);
   const int slices = ceil_div(steps, per);
-  const size_t bytes = size_t(2 * kMods) * slices * n * m_pad;
+  const size_t bytes = crt_result_bytes(m, n, a.k);
   if (rt.crt_res.size() < bytes) rt.crt_res.resize(bytes);
   raise_smem_limit(crt_gemm_kernel, kSmem);
   crt_gemm_kernel<<<dim3(mt, nt, kMods * slices), kThreads, kSmem, st>>>(

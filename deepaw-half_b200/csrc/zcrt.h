@@ -28,6 +28,14 @@ struct CrtPlanes {
 // right-hand operand of products, else the left-hand one.
 CrtPlanes crt_prepare(Runtime& rt, const CrtSide& s, bool as_b, DeviceBuffer<unsigned char>& store);
 
+// Bytes of an operand's planes, and of the residues of an m x n product over k.
+size_t crt_plane_bytes(int rows, int k, bool as_b);
+size_t crt_result_bytes(int m, int n, int k);
+
+// The runtime's buffers grown to these sizes; false where memory does not
+// suffice (the product then goes to ZGEMM).
+bool crt_reserve(Runtime& rt, size_t a, size_t b, size_t result);
+
 // C (a.rows x b.rows, ldc) = alpha A B + beta C; columns from split_col on go
 // to C2 (column 0 on).  upper: tiles below the diagonal are left out.
 void crt_product(Runtime& rt, const CrtPlanes& a, const CrtPlanes& b, double2 alpha, double2 beta, double2* C,
