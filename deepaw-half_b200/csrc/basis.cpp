@@ -42,8 +42,10 @@ Basis build_basis(const Crystal& c, const std::array<int, 3>& shape, double encu
       // A row whose minimum misses the sphere by less than rounding is still looked at.
       if (!(room > -1e-6 * (1.0 + lim / a2))) continue;
       const double half = std::sqrt(std::max(0.0, room)) + 1.01;
-      const int lo = int(std::max(double(-(s3 / 2)), std::floor(mid - half - k[2])));
-      const int hi = int(std::min(double((s3 - 1) / 2), std::ceil(mid + half - k[2])));
+      // clamped to the box before the conversion: a k point far away may put the interval outside int
+      const double first = -(s3 / 2), last = (s3 - 1) / 2;
+      const int lo = int(std::min(std::max(first, std::floor(mid - half - k[2])), last + 1.0));
+      const int hi = int(std::max(std::min(last, std::ceil(mid + half - k[2])), first - 1.0));
       for (int n3 = lo; n3 <= hi; ++n3) {
         const double f2 = n3 + k[2];
         double q[3];
