@@ -294,6 +294,11 @@ struct SmallSolver {
   // SmallEigen::hegv too (cuSOLVER zpotrf / zhetrd / zunmtr around the
   // library's multisection and inverse-iteration kernels)
   bool own_large = false;
+  // FP64 mode: above this order an overlap that is not positive definite is an
+  // error, as it is to zhegvd, which served those orders; the own solver
+  // floors the pivots of the orders that it always served
+  bool strict = false;
+  static constexpr int kFlooredOrder = 164;
   SmallEigen eig;
   SmallSolver(Runtime& r, int m_, double2* a, double2* b, double* w) : rt(r), m(m_) {
     const char* sel = std::getenv("HALF_SMALL_EIG");
@@ -347,7 +352,7 @@ struct SmallSolver {
   // generalized problem of order n; the nev lowest eigenvectors are wanted
   void hegvd(double2* a, double2* b, int n, double* w, int nev) {
     if (own_order(n)) {
-      eig.hegv(rt, a, b, n, nev, w, info.get() + 1, info.get() + 2);
+      eig.hegv(rt, a, b, n, nev, w, info.get() + 1, info.get() + 2, strict && n > kFlooredOrder);
       return;
     }
     if (range) {
@@ -770,6 +775,7 @@ void solve_acc(Context& ctx, KOperatorSet& ks, int nbands, bool want_vectors, So
   sc.idx.upload(order, rt.stream);
   SmallSolver ss(rt, m, sc.hsub.get(), sc.ssub.get(), sc.w.get());
   ss.range = ss.range && guarded;   // the FP64 mode keeps the reference's zhegvd
+  ss.strict = !guarded;
   const double seed_threshold = std::max(cfg.tol * 1e-2, 1e-12);
   std::vector<double> norms;
   // Soft locking (guard-band modes): a requested band whose residual is at or

@@ -21,6 +21,7 @@
 #include "blockops.h"
 #include "context.h"
 #include "devmem.h"
+#include "eig.h"
 #include "staging.h"
 #include "tc_gemm.h"
 #include "zcrt.h"
@@ -1131,6 +1132,29 @@ extern "C" int hb_diag_gram_route(int n, int rows, int cols, int integer) {
 
 extern "C" int hb_diag_update_route(int n, int k, int cols, int integer) {
   return int(zupdate_route(n, k, cols, integer != 0));
+}
+
+// The pencil a y = w b y (order n, upper triangles; a and b are overwritten): the nev lowest pairs to w and a;
+// *status, *chol_status as SmallEigen::hegv's.
+extern "C" int hb_diag_pencil(int n, int nev, int strict, void* a, void* b, void* w, int* status, int* chol_status,
+                              char* error, int cap) {
+  clear_error(error, cap);
+  return guarded(error, cap, [&]() -> int {
+    if (n < 1 || nev < 1 || nev > n || !status || !chol_status) fail(kInvalidArgument, "invalid pencil");
+    if (!device_pointer(a) || !device_pointer(b) || !device_pointer(w)) fail(kInvalidArgument, "operands must be device memory");
+    std::lock_guard<std::mutex> lock(g_diag_mutex);
+    Runtime& rt = diagnostic_runtime();
+    rt.prof.reset();
+    SmallEigen eig;
+    DeviceBuffer<int> info(2);
+    info.zero(rt.stream);
+    eig.hegv(rt, static_cast<double2*>(a), static_cast<double2*>(b), n, nev, static_cast<double*>(w), info.get(),
+             info.get() + 1, strict != 0);
+    const std::vector<int> h = info.download(rt.stream);
+    *status = h[0];
+    *chol_status = h[1];
+    return HALF_SUCCESS;
+  });
 }
 
 // 'G': c (a1 + a2 x b1 + b2, leading dimension ldc) = [a | a_2]^H [b | b_2].  'U': c (n x b1) = beta c + alpha [a | a_2] b.

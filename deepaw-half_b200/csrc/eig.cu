@@ -549,7 +549,7 @@ __global__ void hermitian_fill_kernel(double2* A, int n) {
 // The panel F and the diagonal block travel through global memory (L2): one
 // writer and many readers, where pushes through distributed shared memory
 // cost 6-8 cycles per 16 bytes and target.  Two cluster barriers per block.
-// *status = 1 if a pivot was not finite.
+// *status = 1 if a pivot was not finite or, with floor 0, not positive.
 //
 // Bound by the chain: about 4 us a block.  Measured per solve at orders
 // around 120 (12-atom cell, B200): one CTA with the packed triangle, one
@@ -568,6 +568,7 @@ constexpr int kClThreads = 256;
 constexpr int kClWarps = kClThreads / 32;
 constexpr int kClCols = 4;                        // columns a warp carries at once
 constexpr int kFB = 8;                            // columns per block of the metric factor
+constexpr double kPivotFloor = 1.0e-14;           // of the unit scaled diagonal
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
@@ -643,7 +644,8 @@ __host__ __device__ inline size_t factor_panel(int m) { return size_t(kFB) * m +
 template <bool kGrid>
 __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __restrict__ M, int m, int P,
                                                                    double2* __restrict__ panels,
-                                                                   int* __restrict__ status, int* grid_state) {
+                                                                   int* __restrict__ status, int* grid_state,
+                                                                   double floor) {
   wait_previous();
   const int rank = blockIdx.x;   // the grid is one cluster of P CTAs, or a cooperative launch of P
   const int nblk = (m + kFB - 1) / kFB, nown = nblk > rank ? (nblk - rank + P - 1) / P : 0;
@@ -705,7 +707,7 @@ __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __re
         __syncwarp();
         for (int l = 0; l < kb; ++l) {
           const double p = sD[l * kFB + l].x;
-          const bool dep = !(p > 1.0e-14);   // also true for NaN
+          const bool dep = !(p > floor);   // also true for NaN
           const double invp = dep ? 0.0 : 1.0 / p;
           double2 out[2];
 #pragma unroll
@@ -728,7 +730,7 @@ __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __re
             sC[l * kFB + lane] = cscale(sD[l * kFB + lane], invp);
           }
           if (lane == 0) {
-            if (!isfinite(p)) bad = 1;
+            if (!isfinite(p) || (dep && floor == 0.0)) bad = 1;
             sinv[l] = invp;
             ir[k0 + l] = p;   // 1 / R(k,k) below
           }
@@ -739,7 +741,7 @@ __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __re
         }
         if (lane < kb) {
           const double p = ir[k0 + lane];
-          ir[k0 + lane] = !(p > 1.0e-14) ? 1.0e7 : 1.0 / sqrt(p);
+          ir[k0 + lane] = !(p > floor) ? 1.0e7 : 1.0 / sqrt(p);
         }
         for (int e = lane; e < kFB * kFB; e += 32) {
           const int r = e >> 3, c = e & 7;
@@ -1495,7 +1497,8 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
 
 // Generalized problem A y = lambda B y (itype 1, upper triangles used), B HPD.
 // The nev lowest eigenvectors (Y^H B Y = I) overwrite A[:, :nev].
-void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, double* w, int* status, int* chol_status) {
+void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, double* w, int* status, int* chol_status,
+                      bool strict) {
   reserve(rt, n);
   cudaStream_t s = rt.stream;
   if (n <= kOwnMaxOrder || grid_order(rt, n)) {
@@ -1510,7 +1513,7 @@ void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, doubl
     // 480 to 512 bands of the 12-atom cell at 5e-6 to 4e-5 eV whatever the
     // tolerance; these reach 1e-7 in 9 iterations.)
     if (n <= kOwnMaxOrder) {
-      metric_normalize(rt, B, n, chol_status);
+      metric_normalize(rt, B, n, chol_status, strict);
     } else {
       int p = factor_grid_ctas(rt, n);
       const size_t fsm = factor_smem(n, p, true);
@@ -1519,7 +1522,8 @@ void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, doubl
       raise_smem_limit(metric_factor_kernel<true>, kSmemMax);
       double2* pp = panels.get();
       int* gp = grid_state.get();
-      void* args[] = {&B, &n, &p, &pp, &chol_status, &gp};
+      double floor = strict ? 0.0 : kPivotFloor;
+      void* args[] = {&B, &n, &p, &pp, &chol_status, &gp, &floor};
       HALF_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(metric_factor_kernel<true>), dim3(p),
                                             dim3(kClThreads), args, fsm, s));
       rt.prof.launches += 1;
@@ -1567,12 +1571,12 @@ void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, doubl
 
 // U with (P U)^H S (P U) = I from M = P^H S P, overwriting M (see
 // metric_factor_kernel); false when m is beyond the cluster's shared memory.
-bool SmallEigen::metric_normalize(Runtime& rt, double2* M, int m, int* status) {
+bool SmallEigen::metric_normalize(Runtime& rt, double2* M, int m, int* status, bool strict) {
   if (m > kOwnMaxOrder) return false;
   const int p = factor_ctas(m);
   if (panels.size() < 2 * factor_panel(m)) panels.resize(2 * factor_panel(kOwnMaxOrder));
   launch_cluster(metric_factor_kernel<false>, p, factor_smem(m, p), rt.stream, M, m, p, panels.get(), status,
-                 static_cast<int*>(nullptr));
+                 static_cast<int*>(nullptr), strict ? 0.0 : kPivotFloor);
   rt.prof.launches += 1;
   return true;
 }

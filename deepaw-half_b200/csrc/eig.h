@@ -28,11 +28,14 @@ struct SmallEigen {
   void heev(Runtime& rt, double2* A, int n, int nev, double* w, int* status);
   // A y = lambda B y, B Hermitian positive definite; Y^H B Y = I.
   // *chol_status (device): nonzero when the factor saw a pivot that is not
-  // finite (beyond the grid-wide kernels' orders zpotrf's info)
-  void hegv(Runtime& rt, double2* A, double2* B, int n, int nev, double* w, int* status, int* chol_status);
+  // finite (beyond the grid-wide kernels' orders zpotrf's info).  strict: a
+  // pivot that is not positive is an error, as in zpotrf; otherwise dependent
+  // and negative pivots are floored as in the metric.
+  void hegv(Runtime& rt, double2* A, double2* B, int n, int nev, double* w, int* status, int* chol_status,
+            bool strict = false);
   // ACC correction metric: M = P^H S P (m x m) -> U, upper triangular, with
   // (P U)^H S (P U) = I; returns false (nothing launched) when m is too large.
-  bool metric_normalize(Runtime& rt, double2* M, int m, int* status);
+  bool metric_normalize(Runtime& rt, double2* M, int m, int* status, bool strict = false);
   // Whether an order above kOwnMaxOrder goes through the grid-wide kernels,
   // whose metric factor floors dependent pivots like the cluster kernel's.
   static bool grid_order(const Runtime& rt, int n);
