@@ -499,10 +499,8 @@ struct AccRun {
     if (host[2 * m + 3] != 0.0) tc_check(rt);   // raises
     rt.crt_pending = false;
     mark("residual");
-    if (infos[0] != 0) fail(kInternal, "ACC correction metric eigensolve failed (info " + std::to_string(infos[0]) + ")");
-    if (infos[1] != 0) fail(kInternal, "ACC small generalized eigensolve failed (info " + std::to_string(infos[1]) + ")");
-    if (infos[2] != 0)
-      fail(kInternal, "ACC Rayleigh-Ritz overlap is not positive definite (Cholesky info " + std::to_string(infos[2]) + ")");
+    const std::string failure = pencil_failure(infos);
+    if (!failure.empty()) fail(kInternal, failure);
     order_requested();
     double mx = 0;
     for (int j : req) mx = std::max(mx, norms[j]);

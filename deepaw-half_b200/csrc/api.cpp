@@ -1134,6 +1134,9 @@ extern "C" int hb_diag_update_route(int n, int k, int cols, int integer) {
   return int(zupdate_route(n, k, cols, integer != 0));
 }
 
+// pencil_failure of three status words.
+extern "C" void hb_diag_pencil_failure(const int* infos, char* text, int cap) { export_error(pencil_failure(infos), text, cap); }
+
 // The pencil a y = w b y (order n, upper triangles; a and b are overwritten): the nev lowest pairs to w and a;
 // *status, *chol_status as SmallEigen::hegv's.
 extern "C" int hb_diag_pencil(int n, int nev, int strict, void* a, void* b, void* w, int* status, int* chol_status,

@@ -210,8 +210,8 @@ __device__ double multisect(const double* d, const double* e2, int n, int k, dou
 }
 
 // Eigenvalues 0..ne-1 of T (ascending), one warp each.  Also sets *status for
-// the vector kernel that follows on the stream: 0, or 2 when a grid barrier of
-// the tridiagonalisation gave up.
+// the vector kernel that follows on the stream: 0, or kWaitGaveUp when a grid
+// barrier of the tridiagonalisation gave up.
 __global__ void __launch_bounds__(32 * kValueWarps) tridiag_values_kernel(const double* __restrict__ d_in,
                                                                           const double* __restrict__ e_in, int n,
                                                                           int ne, double* __restrict__ lam,
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(32 * kValueWarps) tridiag_values_kernel(const 
   double* e = d + n;
   double* e2 = e + n;
   __shared__ double s_gl, s_gu, s_norm;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *status = grid_err && *grid_err ? 2 : 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *status = grid_err && *grid_err ? kWaitGaveUp : 0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     d[i] = d_in[i];
     e[i] = i < n - 1 ? e_in[i] : 0.0;
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kVectorThreads) tridiag_vectors_kernel(
       for (int i = 0; i < n; ++i) nrm += x[i * st] * x[i * st];
       nrm = sqrt(nrm);
       if (!(nrm > 0) || !isfinite(nrm)) {
-        atomicExch(status, 1);
+        atomicCAS(status, 0, 1);   // an earlier report stays
         break;
       }
       const double inv = 1.0 / nrm;
@@ -775,7 +775,7 @@ __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __re
     }
     if (k1 >= m) break;   // the last block has no columns to its right
     if (!barrier()) {
-      if (tid == 0) atomicExch(status, 2);
+      if (tid == 0) atomicExch(status, kWaitGaveUp);
       return;
     }
     if (rank != owner) {
@@ -814,7 +814,7 @@ __global__ void __launch_bounds__(kClThreads) metric_factor_kernel(double2* __re
       }
     }
     if (!barrier()) {
-      if (tid == 0) atomicExch(status, 2);
+      if (tid == 0) atomicExch(status, kWaitGaveUp);
       return;
     }
     if constexpr (kGrid) {
@@ -1365,6 +1365,16 @@ __global__ void __launch_bounds__(32 * kValueWarps) tridiag_values_global_kernel
 }
 
 }  // namespace
+
+std::string pencil_failure(const int* infos) {
+  if (infos[1] == kWaitGaveUp || infos[2] == kWaitGaveUp)
+    return "ACC small generalized eigensolve: a grid-wide kernel gave up waiting for its other thread blocks";
+  if (infos[0] != 0) return "ACC correction metric eigensolve failed (info " + std::to_string(infos[0]) + ")";
+  if (infos[2] != 0)
+    return "ACC Rayleigh-Ritz overlap is not positive definite (Cholesky info " + std::to_string(infos[2]) + ")";
+  if (infos[1] != 0) return "ACC small generalized eigensolve failed (info " + std::to_string(infos[1]) + ")";
+  return "";
+}
 
 void SmallEigen::reserve(Runtime& rt, int nmax) {
   if (nmax <= cap) return;

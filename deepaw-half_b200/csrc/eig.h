@@ -1,11 +1,19 @@
 // Device-resident small Hermitian eigensolvers (see eig.cu).
 #pragma once
 
+#include <string>
 #include <vector>
 
 #include "context.h"
 
 namespace hb {
+
+// Status of a pencil whose grid-wide kernel gave up waiting for its other CTAs.
+constexpr int kWaitGaveUp = -100;
+
+// What went wrong in a solver iteration, from its three status words (metric,
+// pencil, factor of the overlap); empty when nothing did.
+std::string pencil_failure(const int* infos);
 
 struct SmallEigen {
   // Orders the cluster kernels serve: the matrix fits the shared memory of 16
