@@ -346,8 +346,10 @@ struct SmallSolver {
   }
   // orders of the own solver; those of the grid-wide tridiagonalisation in the
   // guard-band modes only (the FP64 mode keeps zhegvd there)
-  bool own_order(int n) const {
-    return own && (n <= SmallEigen::kOwnMaxOrder || (range && SmallEigen::grid_order(rt, n)) || own_large);
+  bool own_order(int n) const { return own_floored(n) || (own && own_large); }
+  // those whose dependent pivots it floors
+  bool own_floored(int n) const {
+    return own && (SmallEigen::cluster_order(rt, n) || (range && SmallEigen::grid_order(rt, n)));
   }
   // generalized problem of order n; the nev lowest eigenvectors are wanted
   void hegvd(double2* a, double2* b, int n, double* w, int nev) {
@@ -618,7 +620,7 @@ struct AccRun {
     const int mu = m - nl;
     const long long off = (long long)nl * n;
     const int ord = mu + np;
-    const bool own_pencil = ss.own && (ord <= SmallEigen::kOwnMaxOrder || (ss.range && SmallEigen::grid_order(rt, ord)));
+    const bool own_pencil = ss.own_floored(ord);
     bool skip_metric = guarded && ss.own;
     double2* hs = sc.hsub.get();
     double2* ssb = sc.ssub.get();

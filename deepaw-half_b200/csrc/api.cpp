@@ -1134,6 +1134,19 @@ extern "C" int hb_diag_update_route(int n, int k, int cols, int integer) {
   return int(zupdate_route(n, k, cols, integer != 0));
 }
 
+// Limits of contexts made from here on, and what a new runtime then finds: cluster size | 256 for grid-wide launches.
+extern "C" int hb_diag_limit_pencils(int cluster_ctas, int grid) {
+  limit_pencil_launches(cluster_ctas, grid != 0);
+  int found = -1;
+  guarded(nullptr, 0, [&]() -> int {
+    Runtime rt;
+    SmallEigen::cluster_order(rt, 1);
+    found = rt.cluster_ctas | (rt.grid_pencils ? 256 : 0);
+    return HALF_SUCCESS;
+  });
+  return found;
+}
+
 // pencil_failure of three status words.
 extern "C" void hb_diag_pencil_failure(const int* infos, char* text, int cap) { export_error(pencil_failure(infos), text, cap); }
 

@@ -73,6 +73,8 @@ struct Runtime {
   cublasHandle_t blas = nullptr;
   cusolverDnHandle_t solver = nullptr;
   int sms = 148;         // multiprocessors of the stream's device
+  int cluster_ctas = -1; // largest cluster that the pencil kernels (eig.cu) can be launched with; -1: not asked yet
+  bool grid_pencils = true;   // their cooperative launches over all multiprocessors are possible
   bool bf16x9 = false;   // cuBLAS offers FP32 emulation on BF16 tensor cores
   bool tc_gemm = true;   // complex FP32 GEMMs on the library's tcgen05 kernel (tc_gemm.cu)
   DeviceBuffer<unsigned char> tc_work;   // its split-K partial sums, grow-only

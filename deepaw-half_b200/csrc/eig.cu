@@ -27,6 +27,7 @@
 //
 // Y^H B Y = I, the same normalisation as zhegvd (itype 1, upper).
 #include <algorithm>
+#include <atomic>
 #include <cooperative_groups.h>
 
 #include <cfloat>
@@ -1294,29 +1295,91 @@ constexpr size_t kGridSmem = 227 * 1024 - 2560;   // leaves room for the kernel'
 int hetrd_ctas(int n) { return n <= 40 ? 4 : n <= 176 ? 8 : 16; }
 
 // CTAs for an order-m metric factor: one while its panel update is short.
+int factor_ctas(int m) { return m <= 64 ? 1 : m <= 176 ? 8 : 16; }
+
+// And over the whole GPU: one per column block, at most one per SM.
 int factor_grid_ctas(const Runtime& rt, int m) { return std::min(rt.sms, ceil_div(m, kFB)); }
 
-int factor_ctas(int m) { return m <= 64 ? 1 : m <= 176 ? 8 : 16; }
+// Launch of one cluster of `ctas` CTAs.
+struct ClusterLaunch {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[2];
+  template <typename... KArgs>
+  ClusterLaunch(void (*kernel)(KArgs...), int ctas, size_t smem, cudaStream_t s) {
+    raise_smem_limit(kernel, smem);
+    if (ctas > 8) HALF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(kClThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // as launch_chained
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+  }
+  ClusterLaunch(const ClusterLaunch&) = delete;
+};
 
 template <typename... KArgs, typename... Args>
 void launch_cluster(void (*kernel)(KArgs...), int ctas, size_t smem, cudaStream_t s, Args... args) {
+  ClusterLaunch l(kernel, ctas, smem, s);
+  HALF_CUDA(cudaLaunchKernelEx(&l.cfg, kernel, args...));
+}
+
+template <typename... KArgs>
+bool cluster_fits(void (*kernel)(KArgs...), int ctas, size_t smem) {
+  ClusterLaunch l(kernel, ctas, smem, nullptr);
+  l.cfg.numAttrs = 1;   // the cluster's size alone
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &l.cfg) == cudaSuccess) return clusters > 0;
+  cudaGetLastError();
+  return false;
+}
+
+template <typename... KArgs>
+bool block_fits(void (*kernel)(KArgs...), size_t smem) {
   raise_smem_limit(kernel, smem);
-  if (ctas > 8) HALF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(ctas);
-  cfg.blockDim = dim3(kClThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = ctas;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // as launch_chained
-  at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 2;
-  HALF_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+  int blocks = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, kClThreads, smem) == cudaSuccess) return blocks > 0;
+  cudaGetLastError();
+  return false;
+}
+
+std::atomic<int> g_cluster_limit{16};
+std::atomic<bool> g_grid_limit{true};
+
+// Asks the device, once per runtime, what the pencil kernels can be launched with.
+void ask_pencil_limits(Runtime& rt) {
+  if (rt.cluster_ctas >= 0) return;
+  rt.cluster_ctas = 0;
+  for (const auto [ctas, order] : {std::pair(16, SmallEigen::kOwnMaxOrder), std::pair(8, 176), std::pair(4, 40)}) {
+    if (ctas > g_cluster_limit.load()) continue;
+    if (cluster_fits(hetrd_kernel, ctas, hetrd_smem(order, ctas)) &&
+        cluster_fits(metric_factor_kernel<false>, factor_ctas(order), factor_smem(order, factor_ctas(order)))) {
+      rt.cluster_ctas = ctas;
+      break;
+    }
+  }
+  rt.grid_pencils = g_grid_limit.load() && block_fits(hetrd_grid_kernel, kGridSmem) &&
+                    block_fits(metric_factor_kernel<true>, kSmemMax);
+}
+
+// A cooperative launch; false (nothing launched, and not tried again on this
+// runtime) where the process may not use as many SMs at once.
+bool launch_grid(Runtime& rt, const void* kernel, int ctas, void** args, size_t smem) {
+  const cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(ctas), dim3(kClThreads), args, smem, rt.stream);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    rt.grid_pencils = false;
+    return false;
+  }
+  HALF_CUDA(e);
+  rt.prof.launches += 1;
+  return true;
 }
 
 __global__ void real_to_complex_block_kernel(const double* __restrict__ z, long long count, double2* __restrict__ out) {
@@ -1407,9 +1470,19 @@ void SmallEigen::reserve(Runtime& rt, int nmax) {
   work.resize(size_t(std::max({l1, l2, l3, 1})));
 }
 
-// Whether order n goes through the grid-wide kernels.
-bool SmallEigen::grid_order(const Runtime& rt, int n) {
-  return n > kOwnMaxOrder && n <= kGridMaxOrder && n <= kGridCols * rt.sms && hetrd_grid_smem(n, rt.sms) <= kGridSmem &&
+void limit_pencil_launches(int cluster_ctas, bool grid) {
+  g_cluster_limit.store(cluster_ctas);
+  g_grid_limit.store(grid);
+}
+
+bool SmallEigen::cluster_order(Runtime& rt, int n) {
+  ask_pencil_limits(rt);
+  return n <= kOwnMaxOrder && std::max(hetrd_ctas(n), factor_ctas(n)) <= rt.cluster_ctas;
+}
+
+bool SmallEigen::grid_order(Runtime& rt, int n) {
+  ask_pencil_limits(rt);
+  return rt.grid_pencils && n > kOwnMaxOrder && n <= kGridMaxOrder && n <= kGridCols * rt.sms && hetrd_grid_smem(n, rt.sms) <= kGridSmem &&
          factor_smem(n, factor_grid_ctas(rt, n), true) <= kSmemMax;
 }
 
@@ -1424,10 +1497,12 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
   reserve(rt, n);
   cudaStream_t s = rt.stream;
   const int* gave_up = nullptr;
-  if (n <= kOwnMaxOrder) {   // whole reduction in one cluster
+  bool reduced = false;
+  if (cluster_order(rt, n)) {   // whole reduction in one cluster
     const int p = hetrd_ctas(n);
     launch_cluster(hetrd_kernel, p, hetrd_smem(n, p), s, A, n, d.get(), e.get(), tau.get());
     rt.prof.launches += 1;
+    reduced = true;
   } else if (grid_order(rt, n)) {
     const size_t gsm = hetrd_grid_smem(n, rt.sms);
     if (exchange.size() < 4 * size_t(n)) exchange.resize(4 * size_t(kGridMaxOrder));
@@ -1438,10 +1513,10 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
     double2 *tp = tau.get(), *xp = exchange.get();
     int *cp = grid_state.get(), *gp = cp + 1;
     void* args[] = {&A, &n, &dp, &ep, &tp, &xp, &cp, &gp};
-    HALF_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(hetrd_grid_kernel), dim3(rt.sms),
-                                          dim3(kClThreads), args, gsm, s));
-    rt.prof.launches += 1;
-  } else {
+    reduced = launch_grid(rt, reinterpret_cast<const void*>(hetrd_grid_kernel), rt.sms, args, gsm);
+  }
+  if (!reduced) {
+    gave_up = nullptr;
     cusolver_check(cusolverDnZhetrd(rt.solver, CUBLAS_FILL_MODE_UPPER, n, reinterpret_cast<cuDoubleComplex*>(A), n,
                                     d.get(), e.get(), reinterpret_cast<cuDoubleComplex*>(tau.get()),
                                     reinterpret_cast<cuDoubleComplex*>(work.get()), int(work.size()), info.get()),
@@ -1511,7 +1586,22 @@ void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, doubl
                       bool strict) {
   reserve(rt, n);
   cudaStream_t s = rt.stream;
-  if (n <= kOwnMaxOrder || grid_order(rt, n)) {
+  bool factored = false;
+  if (cluster_order(rt, n)) {
+    factored = metric_normalize(rt, B, n, chol_status, strict);
+  } else if (grid_order(rt, n)) {
+    int p = factor_grid_ctas(rt, n);
+    const size_t fsm = factor_smem(n, p, true);
+    if (panels.size() < 2 * factor_panel(n)) panels.resize(2 * factor_panel(kGridMaxOrder));
+    clear_grid_state(s);
+    raise_smem_limit(metric_factor_kernel<true>, kSmemMax);
+    double2* pp = panels.get();
+    int* gp = grid_state.get();
+    double floor = strict ? 0.0 : kPivotFloor;
+    void* args[] = {&B, &n, &p, &pp, &chol_status, &gp, &floor};
+    factored = launch_grid(rt, reinterpret_cast<const void*>(metric_factor_kernel<true>), p, args, fsm);
+  }
+  if (factored) {
     // B -> X = D R^-1 with X^H B X = I (metric_factor_kernel), C = X^H A X,
     // C V = V Lambda, Y = X V: the same pencil reduction as zhegvd's
     // Cholesky / two triangular solves, with the factor inverted in shared
@@ -1522,22 +1612,6 @@ void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, doubl
     // fixed point relative to its norm, as zcrt.cu does, stop the residuals of
     // 480 to 512 bands of the 12-atom cell at 5e-6 to 4e-5 eV whatever the
     // tolerance; these reach 1e-7 in 9 iterations.)
-    if (n <= kOwnMaxOrder) {
-      metric_normalize(rt, B, n, chol_status, strict);
-    } else {
-      int p = factor_grid_ctas(rt, n);
-      const size_t fsm = factor_smem(n, p, true);
-      if (panels.size() < 2 * factor_panel(n)) panels.resize(2 * factor_panel(kGridMaxOrder));
-      clear_grid_state(s);
-      raise_smem_limit(metric_factor_kernel<true>, kSmemMax);
-      double2* pp = panels.get();
-      int* gp = grid_state.get();
-      double floor = strict ? 0.0 : kPivotFloor;
-      void* args[] = {&B, &n, &p, &pp, &chol_status, &gp, &floor};
-      HALF_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(metric_factor_kernel<true>), dim3(p),
-                                            dim3(kClThreads), args, fsm, s));
-      rt.prof.launches += 1;
-    }
     launch_chained(ceil_div((long long)n * n, 256), 256, 0, s, hermitian_fill_kernel,
         A, n);
     rt.prof.launches += 1;
@@ -1582,7 +1656,7 @@ void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, doubl
 // U with (P U)^H S (P U) = I from M = P^H S P, overwriting M (see
 // metric_factor_kernel); false when m is beyond the cluster's shared memory.
 bool SmallEigen::metric_normalize(Runtime& rt, double2* M, int m, int* status, bool strict) {
-  if (m > kOwnMaxOrder) return false;
+  if (!cluster_order(rt, m)) return false;
   const int p = factor_ctas(m);
   if (panels.size() < 2 * factor_panel(m)) panels.resize(2 * factor_panel(kOwnMaxOrder));
   launch_cluster(metric_factor_kernel<false>, p, factor_smem(m, p), rt.stream, M, m, p, panels.get(), status,

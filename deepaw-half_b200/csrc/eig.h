@@ -11,6 +11,10 @@ namespace hb {
 // Status of a pencil whose grid-wide kernel gave up waiting for its other CTAs.
 constexpr int kWaitGaveUp = -100;
 
+// For tests: runtimes that have not asked the device yet take at most clusters
+// of this size, and no grid-wide launch unless grid (16, true: the device's own limits).
+void limit_pencil_launches(int cluster_ctas, bool grid);
+
 // What went wrong in a solver iteration, from its three status words (metric,
 // pencil, factor of the overlap); empty when nothing did.
 std::string pencil_failure(const int* infos);
@@ -42,11 +46,14 @@ struct SmallEigen {
   void hegv(Runtime& rt, double2* A, double2* B, int n, int nev, double* w, int* status, int* chol_status,
             bool strict = false);
   // ACC correction metric: M = P^H S P (m x m) -> U, upper triangular, with
-  // (P U)^H S (P U) = I; returns false (nothing launched) when m is too large.
+  // (P U)^H S (P U) = I; returns false (nothing launched) when m is not a cluster_order.
   bool metric_normalize(Runtime& rt, double2* M, int m, int* status, bool strict = false);
-  // Whether an order above kOwnMaxOrder goes through the grid-wide kernels,
-  // whose metric factor floors dependent pivots like the cluster kernel's.
-  static bool grid_order(const Runtime& rt, int n);
+  // Whether order n goes through the cluster kernels, or above kOwnMaxOrder
+  // through the grid-wide ones, whose metric factor floors dependent pivots like
+  // the cluster kernel's.  Where the device (or the part of it that the process
+  // may use) cannot hold such a launch, neither does, and the order is cuSOLVER's.
+  static bool cluster_order(Runtime& rt, int n);
+  static bool grid_order(Runtime& rt, int n);
 
  private:
   void clear_grid_state(cudaStream_t s);

@@ -43,6 +43,10 @@ def _solve(a, b, strict):
 def test_indefinite_overlap_is_reported(n):
     a, b = _pencil(n, -0.05, n)
     assert _solve(a, b, True)[2] != 0
+
+
+def test_floored_variant_accepts_it():
+    a, b = _pencil(165, -0.05, 165)
     assert _solve(a, b, False)[2] == 0
 
 
