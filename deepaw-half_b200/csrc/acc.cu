@@ -465,11 +465,11 @@ struct AccRun {
     if constexpr (sizeof(R) == 8) {
       const ZBlock b[2] = {{blk.hx(), m}, {blk.sx(), m}};
       double2* const c[2] = {hs, ssb};
-      zgram(rt, n, {blk.x(), m}, b, c, 2, m, true, zgram_route(n, m, m, integer));
+      zgram(rt, n, {blk.x(), m}, b, c, 2, m, true, zgram_route(rt.sms, n, m, m, integer));
       ss.hegvd(hs, ssb, m, sc.w.get(), m);
       const ZBlock z[3] = {{blk.x(), m}, {blk.hx(), m}, {blk.sx(), m}};
       double2* const out[3] = {blk.X[nx].get(), blk.HX[nx].get(), blk.SX[nx].get()};
-      zupdate(rt, n, z, hs, m, out, m, 3, 1.0, 0.0, zupdate_route(n, m, m, false));
+      zupdate(rt, n, z, hs, m, out, m, 3, 1.0, 0.0, zupdate_route(rt.sms, n, m, m, false));
     } else {
       const auto one = cval<R>(1.0), zero = cval<R>(0.0);
       gemm_to64(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, m, n, blk.x(), n, blk.hx(), n, hs, m);
@@ -596,10 +596,10 @@ struct AccRun {
     if constexpr (sizeof(R) == 8) {
       const ZBlock b = {blk.SP.get(), np};
       double2* const c = blk.small.get();
-      zgram(rt, n, {blk.x(), m}, &b, &c, 1, m, false, zgram_route(n, m, np, integer));
+      zgram(rt, n, {blk.x(), m}, &b, &c, 1, m, false, zgram_route(rt.sms, n, m, np, integer));
       const ZBlock z[3] = {{blk.x(), m}, {blk.hx(), m}, {blk.sx(), m}};
       double2* const out[3] = {blk.P.get(), blk.HP.get(), blk.SP.get()};
-      zupdate(rt, n, z, blk.small.get(), m, out, np, 3, -1.0, 1.0, zupdate_route(n, m, np, integer));
+      zupdate(rt, n, z, blk.small.get(), m, out, np, 3, -1.0, 1.0, zupdate_route(rt.sms, n, m, np, integer));
     } else {
       gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, m, np, n, one, blk.x(), n, blk.SP.get(), n, zero, blk.small.get(), m);
       gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, m, mone, blk.x(), n, blk.small.get(), m, one, blk.P.get(), n);
@@ -639,7 +639,7 @@ struct AccRun {
       if constexpr (sizeof(R) == 8) {
         const ZBlock b[2] = {{blk.hx() + off, mu, hpu, np}, {blk.sx() + off, mu, spu, np}};
         double2* const c[2] = {hs, ssb};
-        zgram(rt, n, {blk.x() + off, mu, pu, np}, b, c, 2, ord, true, zgram_route(n, ord, ord, integer));
+        zgram(rt, n, {blk.x() + off, mu, pu, np}, b, c, 2, ord, true, zgram_route(rt.sms, n, ord, ord, integer));
       } else {
         project_upper(rt, n, mu, np, blk.x() + off, pu, blk.hx() + off, hpu, hs);
         project_upper(rt, n, mu, np, blk.x() + off, pu, blk.sx() + off, spu, ssb);
@@ -673,7 +673,7 @@ struct AccRun {
     if constexpr (sizeof(R) == 8) {
       const ZBlock z[3] = {{blk.x() + off, mu, pu, np}, {blk.hx() + off, mu, hpu, np}, {blk.sx() + off, mu, spu, np}};
       double2* const out[3] = {blk.X[nx].get() + off, blk.HX[nx].get() + off, blk.SX[nx].get() + off};
-      zupdate(rt, n, z, hs, ord, out, mu, 3, 1.0, 0.0, zupdate_route(n, ord, mu, false));
+      zupdate(rt, n, z, hs, ord, out, mu, 3, 1.0, 0.0, zupdate_route(rt.sms, n, ord, mu, false));
     } else {
       rotate(ord, mu, np, off, pu, hpu, spu, hs, nx);
     }
@@ -708,7 +708,7 @@ struct AccRun {
     double2* metric = sc.metric.get();
     if constexpr (sizeof(R) == 8) {
       const ZBlock b = {blk.SP.get(), np};
-      zgram(rt, n, {blk.P.get(), np}, &b, &metric, 1, np, true, zgram_route(n, np, np, integer));
+      zgram(rt, n, {blk.P.get(), np}, &b, &metric, 1, np, true, zgram_route(rt.sms, n, np, np, integer));
     } else {
       gemm_to64(rt, CUBLAS_OP_C, CUBLAS_OP_N, np, np, n, blk.P.get(), n, blk.SP.get(), n, metric, np);
     }
@@ -722,7 +722,7 @@ struct AccRun {
     if constexpr (sizeof(R) == 8) {
       const ZBlock z[3] = {{blk.P.get(), np}, {blk.HP.get(), np}, {blk.SP.get(), np}};
       double2* const out[3] = {blk.PU.get(), blk.HPU.get(), blk.SPU.get()};
-      zupdate(rt, n, z, metric, np, out, np, 3, 1.0, 0.0, zupdate_route(n, np, np, false));
+      zupdate(rt, n, z, metric, np, out, np, 3, 1.0, 0.0, zupdate_route(rt.sms, n, np, np, false));
     } else {
       to_r(metric, np, blk.small.get(), np, np, np);
       gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, np, one, blk.P.get(), n, blk.small.get(), np, zero, blk.PU.get(), n);

@@ -425,7 +425,6 @@ int half_assemble_hs(half_handle handle, const double kpoint[3], int64_t ld, HAL
     if (ld < n) fail(kCapacity, "matrix leading dimension is too small");
     DeviceBuffer<double2> dh((size_t)n * n), ds((size_t)n * n);
     assemble_dense(*ctx, *ks, dh.get(), ds.get());
-    if (ctx->rt->crt_pending) tc_check(*ctx->rt);
     cudaStream_t st = ctx->rt->stream;
     block_to_host(h, ld, dh.get(), n, n, st);
     block_to_host(s, ld, ds.get(), n, n, st);
@@ -1127,11 +1126,11 @@ extern "C" int half_tc_cgemm(char op_a, char op_b, int m, int n, int k, const do
 extern "C" long long hb_diag_refuse_allocations(size_t bytes) { return device_refuse_above(bytes); }
 
 extern "C" int hb_diag_gram_route(int n, int rows, int cols, int integer) {
-  return int(zgram_route(n, rows, cols, integer != 0));
+  return int(zgram_route(148, n, rows, cols, integer != 0));
 }
 
 extern "C" int hb_diag_update_route(int n, int k, int cols, int integer) {
-  return int(zupdate_route(n, k, cols, integer != 0));
+  return int(zupdate_route(148, n, k, cols, integer != 0));
 }
 
 // Limits of contexts made from here on, and what a new runtime then finds: cluster size | 256 for grid-wide launches.

@@ -288,14 +288,14 @@ CrtSide side_of(const ZBlock& b, int n, bool k_is_rows, bool conj) {
 
 }  // namespace
 
-ZRoute zgram_route(int n, int rows, int cols, bool integer) {
+ZRoute zgram_route(int sms, int n, int rows, int cols, bool integer) {
   if (zblock_small(n, std::max(rows, cols))) return ZRoute::kBlock;
-  return integer && zcrt_serves(rows, cols, n) ? ZRoute::kInteger : ZRoute::kLibrary;
+  return integer && zcrt_serves(sms, rows, cols, n) ? ZRoute::kInteger : ZRoute::kLibrary;
 }
 
-ZRoute zupdate_route(int n, int k, int cols, bool integer) {
+ZRoute zupdate_route(int sms, int n, int k, int cols, bool integer) {
   if (zblock_small(n, std::max(k, cols))) return ZRoute::kBlock;
-  return integer && zcrt_serves(n, cols, k) ? ZRoute::kInteger : ZRoute::kLibrary;
+  return integer && zcrt_serves(sms, n, cols, k) ? ZRoute::kInteger : ZRoute::kLibrary;
 }
 
 void zgram(Runtime& rt, int n, const ZBlock& a, const ZBlock* b, double2* const* c, int count, int ldc, bool upper,
@@ -310,7 +310,7 @@ void zgram(Runtime& rt, int n, const ZBlock& a, const ZBlock* b, double2* const*
   if (g.rows <= 0 || g.cols <= 0) return;
   const double2 one = make_double2(1, 0), zero = make_double2(0, 0);
   if (route == ZRoute::kInteger && !crt_reserve(rt, crt_plane_bytes(g.rows, n, false), crt_plane_bytes(g.cols, n, true),
-                                                crt_result_bytes(g.rows, g.cols, n)))
+                                                crt_result_bytes(rt.sms, g.rows, g.cols, n)))
     route = ZRoute::kLibrary;
   if (route == ZRoute::kLibrary) {
     for (int i = 0; i < count; ++i) {
@@ -340,7 +340,7 @@ void zgram(Runtime& rt, int n, const ZBlock& a, const ZBlock* b, double2* const*
   const int tiles = g.tiles * count;
   // about four CTAs per SM, down to slices of one chunk
   const int chunks = ceil_div(n, kGramK);
-  int slices = std::max(1, std::min({ceil_div(4 * 148, tiles), chunks, 64}));
+  int slices = std::max(1, std::min({ceil_div(4 * rt.sms, tiles), chunks, 64}));
   const int kper = ceil_div(chunks, slices) * kGramK;
   slices = ceil_div(n, kper);
   const size_t need = slices > 1 ? size_t(slices) * tiles * kT * kT : 0;
@@ -363,7 +363,7 @@ void zupdate(Runtime& rt, int n, const ZBlock* z, const double2* y, int ldy, dou
   if (n <= 0 || cols <= 0) return;
   const int k = z[0].cols();
   if (route == ZRoute::kInteger && !crt_reserve(rt, crt_plane_bytes(n, k, false), crt_plane_bytes(cols, k, true),
-                                                crt_result_bytes(n, cols, k)))
+                                                crt_result_bytes(rt.sms, n, cols, k)))
     route = ZRoute::kLibrary;
   if (route == ZRoute::kLibrary) {
     const double2 al = make_double2(alpha, 0), one = make_double2(1, 0);

@@ -20,8 +20,8 @@ struct ZBlock {
 // large ones on the integer tensor cores (zcrt.cu) where the caller allows
 // that, every other on ZGEMM.
 enum class ZRoute { kBlock = 1, kInteger = 2, kLibrary = 3 };
-ZRoute zgram_route(int n, int rows, int cols, bool integer);     // A^H B: rows x cols over n
-ZRoute zupdate_route(int n, int k, int cols, bool integer);      // Z Y: n x cols over k
+ZRoute zgram_route(int sms, int n, int rows, int cols, bool integer);     // A^H B: rows x cols over n
+ZRoute zupdate_route(int sms, int n, int k, int cols, bool integer);      // Z Y: n x cols over k
 
 // C_i = A^H B_i for i < count (count 1 or 2, blocks of one shape), written
 // with leading dimension ldc.  upper: only the upper triangle is needed (A

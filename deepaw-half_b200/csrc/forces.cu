@@ -278,7 +278,7 @@ void nonlocal_forces_device(Context& ctx, KOperatorSet& ks, const double2* dvec,
   // sums of at most 256 MB.
   const long long slice_bytes = (long long)nions * 4 * nlm_max * nb * (long long)sizeof(double2);
   const int chunks = (npw + kAdjG - 1) / kAdjG;
-  long long slices = (6LL * 148 + (long long)nions * btiles - 1) / ((long long)nions * btiles);
+  long long slices = (6LL * rt.sms + (long long)nions * btiles - 1) / ((long long)nions * btiles);
   slices = std::min(slices, (long long)std::max(1, chunks / 4));
   slices = std::max(1LL, std::min(slices, (256LL << 20) / slice_bytes));
   const int gper = ceil_div(chunks, slices) * kAdjG;

@@ -883,14 +883,17 @@ void apply_nonlocal(Runtime& rt, KOperator<R>& op, const cplx_t<R>* x, long long
   } else {
     const bool kept = op.crt_bh.planes != nullptr;
     auto room = [&]() {   // for the planes of B and of the blocks, and the residues
-      const bool ok = crt_reserve(rt, 0, std::max(crt_plane_bytes(nb, op.npw, true), crt_plane_bytes(2 * nb, op.np, true)),
-                                  std::max(crt_result_bytes(op.np, nb, op.npw), crt_result_bytes(op.npw, 2 * nb, op.np))) &&
+      const size_t block = std::max(crt_plane_bytes(nb, op.npw, true), crt_plane_bytes(2 * nb, op.np, true));
+      const size_t result = std::max(crt_result_bytes(rt.sms, op.np, nb, op.npw),
+                                     crt_result_bytes(rt.sms, op.npw, 2 * nb, op.np));
+      const bool ok = crt_reserve(rt, 0, block, result) &&
                       op.crt_bh_store.try_reserve(crt_plane_bytes(op.np, op.npw, false)) &&
                       op.crt_b_store.try_reserve(crt_plane_bytes(op.npw, op.np, false));
       if (!ok) release_integer(op);
       return ok;
     };
-    if (op.integer && zcrt_serves(op.np, nb, op.npw, kept) && zcrt_serves(op.npw, 2 * nb, op.np, kept) && room()) {
+    if (op.integer && zcrt_serves(rt.sms, op.np, nb, op.npw, kept) &&
+        zcrt_serves(rt.sms, op.npw, 2 * nb, op.np, kept) && room()) {
       // coeff = B^H X, [H X | S X] += B [DY | QY] on the integer tensor cores
       CrtSide s;
       s.ld = op.npw;

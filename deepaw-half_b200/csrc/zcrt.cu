@@ -47,7 +47,8 @@
 // rate; the residues of one modulus are of no use to another) and by the
 // split and join passes.  Both operands split, one product, ZGEMM / this:
 // X^H Y 600 x 600 x 38,089 3.22 / 1.61 ms, upper half of 1,200 x 1,200 x 38,089
-// 12.5 / 3.4 ms (ZGEMM of the whole matrix), 1,696 x 600 x 38,089 8.91 / 3.49 ms, X C 38,089 x 600 x 600 3.16 / 2.23 ms.
+// 12.5 / 3.4 ms (ZGEMM of the whole matrix), 1,696 x 600 x 38,089 8.91 / 3.49
+// ms, X C 38,089 x 600 x 600 3.16 / 2.23 ms.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -63,7 +64,7 @@ namespace {
 using namespace tc;
 
 constexpr int kMods = 16;
-constexpr int kScaleBits = 62;     // row norms are scaled below 2^62; the products' sums stay below 2^124 < P / 2 = 2^124.4
+constexpr int kScaleBits = 62;     // row norms are scaled below 2^62; the sums stay below 2^124 < P / 2 = 2^124.4
 constexpr int kMod[kMods] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193};
 constexpr int kMaxK = 65000;       // |2 K 128 128| < 2^31
 constexpr int kBM = 128, kBN = 160;   // three int32 accumulators of kBN columns fit Tensor Memory
@@ -469,12 +470,12 @@ int pad_to(int x, int a) { return (x + a - 1) / a * a; }
 
 // Slices of K: the count with the least estimated time of the tiles' waves
 // (about 1 us per step of 128 k and 4 us per CTA) and the longer join.
-int pick_slices(long long tiles, int steps, double mn) {
+int pick_slices(int sms, long long tiles, int steps, double mn) {
   int best = 1;
   double best_t = 0;
   for (int s = 1; s <= std::min(8, steps); ++s) {
     const int per = (steps + s - 1) / s, used = (steps + per - 1) / per;
-    const double waves = double((tiles * used + 147) / 148);
+    const double waves = double((tiles * used + sms - 1) / sms);
     const double tm = waves * (per * 1.0e-6 + 4e-6) + used * mn * 2 * kMods / 2.0e12;
     if (best_t == 0 || tm < best_t) {
       best_t = tm;
@@ -488,16 +489,16 @@ constexpr double kMaxBytes = 8e9;   // planes of one operand, and residues of on
 
 }  // namespace
 
-bool zcrt_serves(int m, int n, int k, bool a_kept) {
+bool zcrt_serves(int sms, int m, int n, int k, bool a_kept) {
   if (m < 1 || n < 1 || k < 1 || k > kMaxK) return false;
   const double M = m, N = n, K = k;
   const long long tiles = (long long)ceil_div(m, kBM) * ceil_div(n, kBN) * kMods;
-  const int steps = ceil_div(k, kKB), s = pick_slices(tiles, steps, M * N), per = ceil_div(steps, s);
+  const int steps = ceil_div(k, kKB), s = pick_slices(sms, tiles, steps, M * N), per = ceil_div(steps, s);
   if (double(std::max(crt_plane_bytes(m, k, false), crt_plane_bytes(n, k, true))) > kMaxBytes ||
-      double(crt_result_bytes(m, n, k)) > kMaxBytes)
+      double(crt_result_bytes(sms, m, n, k)) > kMaxBytes)
     return false;
   const double native = 8.0 * M * N * K / 36.0e12;
-  const double waves = std::ceil(double(tiles) * s / 148.0);
+  const double waves = std::ceil(double(tiles) * s / sms);
   const double crt = 40e-6 + ((a_kept ? 0.0 : M) + N) * K * (2 * 16 + 2 * kMods) / 4.0e12 +
                      waves * (per * 1.0e-6 + 4e-6) + M * N * (4.0 * kMods * s + 16) / 3.0e12;
   return crt < 0.85 * native;
@@ -507,9 +508,9 @@ size_t crt_plane_bytes(int rows, int k, bool as_b) {
   return size_t(2 * kMods) * pad_to(rows, as_b ? kBN : kBM) * pad_to(k, kKB) + size_t(rows) * sizeof(int);
 }
 
-size_t crt_result_bytes(int m, int n, int k) {
+size_t crt_result_bytes(int sms, int m, int n, int k) {
   const int mt = ceil_div(m, kBM), nt = ceil_div(n, kBN), steps = ceil_div(k, kKB);
-  return size_t(2 * kMods) * pick_slices((long long)mt * nt * kMods, steps, double(m) * n) * n * mt * kBM;
+  return size_t(2 * kMods) * pick_slices(sms, (long long)mt * nt * kMods, steps, double(m) * n) * n * mt * kBM;
 }
 
 bool crt_reserve(Runtime& rt, size_t a, size_t b, size_t result) {
@@ -550,9 +551,9 @@ void crt_product(Runtime& rt, const CrtPlanes& a, const CrtPlanes& b, double2 al
   const int m = a.rows, n = b.rows, mt = a.rows_pad / kBM, nt = b.rows_pad / kBN, m_pad = a.rows_pad;
   if (a.k != b.k || a.k > kMaxK) fail(kInternal, "CRT product operands do not match");
   const int steps = a.k_pad / kKB;
-  const int s = pick_slices((long long)mt * nt * kMods, steps, double(m) * n), per = ceil_div(steps, s);
+  const int s = pick_slices(rt.sms, (long long)mt * nt * kMods, steps, double(m) * n), per = ceil_div(steps, s);
   const int slices = ceil_div(steps, per);
-  const size_t bytes = crt_result_bytes(m, n, a.k);
+  const size_t bytes = crt_result_bytes(rt.sms, m, n, a.k);
   if (rt.crt_res.size() < bytes) rt.crt_res.resize(bytes);
   raise_smem_limit(crt_gemm_kernel, kSmem);
   crt_gemm_kernel<<<dim3(mt, nt, kMods * slices), kThreads, kSmem, st>>>(

@@ -30,7 +30,7 @@ CrtPlanes crt_prepare(Runtime& rt, const CrtSide& s, bool as_b, DeviceBuffer<uns
 
 // Bytes of an operand's planes, and of the residues of an m x n product over k.
 size_t crt_plane_bytes(int rows, int k, bool as_b);
-size_t crt_result_bytes(int m, int n, int k);
+size_t crt_result_bytes(int sms, int m, int n, int k);
 
 // The runtime's buffers grown to these sizes; false where memory does not
 // suffice (the product then goes to ZGEMM).
@@ -44,6 +44,6 @@ void crt_product(Runtime& rt, const CrtPlanes& a, const CrtPlanes& b, double2 al
 // Whether an m x n product over k is large enough to gain over ZGEMM (a_kept:
 // the left operand's planes exist already) and within the method's range and
 // memory.
-bool zcrt_serves(int m, int n, int k, bool a_kept = false);
+bool zcrt_serves(int sms, int m, int n, int k, bool a_kept = false);
 
 }  // namespace hb
