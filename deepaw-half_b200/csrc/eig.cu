@@ -266,8 +266,9 @@ __global__ void __launch_bounds__(32 * kValueWarps) tridiag_values_kernel(const 
 __global__ void __launch_bounds__(kVectorThreads) tridiag_vectors_kernel(
     const double* __restrict__ d_in, const double* __restrict__ e_in, int n, int nev, int ne, int per,
     const double* __restrict__ lam_g, double* __restrict__ w, double* __restrict__ Z, double* __restrict__ gscratch,
-    int* __restrict__ status) {
+    int* __restrict__ status, const int* __restrict__ failed) {
   wait_previous();
+  if (failed && *failed) return;
   extern __shared__ double sm[];
   double* d = sm;
   double* e = d + n;
@@ -345,7 +346,7 @@ __global__ void __launch_bounds__(kVectorThreads) tridiag_vectors_kernel(
       nrm = sqrt(nrm);
       if (!(nrm > 0) || !isfinite(nrm)) {
         atomicCAS(status, 0, 1);   // an earlier report stays
-        break;
+        return;                    // the rest of the cluster is of no use either
       }
       const double inv = 1.0 / nrm;
       for (int i = 0; i < n; ++i) x[i * st] *= inv;
@@ -1493,7 +1494,7 @@ void SmallEigen::clear_grid_state(cudaStream_t s) {
 
 // Hermitian eigenproblem of A (n x n, upper triangle used, destroyed); the nev
 // lowest eigenvectors go to V[:, :nev] (leading dimension n), eigenvalues to w.
-void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* status) {
+void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* status, const int* failed) {
   reserve(rt, n);
   cudaStream_t s = rt.stream;
   const int* gave_up = nullptr;
@@ -1546,7 +1547,7 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
   }
   raise_smem_limit(tridiag_vectors_kernel, tsm);
   launch_chained(ceil_div(nev, per), kVectorThreads, tsm, s, tridiag_vectors_kernel,
-      d.get(), e.get(), n, nev, ne, per, lam.get(), w, Z.get(), gs, status);
+      d.get(), e.get(), n, nev, ne, per, lam.get(), w, Z.get(), gs, status, failed);
   HALF_LAUNCH("tridiagonal eigenvectors");
   if (n > kOwnMaxOrder) {
     // large orders: cuSOLVER's blocked back-transformation (zunmtr, Q Z with
@@ -1621,13 +1622,13 @@ void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, doubl
       const ZBlock ba = {A, n}, bb = {B, n}, bv = {v, n};
       zupdate(rt, n, &ba, B, n, &v, n, 1, 1.0, 0.0, ZRoute::kBlock);
       zgram(rt, n, bb, &bv, &A, 1, n, true, ZRoute::kBlock);
-      heev(rt, A, n, nev, w, status);
+      heev(rt, A, n, nev, w, status, chol_status);
       zupdate(rt, n, &bb, v, n, &A, nev, 1, 1.0, 0.0, ZRoute::kBlock);
       return;
     }
     gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, n, n, one, A, n, B, n, zero, V.get(), n);
     gemm(rt, CUBLAS_OP_C, CUBLAS_OP_N, n, n, n, one, B, n, V.get(), n, zero, A, n);
-    heev(rt, A, n, nev, w, status);
+    heev(rt, A, n, nev, w, status, chol_status);
     gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, nev, n, one, B, n, V.get(), n, zero, A, n);
     return;
   }
@@ -1646,7 +1647,7 @@ void SmallEigen::hegv(Runtime& rt, double2* A, double2* B, int n, int nev, doubl
   cublas_check(cublasZtrsm(rt.blas, CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N, CUBLAS_DIAG_NON_UNIT, n, n,
                            &one, Bc, n, Ac, n),
                "ztrsm");
-  heev(rt, A, n, nev, w, status);
+  heev(rt, A, n, nev, w, status, chol_status);
   HALF_CUDA(cudaMemcpyAsync(A, V.get(), size_t(n) * nev * sizeof(double2), cudaMemcpyDeviceToDevice, s));
   cublas_check(cublasZtrsm(rt.blas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N, CUBLAS_DIAG_NON_UNIT, n, nev,
                            &one, Bc, n, Ac, n),

@@ -37,7 +37,9 @@ struct SmallEigen {
   void reserve(Runtime& rt, int nmax);
   // A (n x n, upper triangle, destroyed) -> nev lowest eigenpairs; vectors in
   // V[:, :nev].  *status (device) becomes nonzero if inverse iteration failed.
-  void heev(Runtime& rt, double2* A, int n, int nev, double* w, int* status);
+  // Where *failed (device; null: never) is nonzero the matrix is of no use, and
+  // no eigenvectors are computed.
+  void heev(Runtime& rt, double2* A, int n, int nev, double* w, int* status, const int* failed = nullptr);
   // A y = lambda B y, B Hermitian positive definite; Y^H B Y = I.
   // *chol_status (device): nonzero when the factor saw a pivot that is not
   // finite (beyond the grid-wide kernels' orders zpotrf's info).  strict: a

@@ -5,6 +5,7 @@ numpy.  The floored variant (the smaller orders and the guard-band modes)
 accepts both.  Orders on either side of the cluster kernels' sizes and in the
 grid-wide range."""
 import ctypes as C
+import time
 
 import numpy as np
 import pytest
@@ -39,10 +40,32 @@ def _solve(a, b, strict):
     return w.cpu().numpy(), st.value, chol.value
 
 
+@pytest.fixture(scope="module", autouse=True)
+def started():
+    """torch, the CUDA context and the kernels are loaded before anything is timed."""
+    _solve(*_pencil(40, 0.5, 0), False)
+    _solve(*_pencil(440, 0.5, 0), False)
+
+
 @pytest.mark.parametrize("n", [165, 177, 300, 432, 500])
 def test_indefinite_overlap_is_reported(n):
     a, b = _pencil(n, -0.05, n)
+    t = time.monotonic()
     assert _solve(a, b, True)[2] != 0
+    assert time.monotonic() - t < 5.0   # no eigenvectors of a pencil that has failed
+
+
+@pytest.mark.parametrize("n", [40, 170, 432, 500])
+@pytest.mark.parametrize("where", ["a", "b"])
+def test_pencil_with_nan_is_reported_soon(where, n):
+    """Eigenvalues that are not numbers form one cluster, which a single thread
+    would orthogonalise (25 s at order 500): it stops at the first."""
+    a, b = _pencil(n, 0.5, n)
+    (a if where == "a" else b)[n // 3, n // 2] = np.nan
+    t = time.monotonic()
+    _, st, chol = _solve(a, b, False)
+    assert st != 0 or chol != 0
+    assert time.monotonic() - t < 5.0
 
 
 def test_floored_variant_accepts_it():
