@@ -19,9 +19,9 @@
 //   tridiag_vectors_kernel eigenvectors by inverse iteration on the pivoted
 //                          tridiagonal LU (one thread per eigenvector);
 //                          eigenvalues closer than 1e-7 ||T|| form clusters
-//                          whose members are iterated in order and
-//                          Gram-Schmidt orthogonalised against each other (the
-//                          strategy of LAPACK's dstebz/dstein);
+//                          whose members a warp iterates together and
+//                          Gram-Schmidt orthogonalises in order (after
+//                          LAPACK's dstebz/dstein);
 //   back_transform_kernel  V = Q Z with Q = H(n-1)...H(1), the reflectors
 //                          staged in shared memory, one warp per eigenvector.
 //
@@ -249,26 +249,95 @@ __global__ void __launch_bounds__(32 * kValueWarps) tridiag_values_kernel(const 
   if (lane == 0) lam[k] = v / sc;
 }
 
+// x(i) of a slot, scaled to norm 1; the norm before.
+__device__ double normalise(double* x, int n, int st) {
+  double nrm = 0;
+  for (int i = 0; i < n; ++i) nrm += x[i * st] * x[i * st];
+  nrm = sqrt(nrm);
+  const double inv = 1.0 / nrm;
+  for (int i = 0; i < n; ++i) x[i * st] *= inv;
+  return nrm;
+}
+
+// The same and Gram-Schmidt by the whole warp: lane = slot + per q, and the
+// 32 / per lanes of a slot share its vector (elements q, q + 32 / per, ...).
+__device__ __forceinline__ double slot_sum(double v, int per) {
+  for (int off = per; off < 32; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
+}
+
+__device__ double slot_normalise(double* x, int n, int st, int per, bool on) {
+  const int q = (threadIdx.x & 31) / per, g = 32 / per;
+  double s = 0;
+  for (int i = q; i < n; i += g) s += x[i * st] * x[i * st];
+  const double nrm = sqrt(slot_sum(s, per));
+  if (on) {
+    const double inv = 1.0 / nrm;
+    for (int i = q; i < n; i += g) x[i * st] *= inv;
+  }
+  return nrm;
+}
+
+// x -= sum_j (y_j . x) y_j over NY vectors, stride sy and one after another at distance dy.
+template <int NY>
+__device__ void slot_remove(double* x, int st, const double* y, int sy, size_t dy, int n, int per, bool on) {
+  const int q = (threadIdx.x & 31) / per, g = 32 / per;
+  double s[NY] = {};
+#pragma unroll 4
+  for (int i = q; i < n; i += g) {
+    const double v = x[i * st];
+#pragma unroll
+    for (int j = 0; j < NY; ++j) s[j] += y[j * dy + size_t(i) * sy] * v;
+  }
+#pragma unroll
+  for (int j = 0; j < NY; ++j) s[j] = slot_sum(s[j], per);   // every lane takes part
+  if (!on) return;
+#pragma unroll 4
+  for (int i = q; i < n; i += g) {
+    double v = x[i * st];
+#pragma unroll
+    for (int j = 0; j < NY; ++j) v -= s[j] * y[j * dy + size_t(i) * sy];
+    x[i * st] = v;
+  }
+}
+
+// z = x with its largest component positive.
+__device__ void store_signed(double* __restrict__ z, const double* x, int n, int st) {
+  double big = 0;
+  for (int i = 0; i < n; ++i)
+    if (fabs(x[i * st]) > fabs(big)) big = x[i * st];
+  const double sg = big < 0 ? -1.0 : 1.0;
+  for (int i = 0; i < n; ++i) z[i] = sg * x[i * st];
+}
+
 // Eigenvectors of lam[0..nev) by inverse iteration on the pivoted LU of
 // T - lambda I, one thread per eigenvector.  Eigenvalues (up to ne) closer
-// than 1e-7 ||T|| form clusters; the thread of a cluster's first member
-// computes the whole cluster in order, Gram-Schmidt orthogonalising each
-// member against the earlier ones (the strategy of LAPACK's dstein with a
-// tighter cluster threshold: dstein's 1e-3 ||T|| would serialise the dense
-// Ritz spectra met here).  Outside a cluster inverse iteration alone keeps
-// |<z_i, z_j>| <= eps ||T|| / gap <~ 1e-9.  Scratch: five n-vectors and the
-// pivot flags per thread, interleaved by thread (a warp touches consecutive
-// words), in shared memory after the tables when gscratch is null, else in
-// global memory with one slot per eigenvector.  A CTA takes `per` eigenvectors,
+// than 1e-7 ||T|| form clusters, whose members are orthogonalised against each
+// other (LAPACK's dstein does the same with 1e-3 ||T||, which would take most
+// of the dense Ritz spectra met here).  Outside a cluster inverse iteration
+// alone keeps |<z_i, z_j>| <= eps ||T|| / gap <~ 1e-9.
+//
+// A cluster belongs to the CTA (one warp) of its first member.  The warp takes
+// `per` consecutive values at a time, a lane each: all solve, then modified
+// Gram-Schmidt inside each cluster, in ascending order, against the members
+// that are done (in Z) and those of the batch, all 32 lanes working on the
+// batch's vectors.  Three such rounds, the last one with a second pass.  With
+// one thread for a whole cluster, the solves of the undisplaced 64-atom cell at
+// (1/2, 1/2, 1/2), whose levels are many-fold, took 299 and 740 ms with 160 and
+// 400 bands; like this 111 and 254 ms (with cuSOLVER's pencils 138 and 305).
+//
+// Scratch: five n-vectors and the pivot flags per thread, interleaved by thread
+// (a warp touches consecutive words), in shared memory after the tables when
+// gscratch is null, else in global memory with one slot per eigenvector.  A CTA takes `per` eigenvectors,
 // as many as its shared memory holds (32 at order 138, 8 at order 432): the
 // threads run serial chains, so few of them per SM cost nothing, while
 // scratch in global memory puts a cache miss into every link.
 __global__ void __launch_bounds__(kVectorThreads) tridiag_vectors_kernel(
     const double* __restrict__ d_in, const double* __restrict__ e_in, int n, int nev, int ne, int per,
-    const double* __restrict__ lam_g, double* __restrict__ w, double* __restrict__ Z, double* __restrict__ gscratch,
+    const double* __restrict__ lam_g, double* __restrict__ w, double* Z, double* __restrict__ gscratch,
     int* __restrict__ status, const int* __restrict__ failed) {
   wait_previous();
-  if (failed && *failed) return;
+  const int stop = failed ? *failed : 0;
   extern __shared__ double sm[];
   double* d = sm;
   double* e = d + n;
@@ -279,6 +348,7 @@ __global__ void __launch_bounds__(kVectorThreads) tridiag_vectors_kernel(
     e[i] = i < n - 1 ? e_in[i] : 0.0;
   }
   for (int i = threadIdx.x; i < ne; i += blockDim.x) lam[i] = lam_g[i];
+  if (stop) return;
   __syncthreads();
   double gl, gu, tnorm;   // one warp (kVectorThreads) evaluates, every thread holds the results
   gershgorin(d, e, n, gl, gu, tnorm);
@@ -289,75 +359,102 @@ __global__ void __launch_bounds__(kVectorThreads) tridiag_vectors_kernel(
     cl_first[k] = f;
   }
   __syncthreads();
-  const int k0 = blockIdx.x * per + threadIdx.x;
-  if (int(threadIdx.x) >= per) return;
-  if (k0 < nev) w[k0] = lam[k0];
-  if (k0 >= nev || cl_first[k0] != k0) return;
+  const int lane = threadIdx.x, slot = min(lane, per - 1);
   const double tiny = DBL_EPSILON * tnorm;
   double* ai;
   unsigned char* piv;
   int st;
   if (gscratch) {
     st = gridDim.x * per;
-    ai = gscratch + k0;
-    piv = reinterpret_cast<unsigned char*>(gscratch + 5 * size_t(n) * st) + k0;
+    ai = gscratch + blockIdx.x * per + slot;
+    piv = reinterpret_cast<unsigned char*>(gscratch + 5 * size_t(n) * st) + blockIdx.x * per + slot;
   } else {
     size_t off = (2 * size_t(n) + ne) * sizeof(double) + size_t(ne) * sizeof(int);
     off = (off + 15) & ~size_t(15);
     double* sbase = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(sm) + off);
     st = per;
-    ai = sbase + threadIdx.x;
-    piv = reinterpret_cast<unsigned char*>(sbase + 5 * size_t(n) * st) + threadIdx.x;
+    ai = sbase + slot;
+    piv = reinterpret_cast<unsigned char*>(sbase + 5 * size_t(n) * st) + slot;
   }
   double* b1 = ai + size_t(n) * st;
   double* b2 = b1 + size_t(n) * st;
   double* l = b2 + size_t(n) * st;
   double* x = l + size_t(n) * st;
-  int k1 = k0;
-  while (k1 + 1 < ne && cl_first[k1 + 1] == k0) ++k1;
-  double prev = -HUGE_VAL;
-  for (int k = k0; k <= k1; ++k) {
-    double lk = lam[k];
-    // separate numerically equal eigenvalues of a cluster (dstein)
-    const double sep = 10.0 * DBL_EPSILON * fmax(fabs(lk), tnorm * 1e-3);
-    if (k > k0 && lk - prev < sep) lk = prev + sep;
-    prev = lk;
-    tri_factor(d, e, n, lk, tiny, ai, b1, b2, l, piv, st);
-    unsigned s = 0x9E3779B9u * (k + 1);
-    for (int i = 0; i < n; ++i) {   // deterministic pseudo-random start vector
-      s = s * 1664525u + 1013904223u;
-      x[i * st] = 1.0 + 0.5 * (double(s >> 8) / 16777216.0 - 0.5);
+  if (lane < per && blockIdx.x * per + lane < nev) w[blockIdx.x * per + lane] = lam[blockIdx.x * per + lane];
+  // this CTA's values: the clusters that begin among its `per`, whole
+  auto cluster_start = [&](int k) {
+    while (k < ne && cl_first[k] != k) ++k;
+    return k;
+  };
+  const int kbeg = cluster_start(blockIdx.x * per);
+  const int kend = kbeg < nev ? cluster_start(min((int(blockIdx.x) + 1) * per, nev)) : kbeg;
+  for (int c0 = kbeg; c0 < kend; c0 += per) {
+    const int cnt = min(per, kend - c0), k = c0 + lane;
+    const bool on = lane < cnt;
+    const int f = on ? cl_first[k] : 0;                               // first member
+    const int base = max(f, c0) - c0, pos = on ? lane - base : 0;     // of the batch's members: lane of the first, place
+    int size = on ? 1 : 0;                                            // members in the batch
+    while (on && base + size < cnt && cl_first[c0 + base + size] == f) ++size;
+    const bool clustered = on && (f < k || (k + 1 < ne && cl_first[k + 1] == f));
+    int steps = size;
+    for (int off = 16; off > 0; off >>= 1) steps = max(steps, __shfl_xor_sync(0xffffffffu, steps, off));
+    const bool any = __any_sync(0xffffffffu, clustered);
+    // the Gram-Schmidt's view: slot gs, its vector, cluster and place
+    const int gs = lane & (per - 1);
+    double* const gx = x + (gs - slot);
+    const int gf = __shfl_sync(0xffffffffu, f, gs), gbase = __shfl_sync(0xffffffffu, base, gs);
+    const int gpos = __shfl_sync(0xffffffffu, pos, gs);
+    const bool gclustered = __shfl_sync(0xffffffffu, int(clustered), gs);
+    if (on) {
+      double lk = lam[f];
+      for (int q = f + 1; q <= k; ++q) {   // numerically equal eigenvalues of a cluster are separated (dstein)
+        const double sep = 10.0 * DBL_EPSILON * fmax(fabs(lam[q]), tnorm * 1e-3);
+        lk = lam[q] - lk < sep ? lk + sep : lam[q];
+      }
+      tri_factor(d, e, n, lk, tiny, ai, b1, b2, l, piv, st);
+      unsigned s = 0x9E3779B9u * (k + 1);
+      // deterministic pseudo-random start; of either sign in a cluster, whose members differ by it
+      for (int i = 0; i < n; ++i) {
+        s = s * 1664525u + 1013904223u;
+        const double u = double(s >> 8) / 16777216.0 - 0.5;
+        x[i * st] = clustered ? u : 1.0 + 0.5 * u;
+      }
     }
     // With an eigenvalue accurate to rounding each solve amplifies the wanted
-    // direction by ~gap / (eps ||T||): two solves for an isolated eigenvalue,
-    // three (each followed by Gram-Schmidt against the earlier members) inside
-    // a cluster.
-    const int steps = k1 > k0 ? 3 : 2;
-    for (int it = 0; it < steps; ++it) {
-      tri_solve(n, ai, b1, b2, l, piv, x, st);
-      for (int j = k0; j < k; ++j) {
-        const double* y = Z + (size_t)j * n;
-        double dot = 0;
-        for (int i = 0; i < n; ++i) dot += y[i] * x[i * st];
-        for (int i = 0; i < n; ++i) x[i * st] -= dot * y[i];
+    // direction by ~gap / (eps ||T||): two solves for one by itself, three
+    // (each followed by Gram-Schmidt) inside a cluster.
+    bool ok = true;
+    for (int it = 0; it < (any ? 3 : 2); ++it) {
+      if (on && (clustered || it < 2)) {
+        tri_solve(n, ai, b1, b2, l, piv, x, st);
+        const double nrm = normalise(x, n, st);
+        ok = ok && nrm > 0 && isfinite(nrm);
       }
-      double nrm = 0;
-      for (int i = 0; i < n; ++i) nrm += x[i * st] * x[i * st];
-      nrm = sqrt(nrm);
-      if (!(nrm > 0) || !isfinite(nrm)) {
-        atomicCAS(status, 0, 1);   // an earlier report stays
-        return;                    // the rest of the cluster is of no use either
+      for (int pass = 0; any && pass < (it == 2 ? 2 : 1); ++pass) {
+        __syncwarp();
+        // from here lane = gs + per q works on slot gs
+        int j = cl_first[c0];   // only the batch's first cluster can have members that are done
+        const bool part = gclustered && gf < c0;
+        for (; j + 3 < c0; j += 4) slot_remove<4>(gx, st, Z + (size_t)j * n, 1, n, n, per, part);
+        for (; j < c0; ++j) slot_remove<1>(gx, st, Z + (size_t)j * n, 1, n, n, per, part);
+        __syncwarp();
+        for (int r = 0; r < steps; ++r) {
+          const double nrm = slot_normalise(gx, n, st, per, gclustered && gpos == r);
+          if (gclustered && gpos == r) ok = ok && nrm > 0 && isfinite(nrm);
+          __syncwarp();
+          slot_remove<1>(gx, st, gx + (min(gbase + r, per - 1) - gs), st, 0, n, per, gclustered && gpos > r);
+          __syncwarp();
+        }
       }
-      const double inv = 1.0 / nrm;
-      for (int i = 0; i < n; ++i) x[i * st] *= inv;
     }
-    // sign convention: largest component positive
-    double big = 0;
-    for (int i = 0; i < n; ++i)
-      if (fabs(x[i * st]) > fabs(big)) big = x[i * st];
-    const double sg = big < 0 ? -1.0 : 1.0;
-    double* z = Z + (size_t)k * n;
-    for (int i = 0; i < n; ++i) z[i] = sg * x[i * st];
+    ok = __all_sync(0xffffffffu, ok);
+    __syncwarp();
+    if (!ok) {   // the rest is of no use either
+      if (lane == 0) atomicCAS(status, 0, 1);   // an earlier report stays
+      return;
+    }
+    if (on) store_signed(Z + (size_t)k * n, x, n, st);
+    __syncwarp();
   }
 }
 
