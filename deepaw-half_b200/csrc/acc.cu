@@ -294,10 +294,10 @@ struct SmallSolver {
   // SmallEigen::hegv too (cuSOLVER zpotrf / zhetrd / zunmtr around the
   // library's multisection and inverse-iteration kernels)
   bool own_large = false;
-  // FP64 mode: above this order an overlap that is not positive definite is an
-  // error, as it is to zhegvd, which served those orders; the own solver
-  // floors the pivots of the orders that it always served
-  bool strict = false;
+  // Above this order the own solver reports an overlap that is not positive
+  // definite, as the cuSOLVER calls do that served those orders: the FP64 mode
+  // ends with that error, the guard-band modes redo the step with the metric
+  // normalisation.  Up to it, it floors the dependent pivots.
   static constexpr int kFlooredOrder = 164;
   SmallEigen eig;
   SmallSolver(Runtime& r, int m_, double2* a, double2* b, double* w) : rt(r), m(m_) {
@@ -346,15 +346,15 @@ struct SmallSolver {
   }
   // orders of the own solver; those of the grid-wide tridiagonalisation in the
   // guard-band modes only (the FP64 mode keeps zhegvd there)
-  bool own_order(int n) const { return own_floored(n) || (own && own_large); }
-  // those whose dependent pivots it floors
-  bool own_floored(int n) const {
+  bool own_order(int n) const { return own_kernels(n) || (own && own_large); }
+  // those of its own kernels, which scale the pencil themselves
+  bool own_kernels(int n) const {
     return own && (SmallEigen::cluster_order(rt, n) || (range && SmallEigen::grid_order(rt, n)));
   }
   // generalized problem of order n; the nev lowest eigenvectors are wanted
   void hegvd(double2* a, double2* b, int n, double* w, int nev) {
     if (own_order(n)) {
-      eig.hegv(rt, a, b, n, nev, w, info.get() + 1, info.get() + 2, strict && n > kFlooredOrder);
+      eig.hegv(rt, a, b, n, nev, w, info.get() + 1, info.get() + 2, n > kFlooredOrder);
       return;
     }
     if (range) {
@@ -430,6 +430,7 @@ struct AccRun {
   int mcheck = m;              // bands whose residuals decide convergence (guard bands excluded)
   bool guarded = false;        // guard-band modes: may skip the separate metric normalisation
   int metric_fallbacks = 0;    // Jacobi-scaled pencils whose Cholesky failed (redone with the metric step)
+  int unchecked = 0;           // P columns of a step whose pencil status has not been read yet (redo_if_failed), or 0
   int nl = 0;                  // hard-locked columns, at the front of X, H X, S X
   std::vector<double> wh;      // Ritz values (host copy, physical column order)
   std::vector<int> req;        // requested bands: physical columns of the mcheck lowest Ritz values
@@ -501,6 +502,7 @@ struct AccRun {
     if (host[2 * m + 3] != 0.0) tc_check(rt);   // raises
     rt.crt_pending = false;
     mark("residual");
+    if (redo_if_failed(infos)) return residuals(norms, infos);
     const std::string failure = pencil_failure(infos);
     if (!failure.empty()) fail(kInternal, failure);
     order_requested();
@@ -519,9 +521,32 @@ struct AccRun {
     req.resize(std::min(mcheck, m));
   }
 
-  // the current Ritz values to the host and req from them (after an iteration
-  // that no residual check followed: the iteration bound was reached)
+  // A guard-band pencil of the own solver went ahead unchecked, and its overlap
+  // turned out not to be positive definite (or the solve failed): the step is
+  // redone from the blocks it started from, with the metric normalisation.
+  bool redo_if_failed(const int* infos) {
+    const int np = unchecked;
+    unchecked = 0;
+    if (np == 0 || (infos[1] == 0 && infos[2] == 0)) return false;
+    ++metric_fallbacks;
+    ss.info.zero(rt.stream);
+    blk.cur ^= 1;
+    rayleigh_ritz(np, false);
+    return true;
+  }
+
+  // After an iteration that no residual check followed (the iteration bound was reached).
+  void settle() {
+    if (unchecked == 0) return;
+    int infos[3];
+    HALF_CUDA(cudaMemcpyAsync(infos, ss.info.get(), sizeof infos, cudaMemcpyDeviceToHost, rt.stream));
+    HALF_CUDA(cudaStreamSynchronize(rt.stream));
+    redo_if_failed(infos);
+  }
+
+  // the current Ritz values to the host and req from them (as settle)
   void refresh_values() {
+    settle();
     wh.resize(m);
     HALF_CUDA(cudaMemcpyAsync(wh.data(), sc.w.get(), m * sizeof(double), cudaMemcpyDeviceToHost, rt.stream));
     HALF_CUDA(cudaStreamSynchronize(rt.stream));
@@ -607,21 +632,31 @@ struct AccRun {
       gemm(rt, CUBLAS_OP_N, CUBLAS_OP_N, n, np, m, mone, blk.sx(), n, blk.small.get(), m, one, blk.SP.get(), n);
     }
     mark("orth_gemm");
+    rayleigh_ritz(np, guarded && ss.own);
+  }
+
+  // The rest of the iteration, from P, HP, SP (np columns, S-orthogonal to X):
+  // metric normalisation unless skipped, Rayleigh-Ritz, rotation.
+  void rayleigh_ritz(int np, bool skip_metric) {
+    const auto one = cval<R>(1.0), zero = cval<R>(0.0);
     // In the guard-band modes the separate S-metric normalisation is
-    // skipped.  The library's own pencil solver (to order 1,280) Jacobi-scales
-    // the overlap and floors dependent pivots exactly like the metric step,
-    // so [X P] spans the same space and the Ritz pairs are the same.  Larger
-    // pencils are Jacobi-scaled here and go through a plain Cholesky of the
-    // overlap (SmallEigen::hegv, or cuSOLVER beyond its orders), which then
-    // does the metric step's work; if that Cholesky (or the solve) fails, the step is redone with the metric normalisation.
-    // The FP64 mode keeps the reference's metric step.
+    // skipped.  The pencil is Jacobi-scaled (the library's own kernels do that
+    // themselves) and goes through a plain Cholesky of the overlap, which does
+    // the metric step's work; if that Cholesky (or the solve) fails, the step
+    // is redone with the metric normalisation.  The own kernels' status is read
+    // with the next residuals, the others' here.  To order 164 the own solver
+    // floors dependent pivots exactly like the metric step instead, so [X P]
+    // spans the same space and the Ritz pairs are the same.  (Floored pivots at
+    // larger orders let rounding in the FP32 phase's overlaps through as Ritz
+    // values of -1e9 eV: 600 bands of the 12-atom cell.)  The FP64 mode keeps
+    // the reference's metric step.
     // Rayleigh-Ritz on Z = [X_U PU], X_U = the unlocked columns [nl, m) of X
     // (all of them without hard locking)
     const int mu = m - nl;
     const long long off = (long long)nl * n;
     const int ord = mu + np;
-    const bool own_pencil = ss.own_floored(ord);
-    bool skip_metric = guarded && ss.own;
+    const bool own_pencil = ss.own_kernels(ord);
+    unchecked = skip_metric && own_pencil && ord > SmallSolver::kFlooredOrder ? np : 0;
     double2* hs = sc.hsub.get();
     double2* ssb = sc.ssub.get();
     double* wu = sc.w.get() + nl;
@@ -775,7 +810,6 @@ void solve_acc(Context& ctx, KOperatorSet& ks, int nbands, bool want_vectors, So
   sc.idx.upload(order, rt.stream);
   SmallSolver ss(rt, m, sc.hsub.get(), sc.ssub.get(), sc.w.get());
   ss.range = ss.range && guarded;   // the FP64 mode keeps the reference's zhegvd
-  ss.strict = !guarded;
   const double seed_threshold = std::max(cfg.tol * 1e-2, 1e-12);
   std::vector<double> norms;
   // Soft locking (guard-band modes): a requested band whose residual is at or
@@ -874,6 +908,7 @@ void solve_acc(Context& ctx, KOperatorSet& ks, int nbands, bool want_vectors, So
       advance(run32, lock_frac * switch_tol);
     }
     if (iter > cfg.max_iter) iter = cfg.max_iter;
+    run32.settle();
     op_cols += run32.op_cols;
     fallbacks += run32.metric_fallbacks;
     // promote X, recreate H X and S X in FP64, Rayleigh-Ritz
