@@ -1480,6 +1480,14 @@ bool launch_grid(Runtime& rt, const void* kernel, int ctas, void** args, size_t 
   return true;
 }
 
+constexpr int kUnpolishedOrder = 164;
+
+// g = 3/2 - g / 2
+__global__ void polish_matrix_kernel(double* __restrict__ g, int n) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t < (long long)n * n) g[t] = (t % (n + 1) == 0 ? 1.5 : 0.0) - 0.5 * g[t];
+}
+
 __global__ void real_to_complex_block_kernel(const double* __restrict__ z, long long count, double2* __restrict__ out) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t < count) out[t] = make_double2(z[t], 0.0);
@@ -1646,11 +1654,26 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
   launch_chained(ceil_div(nev, per), kVectorThreads, tsm, s, tridiag_vectors_kernel,
       d.get(), e.get(), n, nev, ne, per, lam.get(), w, Z.get(), gs, status, failed);
   HALF_LAUNCH("tridiagonal eigenvectors");
+  // Inverse iteration leaves |<z_i, z_j>| <= eps ||T|| / gap between clusters:
+  // 1e-13 in the 12-atom cell's wide blocks, 1e-9 at worst.  One step of
+  // Z <- Z (3/2 - Z^T Z / 2) brings that to rounding, which is what cuSOLVER
+  // gave the orders above 164 (25 us of a pencil's 1.5 ms and more).
+  const double* z = Z.get();
+  if (n > kUnpolishedOrder) {
+    double* const g = scratch.get();
+    double* const z2 = g + size_t(nev) * nev;
+    const double one = 1.0, zero = 0.0;
+    cublas_check(cublasDgemm(rt.blas, CUBLAS_OP_T, CUBLAS_OP_N, nev, nev, n, &one, z, n, z, n, &zero, g, nev), "dgemm");
+    polish_matrix_kernel<<<ceil_div((long long)nev * nev, 256), 256, 0, s>>>(g, nev);
+    HALF_LAUNCH("tridiagonal eigenvector overlaps");
+    cublas_check(cublasDgemm(rt.blas, CUBLAS_OP_N, CUBLAS_OP_N, n, nev, nev, &one, z, n, g, nev, &zero, z2, n), "dgemm");
+    rt.prof.launches += 1;
+    z = z2;
+  }
   if (n > kOwnMaxOrder) {
     // large orders: cuSOLVER's blocked back-transformation (zunmtr, Q Z with
     // zhetrd's reflectors) on the complex copy of Z
-    real_to_complex_block_kernel<<<ceil_div((long long)n * nev, 256), 256, 0, s>>>(Z.get(), (long long)n * nev,
-                                                                                   V.get());
+    real_to_complex_block_kernel<<<ceil_div((long long)n * nev, 256), 256, 0, s>>>(z, (long long)n * nev, V.get());
     HALF_LAUNCH("tridiagonal eigenvectors to complex");
     cusolver_check(cusolverDnZunmtr(rt.solver, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N, n, nev,
                                     reinterpret_cast<cuDoubleComplex*>(A), n,
@@ -1667,7 +1690,7 @@ void SmallEigen::heev(Runtime& rt, double2* A, int n, int nev, double* w, int* s
   const size_t bsm = size_t(blocks) * per_block;
   auto back = [&](auto kernel) {
     raise_smem_limit(kernel, bsm);
-    launch_chained(ceil_div(nev, kBackWarps), 32 * kBackWarps, bsm, s, kernel, A, tau.get(), Z.get(), n, nev,
+    launch_chained(ceil_div(nev, kBackWarps), 32 * kBackWarps, bsm, s, kernel, A, tau.get(), z, n, nev,
                    blocks * kBackBlock, V.get());
   };
   if (n <= 64) back(back_transform_kernel<2>);

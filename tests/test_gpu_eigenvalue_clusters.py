@@ -50,10 +50,12 @@ def _values(kind, n, r):
             if len(out) >= n:
                 break
         return np.array(out[:n])
+    if kind == "close":   # tens of values 1e-6 apart, three times what makes a cluster
+        return np.sort(np.repeat(np.linspace(-4.0, 4.0, (n + 9) // 10), 10)[:n]) + 1e-6 * (np.arange(n) % 10)
     return np.sort(np.repeat(r.uniform(-5, 5, size=(n + 29) // 30), 30)[:n]) + 1e-9 * r.normal(size=n)   # "spread"
 
 
-@pytest.mark.parametrize("kind", ["identity", "pairs", "levels", "spread"])
+@pytest.mark.parametrize("kind", ["identity", "pairs", "levels", "spread", "close"])
 @pytest.mark.parametrize("n", [7, 33, 100, 165, 300, 432, 434, 700])
 def test_clusters(n, kind):
     r = rng(n)
@@ -67,6 +69,8 @@ def test_clusters(n, kind):
     a = a / np.outer(s, s)
     bound = 8 * n * 2.0 ** -52 * np.abs(lam).max()
     assert np.abs(w - np.sort(lam)).max() <= bound
-    assert np.abs(y.conj().T @ y - np.eye(n)).max() <= max(1e-9, 8 * n * 2.0 ** -52)   # 1e-9: outside clusters
+    orth = np.abs(y.conj().T @ y - np.eye(n)).max()
+    # up to order 164 what inverse iteration leaves between clusters, above it rounding
+    assert orth <= (4e-9 if n <= 164 else 8 * n * 2.0 ** -52)
     assert np.linalg.norm(a @ y - y * w[None, :], axis=0).max() <= 4 * bound
     assert t < 1.0
