@@ -283,7 +283,7 @@ template <int NY>
 __device__ void slot_remove(double* x, int st, const double* y, int sy, size_t dy, int n, int per, bool on) {
   const int q = (threadIdx.x & 31) / per, g = 32 / per;
   double s[NY] = {};
-#pragma unroll 4
+#pragma unroll 8
   for (int i = q; i < n; i += g) {
     const double v = x[i * st];
 #pragma unroll
@@ -292,7 +292,7 @@ __device__ void slot_remove(double* x, int st, const double* y, int sy, size_t d
 #pragma unroll
   for (int j = 0; j < NY; ++j) s[j] = slot_sum(s[j], per);   // every lane takes part
   if (!on) return;
-#pragma unroll 4
+#pragma unroll 8
   for (int i = q; i < n; i += g) {
     double v = x[i * st];
 #pragma unroll
@@ -310,6 +310,74 @@ __device__ void store_signed(double* __restrict__ z, const double* x, int n, int
   for (int i = 0; i < n; ++i) z[i] = sg * x[i * st];
 }
 
+// Start vector of eigenvector k, deterministic and pseudo-random; of either
+// sign in a cluster, whose members differ by it.
+__device__ void start_vector(double* x, int n, int st, int k, bool clustered) {
+  unsigned s = 0x9E3779B9u * (k + 1);
+  for (int i = 0; i < n; ++i) {
+    s = s * 1664525u + 1013904223u;
+    const double u = double(s >> 8) / 16777216.0 - 0.5;
+    x[i * st] = clustered ? u : 1.0 + 0.5 * u;
+  }
+}
+
+// tridiag_vectors_kernel's work on the cnt values from c0 on when some of them
+// are members of clusters; true when the lane's vector is in order.  A call, so
+// that the kernel's path without clusters keeps its registers.
+__device__ __noinline__ bool cluster_batch(const double* d, const double* e, const double* lam, const int* cl_first,
+                                           int n, int per, int c0, int cnt, bool clustered, double tiny, double tnorm,
+                                           double* ai, double* b1, double* b2, double* l, double* x,
+                                           unsigned char* piv, int st, const double* Z) {
+  const int lane = threadIdx.x, k = c0 + lane, slot = min(lane, per - 1);
+  const bool on = lane < cnt;
+  const int f = on ? cl_first[k] : 0;                               // first member
+  const int base = max(f, c0) - c0, pos = on ? lane - base : 0;     // of the batch's members: lane of the first, place
+  int steps = on ? 1 : 0;                                           // members in the batch
+  while (on && base + steps < cnt && cl_first[c0 + base + steps] == f) ++steps;
+  for (int off = 16; off > 0; off >>= 1) steps = max(steps, __shfl_xor_sync(0xffffffffu, steps, off));
+  // the Gram-Schmidt's view: lane = gs + per q works on slot gs, its vector, cluster and place
+  const int gs = lane & (per - 1);
+  double* const gx = x + (gs - slot);
+  const int gf = __shfl_sync(0xffffffffu, f, gs), gbase = __shfl_sync(0xffffffffu, base, gs);
+  const int gpos = __shfl_sync(0xffffffffu, pos, gs);
+  const bool gclustered = __shfl_sync(0xffffffffu, int(clustered), gs);
+  if (on) {
+    double lk = lam[f];
+    for (int q = f + 1; q <= k; ++q) {   // numerically equal eigenvalues of a cluster are separated (dstein)
+      const double sep = 10.0 * DBL_EPSILON * fmax(fabs(lam[q]), tnorm * 1e-3);
+      lk = lam[q] - lk < sep ? lk + sep : lam[q];
+    }
+    tri_factor(d, e, n, lk, tiny, ai, b1, b2, l, piv, st);
+    start_vector(x, n, st, k, clustered);
+  }
+  bool ok = true;
+  for (int it = 0; it < 3; ++it) {
+    if (on && (clustered || it < 2)) {
+      tri_solve(n, ai, b1, b2, l, piv, x, st);
+      const double nrm = normalise(x, n, st);
+      ok = ok && nrm > 0 && isfinite(nrm);
+    }
+    for (int pass = 0; pass < (it == 2 ? 2 : 1); ++pass) {
+      __syncwarp();
+      int j = cl_first[c0];   // only the batch's first cluster can have members that are done
+      const bool part = gclustered && gf < c0;
+      if (it == 0) j = c0;    // and from the second round on: the first leaves the vectors different enough
+      // four at a time: as many as the L1 beside the scratch holds for the second reading
+      for (; j + 3 < c0; j += 4) slot_remove<4>(gx, st, Z + (size_t)j * n, 1, n, n, per, part);
+      for (; j < c0; ++j) slot_remove<1>(gx, st, Z + (size_t)j * n, 1, n, n, per, part);
+      __syncwarp();
+      for (int r = 0; r < steps; ++r) {
+        const double nrm = slot_normalise(gx, n, st, per, gclustered && gpos == r);
+        if (gclustered && gpos == r) ok = ok && nrm > 0 && isfinite(nrm);
+        __syncwarp();
+        slot_remove<1>(gx, st, gx + (min(gbase + r, per - 1) - gs), st, 0, n, per, gclustered && gpos > r);
+        __syncwarp();
+      }
+    }
+  }
+  return ok;
+}
+
 // Eigenvectors of lam[0..nev) by inverse iteration on the pivoted LU of
 // T - lambda I, one thread per eigenvector.  Eigenvalues (up to ne) closer
 // than 1e-7 ||T|| form clusters, whose members are orthogonalised against each
@@ -324,7 +392,7 @@ __device__ void store_signed(double* __restrict__ z, const double* x, int n, int
 // batch's vectors.  Three such rounds, the last one with a second pass.  With
 // one thread for a whole cluster, the solves of the undisplaced 64-atom cell at
 // (1/2, 1/2, 1/2), whose levels are many-fold, took 299 and 740 ms with 160 and
-// 400 bands; like this 111 and 254 ms (with cuSOLVER's pencils 138 and 305).
+// 400 bands; like this 109 and 246 ms (with cuSOLVER's pencils 138 and 305).
 //
 // Scratch: five n-vectors and the pivot flags per thread, interleaved by thread
 // (a warp touches consecutive words), in shared memory after the tables when
@@ -391,65 +459,22 @@ __global__ void __launch_bounds__(kVectorThreads) tridiag_vectors_kernel(
   for (int c0 = kbeg; c0 < kend; c0 += per) {
     const int cnt = min(per, kend - c0), k = c0 + lane;
     const bool on = lane < cnt;
-    const int f = on ? cl_first[k] : 0;                               // first member
-    const int base = max(f, c0) - c0, pos = on ? lane - base : 0;     // of the batch's members: lane of the first, place
-    int size = on ? 1 : 0;                                            // members in the batch
-    while (on && base + size < cnt && cl_first[c0 + base + size] == f) ++size;
-    const bool clustered = on && (f < k || (k + 1 < ne && cl_first[k + 1] == f));
-    int steps = size;
-    for (int off = 16; off > 0; off >>= 1) steps = max(steps, __shfl_xor_sync(0xffffffffu, steps, off));
-    const bool any = __any_sync(0xffffffffu, clustered);
-    // the Gram-Schmidt's view: slot gs, its vector, cluster and place
-    const int gs = lane & (per - 1);
-    double* const gx = x + (gs - slot);
-    const int gf = __shfl_sync(0xffffffffu, f, gs), gbase = __shfl_sync(0xffffffffu, base, gs);
-    const int gpos = __shfl_sync(0xffffffffu, pos, gs);
-    const bool gclustered = __shfl_sync(0xffffffffu, int(clustered), gs);
-    if (on) {
-      double lk = lam[f];
-      for (int q = f + 1; q <= k; ++q) {   // numerically equal eigenvalues of a cluster are separated (dstein)
-        const double sep = 10.0 * DBL_EPSILON * fmax(fabs(lam[q]), tnorm * 1e-3);
-        lk = lam[q] - lk < sep ? lk + sep : lam[q];
-      }
-      tri_factor(d, e, n, lk, tiny, ai, b1, b2, l, piv, st);
-      unsigned s = 0x9E3779B9u * (k + 1);
-      // deterministic pseudo-random start; of either sign in a cluster, whose members differ by it
-      for (int i = 0; i < n; ++i) {
-        s = s * 1664525u + 1013904223u;
-        const double u = double(s >> 8) / 16777216.0 - 0.5;
-        x[i * st] = clustered ? u : 1.0 + 0.5 * u;
-      }
-    }
-    // With an eigenvalue accurate to rounding each solve amplifies the wanted
-    // direction by ~gap / (eps ||T||): two solves for one by itself, three
-    // (each followed by Gram-Schmidt) inside a cluster.
+    const bool clustered = on && (cl_first[k] < k || (k + 1 < ne && cl_first[k + 1] == k));
     bool ok = true;
-    for (int it = 0; it < (any ? 3 : 2); ++it) {
-      if (on && (clustered || it < 2)) {
+    if (__any_sync(0xffffffffu, clustered)) {
+      ok = cluster_batch(d, e, lam, cl_first, n, per, c0, cnt, clustered, tiny, tnorm, ai, b1, b2, l, x, piv, st, Z);
+    } else if (on) {
+      tri_factor(d, e, n, lam[k], tiny, ai, b1, b2, l, piv, st);
+      start_vector(x, n, st, k, false);
+      // With an eigenvalue accurate to rounding each solve amplifies the wanted
+      // direction by ~gap / (eps ||T||): two are enough.
+      for (int it = 0; it < 2; ++it) {
         tri_solve(n, ai, b1, b2, l, piv, x, st);
         const double nrm = normalise(x, n, st);
         ok = ok && nrm > 0 && isfinite(nrm);
       }
-      for (int pass = 0; any && pass < (it == 2 ? 2 : 1); ++pass) {
-        __syncwarp();
-        // from here lane = gs + per q works on slot gs
-        int j = cl_first[c0];   // only the batch's first cluster can have members that are done
-        const bool part = gclustered && gf < c0;
-        for (; j + 3 < c0; j += 4) slot_remove<4>(gx, st, Z + (size_t)j * n, 1, n, n, per, part);
-        for (; j < c0; ++j) slot_remove<1>(gx, st, Z + (size_t)j * n, 1, n, n, per, part);
-        __syncwarp();
-        for (int r = 0; r < steps; ++r) {
-          const double nrm = slot_normalise(gx, n, st, per, gclustered && gpos == r);
-          if (gclustered && gpos == r) ok = ok && nrm > 0 && isfinite(nrm);
-          __syncwarp();
-          slot_remove<1>(gx, st, gx + (min(gbase + r, per - 1) - gs), st, 0, n, per, gclustered && gpos > r);
-          __syncwarp();
-        }
-      }
     }
-    ok = __all_sync(0xffffffffu, ok);
-    __syncwarp();
-    if (!ok) {   // the rest is of no use either
+    if (!__all_sync(0xffffffffu, ok)) {   // the rest is of no use either
       if (lane == 0) atomicCAS(status, 0, 1);   // an earlier report stays
       return;
     }
