@@ -20,8 +20,8 @@
 //   solver status words (one synchronisation, as in the reference);
 // * with the library's own small solvers (eig.cu, the default) the
 //   correction directions are S-normalised by a Jacobi-scaled Cholesky
-//   factor (pivots floored at 1e-14) instead of the eigenvectors of the
-//   metric; both bases span the same space, so the Rayleigh-Ritz step and
+//   factor (pivots floored at 1e-14; orders to 432) instead of the
+//   eigenvectors of the metric; both bases span the same space, so the Rayleigh-Ritz step and
 //   the Ritz values are those of the reference up to rounding;
 // * precision MIXED runs the iterations on FP32 blocks (FP32 operator,
 //   split-bf16 tcgen05 GEMMs from tc_gemm.cu whose projected matrices land

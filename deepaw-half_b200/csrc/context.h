@@ -80,7 +80,7 @@ struct Runtime {
   DeviceBuffer<unsigned char> tc_work;   // its split-K partial sums, grow-only
   DeviceBuffer<unsigned char> tc_planes; // its operands pre-split into bf16 planes, grow-only
   DeviceBuffer<double2> zwork;           // partial sums of the block products (blockops.cu), grow-only
-  DeviceBuffer<unsigned char> crt_a, crt_b, crt_res;   // residue planes of the FP64 products (zcrt.cu), grow-only
+  DeviceBuffer<unsigned char> crt_a, crt_b, crt_res;   // residue planes of integer products (zcrt.cu), given back when a call ends
   bool crt_pending = false;              // such products ran since the last tc_check
   DeviceBuffer<int> tc_err;              // raised when one of its pipeline waits gave up
   Profile prof;

@@ -58,7 +58,7 @@ struct BoxCell {
 // once per block, and so are the divisors of the Bessel series; cos(m phi) and
 // sin(m phi) once per point and atom instead of once per (l, m).  12-atom cell,
 // s/p/d channels, both species: 203 us with every function evaluated in place,
-// 84 us (138 us of it with the series' divisions).
+// 138 us with only the series' divisions left in, 84 us as it stands.
 constexpr int kDepositThreads = 128;
 constexpr int kBesselTerms = 31;
 inline size_t deposit_smem(int lmax) {

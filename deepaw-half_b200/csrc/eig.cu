@@ -9,7 +9,8 @@
 // Householder tridiagonalisation, Y = X V -- runs in kernels that keep the
 // matrix in the shared memory of a cluster of CTAs (orders to 432):
 //
-//   metric_factor_kernel   X = D R^-1 from a floored Cholesky factorisation;
+//   metric_factor_kernel   X = D R^-1 from a Cholesky factorisation, its pivots
+//                          floored (metrics, pencils to order 164) or reported;
 //   hetrd_kernel           tridiagonalisation (both also over the whole GPU's
 //                          shared memory, orders 434 to 1,280, with cuSOLVER's
 //                          zunmtr behind them);
@@ -21,7 +22,8 @@
 //                          eigenvalues closer than 1e-7 ||T|| form clusters
 //                          whose members a warp iterates together and
 //                          Gram-Schmidt orthogonalises in order (after
-//                          LAPACK's dstebz/dstein);
+//                          LAPACK's dstebz/dstein); above order 164 a step of
+//                          Z (3/2 - Z^T Z / 2) makes them orthogonal to rounding;
 //   back_transform_kernel  V = Q Z with Q = H(n-1)...H(1), the reflectors
 //                          staged in shared memory, one warp per eigenvector.
 //
@@ -686,7 +688,7 @@ __global__ void hermitian_fill_kernel(double2* A, int n) {
 // takes rows of all the CTA's columns and reads their eight panel elements
 // from L2 once.  The 17 pencils of orders 434 to 1,200 of a 480-band solve:
 // 26.6 ms (10 us a block: two grid barriers, the owner's elimination, the
-// update); the solve 561 ms, 577 with cuSOLVER's zpotrf and three ztrsm in
+// update); with that solve at 561 ms, 577 with cuSOLVER's zpotrf and three ztrsm in
 // place of this kernel and three products.
 constexpr int kClThreads = 256;
 constexpr int kClWarps = kClThreads / 32;

@@ -20,7 +20,8 @@
 // chunk stays resident in the 126 MB L2 between the three kernels.  The
 // projector part is one GEMM B^H X over all species and bands, a D/Q mixing
 // kernel and the GEMMs accumulating B DY into H X and B QY into S X.  In FP64
-// B is stored and the GEMMs are cuBLAS ZGEMM (the reference's calls); in FP32
+// B is stored and the GEMMs are cuBLAS ZGEMM (the reference's calls) or, large
+// ones of a mixed solve's FP64 phase, integer products (zcrt.cu); in FP32
 // one pass per k point generates B from a radial-angular table
 // (Omega^-1/2 beta_l(|q|) Y_lm, one row per species channel), the packed
 // plane-wave indices and the ions' b_j.R / 2 pi straight into the bf16 planes
@@ -79,9 +80,10 @@ constexpr int kPlaneThreads = 512;
 template <typename C>
 __device__ __forceinline__ C czero() { C c; c.x = 0; c.y = 0; return c; }
 
-// The local operator's three kernels are bound by instruction issue and
-// shared-memory accesses, not by HBM (a chunk's planes stay in L2), so every
-// pass over a plane or line that can be saved is: the first and last
+// The local operator's three kernels are bound by instruction issue (half of
+// the slots in FP32) and the latency between passes, not by HBM (a chunk's
+// planes stay in L2), so every pass over a plane or line that can be saved is:
+// the first and last
 // transform passes read and write global memory directly, rows known to be
 // zero are neither cleared nor loaded, and rows nobody reads are not stored.
 // Rows of a plane are padded by one element in shared memory so that the z

@@ -57,7 +57,8 @@ typedef struct half_solve_info_v1 {
   double max_residual_eV;
   double setup_ms;             /* basis, projectors, operator tables */
   double solve_ms;             /* iterations through eigenpairs */
-  double operator_ms;          /* time inside H/S applications */
+  double operator_ms;          /* time of H/S applications (= sweep_ms; in a batch of k points an
+                                  event span also covers the other streams' kernels) */
   double device_ms;            /* CUDA-event span on the library stream */
   double local_ms;             /* CUDA-event time of the local-operator kernels */
   double local_bytes;          /* their algorithmic bytes (FFT-path figure per band) */
