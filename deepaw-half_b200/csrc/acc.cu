@@ -381,7 +381,7 @@ struct Blocks {
   using C = cplx_t<R>;
   int n = 0, m = 0;
   DeviceBuffer<C> X[2], HX[2], SX[2];
-  DeviceBuffer<C> P, HP, SP, PU, HPU, SPU;
+  DeviceBuffer<C> P, HP, SP, PU, HPU, SPU;   // PU, HPU, SPU from the first metric step on
   DeviceBuffer<C> small;       // m x m (cross) in this precision
   DeviceBuffer<C> Y;           // 2m x m rotation in this precision
   int cur = 0;
@@ -389,7 +389,7 @@ struct Blocks {
     n = n_; m = m_;
     size_t nm = size_t(n) * m;
     for (int i = 0; i < 2; ++i) { X[i].resize(nm); HX[i].resize(nm); SX[i].resize(nm); }
-    P.resize(nm); HP.resize(nm); SP.resize(nm); PU.resize(nm); HPU.resize(nm); SPU.resize(nm);
+    P.resize(nm); HP.resize(nm); SP.resize(nm);
     small.resize(size_t(m) * m);
     Y.resize(size_t(2) * m * m);
   }
@@ -741,6 +741,7 @@ struct AccRun {
   // (src/half_cuda_iterative_solver.cuf:166-176)
   void normalise_metric(cplx_t<R> one, cplx_t<R> zero, int np) {
     double2* metric = sc.metric.get();
+    for (auto* b : {&blk.PU, &blk.HPU, &blk.SPU}) b->resize(size_t(n) * m);
     if constexpr (sizeof(R) == 8) {
       const ZBlock b = {blk.SP.get(), np};
       zgram(rt, n, {blk.P.get(), np}, &b, &metric, 1, np, true, zgram_route(rt.sms, n, np, np, integer));

@@ -23,10 +23,12 @@ namespace {
 using Key = std::pair<int, size_t>;   // (device, bytes)
 using Pool = std::multimap<Key, void*>;
 
-// Cached bytes kept by one thread (a 216-atom solve takes 17 GB in all) and by
-// the process: what four k-point workers and their caller need.
+// Cached bytes kept by one thread (a 216-atom mixed solve takes 20 GB in all)
+// and by the process: what a batch of four such solves comes back for.  At 80
+// GB a batch freed and allocated 20 to 40 blocks a step and took 550 to 583 ms
+// per k point, at 96 GB 543 to 550.
 constexpr size_t kThreadCap = size_t(32) << 30;
-constexpr size_t kProcessCap = size_t(80) << 30;
+constexpr size_t kProcessCap = size_t(96) << 30;
 
 size_t round_bytes(size_t b) {
   if (b <= (size_t(1) << 20)) return (b + 511) & ~size_t(511);

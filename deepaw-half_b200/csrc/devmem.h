@@ -13,7 +13,7 @@
 //   * a request takes the smallest cached block of at least its (rounded)
 //     size and at most twice it; on an allocation failure every cached block
 //     of every thread is released and the allocation retried once;
-//   * a thread keeps at most 32 GB and the process at most 80 GB: beyond that
+//   * a thread keeps at most 32 GB and the process at most 96 GB: beyond that
 //     a freed block goes back to the driver.
 #pragma once
 
