@@ -20,7 +20,7 @@
 //   solver status words (one synchronisation, as in the reference);
 // * with the library's own small solvers (eig.cu, the default) the
 //   correction directions are S-normalised by a Jacobi-scaled Cholesky
-//   factor (pivots floored at 1e-14; orders to 432) instead of the
+//   factor (pivots floored at 1e-14; orders to 164) instead of the
 //   eigenvectors of the metric; both bases span the same space, so the Rayleigh-Ritz step and
 //   the Ritz values are those of the reference up to rounding;
 // * precision MIXED runs the iterations on FP32 blocks (FP32 operator,
@@ -336,8 +336,7 @@ struct SmallSolver {
     lw_ev = l1;
     lw_gv = std::max(l2, l3);
   }
-  // all n eigenpairs of a (n x n) (cuSOLVER in both modes: the metric of the
-  // own path goes through metric_normalize unless m is beyond its kernel)
+  // all n eigenpairs of a (n x n) (cuSOLVER in all modes: metrics above kFlooredOrder)
   void heevd(double2* a, int n, double* w) {
     cusolver_check(cusolverDnZheevd(rt.solver, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_UPPER, n,
                                     reinterpret_cast<cuDoubleComplex*>(a), n, w,
@@ -749,7 +748,12 @@ struct AccRun {
       gemm_to64(rt, CUBLAS_OP_C, CUBLAS_OP_N, np, np, n, blk.P.get(), n, blk.SP.get(), n, metric, np);
     }
     mark("metric_gemm");
-    if (!(ss.own && ss.eig.metric_normalize(rt, metric, np, ss.info.get()))) {
+    // Above order 164 the reference's eigenvectors with its absolute floor: late
+    // in a solve P is so small that rounding in the metric lies far below that
+    // floor, while the Cholesky factor's, relative to the scaled diagonal, lies
+    // in it, and the step that is redone for an indefinite overlap (rayleigh_ritz)
+    // must not meet one again.
+    if (!(ss.own && np <= SmallSolver::kFlooredOrder && ss.eig.metric_normalize(rt, metric, np, ss.info.get()))) {
       ss.heevd(metric, np, sc.mu.get());
       scale_columns_kernel<<<ceil_div(np * np, 256), 256, 0, rt.stream>>>(metric, np, sc.mu.get(), 1.0e-14);
       ++rt.prof.launches;
