@@ -150,14 +150,19 @@ void begin_call(Runtime& rt) {
   HALF_CUDA(cudaEventRecord(pf.a, rt.stream));
 }
 
+// After the work of a call that may have run integer products: raises if one
+// gave up waiting.  The residue planes go back to the thread's cache: gigabytes
+// that the next context's first call finds there.
+void finish_products(Runtime& rt) {
+  if (rt.crt_pending) tc_check(rt);
+  for (auto* b : {&rt.crt_a, &rt.crt_b, &rt.crt_res}) b->release();
+}
+
 void end_call(Runtime& rt, SolveInfo& info) {
   Profile& pf = rt.prof;
   HALF_CUDA(cudaEventRecord(pf.b, rt.stream));
   HALF_CUDA(cudaEventSynchronize(pf.b));
-  if (rt.crt_pending) tc_check(rt);
-  // The residue planes go back to the thread's cache (the call's work is
-  // done): gigabytes that the next context's first call finds there.
-  for (auto* b : {&rt.crt_a, &rt.crt_b, &rt.crt_res}) b->release();
+  finish_products(rt);
   float ms = 0;
   HALF_CUDA(cudaEventElapsedTime(&ms, pf.a, pf.b));
   pf.collect();
@@ -965,6 +970,7 @@ extern "C" int half_forces(half_handle handle, int nk, const double* kpoints, co
     output_density_device(*ctx, nk, kpoints, kweights, nbands, ptr, lds, occ.data(), rho_out.get(), &aug);
     IonicForces f;
     ionic_forces_device(*ctx, rho_out.get(), true, true, true, true, true, f);
+    finish_products(*ctx->rt);   // none since the solves' own check as things stand
     for (int i = 0; i < 3 * nions; ++i) forces[i] = f.ewald[i] + f.local[i] + nonlocal[i] + f.nlcc[i] + f.harris[i];
     if (components) {
       const std::vector<double>* parts[5] = {&f.ewald, &f.local, &nonlocal, &f.nlcc, &f.harris};
